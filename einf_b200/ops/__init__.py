@@ -1506,6 +1506,48 @@ def recurrence_plan(num_requests: int, max_q_len: Optional[int], heads: int, dim
     return -(-max_q_len // segment_len), segment_len
 
 
+#: tokens that the chunked recurrence takes at a time
+RECURRENCE_CHUNK = 64
+#: shortest longest portion that takes the chunked kernel (kernels alone, us, one request / eight; token by token against
+#: chunked: 16 tokens 7.6 / 10.7 against 9.6 / 11.3 (14 heads of 64 x 64), 9.4 / 15.8 against 9.2 / 11.5 (24 of 128 x 64); 24 tokens
+#: 12.3 / 16.7 against 10.8 / 15.1, 12.1 / 20.1 against 10.1 / 13.9; 64 tokens 20.5 / 30.3 against 14.9 / 21.2)
+RECURRENCE_CHUNK_MIN = 24
+#: bytes that the states of a launch's segments may take (10 an element: the sum and the start state in parts)
+RECURRENCE_SEGMENT_BYTES = 128 << 20
+
+
+def recurrence_takes_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, y: torch.Tensor,
+                            dim: int, vdim: int, max_q_len: Optional[int]) -> bool:
+    """Whether :func:`linear_recurrence` takes the tokens 64 at a time on the tensor cores: bfloat16 inputs whose rows
+    and heads are 8-byte aligned, states of up to 128 rows in 16-byte aligned slots, and a portion long enough."""
+    return bool(
+        max_q_len and max_q_len >= RECURRENCE_CHUNK_MIN and q.dtype == torch.bfloat16
+        and dim <= 128 and dim % 4 == 0 and vdim % 4 == 0
+        and state.stride(0) % 4 == 0 and state.data_ptr() % 16 == 0 and y.data_ptr() % 8 == 0
+        and all(t.stride(0) % 4 == 0 and t.data_ptr() % 8 == 0 for t in (q, k, v))
+    )
+
+
+def recurrence_chunk_plan(tokens: int, num_requests: int, max_q_len: int, heads: int, dim: int, vdim: int) -> tuple[int, int]:
+    """``(segments, segment_len)`` of a chunked recurrence launch; no segments where no portion is longer than one.  A
+    segment is one chunk (longer ones repeat the state's product in both passes: Mamba-2, 24 heads of 128 x 64 over 2,048
+    tokens 70 us with 64, 71 with 128, 83 with 256 tokens) until the segments' states would outgrow the L2."""
+    segment_len = RECURRENCE_CHUNK
+    while segment_len < max_q_len and (
+            10 * heads * dim * vdim * (tokens // segment_len + num_requests) > RECURRENCE_SEGMENT_BYTES
+            or tokens // segment_len + num_requests > 65535):
+        segment_len *= 2
+    return (tokens // segment_len + num_requests if max_q_len > segment_len else 0), segment_len
+
+
+def _recurrence_tiles(dim: int, vdim: int) -> int:
+    """Columns of the state a CTA of the chunked kernel takes, in eights: 64, or 80 where that leaves fewer columns empty
+    and the state is small enough for two CTAs an SM (heads of 64 x 132: 37 us with 80, 42 with 64)."""
+    if vdim <= 32:
+        return 4
+    return 10 if dim <= 64 and -(-vdim // 80) * 80 < -(-vdim // 64) * 64 else 8
+
+
 #: most CTAs that share one head's rows in a step of single tokens
 RECURRENCE_STEP_MAX_SPLITS = 8
 
@@ -1543,6 +1585,7 @@ def linear_recurrence(
     rows: int = 0,
     segment_len: Optional[int] = None,
     columns: int = 0,
+    chunks: Optional[bool] = None,
 ) -> None:
     """Per request and head, over its tokens in order, with a float32 state ``S [dim, vdim]``::
 
@@ -1558,7 +1601,9 @@ def linear_recurrence(
     ``splits`` from :func:`recurrence_step_splits`: the parts of that many CTAs per head, for the
     consumer to add up.  ``max_q_len`` is the longest portion of the step as the host knows it (None: unknown,
     no portion is cut into segments); ``rows`` (0, 4, 8, 16), ``columns`` (0, 1, 2) and ``segment_len``
-    override the launch's own choices (:func:`recurrence_plan`), for tests and measurements."""
+    override the launch's own choices (:func:`recurrence_plan`), for tests and measurements.  ``chunks``: whether the
+    tokens are taken 64 at a time on the tensor cores (None: where :func:`recurrence_takes_chunks` says so and none
+    of the overrides is given; ``segment_len`` is then a multiple of 64)."""
     tokens = v.shape[0]
     if q.shape != (tokens, groups * dim) or k.shape != q.shape or v.shape != (tokens, heads * vdim):
         raise ValueError(f"q, k must be [{tokens}, {groups * dim}] and v [{tokens}, {heads * vdim}]")
@@ -1587,6 +1632,13 @@ def linear_recurrence(
     requests = state_slots.shape[0]
     if tokens == 0 or requests == 0:
         return
+    if chunks is None:
+        chunks = rows == 0 and columns == 0 and segment_len is None and \
+            recurrence_takes_chunks(q, k, v, state, y, dim, vdim, max_q_len)
+    if chunks:
+        _recurrence_chunks(q, k, v, state, q_start, state_slots, y, heads, groups, dim, vdim, head_decay, token_decay,
+                           token_scale, skip, silu_inputs, max_q_len or tokens, segment_len)
+        return
     if segment_len is not None:
         longest = max_q_len or tokens
         segments, segment_len = -(-longest // int(segment_len)), int(segment_len)
@@ -1598,6 +1650,9 @@ def linear_recurrence(
     if segments > 1:
         segment_state = torch.empty((requests * segments, heads, dim, vdim), dtype=torch.float32, device=y.device)
         segment_decay = torch.empty((requests * segments, heads), dtype=torch.float32, device=y.device)
+    global launch_count
+    if segments > 1:
+        launch_count += 2      # the first pass and the walk over the segments
     fn = _fn(
         "einf_linear_recurrence",
         [c_void_p, c_void_p, c_void_p, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p,
@@ -1615,9 +1670,40 @@ def linear_recurrence(
            y_splits, tokens * heads * vdim, _stream()),
         "linear_recurrence",
     )
-    if segments > 1:
-        global launch_count
+
+
+def _recurrence_chunks(q, k, v, state, q_start, state_slots, y, heads, groups, dim, vdim, head_decay, token_decay,
+                       token_scale, skip, silu_inputs, max_q_len, segment_len) -> None:
+    """The chunked form of :func:`linear_recurrence`, which has checked the operands."""
+    global launch_count
+    requests, device = state_slots.shape[0], y.device
+    slots, planned = recurrence_chunk_plan(v.shape[0], requests, max_q_len, heads, dim, vdim)
+    if segment_len is not None:
+        planned = int(segment_len)
+        slots = v.shape[0] // planned + requests if max_q_len > planned else 0
+    segment_state = segment_start = segment_decay = None
+    if slots:
+        segment_state = torch.empty((slots, heads, dim, vdim), dtype=torch.float32, device=device)
+        segment_start = torch.empty((slots, heads, 3, dim, vdim), dtype=torch.bfloat16, device=device)
+        segment_decay = torch.empty((slots, heads), dtype=torch.float32, device=device)
         launch_count += 2      # the first pass and the walk over the segments
+    fn = _fn(
+        "einf_linear_recurrence_chunks",
+        [c_void_p, c_void_p, c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p,
+         c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+         c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
+    )
+    _check(
+        fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), _rows_of(q, "q"), _rows_of(k, "k"), _rows_of(v, "v"),
+           _opt(head_decay, "head_decay", torch.float32), _opt(token_decay, "token_decay", torch.float32),
+           _opt(token_scale, "token_scale", torch.float32), _opt(skip, "skip", torch.float32),
+           state.data_ptr(), state.stride(0), state.shape[0], _opt(q_start, "q_start", torch.int32),
+           _opt(state_slots, "state_slots", torch.int32), requests, _dev(y, "y"), heads, groups, dim, vdim,
+           1 if silu_inputs else 0, _recurrence_tiles(dim, vdim), slots, planned,
+           _opt(segment_state, "segment_state", torch.float32), _opt(segment_start, "segment_start", torch.bfloat16),
+           _opt(segment_decay, "segment_decay", torch.float32), _stream()),
+        "linear_recurrence",
+    )
 
 
 def gated_norm(

@@ -23,6 +23,7 @@ LAUNCHERS = {
     "einf_qkv_norm_store": "pointwise",
     "einf_conv_silu": "recurrence",
     "einf_linear_recurrence": "recurrence",
+    "einf_linear_recurrence_chunks": "recurrence_chunks",
     "einf_gated_norm": "recurrence",
     "einf_paged_attention_generic": "attention_generic",
     "einf_latent_decode_attention": "attention_generic",

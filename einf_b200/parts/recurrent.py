@@ -31,15 +31,19 @@ class _RecurrentMixer(Mixer):
     @classmethod
     def kernel_libraries(cls, spec, runtime):
         return ("pointwise", "recurrence", "gemm_simt") + (
-            ("gemm_tcgen05",) if runtime.dtype == torch.bfloat16 else ()
+            ("gemm_tcgen05", "recurrence_chunks") if runtime.dtype == torch.bfloat16 else ()
         )
 
     #: (heads, rows, columns) of the recurrent state, set by the subclasses
     state_shape: tuple[int, int, int] = (0, 0, 0)
 
     def launch_key(self, ctx: StepContext, page_size: int) -> tuple:
-        """Long portions are cut into segments by the step's longest portion, a host-side figure."""
-        return ops.recurrence_plan(ctx.num_requests, ctx.max_q_len, *self.state_shape)
+        """Long portions are cut into segments by the step's longest portion, a host-side figure (which of the two forms of
+        the recurrence runs goes by it too)."""
+        plan = ops.recurrence_plan(ctx.num_requests, ctx.max_q_len, *self.state_shape)
+        if ctx.max_q_len < ops.RECURRENCE_CHUNK_MIN:
+            return plan
+        return plan + ops.recurrence_chunk_plan(ctx.num_tokens, ctx.num_requests, ctx.max_q_len, *self.state_shape)
 
     def launch_group(self):
         return ("recurrence",) + self.state_shape

@@ -228,6 +228,82 @@ def test_linear_recurrence_keeps_its_state(dev, dtype, heads, groups, dim, vdim,
         torch.testing.assert_close(state_got, state_want, rtol=2e-4, atol=2e-4)
 
 
+@pytest.mark.parametrize("heads, groups, dim, vdim, per_token, silu, pad", [
+    (2, 2, 64, 64, False, True, 8), (4, 1, 128, 64, True, False, 8), (1, 1, 128, 260, True, False, 4), (3, 3, 64, 132, True, True, 4),
+    (2, 2, 16, 12, True, False, 4), (2, 1, 40, 100, False, False, 8), (1, 1, 100, 36, False, True, 4),
+])
+@pytest.mark.parametrize("lengths, segment_len", [
+    ((24,), None), ((63, 1), None), ((64, 0, 65), None), ((130, 16, 1, 193), None), ((130, 16, 1, 193), 128), ((250,), 256),
+])
+def test_chunked_recurrence(dev, heads, groups, dim, vdim, per_token, silu, pad, lengths, segment_len):
+    """The chunked form against the plain loop in 64 bits: portions around its tiles of 16, chunks of 64 and
+    segments, single tokens and an empty request beside them, a request without a slot, decays that are zero, columns of
+    wider matrices on 8- and 16-byte borders, states that fill no tile.  The bound: what both add up are the same products,
+    so an element is off by at most (roundings on its way) x 2^-24 x (the sum of its products' sizes, which the loop on the
+    absolute values gives); a product passes at most 16 rounded sums of 16 in each of two chains, eight roundings of its
+    weight and one per segment."""
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(dim + vdim + sum(lengths))
+    requests = len(lengths)
+    slots = torch.arange(requests, dtype=torch.int32, device=dev)
+    if requests > 2:
+        slots[2] = -1
+    base = torch.randn((requests, 4 + heads * dim * vdim), generator=gen).to(dev)
+    q_start, _ = _packed(lengths, dev)
+    tokens = sum(lengths)
+    wide = (torch.randn((tokens, pad + 2 * groups * dim + heads * vdim + 12), generator=gen) * 0.5).to(torch.bfloat16).to(dev)
+    q, k = wide[:, pad:pad + groups * dim], wide[:, pad + groups * dim:pad + 2 * groups * dim]
+    v = wide[:, pad + 2 * groups * dim:pad + 2 * groups * dim + heads * vdim]
+    kwargs = dict(silu_inputs=silu)
+    if per_token:
+        decay = torch.rand((tokens, heads), generator=gen)
+        decay[torch.rand((tokens, heads), generator=gen) < 0.05] = 0.0
+        kwargs.update(token_decay=decay.to(dev), token_scale=torch.rand((tokens, heads), generator=gen).to(dev),
+                      skip=torch.randn(heads, generator=gen).to(dev))
+    else:
+        kwargs.update(head_decay=(1.0 - 0.1 * torch.rand(heads, generator=gen)).to(dev))
+    state = base.clone()
+    y = torch.full((tokens, heads * vdim), float("nan"), device=dev)
+    view = state[:, 4:].view(requests, heads, dim, vdim)
+    assert ops.recurrence_takes_chunks(q, k, v, view, y, dim, vdim, max(lengths)) == (max(lengths) >= ops.RECURRENCE_CHUNK_MIN)
+    ops.linear_recurrence(q, k, v, view, q_start, slots, y, heads, groups, dim, vdim, max_q_len=max(lengths),
+                          segment_len=segment_len, chunks=True, **kwargs)
+    want = _recurrence64(q, k, v, base[:, 4:].view(requests, heads, dim, vdim), q_start, slots, heads, groups, lambda t: t, **kwargs)
+    size = _recurrence64(q, k, v, base[:, 4:].view(requests, heads, dim, vdim), q_start, slots, heads, groups, torch.abs, **kwargs)
+    bound = (32 + 8 + max(lengths) / 64) * 2.0 ** -24
+    for got, exact, most in zip((y, view), want, size):
+        assert bool(((got.double() - exact).abs() <= bound * most.abs() + 1e-12).all())
+    if requests > 1:
+        assert torch.equal(state[:, :4], base[:, :4])
+
+
+def _recurrence64(q, k, v, state, q_start, slots, heads, groups, of, head_decay=None, token_decay=None, token_scale=None,
+                  skip=None, silu_inputs=False):
+    """y and the states after the loop over tokens in 64 bits, of ``of`` the inputs (torch.abs: the sums of the sizes)."""
+    tokens, dim, vdim = q.shape[0], state.shape[2], state.shape[3]
+    q, k, v = (t.double() for t in (q, k, v))
+    if silu_inputs:
+        q, k, v = (t * torch.sigmoid(t) for t in (q, k, v))
+    head_of = torch.arange(heads, device=q.device) // (heads // groups)
+    q, k = (of(t).view(tokens, groups, dim)[:, head_of] for t in (q, k))
+    v = of(v).view(tokens, heads, vdim)
+    decay = token_decay.double() if head_decay is None else head_decay.double().expand(tokens, heads)
+    scale = torch.ones_like(decay) if token_scale is None else token_scale.double()
+    after, y = state.double().clone(), torch.zeros((tokens, heads, vdim), dtype=torch.float64, device=q.device)
+    for r in range(slots.shape[0]):
+        slot = int(slots[r])
+        S = of(after[slot]) if slot >= 0 else torch.zeros_like(after[0])
+        for t in range(int(q_start[r]), int(q_start[r + 1])):
+            S = decay[t][:, None, None] * S + k[t][:, :, None] * (scale[t][:, None] * v[t])[:, None, :]
+            y[t] = torch.einsum("hd,hdv->hv", q[t], S)
+            if skip is not None:
+                y[t] += of(skip.double())[:, None] * v[t]
+        if slot >= 0 and q_start[r + 1] > q_start[r]:
+            after[slot] = S
+    return y.view(tokens, -1), after
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("width, parts, gate_first, kind", [
     (48, 2, True, "silu"), (64, 1, False, "sigmoid"), (600, 3, True, "silu"), (40, 40, False, "silu"),
