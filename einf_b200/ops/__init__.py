@@ -11,6 +11,7 @@ The plain PyTorch statement of each function lives beside the tests
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import Optional, Tuple
 
@@ -351,16 +352,34 @@ def gemm_simt(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
         raise ValueError("gemm operands must have unit stride in their last dimension")
     if not (x.is_cuda and out.is_cuda):
         raise KernelError("gemm operands must be on a CUDA device: there is no CPU path")
+    share = _gemm_simt_shares(m, n, k)
+    sums = None
+    if share > 1:       # every 256 terms' sums, which a second kernel adds up
+        sums = torch.empty((-(-k // 256), m, n), dtype=torch.float32, device=x.device)
+        global launch_count
+        launch_count += 1
     fn = _fn(
         "einf_gemm_simt",
         [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong,
-         c_longlong, c_void_p],
+         c_longlong, c_int, c_void_p, c_void_p],
     )
     _check(
         fn(x.data_ptr(), _code(x), _dev(weight, "weight"), _code(weight), _opt(bias, "bias", torch.float32),
-           out.data_ptr(), _code(out), m, n, k, x.stride(0), out.stride(0), _stream()),
+           out.data_ptr(), _code(out), m, n, k, x.stride(0), out.stride(0), share,
+           _opt(sums, "sums", torch.float32), _stream()),
         "gemm_simt",
     )
+
+
+#: most bytes of block sums a 32-bit product leaves for its second kernel (beyond that K is not shared: such outputs
+#: have tiles enough)
+GEMM_SIMT_SUM_BYTES = 64 << 20
+
+
+@functools.lru_cache(maxsize=4096)
+def _gemm_simt_shares(m: int, n: int, k: int) -> int:
+    """How many CTAs share K in a 32-bit product of these sizes."""
+    return int(_fn("einf_gemm_simt_shares", [c_int, c_int, c_int, c_longlong])(m, n, k, GEMM_SIMT_SUM_BYTES))
 
 
 def tcgen05_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:

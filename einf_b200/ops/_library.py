@@ -32,6 +32,7 @@ LAUNCHERS = {
     "einf_latent_attention_tcgen05_parts": "attention_latent",
     "einf_gemm_simt": "gemm_simt",
     "einf_gemm_tcgen05": "gemm_tcgen05",
+    "einf_gemm_simt_shares": "gemm_simt",
     "einf_gemm_tcgen05_splits": "gemm_tcgen05",
     "einf_gemm_grouped_tcgen05": "gemm_tcgen05",
     "einf_paged_decode_attention": "attention_bf16",

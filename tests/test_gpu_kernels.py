@@ -270,6 +270,31 @@ def test_silu_mul(dev, dtype):
     torch.testing.assert_close(out, want, **tol(dtype))
 
 
+@pytest.mark.parametrize("m, n, k", [(1, 1, 257), (64, 128, 512), (65, 130, 513), (3, 896, 4864), (200, 129, 1023), (7, 36, 256)])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_gemm_simt_shares_k_without_a_trace(dev, m, n, k, dtype, monkeypatch):
+    """Products whose K several CTAs share give bit for bit what one CTA gives, at the edges of tiles and of the blocks of
+    256 terms; and both are what 64 bits give to within the roundings of a block's sum and of the sum of blocks."""
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(m + n + k)
+    x = torch.randn((m, k), generator=gen).to(dtype).to(dev)
+    w, bias = torch.randn((n, k), generator=gen).to(dev), torch.randn(n, generator=gen).to(dev)
+    shared, alone = torch.empty((m, n), device=dev), torch.empty((m, n), device=dev)
+    ops._gemm_simt_shares.cache_clear()
+    assert ops._gemm_simt_shares(m, n, k) == -(-k // 256)
+    ops.gemm_simt(x, w, bias, shared)
+    monkeypatch.setattr(ops, "GEMM_SIMT_SUM_BYTES", 0)
+    ops._gemm_simt_shares.cache_clear()
+    ops.gemm_simt(x, w, bias, alone)
+    monkeypatch.undo()
+    ops._gemm_simt_shares.cache_clear()
+    assert torch.equal(shared, alone)
+    want = x.double() @ w.double().T + bias.double()
+    size = x.double().abs() @ w.double().abs().T + bias.double().abs()
+    assert bool(((shared.double() - want).abs() <= (256 + k / 256 + 1) * 2.0 ** -24 * size).all())
+
+
 @pytest.mark.parametrize("m, n, k", [(1, 5, 3), (7, 130, 67), (64, 64, 64), (65, 127, 200), (300, 33, 1000)])
 @pytest.mark.parametrize("a_dtype, w_dtype, out_dtype", [
     (torch.float32, torch.float32, torch.float32),
