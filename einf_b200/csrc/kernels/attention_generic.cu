@@ -60,15 +60,17 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
                                int head_size, int value_size, int value_stride, int page_size, int num_pages,
                                int table_width, float scale, int window, int keep_first, int chunk, float softcap,
                                const float* __restrict__ sink, const float* __restrict__ gate,
-                               const T* __restrict__ value_gate, long long value_gate_stride, int* status) {
+                               const T* __restrict__ value_gate, long long value_gate_stride,
+                               const int* __restrict__ tokens, int* status) {
   __shared__ float q_smem[kWarpsPerBlock][kHeadLimit];
   pdl_launch_dependents();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * kWarpsPerBlock + warp;
-  if (row >= num_rows) return;
-  const int t = row / num_heads;
-  const int h = row - t * num_heads;
+  const int listed = blockIdx.x * kWarpsPerBlock + warp;
+  if (listed >= num_rows) return;
+  const int h = listed % num_heads;
+  const int t = tokens ? tokens[listed / num_heads] : listed / num_heads;
+  const int row = t * num_heads + h;
   const int kv_head = h / (num_heads / num_kv_heads);
   const int r = seq_of_token[t];
   const int pos = positions[t];
@@ -165,6 +167,244 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
       o_row[d] = from_float<T>(o);
     }
   }
+}
+
+// ---------------------------------------------------------------------------
+// The same for portions of a prompt, keys and values of up to 128 elements (multiples of four): a CTA has 32
+// neighbouring tokens of one request and one head and takes their keys 64 at a time through shared memory, so that a key
+// row is read once for 32 tokens (the kernel above reads it once for each: 303 us for portions of 512 and 33 tokens, 14
+// heads of 64 in 32 bits, 0.5 GFLOP).  A thread has 4 x 4 of the scores and 4 rows x VALUE / 16 columns of the output; rows
+// of shared memory are four floats longer than a vector, so that eight neighbouring rows meet no bank twice.  The
+// scores are the same sums in the same order; the softmax goes by tiles of 64 keys instead of 32.  Bound by the
+// reads from shared memory and by the longest token's chain of tiles.
+// ---------------------------------------------------------------------------
+constexpr int kPromptRows = 32, kPromptKeys = 64, kPromptThreads = 128;
+
+struct PromptArgs {
+  const void* q; const void* k_cache; const void* v_cache; void* out;
+  const int* block_table; const int* q_tiles;     // [tiles, 4]: request, first token, rows (up to 128), first position
+  const float* sink; const float* gate; const void* value_gate; long long value_gate_stride;
+  int* status;
+  int num_heads, num_kv_heads, head_size, value_size, value_stride, page_size, num_pages, table_width;
+  float scale, softcap;
+  int window, keep_first, chunk;
+};
+
+__device__ __forceinline__ void prompt_copy16(float* smem, const float* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem))), "l"(gmem)
+               : "memory");
+}
+__device__ __forceinline__ void prompt_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void prompt_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// COLS: columns of the output a thread has in groups of four (value sizes up to 64 COLS).
+template <typename T, int COLS>
+__global__ void __launch_bounds__(kPromptThreads)
+paged_attention_prompt_kernel(const __grid_constant__ PromptArgs a) {
+  extern __shared__ __align__(16) float prompt_smem[];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int head_size = a.head_size, value_size = a.value_size;
+  const int key_pitch = head_size + 4, value_pitch = 64 * COLS + 4;
+  constexpr int kScorePitch = kPromptKeys + 4;
+  float* const qs = prompt_smem;                                // [32][key_pitch]
+  float* const ks = qs + kPromptRows * key_pitch;               // [64][key_pitch]
+  float* const vs = ks + kPromptKeys * key_pitch;               // [64][value_pitch]
+  float* const ps = vs + kPromptKeys * value_pitch;             // [32][kScorePitch]
+  __shared__ int pages[kPromptKeys];                            // of the tile's keys: row of the caches, -1 for none
+
+  const int* tile = a.q_tiles + 4 * (blockIdx.x >> 2);
+  const int request = tile[0], sub = (blockIdx.x & 3) * kPromptRows;
+  const int rows = min(kPromptRows, tile[2] - sub);
+  if (rows <= 0) return;
+  const int t0 = tile[1] + sub, pos0 = tile[3] + sub;
+  const int h = blockIdx.y, kv_head = h / (a.num_heads / a.num_kv_heads);
+  const int* table = a.block_table + (long long)request * a.table_width;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;       // scores: rows ty + 8 i, keys tx + 16 j
+  auto low_of = [&](int pos) {
+    int lo = a.window > 0 ? max(0, pos - a.window + 1) : 0;
+    return a.chunk > 0 ? max(lo, pos / a.chunk * a.chunk) : lo;
+  };
+  const int last_pos = pos0 + rows - 1, lowest = low_of(pos0);
+  const int kept = a.window > 0 ? min(a.keep_first, last_pos + 1) : 0;
+  const float inv_cap = a.softcap > 0.f ? 1.f / a.softcap : 0.f;
+
+  // queries, times the scale; rows beyond the portion are zeros
+  const T* qg = (const T*)a.q + ((long long)t0 * a.num_heads + h) * head_size;
+  for (int i = threadIdx.x; i < kPromptRows * head_size; i += kPromptThreads) {
+    const int r = i / head_size, d = i - r * head_size;
+    qs[r * key_pitch + d] = r < rows ? to_float(qg[(long long)r * a.num_heads * head_size + d]) * a.scale : 0.f;
+  }
+  float m[4], l[4], acc[4][COLS][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.f;
+#pragma unroll
+    for (int c = 0; c < COLS; ++c)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][c][e] = 0.f;
+  }
+  bool bad_page = false;
+  // the rows of a tile's keys (or values) into shared memory, zeros where a key has none
+  auto bring = [&](const void* cache, int size, int stride, float* to, int pitch, int width) {
+    const int quads = width / 4;
+    for (int i = threadIdx.x; i < kPromptKeys * quads; i += kPromptThreads) {
+      const int j = i / quads, d = 4 * (i - j * quads);
+      const int page_row = pages[j];
+      float* at = to + j * pitch + d;
+      if (page_row < 0 || d >= size) {
+        *reinterpret_cast<float4*>(at) = make_float4(0.f, 0.f, 0.f, 0.f);
+      } else if constexpr (sizeof(T) == 4) {
+        prompt_copy16(at, (const float*)cache + (long long)page_row * stride + d);
+      } else {
+        const uint2 raw = *reinterpret_cast<const uint2*>((const T*)cache + (long long)page_row * stride + d);
+        *reinterpret_cast<float4*>(at) = make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u),
+                                                     __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u));
+      }
+    }
+    prompt_commit();
+  };
+
+  // the kept first positions' tiles below the window, then the window's
+  const int first_tile = lowest / kPromptKeys, kept_tiles = min(first_tile, (kept + kPromptKeys - 1) / kPromptKeys);
+  const int end_tile = last_pos / kPromptKeys + 1;
+  for (int step = first_tile - kept_tiles; step < end_tile; ++step) {
+    const int base = (step < first_tile ? step - (first_tile - kept_tiles) : step) * kPromptKeys;
+    __syncthreads();                               // the tile before is used up
+    if (threadIdx.x < kPromptKeys) {
+      const int j = base + threadIdx.x;
+      int row = -1;
+      if ((j >= lowest && j <= last_pos) || j < kept) {
+        const int logical = j / a.page_size;
+        const int page = table[logical];
+        if (page < 0 || page >= a.num_pages) bad_page = true;
+        else row = (page * a.num_kv_heads + kv_head) * a.page_size + (j - logical * a.page_size);
+      }
+      pages[threadIdx.x] = row;
+    }
+    __syncthreads();
+    bring(a.k_cache, head_size, head_size, ks, key_pitch, head_size);
+    bring(a.v_cache, value_size, a.value_stride, vs, value_pitch, 64 * COLS);
+    prompt_wait<1>();
+    __syncthreads();
+    float s[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+#pragma unroll 2
+    for (int d = 0; d < head_size; d += 4) {
+      float4 qv[4], kv[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) qv[i] = *reinterpret_cast<const float4*>(qs + (ty + 8 * i) * key_pitch + d);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) kv[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * key_pitch + d);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s[i][j] = fmaf(qv[i].x, kv[j].x, s[i][j]);
+          s[i][j] = fmaf(qv[i].y, kv[j].y, s[i][j]);
+          s[i][j] = fmaf(qv[i].z, kv[j].z, s[i][j]);
+          s[i][j] = fmaf(qv[i].w, kv[j].w, s[i][j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int pos = pos0 + ty + 8 * i, lo = low_of(pos);
+      float top = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int key = base + tx + 16 * j;
+        const bool seen = key <= pos && (key >= lo || key < kept) && pages[tx + 16 * j] >= 0;
+        const float capped = a.softcap > 0.f ? a.softcap * tanhf(s[i][j] * inv_cap) : s[i][j];
+        s[i][j] = seen ? capped : -INFINITY;
+        top = fmaxf(top, s[i][j]);
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+      const float m_new = fmaxf(m[i], top);
+      const float correction = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float p = s[i][j] == -INFINITY ? 0.f : expf(s[i][j] - m_new);
+        ps[(ty + 8 * i) * kScorePitch + tx + 16 * j] = p;
+        sum += p;
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      l[i] = l[i] * correction + sum;
+      m[i] = m_new;
+#pragma unroll
+      for (int c = 0; c < COLS; ++c)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][c][e] *= correction;
+    }
+    prompt_wait<0>();
+    __syncthreads();
+#pragma unroll 2
+    for (int j = 0; j < kPromptKeys; j += 4) {
+      float4 pv[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) pv[i] = *reinterpret_cast<const float4*>(ps + (ty + 8 * i) * kScorePitch + j);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+          const float4 v = *reinterpret_cast<const float4*>(vs + (j + u) * value_pitch + 64 * c + 4 * tx);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float p = u == 0 ? pv[i].x : u == 1 ? pv[i].y : u == 2 ? pv[i].z : pv[i].w;
+            acc[i][c][0] = fmaf(p, v.x, acc[i][c][0]);
+            acc[i][c][1] = fmaf(p, v.y, acc[i][c][1]);
+            acc[i][c][2] = fmaf(p, v.z, acc[i][c][2]);
+            acc[i][c][3] = fmaf(p, v.w, acc[i][c][3]);
+          }
+        }
+    }
+  }
+  if (bad_page) atomicOr(a.status, kStatusBadPage);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = ty + 8 * i;
+    if (r >= rows) continue;
+    const long long row = (long long)(t0 + r) * a.num_heads + h;
+    float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
+    if (a.sink) {
+      // one more term of the denominator, against the larger of the two maxima
+      const float top = fmaxf(m[i], a.sink[h]);
+      const float keys = m[i] == -INFINITY ? 0.f : l[i] * expf(m[i] - top);
+      inv = m[i] == -INFINITY ? 0.f : expf(m[i] - top) / (keys + expf(a.sink[h] - top));
+    }
+    if (a.gate) inv *= a.gate[row];
+    T* out = (T*)a.out + row * value_size;
+#pragma unroll
+    for (int c = 0; c < COLS; ++c)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int d = 64 * c + 4 * tx + e;
+        if (d >= value_size) continue;
+        float o = acc[i][c][e] * inv;
+        if (a.value_gate)
+          o /= 1.f + expf(-to_float(((const T*)a.value_gate)[(t0 + r) * a.value_gate_stride + (long long)h * value_size + d]));
+        out[d] = from_float<T>(o);
+      }
+  }
+}
+
+template <typename T, int COLS>
+static cudaError_t launch_prompt(const PromptArgs& a, int num_tiles, cudaStream_t stream) {
+  auto kernel = paged_attention_prompt_kernel<T, COLS>;
+  auto bytes = [](int head_size) {
+    return (int)sizeof(float) * ((kPromptRows + kPromptKeys) * (head_size + 4) + kPromptKeys * (64 * COLS + 4) +
+                                 kPromptRows * (kPromptKeys + 4));
+  };
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes(128));
+  if (e != cudaSuccess) return e;
+  return launch_pdl(kernel, dim3(4 * num_tiles, a.num_heads), dim3(kPromptThreads), bytes(a.head_size), stream, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -380,6 +620,7 @@ __global__ void latent_decode_merge_kernel(const float* __restrict__ part_acc, c
 
 using namespace einf;
 
+// `tokens`: the tokens to take (num_tokens of them), or null for all.
 extern "C" int einf_paged_attention_generic(const void* q, const void* k_cache, const void* v_cache,
                                             int dtype, const int* block_table, const int* seq_of_token,
                                             const int* positions, void* out, int num_tokens,
@@ -387,7 +628,7 @@ extern "C" int einf_paged_attention_generic(const void* q, const void* k_cache, 
                                             int value_stride, int page_size, int num_pages, int table_width,
                                             float scale, int window, int keep_first, int chunk, float softcap,
                                             const float* sink, const float* gate, const void* value_gate,
-                                            long long value_gate_stride, int* status, cudaStream_t stream) {
+                                            long long value_gate_stride, const int* tokens, int* status, cudaStream_t stream) {
   const int rows = num_tokens * num_heads;
   if (rows == 0) return 0;
   if (head_size > kMaxHeadSize || value_size > kMaxHeadSize || head_size <= 0 || value_size <= 0)
@@ -399,12 +640,12 @@ extern "C" int einf_paged_attention_generic(const void* q, const void* k_cache, 
       paged_attention_generic_kernel<T, 256><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(
           (const T*)q, (const T*)k_cache, (const T*)v_cache, block_table, seq_of_token, positions, (T*)out,
           rows, num_heads, num_kv_heads, head_size, value_size, value_stride, page_size, num_pages, table_width,
-          scale, window, keep_first, chunk, softcap, sink, gate, (const T*)value_gate, value_gate_stride, status);
+          scale, window, keep_first, chunk, softcap, sink, gate, (const T*)value_gate, value_gate_stride, tokens, status);
     } else {
       paged_attention_generic_kernel<T, kMaxHeadSize><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(
           (const T*)q, (const T*)k_cache, (const T*)v_cache, block_table, seq_of_token, positions, (T*)out,
           rows, num_heads, num_kv_heads, head_size, value_size, value_stride, page_size, num_pages, table_width,
-          scale, window, keep_first, chunk, softcap, sink, gate, (const T*)value_gate, value_gate_stride, status);
+          scale, window, keep_first, chunk, softcap, sink, gate, (const T*)value_gate, value_gate_stride, tokens, status);
     }
   })
   return (int)cudaGetLastError();
@@ -457,5 +698,34 @@ extern "C" int einf_latent_decode_merge(const float* part_acc, const float* part
   EINF_DISPATCH_2(dtype, T, {
     return (int)launch_pdl(latent_decode_merge_kernel<T>, dim3(num_tokens * num_heads), dim3(128), 0, stream, part_acc,
                            part_ml, (T*)out, splits, value_size, num_heads, sink, gate, token_list);
+  })
+}
+
+// Portions of prompts: the tokens that `q_tiles` lists.  Key and value sizes up to 128, multiples of four.
+extern "C" int einf_paged_attention_prompt(const void* q, const void* k_cache, const void* v_cache, int dtype,
+                                           const int* block_table, const int* q_tiles, int num_tiles, void* out,
+                                           int num_heads, int num_kv_heads, int head_size, int value_size, int value_stride,
+                                           int page_size, int num_pages, int table_width, float scale, int window,
+                                           int keep_first, int chunk, float softcap, const float* sink, const float* gate,
+                                           const void* value_gate, long long value_gate_stride, int* status,
+                                           cudaStream_t stream) {
+  if (num_tiles == 0) return 0;
+  if (head_size <= 0 || head_size > 128 || head_size % 4 || value_size <= 0 || value_size > 128 || value_size % 4 ||
+      value_stride < value_size || value_stride % 4 || num_heads <= 0 || num_heads > 65535 || num_kv_heads <= 0 ||
+      num_heads % num_kv_heads || num_tiles > (1 << 28) || ((uintptr_t)k_cache & 15) || ((uintptr_t)v_cache & 15) ||
+      (long long)num_pages * num_kv_heads * page_size > 0x7fffffff)
+    return (int)cudaErrorInvalidValue;
+  PromptArgs a;
+  a.q = q; a.k_cache = k_cache; a.v_cache = v_cache; a.out = out;
+  a.block_table = block_table; a.q_tiles = q_tiles;
+  a.sink = sink; a.gate = gate; a.value_gate = value_gate; a.value_gate_stride = value_gate_stride;
+  a.status = status;
+  a.num_heads = num_heads; a.num_kv_heads = num_kv_heads; a.head_size = head_size; a.value_size = value_size;
+  a.value_stride = value_stride; a.page_size = page_size; a.num_pages = num_pages; a.table_width = table_width;
+  a.scale = scale; a.softcap = softcap;
+  a.window = window; a.keep_first = window > 0 ? keep_first : 0; a.chunk = chunk;
+  EINF_DISPATCH_2(dtype, T, {
+    if (value_size <= 64) return (int)launch_prompt<T, 1>(a, num_tiles, stream);
+    return (int)launch_prompt<T, 2>(a, num_tiles, stream);
   })
 }

@@ -589,6 +589,8 @@ def paged_attention_generic(
     sink: Optional[torch.Tensor] = None,
     gate: Optional[torch.Tensor] = None,
     value_gate: Optional[torch.Tensor] = None,
+    q_tiles: Optional[torch.Tensor] = None,
+    single_tokens: Optional[torch.Tensor] = None,
 ) -> None:
     """Causal attention of every token of the batch over the pages of its request.
 
@@ -604,6 +606,10 @@ def paged_attention_generic(
     unscaled, with no key and no value.  ``gate`` (float32 ``[tokens, heads]``): a head's mixed row is multiplied
     by it before it is rounded.  ``value_gate`` (q's dtype, ``[tokens, heads * value_size]``, rows may be columns of
     a wider matrix): every element of the mixed heads is multiplied by the sigmoid of its own logit.
+
+    ``q_tiles`` (int32 ``[tiles, 4]``: request, first token, rows up to 128, first position) and ``single_tokens``
+    (int32) list the step's tokens by portions: portions of ``PROMPT_TILE_MIN`` tokens a tile or more, on average, then
+    take a kernel that shares key rows between their tokens, where it takes the sizes.
     """
     tokens, num_heads, head_size = q.shape
     if sink is not None and (sink.dtype != torch.float32 or sink.shape != (num_heads,)):
@@ -629,21 +635,57 @@ def paged_attention_generic(
         raise TypeError("q, caches and out must share one dtype")
     if out.shape != (tokens, num_heads, value_size):
         raise ValueError(f"out must be {(tokens, num_heads, value_size)}, got {tuple(out.shape)}")
+    options = (float(scale), int(window) if window else 0, int(keep_first) if window else 0, int(chunk) if chunk else 0,
+               float(softcap) if softcap else 0.0, _opt(sink, "sink", torch.float32), _opt(gate, "gate", torch.float32),
+               *_value_gate(value_gate, q, value_size, False))
+    singles = None
+    if q_tiles is not None and single_tokens is not None and _takes_prompt_tiles(
+            q_tiles, tokens - single_tokens.shape[0], head_size, value_size, value_stride, k_cache, v_cache):
+        fn = _fn(
+            "einf_paged_attention_prompt",
+            [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int,
+             c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p, c_longlong,
+             c_void_p, c_void_p],
+        )
+        _check(
+            fn(_dev(q, "q"), _dev(k_cache, "k_cache"), _dev(v_cache, "v_cache"), _code(q),
+               _opt(block_table, "block_table", torch.int32), _opt(q_tiles, "q_tiles", torch.int32), q_tiles.shape[0],
+               _dev(out, "out"), num_heads, num_kv_heads, head_size, value_size, value_stride, page_size, num_pages,
+               block_table.shape[1], *options, _dev(status, "status"), _stream()),
+            "paged_attention_prompt",
+        )
+        tokens = single_tokens.shape[0]
+        if tokens == 0:
+            return
+        singles = single_tokens
     fn = _fn(
         "einf_paged_attention_generic",
         [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
          c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p,
-         c_longlong, c_void_p, c_void_p],
+         c_longlong, c_void_p, c_void_p, c_void_p],
     )
     _check(
         fn(_dev(q, "q"), _dev(k_cache, "k_cache"), _dev(v_cache, "v_cache"), _code(q),
            _opt(block_table, "block_table", torch.int32), _opt(seq_of_token, "seq_of_token", torch.int32),
            _opt(positions, "positions", torch.int32), _dev(out, "out"), tokens, num_heads, num_kv_heads,
-           head_size, value_size, value_stride, page_size, num_pages, block_table.shape[1], float(scale),
-           int(window) if window else 0, int(keep_first) if window else 0, int(chunk) if chunk else 0,
-           float(softcap) if softcap else 0.0, _opt(sink, "sink", torch.float32), _opt(gate, "gate", torch.float32),
-           *_value_gate(value_gate, q, value_size, False), _dev(status, "status"), _stream()),
+           head_size, value_size, value_stride, page_size, num_pages, block_table.shape[1], *options,
+           _opt(singles, "single_tokens", torch.int32), _dev(status, "status"), _stream()),
         "paged_attention_generic",
+    )
+
+
+#: tokens of prompt portions per tile of ``q_tiles``, on average, from which they take the kernel that shares key rows (a
+#: tile of fewer leaves most of its 32 rows empty, and the warps of the general kernel walk the keys side by side)
+PROMPT_TILE_MIN = 8
+
+
+def _takes_prompt_tiles(q_tiles: torch.Tensor, tokens: int, head_size: int, value_size: int, value_stride: int,
+                        k_cache: torch.Tensor, v_cache: torch.Tensor) -> bool:
+    return (
+        q_tiles.shape[0] > 0 and tokens >= PROMPT_TILE_MIN * q_tiles.shape[0] and head_size <= 128 and head_size % 4 == 0
+        and value_size <= 128 and value_size % 4 == 0 and value_stride % 4 == 0
+        and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0
+        and k_cache.shape[0] * k_cache.shape[1] * k_cache.shape[2] <= 0x7fffffff
     )
 
 

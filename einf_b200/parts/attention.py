@@ -382,5 +382,5 @@ class PagedAttention(Mixer):
         ops.paged_attention_generic(
             q, cache.k, cache.v, ctx.block_tables[cache.group], ctx.seq_of_token, ctx.positions,
             out, self.scale, self.window, ctx.status, chunk=self.chunk, softcap=self.softcap,
-            keep_first=self.keep_first, sink=self.sink, value_gate=gate,
+            keep_first=self.keep_first, sink=self.sink, value_gate=gate, **ctx.portions(),
         )

@@ -211,6 +211,13 @@ class StepContext:
     decode_only: bool = False
     extras: dict[str, Any] = field(default_factory=dict)
 
+    def portions(self) -> dict:
+        """What the general attention kernels take to tell portions of prompts from single tokens (nothing off the GPU:
+        the plain statements that stand in for them there take every token alone)."""
+        if not self.q_tiles.is_cuda:
+            return {}
+        return {"q_tiles": self.q_tiles, "single_tokens": self.single_tokens}
+
 
 class Part:
     """Base of all parts."""

@@ -235,7 +235,7 @@ class LatentAttention(Mixer):
             mixed_latent = torch.empty((tokens, heads, self.kv_rank), dtype=dtype, device=device)
             ops.paged_attention_generic(
                 q_full, cache.k, None, table, ctx.seq_of_token, ctx.positions, mixed_latent,
-                self.scale, self.window, ctx.status, values_in_keys=self.kv_rank, sink=self.sink, gate=gate,
+                self.scale, self.window, ctx.status, values_in_keys=self.kv_rank, sink=self.sink, gate=gate, **ctx.portions(),
             )
         mixed = torch.empty((tokens, heads, self.value_size), dtype=dtype, device=device)
         ops.per_head_project(mixed_latent, self.v_up, mixed)

@@ -142,6 +142,58 @@ def test_tcgen05_attention_with_chunks_and_caps(dev, first_case):
         torch.testing.assert_close(out, want, **tol(torch.bfloat16), msg=lambda m: f"case {case}: {m}")
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads, kv_heads, size, value_size, page, options", [
+    (2, 1, 64, 64, 16, {}), (3, 3, 128, 128, 8, {"window": 50}), (2, 2, 4, 68, 16, {"window": 40, "keep_first": 70}),
+    (4, 2, 36, 20, 64, {"chunk": 48, "softcap": 4.0}), (2, 1, 96, 64, 16, {"in_keys": True, "sink": True, "gate": True}),
+    (2, 1, 64, 100, 16, {"sink": True, "value_gate": True, "window": 64}),
+])
+@pytest.mark.parametrize("requests", [[(0, 8)], [(0, 33), (70, 1), (61, 67)], [(5, 129), (0, 32), (0, 1)]])
+def test_attention_of_portions_shares_keys(dev, dtype, heads, kv_heads, size, value_size, page, options, requests):
+    """Portions of prompts through the kernel that reads a key row once for 32 tokens, single tokens beside them,
+    against the plain statement: rows around its tiles of 32 tokens and 64 keys, every option of the general kernel."""
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(size + value_size + len(requests))
+    options = dict(options)
+    window, in_keys = options.pop("window", None), options.pop("in_keys", False)
+    tokens = sum(n for _, n in requests)
+    if options.pop("sink", False):
+        options["sink"] = torch.randn(heads, generator=gen).to(dev)
+    if options.pop("gate", False):
+        options["gate"] = torch.rand((tokens, heads), generator=gen).to(dev)
+    if options.pop("value_gate", False):
+        options["value_gate"] = torch.randn((tokens, heads * value_size), generator=gen).to(dtype).to(dev)
+    pages = [-(-(start + n) // page) for start, n in requests]
+    order = torch.randperm(sum(pages), generator=gen).to(torch.int32)
+    table = torch.full((len(requests), max(pages)), -1, dtype=torch.int32)
+    seq, pos, tiles, singles = [], [], [], []
+    for r, ((start, n), own) in enumerate(zip(requests, torch.split(order, pages))):
+        table[r, :own.shape[0]] = own
+        if n == 1:
+            singles.append(len(seq))
+        else:
+            tiles += [(r, len(seq) + first, min(128, n - first), start + first) for first in range(0, n, 128)]
+        seq, pos = seq + [r] * n, pos + list(range(start, start + n))
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device=dev)  # noqa: E731
+    q = torch.randn((tokens, heads, size), generator=gen).to(dtype).to(dev)
+    k = torch.randn((sum(pages), kv_heads, page, size), generator=gen).to(dtype).to(dev)
+    v = None if in_keys else torch.randn((sum(pages), kv_heads, page, value_size), generator=gen).to(dtype).to(dev)
+    if in_keys:
+        options["values_in_keys"] = value_size
+    st = status(dev)
+    out, want = (torch.full((tokens, heads, value_size), float("nan"), dtype=dtype, device=dev) for _ in range(2))
+    assert ops._takes_prompt_tiles(ints(tiles).view(-1, 4), tokens - len(singles), size, value_size,
+                                   size if in_keys else value_size, k, k if in_keys else v)
+    before = ops.launch_count
+    ops.paged_attention_generic(q, k, v, table.to(dev), ints(seq), ints(pos), out, size ** -0.5, window, st,
+                                q_tiles=ints(tiles).view(-1, 4), single_tokens=ints(singles), **options)
+    assert ops.launch_count - before == 1 + bool(singles)
+    ref.paged_attention_generic(q, k, v, table.to(dev), ints(seq), ints(pos), want, size ** -0.5, window, st, **options)
+    assert int(st) == 0
+    close(out, want, dtype)
+
+
 def _packed(lengths, dev):
     starts = [0]
     seq = []
