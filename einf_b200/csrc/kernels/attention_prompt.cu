@@ -1,0 +1,329 @@
+// Causal attention of prompts that start in this step over keys and values of their own per head, as a latent cache's rows
+// give them when its up-projections are applied to the rows (bfloat16, mma.sync, 32-bit sums and softmax).
+//
+// A latent cache holds one row [c | r] for all heads, and attention can run on the rows as they are, with the key
+// up-projection absorbed into the queries (attention_latent.cu): 2 kv_rank + rot_dim multiply-adds a (head, query, key).
+// Head by head, with keys [W_uk c | r] and values W_uv c, it is dim + rot_dim + value_size, a third of that at rows of
+// 512 + 64 and heads of 128, for one more product over the rows.  That pays for a prompt that is all there: every row is
+// projected once and met by all later queries.  (A portion with cached tokens before it would project those anew in
+// every step, a single token would project all it sees: both stay on the rows.)
+//
+// A CTA has 64 queries of one head, a warp 16 of them with its queries in registers; 64 keys a tile; the next tile's keys
+// are brought while this one's values are used and the other way round.  Keys come from two places (the head's plain part
+// and the rotated part that all heads share), queries too.  Three CTAs an SM hide one another's waits (two warps of 32
+// rows, which read half as much shared memory, have no registers left to load ahead of their products).
+//
+// Measured (B200): 12 heads, keys of 128 + 64, values of 128, 2,048 tokens (16 GFLOP): 116 us, against 336 us of
+// attention_latent.cu on the rows of 512 + 64 (55 GFLOP); two warps of 32 rows 184 us.  The mixer as a whole 403 -> 176 us.
+// What bounds it: the chain of a tile (products, softmax, products) in the CTAs with the most keys, three of which share
+// an SM, and the reads of shared memory (92 a tile and warp, 512 bytes each, against 160 products).
+#include <type_traits>
+
+#include "mma_sync.cuh"
+
+namespace einf {
+
+constexpr int kPromptRows = 64, kPromptKeys = 64, kPromptThreads = 128;
+
+struct HeadPromptArgs {
+  const __nv_bfloat16* q_plain; long long q_plain_token, q_plain_head;     // strides in elements
+  const __nv_bfloat16* q_rot; long long q_rot_token, q_rot_head;
+  const __nv_bfloat16* k_plain; long long k_token, k_head;
+  const __nv_bfloat16* k_rot;                                              // [tokens, rot_dim]
+  const __nv_bfloat16* v; long long v_token, v_head;
+  const int4* tiles;                 // request, first token, tokens (up to 128), first position
+  __nv_bfloat16* out;                // [tokens, heads, value_size]
+  const float* sink; const float* gate;
+  int heads, dim, rot_dim, value_size, window, wave;
+  float scale_log2;
+};
+
+// Byte of a 16-byte piece of a row whose rows are 128-byte lines: exchanged by the row's last three bits, so that the eight
+// rows of an ldmatrix meet no bank twice.
+__device__ __forceinline__ uint32_t swizzled(int row, int piece, int pitch) {
+  return (uint32_t)(row * pitch + ((piece & ~7) | ((piece ^ row) & 7)) * 16);
+}
+
+// KEY: dim + rot_dim filled up to 128 or 192; VALUE: value_size filled up to 64 or 128.
+template <int KEY, int VALUE>
+__global__ void __launch_bounds__(kPromptThreads, 3)
+head_prompt_attention_kernel(const __grid_constant__ HeadPromptArgs a) {
+  extern __shared__ __align__(128) unsigned char prompt_smem[];
+  constexpr int kKeyPitch = KEY * 2, kValuePitch = VALUE * 2;
+  constexpr int kK = 0, kV = kPromptKeys * kKeyPitch;
+  pdl_launch_dependents();
+  // Which rows: (tile, head) pairs in the order of their keys, the last tiles first; every second wave of CTAs takes them
+  // from the other end, so that an SM's CTAs, which all run at once, are long and short ones.
+  const int total = (int)gridDim.x, wave = (int)blockIdx.x / a.wave, place = (int)blockIdx.x - wave * a.wave;
+  const int rank = wave & 1 ? total - 1 - ((wave >> 1) * a.wave + place) : ((wave + 1) >> 1) * a.wave + place;
+  const int row_tiles = total / a.heads, row_tile = row_tiles - 1 - rank / a.heads, h = rank % a.heads;
+  const int4 tile = a.tiles[row_tile >> 1];
+  const int sub = (row_tile & 1) * kPromptRows;
+  const int rows = min(kPromptRows, tile.z - sub);
+  if (rows <= 0) {
+    pdl_wait();
+    return;
+  }
+  const int t0 = tile.y + sub, pos0 = tile.w + sub;
+  const int key_token = tile.y - tile.w;                  // packed index of the request's position 0
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, q2 = (lane & 3) * 2;
+  const uint32_t base = smem_address(prompt_smem);
+  const int last_pos = pos0 + rows - 1;
+  const int first_tile = a.window > 0 ? max(0, pos0 - a.window + 1) / kPromptKeys : 0, end_tile = last_pos / kPromptKeys + 1;
+  pdl_wait();
+
+  // 64 rows of a plain and a rotated part, zeros from row `count` on: a thread has one 16-byte piece of every 128-byte
+  // line of four rows
+  auto bring = [&](uint32_t at, auto lines_tag, const __nv_bfloat16* plain, long long plain_stride, int plain_size,
+                   const __nv_bfloat16* rot, long long rot_stride, int rot_size, int count) {
+    constexpr int kLines = decltype(lines_tag)::value, kPitch = 128 * kLines;
+    const int r0 = threadIdx.x >> 3, piece = threadIdx.x & 7;
+#pragma unroll
+    for (int line = 0; line < kLines; ++line) {
+      const int e = 64 * line + 8 * piece;
+      const bool in_plain = e < plain_size, in_rot = !in_plain && e - plain_size < rot_size;
+      const __nv_bfloat16* from = plain;
+      if (in_plain) from = plain + r0 * plain_stride + e;
+      else if (in_rot) from = rot + r0 * rot_stride + (e - plain_size);
+      const long long step = in_plain ? 16 * plain_stride : in_rot ? 16 * rot_stride : 0;
+      const uint32_t to = at + r0 * kPitch + 128 * line + ((piece ^ r0) & 7) * 16;       // rows 16 apart exchange alike
+      const bool any = in_plain || in_rot;
+#pragma unroll
+      for (int u = 0; u < 4; ++u, from += step) {
+        const bool there = any && r0 + 16 * u < count;
+        cp_async16(to + u * 16 * kPitch, there ? from : plain, there ? 16 : 0);
+      }
+    }
+  };
+  using KeyLines = std::integral_constant<int, KEY / 64>;
+  using ValueLines = std::integral_constant<int, VALUE / 64>;
+  auto bring_keys = [&](int t) {
+    const int j0 = t * kPromptKeys;
+    bring(base + kK, KeyLines{}, a.k_plain + (key_token + j0) * a.k_token + h * a.k_head, a.k_token, a.dim,
+          a.k_rot + (long long)(key_token + j0) * a.rot_dim, a.rot_dim, a.rot_dim, last_pos + 1 - j0);
+    cp_async_commit_group();
+  };
+  auto bring_values = [&](int t) {
+    const int j0 = t * kPromptKeys;
+    bring(base + kV, ValueLines{}, a.v + (key_token + j0) * a.v_token + h * a.v_head, a.v_token, a.value_size, nullptr, 0, 0,
+          last_pos + 1 - j0);
+    cp_async_commit_group();
+  };
+  const int in8 = lane & 7, second = (lane >> 3) & 1, third = lane >> 4;
+  // the queries come through the keys' place
+  bring(base + kK, KeyLines{}, a.q_plain + t0 * a.q_plain_token + h * a.q_plain_head, a.q_plain_token, a.dim,
+        a.q_rot + t0 * a.q_rot_token + h * a.q_rot_head, a.q_rot_token, a.rot_dim, rows);
+  cp_async_commit_group();
+  cp_async_wait_groups<0>();
+  __syncthreads();
+  uint32_t Q[KEY / 16][4];
+#pragma unroll
+  for (int kk = 0; kk < KEY / 16; ++kk)
+    ldsm_x4(Q[kk], base + kK + swizzled(16 * warp + in8 + 8 * second, 2 * kk + third, kKeyPitch));
+  __syncthreads();
+  bring_keys(first_tile);
+  bring_values(first_tile);
+
+  float O[VALUE / 8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < VALUE / 8; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) O[j][e] = 0.f;
+  const int warp_first = pos0 + 16 * warp, warp_last = warp_first + 15;
+
+  for (int t = first_tile; t < end_tile; ++t) {
+    const int j0 = t * kPromptKeys;
+    // a warp none of whose rows sees a key of the tile sits the products out
+    const bool seen = j0 <= warp_last && (a.window <= 0 || j0 + kPromptKeys - 1 > warp_first - a.window);
+    cp_async_wait_groups<1>();                             // the keys are there
+    __syncthreads();
+    float S[8][4];
+    if (seen) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[j][e] = 0.f;
+#pragma unroll
+      for (int kk = 0; kk < KEY / 16; ++kk) {
+        uint32_t kf[4][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          ldsm_x4(kf[j], base + kK + swizzled(16 * j + in8 + 8 * third, 2 * kk + second, kKeyPitch));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          mma_bf16_16816(S[2 * j], Q[kk], kf[j][0], kf[j][1]);
+          mma_bf16_16816(S[2 * j + 1], Q[kk], kf[j][2], kf[j][3]);
+        }
+      }
+    }
+    __syncthreads();                                       // the keys are used up
+    if (t + 1 < end_tile) bring_keys(t + 1);
+    else cp_async_commit_group();                          // an empty group: the values are always the second youngest
+    if (seen) {
+      const bool masks = j0 + kPromptKeys - 1 > warp_first || (a.window > 0 && j0 <= warp_last - a.window);
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {               // rows g and g + 8 of the 16
+        const int pos = warp_first + g + 8 * half;
+        float top = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float z = S[j][2 * half + e] * a.scale_log2;
+            if (masks) {
+              const int key = j0 + 8 * j + q2 + e;
+              z = (key <= pos && (a.window <= 0 || key > pos - a.window)) ? z : -INFINITY;
+            }
+            S[j][2 * half + e] = z;
+            top = fmaxf(top, z);
+          }
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+        const float to = fmaxf(m[half], top);
+        const float shift = to == -INFINITY ? 0.f : to;
+        const float factor = exp2f(m[half] - shift);       // nothing seen so far: zero
+        m[half] = to;
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float w;
+            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(w) : "f"(S[j][2 * half + e] - shift));
+            S[j][2 * half + e] = w;
+            sum += w;
+          }
+        l[half] = l[half] * factor + sum;                  // this lane's share; the row's lanes are added at the end
+        if (__any_sync(0xffffffffu, factor != 1.f)) {
+#pragma unroll
+          for (int j = 0; j < VALUE / 8; ++j) {
+            O[j][2 * half] *= factor;
+            O[j][2 * half + 1] *= factor;
+          }
+        }
+      }
+    }
+    cp_async_wait_groups<1>();                             // the values are there
+    __syncthreads();
+    if (seen) {
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {                     // the weights are the first operand as they lie in registers
+        const uint32_t P[4] = {pack_pair(S[2 * kk][0], S[2 * kk][1]), pack_pair(S[2 * kk][2], S[2 * kk][3]),
+                               pack_pair(S[2 * kk + 1][0], S[2 * kk + 1][1]), pack_pair(S[2 * kk + 1][2], S[2 * kk + 1][3])};
+#pragma unroll
+        for (int j0v = 0; j0v < VALUE / 16; j0v += 4) {
+          uint32_t vf[4][4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            ldsm_x4_trans(vf[j], base + kV + swizzled(16 * kk + in8 + 8 * second, 2 * (j0v + j) + third, kValuePitch));
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            mma_bf16_16816(O[2 * (j0v + j)], P, vf[j][0], vf[j][1]);
+            mma_bf16_16816(O[2 * (j0v + j) + 1], P, vf[j][2], vf[j][3]);
+          }
+        }
+      }
+    }
+    __syncthreads();                                       // the values are used up
+    if (t + 1 < end_tile) bring_values(t + 1);
+    else cp_async_commit_group();
+  }
+  cp_async_wait_groups<0>();
+
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const int r = 16 * warp + g + 8 * half;
+    float sum = l[half];
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    if (r >= rows) continue;
+    if (a.sink) sum += exp2f(a.sink[h] * 1.4426950408889634f - m[half]);
+    const long long row = (long long)(t0 + r) * a.heads + h;
+    float factor = sum > 0.f ? 1.f / sum : 0.f;
+    if (a.gate) factor *= a.gate[row];
+    __nv_bfloat16* out = a.out + row * a.value_size;
+#pragma unroll
+    for (int j = 0; j < VALUE / 8; ++j) {
+      const int column = 8 * j + q2;
+      if (column < a.value_size)
+        *reinterpret_cast<uint32_t*>(out + column) = pack_pair(O[j][2 * half] * factor, O[j][2 * half + 1] * factor);
+    }
+  }
+}
+
+// Cached rows of the step's tokens, taken apart: rows[t] = the first `first` elements of the row in slot t, rest[t] the next
+// `second` (multiples of eight; a token without a slot gets zeros).
+__global__ void __launch_bounds__(256)
+latent_rows_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restrict__ slots, long long num_rows, int row_size,
+                   __nv_bfloat16* __restrict__ rows, int first, __nv_bfloat16* __restrict__ rest, int second, int tokens) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int pieces = (first + second) / 8;
+  const long long total = (long long)tokens * pieces;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const int t = (int)(i / pieces), e = 8 * (int)(i - (long long)t * pieces);
+    const int slot = slots[t];
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (slot >= 0 && slot < num_rows) v = *reinterpret_cast<const uint4*>(cache + (long long)slot * row_size + e);
+    __nv_bfloat16* to = e < first ? rows + (long long)t * first + e : rest + (long long)t * second + (e - first);
+    *reinterpret_cast<uint4*>(to) = v;
+  }
+}
+
+template <int KEY, int VALUE>
+static cudaError_t launch_head_prompt(const HeadPromptArgs& a, int num_tiles, cudaStream_t stream) {
+  auto kernel = head_prompt_attention_kernel<KEY, VALUE>;
+  constexpr int kBytes = kPromptKeys * (KEY + VALUE) * 2;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+  if (e != cudaSuccess) return e;
+  return launch_pdl(kernel, dim3(2 * num_tiles * a.heads), dim3(kPromptThreads), kBytes, stream, a);
+}
+
+}  // namespace einf
+
+using namespace einf;
+
+extern "C" int einf_latent_rows(const void* cache, const int* slots, long long num_rows, int row_size, void* rows, int first,
+                                void* rest, int second, int tokens, cudaStream_t stream) {
+  if (tokens == 0) return 0;
+  if (first % 8 || second % 8 || row_size % 8 || first <= 0 || second < 0 || first + second > row_size ||
+      (((uintptr_t)cache | (uintptr_t)rows | (uintptr_t)rest) & 15))
+    return (int)cudaErrorInvalidValue;
+  const long long ctas = ((long long)tokens * ((first + second) / 8) + 255) / 256;
+  return (int)launch_pdl(latent_rows_kernel, dim3((unsigned)(ctas < 148 * 8 ? ctas : 148 * 8)), dim3(256), 0, stream,
+                         (const __nv_bfloat16*)cache, slots, num_rows, row_size, (__nv_bfloat16*)rows, first,
+                         (__nv_bfloat16*)rest, second, tokens);
+}
+
+// Every request listed in `tiles` starts at position 0 in this step, its tokens packed one after the other.  Sizes and
+// strides in multiples of eight elements, pointers on 16-byte borders; dim + rot_dim up to 192, value_size up to 128.
+// `wave`: multiprocessors of the device.
+extern "C" int einf_head_prompt_attention(const void* q_plain, long long q_plain_token, long long q_plain_head,
+                                          const void* q_rot, long long q_rot_token, long long q_rot_head, const void* k_plain,
+                                          long long k_token, long long k_head, const void* k_rot, const void* v,
+                                          long long v_token, long long v_head, const int* tiles, int num_tiles, void* out,
+                                          const float* sink, const float* gate, int heads, int dim, int rot_dim,
+                                          int value_size, int window, float scale, int wave, cudaStream_t stream) {
+  if (num_tiles == 0) return 0;
+  const long long strides = q_plain_token | q_plain_head | q_rot_token | q_rot_head | k_token | k_head | v_token | v_head;
+  if (heads <= 0 || 2ll * num_tiles * heads > 0x7fffffff || dim <= 0 || rot_dim < 0 || dim + rot_dim > 192 ||
+      value_size <= 0 || value_size > 128 || ((dim | rot_dim | value_size) & 7) || (strides & 7) || wave <= 0 ||
+      (((uintptr_t)q_plain | (uintptr_t)q_rot | (uintptr_t)k_plain | (uintptr_t)k_rot | (uintptr_t)v | (uintptr_t)out |
+        (uintptr_t)tiles) & 15))
+    return (int)cudaErrorInvalidValue;
+  HeadPromptArgs a;
+  a.q_plain = (const __nv_bfloat16*)q_plain; a.q_plain_token = q_plain_token; a.q_plain_head = q_plain_head;
+  a.q_rot = (const __nv_bfloat16*)q_rot; a.q_rot_token = q_rot_token; a.q_rot_head = q_rot_head;
+  a.k_plain = (const __nv_bfloat16*)k_plain; a.k_token = k_token; a.k_head = k_head;
+  a.k_rot = (const __nv_bfloat16*)k_rot;
+  a.v = (const __nv_bfloat16*)v; a.v_token = v_token; a.v_head = v_head;
+  a.tiles = (const int4*)tiles; a.out = (__nv_bfloat16*)out; a.sink = sink; a.gate = gate;
+  a.heads = heads; a.dim = dim; a.rot_dim = rot_dim; a.value_size = value_size; a.window = window; a.wave = wave;
+  a.scale_log2 = scale * 1.4426950408889634f;
+  if (dim + rot_dim <= 128)
+    return (int)(value_size <= 64 ? launch_head_prompt<128, 64>(a, num_tiles, stream)
+                                  : launch_head_prompt<128, 128>(a, num_tiles, stream));
+  return (int)(value_size <= 64 ? launch_head_prompt<192, 64>(a, num_tiles, stream)
+                                : launch_head_prompt<192, 128>(a, num_tiles, stream));
+}

@@ -859,6 +859,87 @@ def latent_attention(
         launch(q_tiles, None, q_tiles.shape[0], 1, (0, 0))
 
 
+#: most elements of a head's key (plain and rotated part) and of its value that the prompts' kernel takes
+HEAD_PROMPT_MAX_KEY, HEAD_PROMPT_MAX_VALUE = 192, 128
+
+
+def takes_head_prompts(dtype: torch.dtype, dim: int, rot_dim: int, value_size: int, kv_rank: int) -> bool:
+    """Whether a latent layer of these sizes can run prompts head by head (:func:`head_prompt_attention`): bfloat16 and
+    whole 16-byte pieces."""
+    return (
+        dtype == torch.bfloat16 and dim + rot_dim <= HEAD_PROMPT_MAX_KEY and value_size <= HEAD_PROMPT_MAX_VALUE
+        and all(n % 8 == 0 for n in (dim, rot_dim, value_size, kv_rank))
+    )
+
+
+def latent_rows(cache: torch.Tensor, slots: torch.Tensor, rows: torch.Tensor, rest: torch.Tensor) -> None:
+    """The step's tokens' cached rows, taken apart: of the row in slot ``slots[t]`` of ``cache [pages, 1, page_size, row]``
+    the first elements go to ``rows [tokens, n]``, the next to ``rest [tokens, m]`` (zeros for a token without a slot)."""
+    tokens = slots.shape[0]
+    pages, kv_heads, page_size, row = cache.shape
+    if kv_heads != 1 or rows.shape[0] != tokens or rest.shape[0] != tokens or rows.shape[1] + rest.shape[1] > row:
+        raise ValueError(f"latent_rows: cache {tuple(cache.shape)}, rows {tuple(rows.shape)}, rest {tuple(rest.shape)}")
+    if not (cache.dtype == rows.dtype == rest.dtype == torch.bfloat16):
+        raise TypeError("latent_rows takes bfloat16")
+    fn = _fn("einf_latent_rows", [c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p])
+    _check(
+        fn(_dev(cache, "cache"), _opt(slots, "slots", torch.int32), pages * page_size, row, _dev(rows, "rows"), rows.shape[1],
+           _dev(rest, "rest"), rest.shape[1], tokens, _stream()),
+        "latent_rows",
+    )
+
+
+def head_prompt_attention(
+    q_plain: torch.Tensor,
+    q_rot: torch.Tensor,
+    k_plain: torch.Tensor,
+    k_rot: torch.Tensor,
+    v: torch.Tensor,
+    q_tiles: torch.Tensor,
+    out: torch.Tensor,
+    scale: float,
+    window: Optional[int],
+    sink: Optional[torch.Tensor] = None,
+    gate: Optional[torch.Tensor] = None,
+) -> None:
+    """Causal attention of prompts that start in this step, every head with keys and values of its own: query head h
+    scores key head h, ``q_plain . k_plain + q_rot . k_rot``, where all heads share ``k_rot``.  ``q_plain``, ``k_plain``
+    ``[tokens, heads, dim]``, ``q_rot [tokens, heads, rot]``, ``v [tokens, heads, value]`` (views of wider rows are fine),
+    ``k_rot [tokens, rot]``, ``out [tokens, heads, value]``, all bfloat16; ``q_tiles`` as for
+    :func:`paged_prefill_attention`, of requests whose first token in the step is at position 0.  ``window``, ``sink`` and
+    ``gate``: see :func:`paged_attention_generic`."""
+    tokens, heads, dim = q_plain.shape
+    rot_dim, value_size = q_rot.shape[2], v.shape[2]
+    if q_rot.shape[:2] != (tokens, heads) or k_plain.shape != (tokens, heads, dim) or k_rot.shape != (tokens, rot_dim) or \
+            v.shape[:2] != (tokens, heads) or out.shape != v.shape:
+        raise ValueError("head_prompt_attention: q, k, v and out must agree in tokens, heads and sizes")
+    if any(t.dtype != torch.bfloat16 for t in (q_plain, q_rot, k_plain, k_rot, v, out)):
+        raise TypeError("head_prompt_attention takes bfloat16")
+    if any(t.stride(2) != 1 for t in (q_plain, q_rot, k_plain, v)):
+        raise ValueError("heads need unit stride in their last dimension")
+    if dim + rot_dim > HEAD_PROMPT_MAX_KEY or value_size > HEAD_PROMPT_MAX_VALUE:
+        raise UnsupportedSize(f"keys of {dim + rot_dim} and values of {value_size} elements a head")
+    if q_tiles.dim() != 2 or q_tiles.shape[1] != 4:
+        raise ValueError("q_tiles must be int32 [tiles, 4]")
+    if sink is not None and (sink.dtype != torch.float32 or sink.shape != (heads,)):
+        raise ValueError(f"sink must be float32 [{heads}]")
+    _check_gate(gate, tokens, heads)
+    fn = _fn(
+        "einf_head_prompt_attention",
+        [c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p,
+         c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+         c_float, c_int, c_void_p],
+    )
+    _check(
+        fn(q_plain.data_ptr(), q_plain.stride(0), q_plain.stride(1), q_rot.data_ptr(), q_rot.stride(0), q_rot.stride(1),
+           k_plain.data_ptr(), k_plain.stride(0), k_plain.stride(1), _dev(k_rot, "k_rot"), v.data_ptr(), v.stride(0),
+           v.stride(1), _opt(q_tiles, "q_tiles", torch.int32), q_tiles.shape[0], _dev(out, "out"),
+           _opt(sink, "sink", torch.float32), _opt(gate, "gate", torch.float32), heads, dim, rot_dim, value_size,
+           int(window) if window else 0, float(scale), _sm_count(), _stream()),
+        "head_prompt_attention",
+    )
+
+
 #: activations of :func:`activation` by name
 ACTIVATIONS = {"relu2": 0, "gelu_tanh": 1, "silu": 2, "relu": 3, "gelu": 4}
 

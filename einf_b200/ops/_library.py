@@ -31,6 +31,8 @@ LAUNCHERS = {
     "einf_latent_decode_merge": "attention_generic",
     "einf_latent_attention_tcgen05": "attention_latent",
     "einf_latent_attention_tcgen05_parts": "attention_latent",
+    "einf_latent_rows": "attention_prompt",
+    "einf_head_prompt_attention": "attention_prompt",
     "einf_gemm_simt": "gemm_simt",
     "einf_gemm_simt_shares": "gemm_simt",
     "einf_gemm_tcgen05": "gemm_tcgen05",

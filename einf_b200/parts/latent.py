@@ -24,6 +24,10 @@ reads keys and values out of one tile.  Rows of 64 and 128 elements take the ker
 the cached rows as keys and values at once: the mixed rows then carry ``rot_dim`` elements more than the value up-projection
 reads (a fifth to a quarter more work in the second product, none in memory traffic).  Other row
 sizes, and the 32-bit path, run the general kernel, which reads the values out of the key rows.
+
+A step of prompts alone that all start in it (no cached tokens before them, no single tokens beside them) runs head
+by head instead where the layer is not on the attention mixer's kernels: the up-projections are applied to the step's
+rows, one product for keys and values, and ``ops.head_prompt_attention`` meets queries and keys as they are.
 """
 from __future__ import annotations
 
@@ -70,6 +74,8 @@ class LatentAttention(Mixer):
             fast = (f"attention_tcgen05:HEAD_SIZE={row}",)
         elif ops.has_latent_attention(runtime.dtype, row, ops.LATENT_PAGE):
             fast = ("attention_latent",)
+        if cls._prompts_by_heads(spec, row, runtime.dtype):
+            fast += ("attention_prompt",)
         return ("pointwise", "latent", "attention_generic", "gemm_simt") + \
             (("gemm_tcgen05",) if runtime.dtype == torch.bfloat16 else ()) + fast
 
@@ -85,6 +91,13 @@ class LatentAttention(Mixer):
     @staticmethod
     def _row_on_tensor_cores(row: int, dtype) -> bool:
         return dtype == torch.bfloat16 and row in (64, 128)
+
+    @classmethod
+    def _prompts_by_heads(cls, spec, row: int, dtype) -> bool:
+        """Whether prompts that start in a step can run head by head (see the top of the file).  Not where the cached rows
+        are of a size that the attention mixer's kernels take: those meet a row of 64 or 128 elements as one wide head."""
+        return not cls._row_on_tensor_cores(row, dtype) and ops.takes_head_prompts(
+            dtype, int(spec["head_size"]), int(spec["rotary_size"]), int(spec["value_head_size"]), int(spec["kv_rank"]))
 
     def __init__(self, spec, tensors, runtime):
         super().__init__(spec, tensors, runtime)
@@ -133,7 +146,14 @@ class LatentAttention(Mixer):
         # absorbed into the query: per head [kv_rank, dim], the transpose of the key up-projection
         k_up = tensors["k_up.weight"].reshape(heads, self.dim, self.kv_rank)
         self.k_up_t = runtime.matrix(k_up.transpose(1, 2).contiguous())
-        self.v_up = runtime.matrix(tensors["v_up.weight"].reshape(heads, self.value_size, self.kv_rank))
+        self.by_heads = self._prompts_by_heads(spec, self.row, runtime.dtype)
+        if self.by_heads and tensors["k_up.weight"].dtype == tensors["v_up.weight"].dtype == runtime.dtype:
+            # both up-projections as one matrix [heads * dim | heads * value, kv_rank]; the values' also serve alone
+            self.kv_up = runtime.matrix(torch.cat([tensors["k_up.weight"], tensors["v_up.weight"]], dim=0))
+            self.v_up = self.kv_up[heads * self.dim:].view(heads, self.value_size, self.kv_rank)
+        else:
+            self.by_heads = False
+            self.v_up = runtime.matrix(tensors["v_up.weight"].reshape(heads, self.value_size, self.kv_rank))
         self.out_weight = runtime.matrix(tensors["o_proj.weight"])
         self.fast = self._row_on_tensor_cores(self.row, runtime.dtype)
 
@@ -141,7 +161,7 @@ class LatentAttention(Mixer):
         """As for the attention mixer: the decode kernel's shape follows the batch and the longest context."""
         singles = int(ctx.single_tokens.shape[0])
         if not singles:
-            return ()
+            return ("heads",) if self._runs_by_heads(ctx) else ()
         context = self._visible(ctx.max_context_len)
         if not self.fast and ops.has_latent_attention(self.runtime.dtype, self.row, page_size):
             return ("latent", ops.latent_attention_splits(singles, self.num_heads, self.kv_rank, context))
@@ -149,6 +169,28 @@ class LatentAttention(Mixer):
             # the shared-row decode kernel cuts a token's keys by the batch and the longest context
             return ("shares", ops.latent_decode_splits(singles, self.num_heads, context)) if ctx.decode_only else ()
         return ops.decode_plan(singles, self.num_heads, 1, self.row, page_size, context)
+
+    def _runs_by_heads(self, ctx: StepContext) -> bool:
+        """A step of prompts alone that all start in it."""
+        return self.by_heads and not ctx.single_tokens.shape[0] and ctx.q_tiles.shape[0] > 0 \
+            and ctx.max_portion_start == 0 and ctx.q_tiles.is_cuda
+
+    def _prompts(self, q_plain, q_full, gate, ctx: StepContext, cache: CacheView) -> torch.Tensor:
+        """Prompts head by head: the step's rows through both up-projections, then attention; ``[T, H, value]``."""
+        tokens, heads, device = q_full.shape[0], self.num_heads, q_full.device
+        rows = torch.empty((tokens, self.kv_rank), dtype=q_full.dtype, device=device)
+        part = torch.empty((tokens, self.rot_dim), dtype=q_full.dtype, device=device)
+        ops.latent_rows(cache.k, ctx.slots[cache.group], rows, part)
+        kv = torch.empty((tokens, self.kv_up.shape[0]), dtype=q_full.dtype, device=device)
+        ops.linear(rows, self.kv_up, None, kv)
+        keys = heads * self.dim
+        mixed = torch.empty((tokens, heads, self.value_size), dtype=q_full.dtype, device=device)
+        ops.head_prompt_attention(
+            q_plain, q_full[:, :, self.kv_rank:self.kv_rank + self.rot_dim], kv[:, :keys].unflatten(1, (heads, self.dim)),
+            part, kv[:, keys:].unflatten(1, (heads, self.value_size)), ctx.q_tiles, mixed, self.scale, self.window,
+            sink=self.sink, gate=gate,
+        )
+        return mixed
 
     def _visible(self, context: int) -> int:
         return min(context, self.window) if self.window else context
@@ -199,6 +241,9 @@ class LatentAttention(Mixer):
         dtype, device = self.runtime.dtype, x.device
         heads = self.num_heads
         q_plain, q_full, gate = self._queries_and_store(x, ctx, cache)
+        if self._runs_by_heads(ctx):
+            mixed = self._prompts(q_plain, q_full, gate, ctx, cache)
+            return ops.project(mixed.view(tokens, -1), self.out_weight, ctx.status)
         ops.per_head_project(q_plain, self.k_up_t, q_full[:, :, : self.kv_rank])
         table = ctx.block_tables[cache.group]
         if self.fast and ops.has_tcgen05_attention(self.row, cache.k.shape[2]):

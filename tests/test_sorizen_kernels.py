@@ -316,3 +316,63 @@ def test_latent_attention_reports_a_page_outside_the_pool(dev):
     tiles = torch.tensor([[0, 0, 60, 0]], dtype=torch.int32, device=dev)
     ops.latent_attention(q, k, table, seq, pos, tiles, None, 0, out, scale, None, st)
     assert int(st) == ops.STATUS_BAD_PAGE and torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("heads, dim, rot, value", [(3, 128, 64, 128), (2, 64, 64, 64), (1, 40, 24, 72), (5, 136, 8, 8), (2, 16, 0, 128)])
+@pytest.mark.parametrize("window", [None, 5, 100])
+@pytest.mark.parametrize("lengths", [(2,), (63, 64, 65), (130, 2, 257)])
+@pytest.mark.parametrize("options", [False, True])
+def test_prompts_head_by_head(dev, heads, dim, rot, value, window, lengths, options):
+    """Prompts with keys and values of their own per head against the plain statement in 32 bits: lengths around the
+    kernel's tiles of 64 and the tiles of 128 it is given, keys that fill no tile of 64 elements, views of wider rows."""
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(dim + sum(lengths))
+    tokens = sum(lengths)
+    draw = lambda *shape: torch.randn(shape, generator=gen).to(torch.bfloat16).to(dev)  # noqa: E731
+    wide, kv = draw(tokens, heads, dim + rot + 8), draw(tokens, heads * (dim + value) + 8)
+    q_plain, q_rot = wide[:, :, :dim], draw(tokens, heads, rot + 16)[:, :, 8:8 + rot]
+    k_plain = kv[:, :heads * dim].unflatten(1, (heads, dim))
+    v = kv[:, heads * dim:heads * (dim + value)].unflatten(1, (heads, value))
+    k_rot = draw(tokens, rot)
+    sink = torch.randn(heads, generator=gen).to(dev) if options else None
+    gate = torch.rand((tokens, heads), generator=gen).to(dev) if options else None
+    tiles, first = [], 0
+    for r, n in enumerate(lengths):
+        tiles += [(r, first + at, min(128, n - at), at) for at in range(0, n, 128)]
+        first += n
+    out = torch.full((tokens, heads, value), float("nan"), dtype=torch.bfloat16, device=dev)
+    scale = (dim + rot) ** -0.5
+    ops.head_prompt_attention(q_plain, q_rot, k_plain, k_rot, v, torch.tensor(tiles, dtype=torch.int32, device=dev), out, scale,
+                              window, sink=sink, gate=gate)
+    first = 0
+    for n in lengths:
+        part = slice(first, first + n)
+        scores = torch.einsum("ihd,jhd->hij", q_plain[part].float(), k_plain[part].float())
+        scores = (scores + torch.einsum("ihr,jr->hij", q_rot[part].float(), k_rot[part].float())) * scale
+        i, j = torch.arange(n, device=dev)[:, None], torch.arange(n, device=dev)[None, :]
+        seen = (j <= i) if window is None else (j <= i) & (j > i - window)
+        scores = scores.masked_fill(~seen, float("-inf"))
+        if sink is not None:
+            scores = torch.cat([scores, sink[:, None, None].expand(heads, n, 1)], dim=2)
+        weights = torch.softmax(scores, dim=2)[:, :, :n]
+        want = torch.einsum("hij,jhv->ihv", weights, v[part].float())
+        if gate is not None:
+            want = want * gate[part][:, :, None]
+        torch.testing.assert_close(out[part].float(), want, rtol=2e-2, atol=2e-2)
+        first += n
+
+
+def test_latent_rows(dev):
+    """Cached rows taken apart, a token without a slot among them."""
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(3)
+    cache = torch.randn((5, 1, 8, 96), generator=gen).to(torch.bfloat16).to(dev)
+    slots = torch.tensor([39, 0, -1, 17, 8], dtype=torch.int32, device=dev)
+    rows, rest = (torch.full((5, n), float("nan"), dtype=torch.bfloat16, device=dev) for n in (64, 24))
+    ops.latent_rows(cache, slots, rows, rest)
+    want = cache.view(40, 96)[slots.long().clamp(min=0)]
+    want[2] = 0
+    assert torch.equal(torch.cat([rows, rest], dim=1), want[:, :88])
+
