@@ -1,0 +1,353 @@
+// Score-mixing attention (the statement is at the top of attention_mixed.cu) of bfloat16 prompt portions with the mixing in
+// the queries.  The mixed score of head h,
+//   sum_g talk[h, g] (scale q_g . k_(kv of g) - slope_g distance),
+// is a score of its own: with q'_(h, c) = scale sum_(g reads key head c) talk[h, g] q_g and slope'_h = sum_g talk[h, g] slope_g
+// it is sum_c q'_(h, c) . k_c - slope'_h distance, one query [q'_(h, 0) | q'_(h, 1) ..] against the key heads' rows end to end.
+// So the heads meet in the queries, once a query, and not in every score (heads^2 FMAs a key, which with the exchange of all
+// heads' scores through shared memory bounded the kernel of attention_mixed_tiled.cu), and a head's softmax and values
+// are those of plain attention.  q' is 32-bit and enters the products as three bfloat16 parts (mma_sync.cuh), the weights
+// enter the second product as two, as they did; scores, sums and the output are 32-bit.
+//
+// A CTA has 64 queries of one head, a warp 16 of them; 64 keys a tile; the next tile's keys are brought while this one's
+// values are used and the other way round.  The parts of q' stay in shared memory: in registers (96 of them) they leave two
+// CTAs an SM and no room for sums that do not wait for one another.  Takes key heads of together up to 128 elements (a
+// multiple of 16 each) and value heads up to 64 or 128 (a multiple of 8).
+//
+// Measured (B200): 14 heads of 64 on 2 key heads, window 1,024, 2,048 tokens: 283 -> 128 us (with q' in registers 163); 32
+// heads of 32 on 4, 1,024 tokens: 685 -> 119 us.  Of the products (256 a tile and warp) a third of the time; the rest is
+// the softmax between them and what a tile's four barriers cost three CTAs an SM.
+#include <type_traits>
+
+#include "mma_sync.cuh"
+
+namespace einf {
+
+constexpr int kMixRows = 64, kMixKeys = 64, kMixThreads = 128;
+constexpr int kMixKeySize = 128;                       // key heads end to end, filled up
+
+struct MixArgs {
+  const __nv_bfloat16* q;            // [tokens, heads, dim]
+  const __nv_bfloat16* k_cache; const __nv_bfloat16* v_cache;
+  const int* block_table; int table_width;
+  const int4* tiles;                 // request, first token, tokens (up to 128), first position
+  __nv_bfloat16* out;                // [tokens, heads, vdim]
+  const float* slopes; const float* talk; const float* sink;
+  int* status;
+  int heads, kv_heads, dim, vdim, page_size, num_pages, window, wave;
+  float scale_log2, out_scale;
+};
+
+__device__ __forceinline__ uint32_t swizzled(int row, int piece, int pitch) {
+  return (uint32_t)(row * pitch + ((piece & ~7) | ((piece ^ row) & 7)) * 16);
+}
+
+// Three parts of q', a tile's keys, its values.
+template <int VALUE>
+constexpr int kMixSmem = 3 * kMixRows * kMixKeySize * 2 + kMixKeys * (kMixKeySize + VALUE) * 2;
+
+// VALUE: vdim filled up to 64 or 128.
+template <int VALUE>
+__global__ void __launch_bounds__(kMixThreads, VALUE <= 64 ? 3 : 2)
+mixed_prompt_attention_kernel(const __grid_constant__ MixArgs a) {
+  extern __shared__ __align__(128) unsigned char mix_smem[];
+  __shared__ int places[2][kMixKeys];                  // of a tile's keys: the page's first row of head 0 + slot in it, -1: none
+  constexpr int kKeyPitch = kMixKeySize * 2, kValuePitch = VALUE * 2;
+  constexpr int kQPart = kMixRows * kKeyPitch, kK = 3 * kQPart, kV = kK + kMixKeys * kKeyPitch, kSteps = kMixKeySize / 16;
+  pdl_launch_dependents();
+  // which rows: see attention_prompt.cu
+  const int total = (int)gridDim.x, wave = (int)blockIdx.x / a.wave, place = (int)blockIdx.x - wave * a.wave;
+  const int rank = wave & 1 ? total - 1 - ((wave >> 1) * a.wave + place) : ((wave + 1) >> 1) * a.wave + place;
+  const int row_tiles = total / a.heads, row_tile = row_tiles - 1 - rank / a.heads, h = rank % a.heads;
+  const int4 tile = a.tiles[row_tile >> 1];
+  const int sub = (row_tile & 1) * kMixRows;
+  const int rows = min(kMixRows, tile.z - sub);
+  if (rows <= 0) {
+    pdl_wait();
+    return;
+  }
+  const int t0 = tile.y + sub, pos0 = tile.w + sub;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, q2 = (lane & 3) * 2;
+  const int in8 = lane & 7, second = (lane >> 3) & 1, third = lane >> 4;
+  const uint32_t base = smem_address(mix_smem);
+  const int dim = a.dim, vdim = a.vdim, heads = a.heads, per = heads / a.kv_heads;
+  const int last_pos = pos0 + rows - 1;
+  const int lowest = a.window > 0 ? max(0, pos0 - a.window + 1) : 0;
+  const int first_tile = lowest / kMixKeys, end_tile = last_pos / kMixKeys + 1;
+  const int* table = a.block_table + (long long)tile.x * a.table_width;
+  bool bad_page = false;
+  auto find_places = [&](int t) {
+    if (threadIdx.x < kMixKeys) {
+      const int j = t * kMixKeys + threadIdx.x;
+      int row = -1;
+      if (j >= lowest && j <= last_pos) {
+        const int logical = j / a.page_size, page = table[logical];
+        if (page < 0 || page >= a.num_pages) bad_page = true;
+        else row = page * a.kv_heads * a.page_size + (j - logical * a.page_size);
+      }
+      places[t & 1][threadIdx.x] = row;
+    }
+  };
+  find_places(first_tile);
+
+  // ---- q', summed in registers in the layout of a product's first operand.  All heads' queries of these rows come through
+  // shared memory, as many heads at a time as it holds; rows of an odd number of 16-byte pieces.
+  const int q_pitch = dim * 2 + 16, at_once = kMixSmem<VALUE> / (kMixRows * q_pitch);
+  float mixed[kSteps][8];
+#pragma unroll
+  for (int kk = 0; kk < kSteps; ++kk)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) mixed[kk][e] = 0.f;
+  float slope = 0.f;
+  pdl_wait();
+  for (int g0 = 0; g0 < heads; g0 += at_once) {
+    const int count = min(at_once, heads - g0), pieces = dim / 8;
+    if (g0) __syncthreads();
+    for (int i = threadIdx.x; i < kMixRows * count * pieces; i += kMixThreads) {
+      const int r = i / (count * pieces), rest = i - r * (count * pieces), head = rest / pieces, piece = rest - head * pieces;
+      const bool there = r < rows;
+      cp_async16(base + (head * kMixRows + r) * q_pitch + piece * 16,
+                 a.q + ((long long)(t0 + (there ? r : 0)) * heads + g0 + head) * dim + piece * 8, there ? 16 : 0);
+    }
+    cp_async_commit_group();
+    cp_async_wait_groups<0>();
+    __syncthreads();
+    for (int u = 0; u < count; ++u) {
+      const int other = g0 + u, c = other / per;
+      const float w = a.talk ? a.talk[h * heads + other] : (other == h ? 1.f : 0.f);
+      if (a.slopes) slope = fmaf(w, a.slopes[other], slope);
+#pragma unroll
+      for (int kk = 0; kk < kSteps; ++kk) {
+        const int d = 16 * kk - c * dim;               // this head's 16 elements, if they are
+        if (d < 0 || d >= dim) continue;
+        uint32_t f[4];
+        ldsm_x4(f, base + (u * kMixRows + 16 * warp + in8 + 8 * second) * q_pitch + (d / 8 + third) * 16);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          mixed[kk][2 * e] = fmaf(w, low_bf16(f[e]), mixed[kk][2 * e]);
+          mixed[kk][2 * e + 1] = fmaf(w, high_bf16(f[e]), mixed[kk][2 * e + 1]);
+        }
+      }
+    }
+  }
+  slope *= 1.4426950408889634f;
+  __syncthreads();                                     // everyone has used the queries: their place takes the parts of q'
+#pragma unroll
+  for (int kk = 0; kk < kSteps; ++kk)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      uint32_t part[3];
+      split3(mixed[kk][2 * e] * a.scale_log2, mixed[kk][2 * e + 1] * a.scale_log2, part);
+      const uint32_t at = base + swizzled(16 * warp + g + 8 * (e & 1), 2 * kk + (e >> 1), kKeyPitch) + q2 * 2;
+#pragma unroll
+      for (int p = 0; p < 3; ++p) sts_u32(at + p * kQPart, part[p]);
+    }
+  __syncwarp();                                        // a warp's rows are its own
+
+  // 64 rows: a thread has one 16-byte piece of every 128-byte line of four rows
+  const int r0 = threadIdx.x >> 3, piece = threadIdx.x & 7;
+  auto bring = [&](uint32_t at, auto lines_tag, const __nv_bfloat16* cache, int size, int first_head, int width, int t) {
+    constexpr int kLines = decltype(lines_tag)::value, kPitch = 128 * kLines;
+    int row[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) row[u] = places[t & 1][r0 + 16 * u];
+#pragma unroll
+    for (int line = 0; line < kLines; ++line) {
+      const int e = 64 * line + 8 * piece, c = e / size;
+      const bool inside = e < width;
+      const __nv_bfloat16* from = cache + (long long)(first_head + c) * a.page_size * size + (e - c * size);
+      const uint32_t to = at + r0 * kPitch + 128 * line + ((piece ^ r0) & 7) * 16;       // rows 16 apart exchange alike
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool there = inside && row[u] >= 0;
+        cp_async16(to + u * 16 * kPitch, there ? from + (long long)row[u] * size : cache, there ? 16 : 0);
+      }
+    }
+    cp_async_commit_group();
+  };
+  auto bring_keys = [&](int t) {
+    bring(base + kK, std::integral_constant<int, kMixKeySize / 64>{}, a.k_cache, dim, 0, a.kv_heads * dim, t);
+  };
+  auto bring_values = [&](int t) {
+    bring(base + kV, std::integral_constant<int, VALUE / 64>{}, a.v_cache, vdim, h / per, vdim, t);
+  };
+  bring_keys(first_tile);
+  bring_values(first_tile);
+
+  float O[VALUE / 8][4], m[2], l[2];
+#pragma unroll
+  for (int j = 0; j < VALUE / 8; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) O[j][e] = 0.f;
+  // the sink is the first term of every row's sum (counted once, by the first of the row's four lanes)
+  m[0] = m[1] = a.sink ? a.sink[h] * 1.4426950408889634f : -INFINITY;
+  l[0] = l[1] = a.sink && q2 == 0 ? 1.f : 0.f;
+  const int warp_first = pos0 + 16 * warp, warp_last = warp_first + 15;
+
+  for (int t = first_tile; t < end_tile; ++t) {
+    const int j0 = t * kMixKeys;
+    // a warp none of whose rows sees a key of the tile sits the products out
+    const bool seen = j0 <= warp_last && (a.window <= 0 || j0 + kMixKeys - 1 > warp_first - a.window);
+    if (t + 1 < end_tile) find_places(t + 1);
+    cp_async_wait_groups<1>();                         // the keys are there
+    __syncthreads();
+    float S[8][4];
+    if (seen) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[j][e] = 0.f;
+#pragma unroll 2
+      for (int kk = 0; kk < kSteps; ++kk) {
+        // as mma_parts does it, the eight column tiles side by side: small parts first, the sum of 16 elements added
+        // to the running one by a rounded addition
+        uint32_t qf[3][4], kf[4][4];
+        float sum[8][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          ldsm_x4(kf[j], base + kK + swizzled(16 * j + in8 + 8 * third, 2 * kk + second, kKeyPitch));
+#pragma unroll
+        for (int p = 2; p >= 0; --p) {
+          ldsm_x4(qf[p], base + p * kQPart + swizzled(16 * warp + in8 + 8 * second, 2 * kk + third, kKeyPitch));
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if (p == 2) mma_bf16_16816_zero(sum[j], qf[p], kf[j >> 1][2 * (j & 1)], kf[j >> 1][2 * (j & 1) + 1]);
+            else mma_bf16_16816(sum[j], qf[p], kf[j >> 1][2 * (j & 1)], kf[j >> 1][2 * (j & 1) + 1]);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) S[j][e] += sum[j][e];
+      }
+    }
+    __syncthreads();                                   // the keys are used up
+    if (t + 1 < end_tile) bring_keys(t + 1);
+    else cp_async_commit_group();                      // an empty group: the values are always the second youngest
+    if (seen) {
+      const bool masks = j0 + kMixKeys - 1 > warp_first || (a.window > 0 && j0 <= warp_last - a.window);
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {           // rows g and g + 8 of the 16
+        const int pos = warp_first + g + 8 * half;
+        float top = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int key = j0 + 8 * j + q2 + e;
+            float z = S[j][2 * half + e] - slope * (float)(pos - key);
+            if (masks) z = (key <= pos && (a.window <= 0 || key > pos - a.window)) ? z : -INFINITY;
+            S[j][2 * half + e] = z;
+            top = fmaxf(top, z);
+          }
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+        const float to = fmaxf(m[half], top);
+        const float shift = to == -INFINITY ? 0.f : to;
+        const float factor = exp2f(m[half] - shift);   // nothing seen so far: zero
+        m[half] = to;
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float w = exp2f(S[j][2 * half + e] - shift);
+            S[j][2 * half + e] = w;
+            sum += w;
+          }
+        l[half] = l[half] * factor + sum;              // this lane's share; the row's lanes are added at the end
+        if (__any_sync(0xffffffffu, factor != 1.f)) {
+#pragma unroll
+          for (int j = 0; j < VALUE / 8; ++j) {
+            O[j][2 * half] *= factor;
+            O[j][2 * half + 1] *= factor;
+          }
+        }
+      }
+    }
+    cp_async_wait_groups<1>();                         // the values are there
+    __syncthreads();
+    if (seen) {
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {                 // the weights are the first operand as they lie in registers, two parts
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float x = S[2 * kk + (e >> 1)][2 * (e & 1)], y = S[2 * kk + (e >> 1)][2 * (e & 1) + 1];
+          hi[e] = pack_pair(x, y);
+          lo[e] = pack_pair(x - low_bf16(hi[e]), y - high_bf16(hi[e]));
+        }
+#pragma unroll
+        for (int j0v = 0; j0v < VALUE / 16; j0v += 4) {
+          uint32_t vf[4][4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            ldsm_x4_trans(vf[j], base + kV + swizzled(16 * kk + in8 + 8 * second, 2 * (j0v + j) + third, kValuePitch));
+#pragma unroll
+          for (int j = 0; j < 8; ++j) mma_bf16_16816(O[2 * j0v + j], lo, vf[j >> 1][2 * (j & 1)], vf[j >> 1][2 * (j & 1) + 1]);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) mma_bf16_16816(O[2 * j0v + j], hi, vf[j >> 1][2 * (j & 1)], vf[j >> 1][2 * (j & 1) + 1]);
+        }
+      }
+    }
+    __syncthreads();                                   // the values are used up
+    if (t + 1 < end_tile) bring_values(t + 1);
+    else cp_async_commit_group();
+  }
+  cp_async_wait_groups<0>();
+  if (bad_page) atomicOr(a.status, kStatusBadPage);
+
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const int r = 16 * warp + g + 8 * half;
+    float sum = l[half];
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    if (r >= rows) continue;
+    const float factor = sum > 0.f ? a.out_scale / sum : 0.f;
+    __nv_bfloat16* out = a.out + ((long long)(t0 + r) * heads + h) * vdim;
+#pragma unroll
+    for (int j = 0; j < VALUE / 8; ++j) {
+      const int column = 8 * j + q2;
+      if (column < vdim)
+        *reinterpret_cast<uint32_t*>(out + column) = pack_pair(O[j][2 * half] * factor, O[j][2 * half + 1] * factor);
+    }
+  }
+}
+
+template <int VALUE>
+static cudaError_t launch_mixed_prompt(const MixArgs& a, int num_tiles, cudaStream_t stream) {
+  auto kernel = mixed_prompt_attention_kernel<VALUE>;
+  constexpr int kBytes = kMixSmem<VALUE>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+  if (e != cudaSuccess) return e;
+  return launch_pdl(kernel, dim3(2 * num_tiles * a.heads), dim3(kMixThreads), kBytes, stream, a);
+}
+
+}  // namespace einf
+
+using namespace einf;
+
+// The portions of up to 128 tokens that `tiles` lists; `wave`: multiprocessors of the device.
+extern "C" int einf_mixed_prompt_attention(const void* q, const void* k_cache, const void* v_cache, const int* block_table,
+                                           int table_width, const int* tiles, int num_tiles, void* out, int heads, int kv_heads,
+                                           int dim, int vdim, int page_size, int num_pages, float scale, int window,
+                                           const float* slopes, const float* talk, const float* sink, float out_scale, int wave,
+                                           int* status, cudaStream_t stream) {
+  if (num_tiles == 0) return 0;
+  if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || dim <= 0 || dim % 16 || kv_heads * dim > kMixKeySize || vdim <= 0 ||
+      vdim % 8 || vdim > 128 || 2ll * num_tiles * heads > 0x7fffffff || wave <= 0 ||
+      (long long)num_pages * kv_heads * page_size > 0x7fffffff ||
+      (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)tiles) & 15) || ((uintptr_t)out & 3))
+    return (int)cudaErrorInvalidValue;
+  MixArgs a;
+  a.q = (const __nv_bfloat16*)q;
+  a.k_cache = (const __nv_bfloat16*)k_cache; a.v_cache = (const __nv_bfloat16*)v_cache;
+  a.block_table = block_table; a.table_width = table_width;
+  a.tiles = (const int4*)tiles; a.out = (__nv_bfloat16*)out;
+  a.slopes = slopes; a.talk = talk; a.sink = sink; a.status = status;
+  a.heads = heads; a.kv_heads = kv_heads; a.dim = dim; a.vdim = vdim; a.page_size = page_size; a.num_pages = num_pages;
+  a.window = window; a.wave = wave;
+  a.scale_log2 = scale * 1.4426950408889634f; a.out_scale = out_scale;
+  return (int)(vdim <= 64 ? launch_mixed_prompt<64>(a, num_tiles, stream) : launch_mixed_prompt<128>(a, num_tiles, stream));
+}

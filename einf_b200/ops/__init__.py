@@ -2326,6 +2326,34 @@ def mixed_tiled_splits(blocks: int, rows: int, window: Optional[int], max_contex
     return max(1, min(-(-keys // MIXED_KEYS_PER_SPLIT), (NUM_SMS * per_sm) // max(1, blocks), 64))
 
 
+#: elements of a token's key heads end to end that the prompts' score-mixing kernel takes
+MIXED_PROMPT_KEYS = 128
+#: CTAs (64 queries of a head each) from which it takes prompt portions whatever they see, and keys a query may see for it
+#: to take fewer.  It does not share a query's keys between CTAs as the other kernel does (14 heads of 64, us, the other /
+#: this one: 64, 256, 512 tokens at the start of a prompt 33 / 22, 37 / 33, 49 / 51; 128, 256 tokens behind 1,500 41 / 85,
+#: 53 / 85; 4 heads of 32, 2,048 tokens, 128 CTAs 72 / 81; 32 heads of 32, 1,024 tokens 685 / 119).
+MIXED_PROMPT_CTAS, MIXED_PROMPT_FEW_KEYS = 148, 256
+
+
+def mixed_prompt_pays(num_tiles: int, heads: int, window: Optional[int], max_context: int) -> bool:
+    """Whether so many prompt tiles are worth the kernel with the mixing in the queries (host-side figures only)."""
+    keys = min(max_context or (1 << 30), window or (1 << 30))
+    return 2 * num_tiles * heads >= MIXED_PROMPT_CTAS or keys <= MIXED_PROMPT_FEW_KEYS
+
+
+def mixed_prompt_takes(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, out: torch.Tensor, num_tiles: int,
+                       window: Optional[int], max_context: int) -> bool:
+    """Whether prompt portions run with the mixing in the queries: bfloat16, a token's key heads of together up to 128
+    elements, in multiples of 16 each, value heads of up to 128, in multiples of eight."""
+    heads, dim, kv_heads, value_size = q.shape[1], q.shape[2], k_cache.shape[1], v_cache.shape[3]
+    return (
+        q.dtype == torch.bfloat16 and dim % 16 == 0 and kv_heads * dim <= MIXED_PROMPT_KEYS
+        and value_size % 8 == 0 and value_size <= 128 and mixed_prompt_pays(num_tiles, heads, window, max_context)
+        and all(t.data_ptr() % 16 == 0 for t in (q, k_cache, v_cache, out))
+        and k_cache.shape[0] * kv_heads * k_cache.shape[2] <= 0x7fffffff
+    )
+
+
 def _mixed_tiled(q, k_cache, v_cache, block_table, seq_of_token, positions, out, scale, window, slopes, talk, sink,
                  out_scale, status, q_tiles, single_tokens, num_singles, max_context) -> bool:
     tokens, heads, key_size = q.shape
@@ -2337,10 +2365,27 @@ def _mixed_tiled(q, k_cache, v_cache, block_table, seq_of_token, positions, out,
     launches = []
     if num_singles:
         launches.append((single_tokens, num_singles, 1, mixed_tiled_rows(heads, kv_heads, key_size, value_size, True, q.dtype)))
-    if num_tiles:
+    by_heads = num_tiles and mixed_prompt_takes(q, k_cache, v_cache, out, num_tiles, window, max_context)
+    if num_tiles and not by_heads:
         launches.append((q_tiles, num_tiles, 0, mixed_tiled_rows(heads, kv_heads, key_size, value_size, False, q.dtype)))
-    if not launches or any(rows == 0 for _, _, _, rows in launches):
+    if not (launches or by_heads) or any(rows == 0 for _, _, _, rows in launches):
         return False
+    if by_heads:
+        fn = _fn(
+            "einf_mixed_prompt_attention",
+            [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+             c_float, c_int, c_void_p, c_void_p, c_void_p, c_float, c_int, c_void_p, c_void_p],
+        )
+        _check(
+            fn(_dev(q, "q"), _dev(k_cache, "k_cache"), _dev(v_cache, "v_cache"),
+               _opt(block_table, "block_table", torch.int32), block_table.shape[1], _opt(q_tiles, "q_tiles", torch.int32),
+               num_tiles, _dev(out, "out"), heads, kv_heads, key_size, value_size, page_size, num_pages, float(scale),
+               int(window or 0), _opt(slopes, "slopes", torch.float32), _opt(talk, "talk", torch.float32),
+               _opt(sink, "sink", torch.float32), float(out_scale), _sm_count(), _dev(status, "status"), _stream()),
+            "mixed_prompt_attention",
+        )
+        if not launches:
+            return True
     variant = mixed_tiled_variant(heads)
     fn = _fn(
         "einf_paged_attention_mixed_tiled",

@@ -122,6 +122,8 @@ class PagedAttention(Mixer):
             tiled = ()
             if int(spec["num_heads"]) <= ops.MIXED_MAX_HEADS:
                 tiled = ("attention_mixed_tiled:" + ops.mixed_tiled_variant(int(spec["num_heads"])),)
+            if runtime.dtype == torch.bfloat16:
+                tiled += ("attention_mixed_mma",)
             return ("pointwise", "attention_mixed", "gemm_simt") + tiled + cls._product_libraries(runtime)
         if cls._is_general(spec):
             fast = (f"attention_tcgen05:HEAD_SIZE={int(spec['head_size'])}",) \
@@ -335,8 +337,12 @@ class PagedAttention(Mixer):
         of the longest context: kernel, cluster size and clusters per token."""
         singles = int(ctx.single_tokens.shape[0])
         if self.mixes_scores:
-            # the tiled kernel splits the keys of single tokens by their number and the longest context
-            return ("mixed", ops.mixed_tiled_splits(singles, 1, self.window, ctx.max_context_len)) if singles else ()
+            # the tiled kernel splits the keys of single tokens by their number and the longest context, and which
+            # kernel takes the prompt portions goes by what they see
+            splits = ops.mixed_tiled_splits(singles, 1, self.window, ctx.max_context_len) if singles else 0
+            tiles = int(ctx.q_tiles.shape[0])
+            return ("mixed", splits, bool(tiles) and ops.mixed_prompt_pays(tiles, self.num_heads, self.window,
+                                                                           ctx.max_context_len))
         if not (self.fast or (self.general_fast and ops.has_tcgen05_attention(self.head_size, page_size))) or not singles:
             return ()
         context = ctx.max_context_len

@@ -75,6 +75,64 @@ def test_tiled_score_mixing_attention(dev, dtype, heads, kv_heads, size, vsize, 
         torch.testing.assert_close(out.cpu(), want_cpu, **close)
 
 
+@pytest.mark.parametrize("heads, kv_heads, size, vsize, window", [
+    (14, 2, 64, 64, 100), (6, 3, 32, 128, None), (5, 1, 16, 8, 64), (8, 8, 16, 72, 1), (32, 1, 112, 64, 63),
+])
+@pytest.mark.parametrize("parts", ["all", "no slopes", "no mixing"])
+def test_mixing_in_the_queries(dev, heads, kv_heads, size, vsize, window, parts):
+    """The kernel with the mixing in the queries and the kernel that mixes scores, on the same portions (rows around the tiles
+    of 64, portions behind cached tokens): each off the statement in 64 bits by little more than the output's rounding."""
+    from einf_b200 import ops
+
+    requests = [(0, 2), (0, 63), (0, 64), (5, 65), (300, 129), (61, 19)]
+    (q, k, v, table, seq, pos), scale, window = _attention_case(dev, torch.bfloat16, heads, kv_heads, size, 16, requests, window)
+    generator = torch.Generator().manual_seed(11)
+    v = torch.randn((*v.shape[:3], vsize), generator=generator).to(torch.bfloat16).to(dev)
+    slopes, talk, sink = _mixing(heads, generator, dev)
+    slopes, talk = None if parts == "no slopes" else slopes, None if parts == "no mixing" else talk
+    q_tiles, singles = _step_split(requests)
+    contexts = [start + n for start, n in requests]
+    assert ops.mixed_prompt_takes(q, k, v, q, q_tiles.shape[0], 1, 1)
+    outs = []
+    for tiles_pay in (True, False):
+        out = torch.full((q.shape[0], heads, vsize), float("nan"), dtype=torch.bfloat16, device=dev)
+        st = status(dev)
+        before = ops.MIXED_PROMPT_CTAS, ops.MIXED_PROMPT_FEW_KEYS
+        try:
+            ops.MIXED_PROMPT_CTAS, ops.MIXED_PROMPT_FEW_KEYS = (0, 0) if tiles_pay else (1 << 30, 0)
+            ops.paged_attention_mixed(q, k, v, table, seq, pos, out, scale, window, slopes, talk, sink, 0.7, st,
+                                      q_tiles=q_tiles.to(dev), single_tokens=singles.to(dev), num_singles=0,
+                                      max_context=max(contexts))
+        finally:
+            ops.MIXED_PROMPT_CTAS, ops.MIXED_PROMPT_FEW_KEYS = before
+        assert int(st) == 0
+        outs.append(out)
+    # 64 bits, request by request
+    group = torch.arange(heads, device=dev) // (heads // kv_heads)
+    first = 0
+    for r, (start, n) in enumerate(requests):
+        end, rows = start + n, slice(first, first + n)
+        pages = table[r, :-(-end // 16)].long()
+        if window is not None:
+            pages = pages.clamp(min=0)
+        keys = k[pages].transpose(1, 2).reshape(-1, kv_heads, size)[:end].double()[:, group]
+        values = v[pages].transpose(1, 2).reshape(-1, kv_heads, vsize)[:end].double()[:, group]
+        i = torch.arange(start, end, device=dev)[:, None]
+        j = torch.arange(end, device=dev)[None, :]
+        raw = torch.einsum("ihd,jhd->hij", q[rows].double(), keys) * scale
+        if slopes is not None:
+            raw = raw - slopes.double()[:, None, None] * (i - j)
+        if talk is not None:
+            raw = torch.einsum("hg,gij->hij", talk.double(), raw)
+        seen = (j <= i) if window is None else (j <= i) & (i - j < window)
+        raw = torch.cat([raw.masked_fill(~seen, float("-inf")), sink.double()[:, None, None].expand(heads, n, 1)], dim=2)
+        want = 0.7 * torch.einsum("hij,jhv->ihv", torch.softmax(raw, dim=2)[:, :, :-1], values)
+        # bfloat16 rounding of the output: 2^-9 of an element; weights of two bfloat16 parts and 32-bit sums: far below
+        for out in outs:
+            assert bool(((out[rows].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-4).all())
+        first += n
+
+
 @pytest.mark.parametrize("batch, context, window", [(1, 3000, None), (3, 1500, 1024), (64, 300, 128), (2, 40, 64)])
 def test_tiled_score_mixing_decode_splits_its_keys(dev, batch, context, window):
     """Single tokens with long contexts: the keys of a token are split over CTAs and joined with the sink."""
