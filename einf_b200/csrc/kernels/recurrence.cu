@@ -8,7 +8,7 @@
 // order of additions: what a position computes does not depend on how the prompt was cut.
 #include <type_traits>
 
-#include "common.cuh"
+#include "conv_run.cuh"
 
 namespace einf {
 
@@ -65,6 +65,41 @@ __global__ void conv_silu_kernel(const T* __restrict__ in, long long in_stride, 
     }
     out[(long long)t * channels + c] = from_float<T>(act ? silu_f(acc) : acc);
   }
+}
+
+// The same for steps of many tokens, up to four taps and channels in groups of four (conv_run.cuh); the step sizes' columns
+// are the work of the threads behind the channels'.
+template <typename T>
+__global__ void __launch_bounds__(128)
+conv_silu_run_kernel(const T* __restrict__ in, long long in_stride, const float* __restrict__ weight,
+                     const float* __restrict__ bias, const float* __restrict__ conv_state, long long state_stride,
+                     const int* __restrict__ seq_of_token, const int* __restrict__ q_start,
+                     const int* __restrict__ state_slots, int num_slots, T* __restrict__ out, int channels, int taps,
+                     int num_tokens, const T* __restrict__ dt_in, const float* __restrict__ dt_bias,
+                     const float* __restrict__ a_log, float* __restrict__ dt_out, float* __restrict__ decay_out, int heads,
+                     int act, const float* __restrict__ input_bias) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int pieces = channels / 4, runs = (num_tokens + kRunTokens - 1) / kRunTokens;
+  const int index = blockIdx.x * blockDim.x + threadIdx.x;          // below 2^31 by the launch
+  if (index < pieces * runs) {
+    const int run = index / pieces, c = 4 * (index - run * pieces);
+    float4 start = make_float4(0.f, 0.f, 0.f, 0.f), before = start;
+    if (bias) start = make_float4(bias[c], bias[c + 1], bias[c + 2], bias[c + 3]);
+    if (input_bias) before = make_float4(input_bias[c], input_bias[c + 1], input_bias[c + 2], input_bias[c + 3]);
+    conv_run<T, false>(in, in_stride, c, run * kRunTokens, num_tokens, taps, weight, before, start, conv_state, state_stride,
+                       channels, seq_of_token, q_start, state_slots, num_slots, [&](int t, float4 v) {
+                         if (act) v = make_float4(silu_f(v.x), silu_f(v.y), silu_f(v.z), silu_f(v.w));
+                         store_quad(out + (long long)t * channels + c, v);
+                       });
+    return;
+  }
+  const int rest = index - pieces * runs;
+  if (rest >= num_tokens * heads) return;
+  const int t = rest / heads, h = rest - t * heads;
+  const float dt = softplus_f(to_float(dt_in[(long long)t * in_stride + h]) + dt_bias[h]);
+  dt_out[(long long)t * heads + h] = dt;
+  decay_out[(long long)t * heads + h] = expf(-expf(a_log[h]) * dt);
 }
 
 // After the convolution: the request's last taps-1 inputs become its convolution state (a portion
@@ -534,6 +569,50 @@ __global__ void gated_norm_kernel(const float* __restrict__ y, const T* __restri
   }
 }
 
+// The same for steps of many tokens: a warp per (token, part), the part's elements in registers from their one load (four at a
+// time) to the output; parts of up to 128 N elements, a multiple of four.
+template <typename T, int N>
+__global__ void __launch_bounds__(128)
+gated_norm_warp_kernel(const float* __restrict__ y, const T* __restrict__ gate, long long gate_stride,
+                       const float* __restrict__ weight, T* __restrict__ out, int width, int parts, float eps,
+                       int gate_first, int gate_kind, int rows) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, row = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int t = row / parts, part = row - t * parts, size = width / parts, base = part * size;
+  const float* from = y + (long long)t * width + base;
+  const T* g_row = gate + (long long)t * gate_stride + base;
+  float4 u[N], g[N];
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int i = 128 * n + 4 * lane;
+    u[n] = g[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < size) {
+      u[n] = *reinterpret_cast<const float4*>(from + i);
+      g[n] = load_quad(g_row + i);
+    }
+  }
+  auto open = [&](float z) { return gate_kind == 0 ? silu_f(z) : 1.f / (1.f + expf(-z)); };
+  float ss = 0.f;
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    g[n] = make_float4(open(g[n].x), open(g[n].y), open(g[n].z), open(g[n].w));
+    if (gate_first) u[n] = make_float4(u[n].x * g[n].x, u[n].y * g[n].y, u[n].z * g[n].z, u[n].w * g[n].w);
+    ss += u[n].x * u[n].x + u[n].y * u[n].y + (u[n].z * u[n].z + u[n].w * u[n].w);
+  }
+  const float factor = rsqrtf(warp_sum(ss) / (float)size + eps);
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int i = 128 * n + 4 * lane;
+    if (i >= size) continue;
+    const float4 w = *reinterpret_cast<const float4*>(weight + base + i);
+    float4 v = make_float4(u[n].x * factor * w.x, u[n].y * factor * w.y, u[n].z * factor * w.z, u[n].w * factor * w.w);
+    if (!gate_first) v = make_float4(v.x * g[n].x, v.y * g[n].y, v.z * g[n].z, v.w * g[n].w);
+    store_quad(out + (long long)t * width + base + i, v);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // The gates of a matrix memory with exponential gating.  Per request and head, token after token:
 //   i = cap tanh((z_i + b_i) / cap),  f = logsigmoid(cap tanh((z_f + b_f) / cap)),
@@ -732,6 +811,51 @@ __global__ void memory_output_kernel(const float* __restrict__ y, const float* _
   }
 }
 
+// The same where y comes as one part: four elements a load, the head's row in registers between the norm and the output;
+// heads of up to 128 N elements.  2,548 tokens of 4 heads of 256: 17 -> 9 us.
+template <typename T, int N>
+__global__ void __launch_bounds__(128)
+memory_output_quads_kernel(const float* __restrict__ y, const float* __restrict__ floor, const T* __restrict__ gate,
+                           long long gate_stride, const float* __restrict__ weight, T* __restrict__ out, long long pairs,
+                           int heads, int vdim, int columns, float query_scale, float eps, float denominator_eps) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const long long pair = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (pair >= pairs) return;
+  const int t = (int)(pair / heads), h = (int)(pair - (long long)t * heads);
+  const float* row = y + pair * columns;
+  const T* g_row = gate + t * gate_stride + (long long)h * vdim;
+  float4 u[N], g[N];
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int d = 128 * n + 4 * lane;
+    u[n] = g[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (d < vdim) {
+      u[n] = *reinterpret_cast<const float4*>(row + d);
+      g[n] = load_quad(g_row + d);
+    }
+  }
+  const float factor = query_scale / (fmaxf(fabsf(query_scale * row[vdim]), floor[pair]) + denominator_eps);
+  float ss = 0.f;
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    u[n] = make_float4(u[n].x * factor, u[n].y * factor, u[n].z * factor, u[n].w * factor);
+    ss += u[n].x * u[n].x + u[n].y * u[n].y + (u[n].z * u[n].z + u[n].w * u[n].w);
+  }
+  const float unit = rsqrtf(warp_sum(ss) / (float)vdim + eps);
+  auto open = [](float z) { return 1.f / (1.f + expf(-z)); };
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int d = 128 * n + 4 * lane;
+    if (d >= vdim) continue;
+    const float4 w = *reinterpret_cast<const float4*>(weight + h * vdim + d);
+    store_quad(out + pair * vdim + d,
+               make_float4(u[n].x * unit * w.x * open(g[n].x), u[n].y * unit * w.y * open(g[n].y),
+                           u[n].z * unit * w.z * open(g[n].z), u[n].w * unit * w.w * open(g[n].w)));
+  }
+}
+
 // ---------------------------------------------------------------------------
 // A gated linear recurrence with one state value per channel (a real-gated linear recurrent
 // unit).  Per request and channel c of block b = c / part, token after token:
@@ -867,6 +991,24 @@ extern "C" int einf_conv_silu(const void* in, int dtype, long long in_stride, co
   const long long total = (long long)num_tokens * (channels + heads);
   long long blocks = (total + threads - 1) / threads;
   if (blocks > 148 * 32) blocks = 148 * 32;
+  // Portions of 64 tokens and more on average, rows that four elements divide: 2,048 tokens of 3,328 channels 34 -> 17 us.
+  // 64 single tokens of 896 channels took 17 us this way, every thread one chain of state rows, against 7.
+  const size_t quad = dtype == kFloat32 ? 16 : 8;
+  const long long run_threads = (long long)((num_tokens + kRunTokens - 1) / kRunTokens) * (channels / 4) +
+                                (long long)num_tokens * heads;
+  if (num_tokens >= 64ll * num_requests && taps <= kRunTaps && channels % 4 == 0 && in_stride % 4 == 0 && run_threads < (1ll << 31) &&
+      (uintptr_t)in % quad == 0 && (uintptr_t)out % quad == 0) {
+    EINF_DISPATCH_2(dtype, T, {
+      cudaError_t e = launch_pdl(conv_silu_run_kernel<T>, (int)((run_threads + 127) / 128), 128, 0, stream, (const T*)in,
+                                 in_stride, weight, bias, (const float*)conv_state, state_stride, seq_of_token, q_start,
+                                 state_slots, num_slots, (T*)out, channels, taps, num_tokens, (const T*)dt_in, dt_bias, a_log,
+                                 dt_out, decay_out, heads, act, input_bias);
+      if (e != cudaSuccess || taps == 1) return (int)e;
+      const dim3 grid((channels + 127) / 128, num_requests);
+      return (int)launch_pdl(conv_state_update_kernel<T>, grid, 128, 0, stream, (const T*)in, in_stride, conv_state,
+                             state_stride, q_start, state_slots, num_slots, channels, taps, input_bias);
+    })
+  }
   EINF_DISPATCH_2(dtype, T, {
     cudaError_t e = launch_pdl(conv_silu_kernel<T>, (int)blocks, threads, 0, stream, (const T*)in, in_stride, weight,
                                bias, (const float*)conv_state, state_stride, seq_of_token, q_start, state_slots,
@@ -980,6 +1122,20 @@ extern "C" int einf_gated_norm(const float* y, const void* gate, int dtype, long
   while (threads < size && threads < 256) threads <<= 1;
   const long long blocks = (long long)num_tokens * parts;
   if (blocks >= (1ll << 31)) return (int)cudaErrorInvalidValue;
+  // Rows for all warps of the GPU to have one and more (fewer want a CTA's threads for a row), whole aligned groups of four:
+  // 5,096 rows of 896 24 -> 15 us.  Rows above 1,024 keep their CTA: 2,048 of 3,072 took 26 us by warps, against 16.
+  const size_t quad = dtype == kFloat32 ? 16 : 8;
+  if (blocks >= 148 * 4 && size % 4 == 0 && size <= 1024 && gate_stride % 4 == 0 && (uintptr_t)gate % quad == 0 &&
+      (uintptr_t)out % quad == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)weight % 16 == 0) {
+    EINF_DISPATCH_2(dtype, T, {
+      auto launch = [&](auto kernel) {
+        return (int)launch_pdl(kernel, (int)((blocks + 3) / 4), 128, 0, stream, y, (const T*)gate, gate_stride, weight,
+                               (T*)out, width, parts, eps, gate_first, gate_kind, (int)blocks);
+      };
+      if (size <= 256) return launch(gated_norm_warp_kernel<T, 2>);
+      return launch(gated_norm_warp_kernel<T, 8>);
+    })
+  }
   EINF_DISPATCH_2(dtype, T, {
     return (int)launch_pdl(gated_norm_kernel<T>, (int)blocks, threads, 0, stream, y, (const T*)gate, gate_stride, weight,
                            (T*)out, width, parts, eps, gate_first, gate_kind);
@@ -1041,6 +1197,18 @@ extern "C" int einf_memory_output(const float* y, const float* floor, const void
   const int threads = 128;
   const long long blocks = (pairs * 32 + threads - 1) / threads;
   if (blocks >= (1ll << 31)) return (int)cudaErrorInvalidValue;
+  const size_t quad = dtype == kFloat32 ? 16 : 8;
+  if (y_splits == 1 && vdim % 4 == 0 && columns % 4 == 0 && vdim <= 1024 && gate_stride % 4 == 0 && (uintptr_t)gate % quad == 0 &&
+      (uintptr_t)out % quad == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)weight % 16 == 0) {
+    EINF_DISPATCH_2(dtype, T, {
+      auto launch = [&](auto kernel) {
+        return (int)launch_pdl(kernel, (int)blocks, threads, 0, stream, y, floor, (const T*)gate, gate_stride, weight, (T*)out,
+                               pairs, heads, vdim, columns, query_scale, eps, denominator_eps);
+      };
+      if (vdim <= 256) return launch(memory_output_quads_kernel<T, 2>);
+      return launch(memory_output_quads_kernel<T, 8>);
+    })
+  }
   EINF_DISPATCH_2(dtype, T, {
     if (y_splits == 1)
       return (int)launch_pdl(memory_output_kernel<T, false>, (int)blocks, threads, 0, stream, y, floor, (const T*)gate,

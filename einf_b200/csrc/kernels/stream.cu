@@ -10,7 +10,7 @@
 // row is computed by one CTA from the row's own request alone.
 #include <cstdint>
 
-#include "common.cuh"
+#include "conv_run.cuh"
 
 namespace einf {
 
@@ -49,6 +49,42 @@ __device__ __forceinline__ float pending_sum(const Pending& p, size_t idx) {
   float v = 0.f;
   if (p.a) v = pending_term(p.a, p.a_dtype, p.a_splits, p.a_stride, idx);
   if (p.b) v += pending_term(p.b, p.b_dtype, p.b_splits, p.b_stride, idx);
+  return v;
+}
+
+// kBatch: partial sums of which all loads are in flight at once (they sit in L2); 1: there are none
+template <int kBatch>
+__device__ __forceinline__ float4 pending4(const void* p, int dtype, int splits, long long stride, size_t idx) {
+  if (dtype == kBFloat16) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < (kBatch == 1 ? 1 : splits); ++s) {
+      const uint2 raw = *(const uint2*)((const __nv_bfloat16*)p + (size_t)s * stride + idx);
+      const float2 a = __bfloat1622float2(*(const __nv_bfloat162*)&raw.x), b = __bfloat1622float2(*(const __nv_bfloat162*)&raw.y);
+      v.x += a.x; v.y += a.y; v.z += b.x; v.w += b.y;
+    }
+    return v;
+  }
+  const float* q = (const float*)p + idx;
+  if (kBatch == 1 || splits == 1) return *(const float4*)q;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s0 = 0; s0 < splits; s0 += kBatch) {
+    float4 part[kBatch];
+#pragma unroll
+    for (int e = 0; e < kBatch; ++e) part[e] = *(const float4*)(q + (size_t)min(s0 + e, splits - 1) * stride);
+#pragma unroll
+    for (int e = 0; e < kBatch; ++e)
+      if (s0 + e < splits) { v.x += part[e].x; v.y += part[e].y; v.z += part[e].z; v.w += part[e].w; }
+  }
+  return v;
+}
+
+template <int kBatch>
+__device__ __forceinline__ float4 pending4_sum(const Pending& p, size_t idx) {
+  float4 v = pending4<kBatch>(p.a, p.a_dtype, p.a_splits, p.a_stride, idx);
+  if (p.b) {
+    const float4 more = pending4<kBatch>(p.b, p.b_dtype, p.b_splits, p.b_stride, idx);
+    v.x += more.x; v.y += more.y; v.z += more.z; v.w += more.w;
+  }
   return v;
 }
 
@@ -128,6 +164,75 @@ __global__ void norm_row_kernel(const __grid_constant__ Pending pending, float s
   }
 }
 
+// Mode 1 for up to four taps and widths in groups of four: a thread has kVec groups of four columns and brings the row, the
+// state's rows and the taps before the sum of squares, so their latencies run side by side instead of one behind the
+// other: 64 tokens of 896 columns 9.3 -> 4 us.
+template <typename TOut, int kVec>
+__global__ void __launch_bounds__(512)
+norm_single_quads_kernel(const __grid_constant__ Pending pending, float scale, float* __restrict__ residual,
+                         const float* __restrict__ weight, float eps, const float* __restrict__ conv_weight, int taps,
+                         float* __restrict__ conv_state, long long state_stride, int num_slots,
+                         const int* __restrict__ seq_of_token, const int* __restrict__ state_slots, TOut* __restrict__ out,
+                         int hidden) {
+  __shared__ float red[33];
+  pdl_launch_dependents();
+  const int t = blockIdx.x;
+  const size_t base = (size_t)t * hidden;
+  const int keep = taps - 1;                            // 1 to 3
+  auto column = [&](int j) { return (j * (int)blockDim.x + (int)threadIdx.x) * 4; };
+  pdl_wait();
+  const int slot = state_slots[seq_of_token[t]];
+  float* state = (slot >= 0 && slot < num_slots) ? conv_state + (long long)slot * state_stride : nullptr;
+  float4 x[kVec], line[kVec][3];
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < kVec; ++j) {
+    const int c = column(j);
+    x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c >= hidden) continue;
+    x[j] = *(const float4*)(residual + base + c);
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+      line[j][u] = u < keep && state ? *(const float4*)(state + (size_t)u * hidden + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (pending.a) {
+      const float4 y = pending4_sum<8>(pending, base + c);
+      x[j].x = fmaf(scale, y.x, x[j].x); x[j].y = fmaf(scale, y.y, x[j].y);
+      x[j].z = fmaf(scale, y.z, x[j].z); x[j].w = fmaf(scale, y.w, x[j].w);
+      *(float4*)(residual + base + c) = x[j];
+    }
+    ss += x[j].x * x[j].x + x[j].y * x[j].y + x[j].z * x[j].z + x[j].w * x[j].w;
+  }
+  const float inv = rsqrtf(block_sum(ss, red) / (float)hidden + eps);
+#pragma unroll
+  for (int j = 0; j < kVec; ++j) {
+    const int c = column(j);
+    if (c >= hidden) continue;
+    const float4 w = *(const float4*)(weight + c);
+    const float4 h = make_float4(x[j].x * inv * w.x, x[j].y * inv * w.y, x[j].z * inv * w.z, x[j].w * inv * w.w);
+    const float* tap = conv_weight + (size_t)c * taps;
+    float4 acc = h;
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      if (u >= keep) continue;
+      acc.x = fmaf(tap[u], line[j][u].x, acc.x);
+      acc.y = fmaf(tap[taps + u], line[j][u].y, acc.y);
+      acc.z = fmaf(tap[2 * taps + u], line[j][u].z, acc.z);
+      acc.w = fmaf(tap[3 * taps + u], line[j][u].w, acc.w);
+    }
+    acc.x = fmaf(tap[keep], h.x, acc.x);
+    acc.y = fmaf(tap[taps + keep], h.y, acc.y);
+    acc.z = fmaf(tap[2 * taps + keep], h.z, acc.z);
+    acc.w = fmaf(tap[3 * taps + keep], h.w, acc.w);
+    store_quad(out + base + c, acc);
+    if (state) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (u + 1 < keep) *(float4*)(state + (size_t)u * hidden + c) = line[j][u + 1];
+      *(float4*)(state + (size_t)(keep - 1) * hidden + c) = h;
+    }
+  }
+}
+
 // out[t, c] = h[t, c] + sum_j w[c, j] * h[t - (taps - 1) + j, c] over the tokens of t's request, with
 // the request's state rows (its last taps - 1 inputs, oldest first) in front of its first token.
 template <typename TOut>
@@ -157,6 +262,25 @@ __global__ void conv_rows_kernel(const float* __restrict__ h, const float* __res
     }
     out[idx] = from_float<TOut>(acc);
   }
+}
+
+// The same over runs of tokens, four channels a thread (conv_run.cuh).
+template <typename TOut>
+__global__ void __launch_bounds__(128)
+conv_rows_run_kernel(const float* __restrict__ h, const float* __restrict__ conv_weight, int taps,
+                     const float* __restrict__ conv_state, long long state_stride, int num_slots,
+                     const int* __restrict__ seq_of_token, const int* __restrict__ q_start,
+                     const int* __restrict__ state_slots, TOut* __restrict__ out, int hidden, int num_tokens) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int pieces = hidden / 4, runs = (num_tokens + kRunTokens - 1) / kRunTokens;
+  const int index = blockIdx.x * blockDim.x + threadIdx.x;          // below 2^31 by the launch
+  if (index >= pieces * runs) return;
+  const int run = index / pieces, c = 4 * (index - run * pieces);
+  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+  conv_run<float, true>(h, hidden, c, run * kRunTokens, num_tokens, taps, conv_weight, none, none, conv_state, state_stride,
+                        hidden, seq_of_token, q_start, state_slots, num_slots,
+                        [&](int t, float4 v) { store_quad(out + (size_t)t * hidden + c, v); });
 }
 
 // Afterwards the request's last taps - 1 inputs become its state (a portion shorter than that keeps
@@ -197,41 +321,6 @@ __global__ void conv_rows_state_kernel(const float* __restrict__ h, float* __res
 // first, without a branch between them (an index past the row is clamped, its value unused), so that
 // a whole row is in flight at once.
 // ---------------------------------------------------------------------------
-// kBatch: partial sums of which all loads are in flight at once (they sit in L2); 1: there are none
-template <int kBatch>
-__device__ __forceinline__ float4 pending4(const void* p, int dtype, int splits, long long stride, size_t idx) {
-  if (dtype == kBFloat16) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s < (kBatch == 1 ? 1 : splits); ++s) {
-      const uint2 raw = *(const uint2*)((const __nv_bfloat16*)p + (size_t)s * stride + idx);
-      const float2 a = __bfloat1622float2(*(const __nv_bfloat162*)&raw.x), b = __bfloat1622float2(*(const __nv_bfloat162*)&raw.y);
-      v.x += a.x; v.y += a.y; v.z += b.x; v.w += b.y;
-    }
-    return v;
-  }
-  const float* q = (const float*)p + idx;
-  if (kBatch == 1 || splits == 1) return *(const float4*)q;
-  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int s0 = 0; s0 < splits; s0 += kBatch) {
-    float4 part[kBatch];
-#pragma unroll
-    for (int e = 0; e < kBatch; ++e) part[e] = *(const float4*)(q + (size_t)min(s0 + e, splits - 1) * stride);
-#pragma unroll
-    for (int e = 0; e < kBatch; ++e)
-      if (s0 + e < splits) { v.x += part[e].x; v.y += part[e].y; v.z += part[e].z; v.w += part[e].w; }
-  }
-  return v;
-}
-
-__device__ __forceinline__ void store_row4(float* p, const float4& v) { *(float4*)p = v; }
-__device__ __forceinline__ void store_row4(__nv_bfloat16* p, const float4& v) {
-  const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
-  uint2 raw;
-  raw.x = *(const uint32_t*)&a;
-  raw.y = *(const uint32_t*)&b;
-  *(uint2*)p = raw;
-}
-
 template <typename TOut, int kTeam, int kVec>
 __global__ void stream_norm_kernel(const __grid_constant__ Pending pending, float scale, const float* __restrict__ post,
                                    float post_eps, float* __restrict__ residual, const float* __restrict__ weight,
@@ -254,7 +343,7 @@ __global__ void stream_norm_kernel(const __grid_constant__ Pending pending, floa
     float4 y[kVec];
 #pragma unroll
     for (int j = 0; j < kVec; ++j)
-      y[j] = pending4<kBatch>(pending.a, pending.a_dtype, pending.a_splits, pending.a_stride, base + min(column(j), hidden - 4));
+      y[j] = pending4_sum<kBatch>(pending, base + min(column(j), hidden - 4));
     if (post) {
       float ss = 0.f;
 #pragma unroll
@@ -291,11 +380,11 @@ __global__ void stream_norm_kernel(const __grid_constant__ Pending pending, floa
       const float4 w = *(const float4*)(weight + column(j));
       v.x *= inv * w.x; v.y *= inv * w.y; v.z *= inv * w.z; v.w *= inv * w.w;
     }
-    store_row4(out + base + column(j), v);
+    store_quad(out + base + column(j), v);
   }
 }
 
-// The same for two pending terms, and for widths that are no multiple of four or too wide for registers: one CTA
+// The same for widths that are no multiple of four or too wide for registers: one CTA
 // per row, in shared memory.
 template <typename TOut>
 __global__ void stream_norm_any_kernel(const __grid_constant__ Pending pending, float scale, const float* __restrict__ post,
@@ -620,6 +709,40 @@ static int row_threads(int hidden) {
 
 using namespace einf;
 
+// A row in registers: aligned groups of four columns.  False: the caller's kernel in shared memory.
+static bool norm_in_registers(const Pending& p, const float* residual, const float* post, const float* weight, const void* out,
+                              int out_dtype, int hidden) {
+  // four columns an access: 16 bytes of floats, 8 of bfloat16
+  auto pieces = [](const void* at, int dtype, int splits, long long stride) {
+    return (uintptr_t)at % (dtype == kBFloat16 ? 8 : 16) == 0 && (splits <= 1 || stride % 4 == 0);
+  };
+  return hidden % 4 == 0 && hidden <= 8192 && (p.a || !p.b) && pieces(p.a, p.a_dtype, p.a_splits, p.a_stride) &&
+         pieces(p.b, p.b_dtype, p.b_splits, p.b_stride) &&
+         pieces(residual, kFloat32, 1, 0) && pieces(post, kFloat32, 1, 0) && pieces(weight, kFloat32, 1, 0) &&
+         pieces(out, out_dtype, 1, 0);
+}
+
+template <typename T>
+static cudaError_t launch_stream_norm(const Pending& pending, float scale, const float* post, float post_eps, float* residual,
+                                      const float* weight, float eps, T* out, int num_tokens, int hidden,
+                                      cudaStream_t stream) {
+#define EINF_STREAM_NORM(TEAM, VEC, GRID, THREADS)                                                                      \
+  return launch_pdl(stream_norm_kernel<T, TEAM, VEC>, GRID, THREADS, 0, stream, pending, scale, post, post_eps,         \
+                    residual, weight, eps, out, hidden, num_tokens)
+  // partial sums want every load of a row in flight: a warp a row only where there are none
+  if (num_tokens >= 256 && hidden <= 2048 && pending.a_splits <= 1 && pending.b_splits <= 1) {
+    const int grid = (num_tokens + 3) / 4;
+    if (hidden <= 1024) EINF_STREAM_NORM(32, 8, grid, 128);
+    if (hidden <= 1536) EINF_STREAM_NORM(32, 12, grid, 128);
+    EINF_STREAM_NORM(32, 16, grid, 128);
+  }
+  if (hidden <= 512) EINF_STREAM_NORM(128, 1, num_tokens, 128);
+  if (hidden <= 1024) EINF_STREAM_NORM(256, 1, num_tokens, 256);
+  if (hidden <= 2048) EINF_STREAM_NORM(512, 1, num_tokens, 512);
+  EINF_STREAM_NORM(512, 4, num_tokens, 512);
+#undef EINF_STREAM_NORM
+}
+
 extern "C" int einf_norm_conv(const void* pend_a, int a_dtype, int a_splits, long long a_stride, const void* pend_b,
                               int b_dtype, int b_splits, long long b_stride, float scale, float* residual,
                               const float* weight, float eps, const float* conv_weight, int taps, float* conv_state,
@@ -634,21 +757,47 @@ extern "C" int einf_norm_conv(const void* pend_a, int a_dtype, int a_splits, lon
   const int mode = !conv ? 0 : (single_tokens ? 1 : 2);
   const int threads = row_threads(hidden);
   const size_t smem = (size_t)(hidden + 33) * sizeof(float);
+  const bool registers = norm_in_registers(pending, residual, nullptr, weight, mode == 2 ? scratch : out,
+                                           mode == 2 ? kFloat32 : out_dtype, hidden);
+  const bool quads = taps <= kRunTaps && hidden % 4 == 0 && (uintptr_t)out % (out_dtype == kFloat32 ? 16 : 8) == 0;
+  if (mode == 1 && registers && quads && (uintptr_t)conv_state % 16 == 0 && state_stride % 4 == 0) {
+    EINF_DISPATCH_2(out_dtype, T, {
+      auto launch = [&](auto kernel, int size) {
+        return (int)launch_pdl(kernel, num_tokens, size, 0, stream, pending, scale, residual, weight, eps, conv_weight, taps,
+                               conv_state, state_stride, num_slots, seq_of_token, state_slots, (T*)out, hidden);
+      };
+      if (hidden <= 512) return launch(norm_single_quads_kernel<T, 1>, 128);
+      if (hidden <= 1024) return launch(norm_single_quads_kernel<T, 1>, 256);
+      if (hidden <= 2048) return launch(norm_single_quads_kernel<T, 1>, 512);
+      return launch(norm_single_quads_kernel<T, 4>, 512);
+    })
+  }
   EINF_DISPATCH_2(out_dtype, T, {
     if (smem > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(norm_row_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return (int)e;
     }
-    cudaError_t e = launch_pdl(norm_row_kernel<T>, num_tokens, threads, smem, stream, pending, scale, residual, weight,
-                               eps, conv_weight, taps, conv_state, state_stride, num_slots, seq_of_token, state_slots,
-                               (T*)out, scratch, hidden, mode);
+    cudaError_t e = cudaSuccess;
+    if (mode == 2 && registers)
+      e = launch_stream_norm<float>(pending, scale, nullptr, 0.f, residual, weight, eps, scratch, num_tokens, hidden, stream);
+    else
+      e = launch_pdl(norm_row_kernel<T>, num_tokens, threads, smem, stream, pending, scale, residual, weight, eps, conv_weight,
+                     taps, conv_state, state_stride, num_slots, seq_of_token, state_slots, (T*)out, scratch, hidden, mode);
     if (e != cudaSuccess || mode != 2) return (int)e;
-    const long long total = (long long)num_tokens * hidden;
-    long long blocks = (total + 255) / 256;
-    if (blocks > 148 * 32) blocks = 148 * 32;
-    e = launch_pdl(conv_rows_kernel<T>, (int)blocks, 256, 0, stream, (const float*)scratch, conv_weight, taps,
-                   (const float*)conv_state, state_stride, num_slots, seq_of_token, q_start, state_slots, (T*)out,
-                   hidden, num_tokens);
+    // runs of eight tokens for portions of 64 and more on average: 2,048 tokens of 896 channels 16 -> 7.4 us
+    const long long run_threads = (long long)((num_tokens + kRunTokens - 1) / kRunTokens) * (hidden / 4);
+    if (quads && num_tokens >= 64ll * num_requests && run_threads < (1ll << 31)) {
+      e = launch_pdl(conv_rows_run_kernel<T>, (int)((run_threads + 127) / 128), 128, 0, stream, (const float*)scratch,
+                     conv_weight, taps, (const float*)conv_state, state_stride, num_slots, seq_of_token, q_start, state_slots,
+                     (T*)out, hidden, num_tokens);
+    } else {
+      const long long total = (long long)num_tokens * hidden;
+      long long blocks = (total + 255) / 256;
+      if (blocks > 148 * 32) blocks = 148 * 32;
+      e = launch_pdl(conv_rows_kernel<T>, (int)blocks, 256, 0, stream, (const float*)scratch, conv_weight, taps,
+                     (const float*)conv_state, state_stride, num_slots, seq_of_token, q_start, state_slots, (T*)out, hidden,
+                     num_tokens);
+    }
     if (e != cudaSuccess) return (int)e;
     const dim3 grid((hidden + 127) / 128, num_requests);
     return (int)launch_pdl(conv_rows_state_kernel, grid, 128, 0, stream, (const float*)scratch, conv_state,
@@ -663,30 +812,10 @@ extern "C" int einf_stream_norm(const void* pend_a, int a_dtype, int a_splits, l
   if (num_tokens == 0) return 0;
   if (hidden <= 0) return (int)cudaErrorInvalidValue;
   const Pending pending{pend_a, a_dtype, a_splits, a_stride, pend_b, b_dtype, b_splits, b_stride};
-  // four columns an access: 16 bytes of floats, 8 of bfloat16
-  auto pieces = [](const void* p, int dtype, int splits, long long stride) {
-    return (uintptr_t)p % (dtype == kBFloat16 ? 8 : 16) == 0 && (splits <= 1 || stride % 4 == 0);
-  };
-  const bool vectors = hidden % 4 == 0 && hidden <= 8192 && !pend_b && pieces(pend_a, a_dtype, a_splits, a_stride) &&
-                       pieces(residual, kFloat32, 1, 0) &&
-                       pieces(post, kFloat32, 1, 0) && pieces(weight, kFloat32, 1, 0) && pieces(out, out_dtype, 1, 0);
-#define EINF_STREAM_NORM(TEAM, VEC, GRID, THREADS)                                                                      \
-  return (int)launch_pdl(stream_norm_kernel<T, TEAM, VEC>, GRID, THREADS, 0, stream, pending, scale, post, post_eps,    \
-                         residual, weight, eps, (T*)out, hidden, num_tokens)
   EINF_DISPATCH_2(out_dtype, T, {
-    if (vectors) {
-      // partial sums want every load of a row in flight: a warp a row only where there are none
-      if (num_tokens >= 256 && hidden <= 2048 && a_splits <= 1) {
-        const int grid = (num_tokens + 3) / 4;
-        if (hidden <= 1024) EINF_STREAM_NORM(32, 8, grid, 128);
-        if (hidden <= 1536) EINF_STREAM_NORM(32, 12, grid, 128);
-        EINF_STREAM_NORM(32, 16, grid, 128);
-      }
-      if (hidden <= 512) EINF_STREAM_NORM(128, 1, num_tokens, 128);
-      if (hidden <= 1024) EINF_STREAM_NORM(256, 1, num_tokens, 256);
-      if (hidden <= 2048) EINF_STREAM_NORM(512, 1, num_tokens, 512);
-      EINF_STREAM_NORM(512, 4, num_tokens, 512);
-    }
+    if (norm_in_registers(pending, residual, post, weight, out, out_dtype, hidden))
+      return (int)launch_stream_norm<T>(pending, scale, post, post_eps, residual, weight, eps, (T*)out, num_tokens, hidden,
+                                        stream);
     const size_t smem = (size_t)(hidden + 33) * sizeof(float);
     if (smem > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(stream_norm_any_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -695,7 +824,6 @@ extern "C" int einf_stream_norm(const void* pend_a, int a_dtype, int a_splits, l
     return (int)launch_pdl(stream_norm_any_kernel<T>, num_tokens, row_threads(hidden), smem, stream, pending, scale, post,
                            post_eps, residual, weight, eps, (T*)out, hidden);
   })
-#undef EINF_STREAM_NORM
 }
 
 extern "C" int einf_side_gate(const void* product, int in_dtype, int splits, long long split_stride, const void* table,

@@ -256,3 +256,37 @@ def test_end_of_a_layer(dev, dtype, tokens, hidden, side, layers_done, parts):
     torch.testing.assert_close(got[0].cpu(), want[0], **close)
     if use_depth:
         torch.testing.assert_close(got[5][0].cpu(), want[5][0], **close)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hidden, taps, lengths", [
+    (64, 4, (1, 190, 2, 69)), (516, 2, (8, 8, 264, 3)), (1540, 3, (300,)), (2052, 4, (130, 1)), (72, 5, (66, 2)), (70, 3, (80,)),
+    (64, 4, (1, 1, 1)), (516, 2, (1, 1)), (896, 3, (1, 1, 1, 1)), (2052, 4, (1,)), (72, 5, (1, 1)),
+])
+def test_norm_and_convolution(dev, dtype, hidden, taps, lengths):
+    """Rows in registers and runs of eight tokens (widths in groups of four, up to four taps), the kernels for the other
+    widths and taps, and single tokens, whose launch moves the state on as well."""
+    from einf_b200 import ops
+
+    generator = torch.Generator().manual_seed(hidden + taps)
+    tokens = sum(lengths)
+    starts = torch.tensor([0] + list(torch.tensor(lengths).cumsum(0)), dtype=torch.int32)
+    seq = torch.repeat_interleave(torch.arange(len(lengths)), torch.tensor(lengths)).to(torch.int32)
+    slots = torch.tensor([2, 0, -1, 3], dtype=torch.int32)[:len(lengths)]
+    residual = torch.randn((tokens, hidden), generator=generator)
+    pending = [torch.randn((tokens, hidden), generator=generator).to(dtype),
+               torch.randn((3, tokens, hidden), generator=generator)][:1 + taps % 2]
+    weight = torch.rand((hidden,), generator=generator) + 0.5
+    conv = torch.randn((hidden, taps), generator=generator)
+    state = torch.randn((5, taps - 1, hidden), generator=generator)
+    single = max(lengths) == 1
+
+    def run(module, move):
+        row, line, out = move(residual.clone()), move(state.clone()), move(torch.empty((tokens, hidden), dtype=dtype))
+        module.norm_conv([move(t) for t in pending], 0.7, row, move(weight), 1e-5, move(conv), line, move(seq), move(starts),
+                         move(slots), out, single_tokens=single)
+        return row.cpu(), line.cpu(), out.cpu()
+
+    for got, want in zip(run(ops, lambda t: t.to(dev)), run(ref, lambda t: t)):
+        close = dict(rtol=1e-4, atol=2e-5) if got.dtype == torch.float32 else tol(dtype)
+        torch.testing.assert_close(got, want, **close)

@@ -373,3 +373,68 @@ def test_gated_norm(dev, dtype, width, parts, gate_first, kind):
     ops.gated_norm(y, gate, weight, out, parts, 1e-5, gate_first, kind)
     ref.gated_norm(y, gate, weight, want, parts, 1e-5, gate_first, kind)
     close(out, want, dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("channels, taps, heads, lengths", [
+    (24, 4, 3, (1, 190, 2, 69)), (40, 2, 0, (8, 8, 264, 3)), (64, 1, 1, (65,)), (132, 3, 2, (3, 1, 191)),
+])
+def test_conv_silu_over_runs_of_tokens(dev, dtype, channels, taps, heads, lengths):
+    """Portions of 64 tokens and more on average, four channels of eight tokens a thread: requests that begin inside a run, a
+    request without a slot, a last run that is not full."""
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(8)
+    slots = torch.tensor([2, 0, -1, 3], dtype=torch.int32, device=dev)[:len(lengths)]
+    q_start, seq = _packed(lengths, dev)
+    tokens = sum(lengths)
+    wide = torch.randn((tokens, 4 + channels + 4), generator=gen).to(dtype).to(dev)
+    x, dt_raw = wide[:, 4:4 + channels], wide[:, 4 + channels:4 + channels + heads]
+    weight, bias = torch.randn((channels, taps), generator=gen).to(dev), torch.randn(channels, generator=gen).to(dev)
+    dt_bias, a_log = torch.randn(heads, generator=gen).to(dev), torch.randn(heads, generator=gen).to(dev)
+    state = torch.randn((5, 9 + (taps - 1) * channels), generator=gen).to(dev)
+    results = []
+    for fn in (ops.conv_silu, ref.conv_silu):
+        out = torch.empty((tokens, channels), dtype=dtype, device=dev)
+        dt, decay = torch.empty((tokens, heads), device=dev), torch.empty((tokens, heads), device=dev)
+        mine = state.clone()
+        extra = (dt_raw, dt_bias, a_log, dt, decay) if heads else (None,) * 5
+        fn(x, weight, bias, mine[:, 9:].view(5, taps - 1, channels), seq, q_start, slots, out, *extra, activation=taps != 3,
+           input_bias=bias if taps == 2 else None)
+        results.append((out, dt, decay, mine) if heads else (out, mine))
+    for got, want in zip(*results):
+        close(got, want, dtype if got.dtype == dtype else torch.float32)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width, parts, kind", [(252, 1, "silu"), (1280, 2, "sigmoid"), (1024, 1, "silu"), (1028, 1, "silu")])
+def test_gated_norm_a_warp_a_row(dev, dtype, width, parts, kind):
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(9)
+    tokens = 593
+    y = torch.randn((tokens, width), generator=gen).to(dev)
+    gate = torch.randn((tokens, width + 24), generator=gen).to(dtype).to(dev)[:, 8:8 + width]
+    weight = torch.randn(width, generator=gen).to(dev)
+    for first in (True, False):
+        out, want = (torch.empty((tokens, width), dtype=dtype, device=dev) for _ in range(2))
+        ops.gated_norm(y, gate, weight, out, parts, 1e-5, first, kind)
+        ref.gated_norm(y, gate, weight, want, parts, 1e-5, first, kind)
+        close(out, want, dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads, vdim", [(3, 4), (2, 128), (1, 252), (2, 1024)])
+def test_memory_output_four_elements_a_load(dev, dtype, heads, vdim):
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(10)
+    tokens, columns = 7, ops.memory_value_columns(vdim)
+    y = torch.randn((tokens, heads * columns), generator=gen).to(dev)
+    floor = torch.rand((tokens, heads), generator=gen).to(dev)
+    gate = torch.randn((tokens, heads * vdim + 8), generator=gen).to(dtype).to(dev)[:, 4:4 + heads * vdim]
+    weight = torch.randn(heads * vdim, generator=gen).to(dev)
+    out, want = (torch.empty((tokens, heads * vdim), dtype=dtype, device=dev) for _ in range(2))
+    for fn, to in ((ops.memory_output, out), (ref.memory_output, want)):
+        fn(y, floor, gate, weight, to, heads, vdim, 0.125, 1e-5, 1e-6)
+    close(out, want, dtype)
