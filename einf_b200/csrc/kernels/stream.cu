@@ -11,6 +11,7 @@
 #include <cstdint>
 
 #include "conv_run.cuh"
+#include "mma_sync.cuh"
 
 namespace einf {
 
@@ -699,6 +700,192 @@ stream_tail_tokens_kernel(float* __restrict__ residual, const __grid_constant__ 
   }
 }
 
+// The same end of a layer on the tensor cores, for bfloat16 matrices and up to 16 tokens a CTA.  x and g stay 32-bit: each goes
+// into a product as three bfloat16 parts (24 bits) against the exact matrix, so a product's error is that of its 32-bit
+// additions.  s = gate x: the warps share x's columns, their sums meet in shared memory in warp order.  y = proj_t^T g: a warp
+// has 32 columns at a time; a lane reads four neighbouring ones of a row of proj_t, and the four go to four tiles, so the
+// pieces are whole sectors and a lane's results are eight neighbouring columns.  x's rows and the depth average are float4
+// throughout.  One wave of CTAs (the launcher's `each`); a product's unused rows are never read back.
+// Bound by latency (a CTA's chain of five short phases); the FMA kernel above is bound by its shared-memory reads.  Measured
+// (B200): 2,048 tokens, 896 columns, 64 token-input elements 101 -> 34 us.
+constexpr int kTailRows = 16;
+constexpr int kTailWarps = kTailThreads / 32;
+
+static int tail_stride(int hidden) { return hidden + (40 - hidden % 32) % 32; }     // 8 modulo 32: fragment reads without conflicts
+static size_t tail_mma_bytes(int hidden, int side) {
+  const size_t rows = (size_t)kTailRows * tail_stride(hidden), partial = (size_t)kTailWarps * kTailRows * (side + 8);
+  return (rows + (rows > partial ? rows : partial) + kTailRows * (side + 8) + kTailWarps) * sizeof(float);
+}
+
+template <int KS>                    // side = 16 KS
+__global__ void __launch_bounds__(kTailThreads)
+stream_tail_mma_kernel(float* __restrict__ residual, const __grid_constant__ Pending pending, float scale,
+                       const int* __restrict__ token_ids, const __nv_bfloat16* __restrict__ table,
+                       const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ proj_t,
+                       const float* __restrict__ norm, int vocab, float eps, float* __restrict__ history, int depth_index,
+                       const float* __restrict__ depth_weight, long long history_stride, int hidden, int stride, int pool,
+                       int num_tokens, int each) {
+  constexpr int kSide = 16 * KS, kGStride = kSide + 8;
+  extern __shared__ float4 smem4[];
+  float* x = (float*)smem4;                              // [16, stride]
+  float* y = x + kTailRows * stride;                     // [16, stride]; before that the warps' parts of s
+  float* g = y + pool;                                   // [16, side + 8]
+  float* red = g + kTailRows * kGStride;                 // [warps]
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lr = lane >> 2, lq = lane & 3;
+  const int t0 = blockIdx.x * each, count = min(each, num_tokens - t0);
+  const int per_row = kTailWarps / each, row = warp / per_row, sub = warp - row * per_row;
+  const bool adds = pending.a != nullptr || pending.b != nullptr;
+  const int chunks = hidden / 16;
+  uint32_t b[2 * KS][1][2];                              // a chunk of gate: weights, read before the step's data are there
+  auto load_gate = [&](int chunk) {
+#pragma unroll
+    for (int n = 0; n < 2 * KS; ++n) {
+      const __nv_bfloat16* at = gate + (size_t)(8 * n + lr) * hidden + 16 * chunk + 2 * lq;
+      b[n][0][0] = *(const uint32_t*)at;
+      b[n][0][1] = *(const uint32_t*)(at + 8);
+    }
+  };
+  if (warp < chunks) load_gate(warp);
+  pdl_wait();
+  const size_t base = (size_t)(t0 + row) * hidden;
+  if (row < count) {
+#pragma unroll 2
+    for (int c = 4 * (32 * sub + lane); c < hidden; c += 128 * per_row) {
+      float4 v = *(const float4*)(residual + base + c);
+      if (adds) {
+        const float4 more = pending4_sum<4>(pending, base + c);
+        v.x = fmaf(scale, more.x, v.x); v.y = fmaf(scale, more.y, v.y);
+        v.z = fmaf(scale, more.z, v.z); v.w = fmaf(scale, more.w, v.w);
+      }
+      *(float4*)(x + row * stride + c) = v;
+    }
+  }
+  __syncthreads();
+  float s[2 * KS][4];
+#pragma unroll
+  for (int n = 0; n < 2 * KS; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[n][e] = 0.f;
+  for (int chunk = warp; chunk < chunks; chunk += kTailWarps) {
+    uint32_t a[3][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 v = *(const float2*)(x + (lr + 8 * (e & 1)) * stride + 16 * chunk + 8 * (e >> 1) + 2 * lq);
+      uint32_t part[3];
+      split3(v.x, v.y, part);
+#pragma unroll
+      for (int p = 0; p < 3; ++p) a[p][e] = part[p];
+    }
+    uint32_t now[2 * KS][1][2];
+#pragma unroll
+    for (int n = 0; n < 2 * KS; ++n) { now[n][0][0] = b[n][0][0]; now[n][0][1] = b[n][0][1]; }
+    if (chunk + kTailWarps < chunks) load_gate(chunk + kTailWarps);
+#pragma unroll
+    for (int n = 0; n < 2 * KS; ++n) mma_parts<3, 1>(s[n], a, now[n]);
+  }
+#pragma unroll
+  for (int n = 0; n < 2 * KS; ++n)
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+      *(float2*)(y + (warp * kTailRows + lr + 8 * half) * kGStride + 8 * n + 2 * lq) = make_float2(s[n][2 * half], s[n][2 * half + 1]);
+  __syncthreads();
+  for (int idx = tid; idx < count * kSide; idx += kTailThreads) {
+    const int i = idx / kSide, d = idx - i * kSide;
+    int token = token_ids[t0 + i];
+    token = token < 0 ? 0 : (token >= vocab ? vocab - 1 : token);     // a bad id was reported by the embedding
+    const float entry = __bfloat162float(table[(size_t)token * kSide + d]);
+    float total = 0.f;
+#pragma unroll
+    for (int w = 0; w < kTailWarps; ++w) total += y[(w * kTailRows + i) * kGStride + d];
+    g[i * kGStride + d] = gelu_tanh_f(total) * entry;
+  }
+  __syncthreads();
+  uint32_t a[KS][3][4];
+#pragma unroll
+  for (int k = 0; k < KS; ++k)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 v = *(const float2*)(g + (lr + 8 * (e & 1)) * kGStride + 16 * k + 8 * (e >> 1) + 2 * lq);
+      uint32_t part[3];
+      split3(v.x, v.y, part);
+#pragma unroll
+      for (int p = 0; p < 3; ++p) a[k][p][e] = part[p];
+    }
+  for (int first = 32 * warp; first < hidden; first += 32 * kTailWarps) {
+    const int c = first + 4 * lr;
+    uint2 w[KS][4];                                      // rows 2 lq, 2 lq + 1 and the two eight below, four columns of each
+#pragma unroll
+    for (int k = 0; k < KS; ++k)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        w[k][e] = c < hidden ? *(const uint2*)(proj_t + (size_t)(16 * k + 2 * lq + (e & 1) + 8 * (e >> 1)) * hidden + c) : make_uint2(0, 0);
+    float out[4][4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) out[n][e] = 0.f;
+#pragma unroll
+      for (int k = 0; k < KS; ++k) {
+        const uint32_t pick = n & 1 ? 0x7632 : 0x5410;
+        uint32_t column[1][2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          column[0][e] = n < 2 ? __byte_perm(w[k][2 * e].x, w[k][2 * e + 1].x, pick) : __byte_perm(w[k][2 * e].y, w[k][2 * e + 1].y, pick);
+        mma_parts<3, 1>(out[n], a[k], column);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int at = first + 8 * lq + 4 * (e & 1);
+      if (at < hidden) *(float4*)(y + (lr + 8 * (e >> 1)) * stride + at) = make_float4(out[0][e], out[1][e], out[2][e], out[3][e]);
+    }
+  }
+  __syncthreads();
+  float ss = 0.f;
+  if (row < count)
+    for (int c = 4 * (32 * sub + lane); c < hidden; c += 128 * per_row) {
+      const float4 v = *(const float4*)(y + row * stride + c);
+      ss += v.x * v.x + v.y * v.y + (v.z * v.z + v.w * v.w);
+    }
+  ss = warp_sum(ss);
+  if (lane == 0) red[warp] = ss;
+  __syncthreads();
+  if (row >= count) return;
+  float total = 0.f;
+  for (int w = 0; w < per_row; ++w) total += red[row * per_row + w];
+  const float factor = scale * rsqrtf(total / (float)hidden + eps);
+  const float newest = history ? depth_weight[depth_index + 1] : 0.f;
+  for (int c = 4 * (32 * sub + lane); c < hidden; c += 128 * per_row) {
+    const float4 u = *(const float4*)(y + row * stride + c), w = *(const float4*)(norm + c);
+    float4 v = *(const float4*)(x + row * stride + c);
+    v.x = fmaf(factor * w.x, u.x, v.x); v.y = fmaf(factor * w.y, u.y, v.y);
+    v.z = fmaf(factor * w.z, u.z, v.z); v.w = fmaf(factor * w.w, u.w, v.w);
+    if (history) {
+      *(float4*)(history + (size_t)(depth_index + 1) * history_stride + base + c) = v;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      constexpr int kBatch = 8;                          // earlier layers' results: several loads in flight
+      for (int j0 = 0; j0 <= depth_index; j0 += kBatch) {
+        float4 earlier[kBatch];
+#pragma unroll
+        for (int e = 0; e < kBatch; ++e)
+          earlier[e] = j0 + e <= depth_index ? *(const float4*)(history + (size_t)(j0 + e) * history_stride + base + c)
+                                             : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int e = 0; e < kBatch; ++e) {
+          if (j0 + e > depth_index) continue;
+          const float dw = depth_weight[j0 + e];
+          acc.x = fmaf(dw, earlier[e].x, acc.x); acc.y = fmaf(dw, earlier[e].y, acc.y);
+          acc.z = fmaf(dw, earlier[e].z, acc.z); acc.w = fmaf(dw, earlier[e].w, acc.w);
+        }
+      }
+      v.x = fmaf(newest, v.x, acc.x); v.y = fmaf(newest, v.y, acc.y);
+      v.z = fmaf(newest, v.z, acc.z); v.w = fmaf(newest, v.w, acc.w);
+    }
+    *(float4*)(residual + base + c) = v;
+  }
+}
+
 static int row_threads(int hidden) {
   int threads = 64;
   while (threads < hidden / 4 && threads < 512) threads <<= 1;
@@ -853,6 +1040,35 @@ extern "C" int einf_stream_tail(float* residual, const void* pend_a, int a_dtype
   if (num_tokens == 0) return 0;
   if (hidden <= 0 || side < 0) return (int)cudaErrorInvalidValue;
   const Pending pending{pend_a, a_dtype, a_splits, a_stride, pend_b, b_dtype, b_splits, b_stride};
+  auto quads = [](const void* p, int dtype, int splits, long long stride) {
+    return (uintptr_t)p % (dtype == kBFloat16 ? 8 : 16) == 0 && (splits <= 1 || stride % 4 == 0);
+  };
+  // the tensor cores where three bfloat16 parts can state a product exactly and 16 rows of x and y fit; not while every token
+  // has an SM of its own, where 15 of a product's 16 rows would be idle (64 tokens 19.8 us, 16.6 by the FMA kernel)
+  if (num_tokens > 148 && weight_dtype == kBFloat16 && side > 0 && side % 16 == 0 && side <= 64 && hidden % 16 == 0 &&
+      tail_mma_bytes(hidden, side) <= 220 * 1024 && (pend_a || !pend_b) && quads(pend_a, a_dtype, a_splits, a_stride) &&
+      quads(pend_b, b_dtype, b_splits, b_stride) && history_stride % 4 == 0 &&
+      ((uintptr_t)gate | (uintptr_t)proj_t | (uintptr_t)residual | (uintptr_t)norm | (uintptr_t)history) % 16 == 0) {
+    int each = 2;
+    while (each < kTailRows && num_tokens > 148 * each) each *= 2;
+    const size_t bytes = tail_mma_bytes(hidden, side);
+    const int stride = tail_stride(hidden), partial = kTailWarps * kTailRows * (side + 8);
+    const int pool = kTailRows * stride > partial ? kTailRows * stride : partial;
+    auto launch = [&](auto kernel) {
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      if (e != cudaSuccess) return (int)e;
+      return (int)launch_pdl(kernel, (num_tokens + each - 1) / each, kTailThreads, bytes, stream, residual, pending, scale,
+                             token_ids, (const __nv_bfloat16*)table, (const __nv_bfloat16*)gate,
+                             (const __nv_bfloat16*)proj_t, norm, vocab, eps, history, depth_index, depth_weight,
+                             history_stride, hidden, stride, pool, num_tokens, each);
+    };
+    switch (side / 16) {
+      case 1: return launch(stream_tail_mma_kernel<1>);
+      case 2: return launch(stream_tail_mma_kernel<2>);
+      case 3: return launch(stream_tail_mma_kernel<3>);
+      default: return launch(stream_tail_mma_kernel<4>);
+    }
+  }
   if (hidden % 8 == 0 && side > 0 && ((uintptr_t)gate | (uintptr_t)proj_t) % 16 == 0) {
     // tokens a CTA: eight for a long step where they fit beside a second CTA, else four; one while every token
     // still gets an SM of its own (the step is then bound by one CTA's instructions, not by the matrices' bytes)

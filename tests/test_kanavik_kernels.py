@@ -258,6 +258,43 @@ def test_end_of_a_layer(dev, dtype, tokens, hidden, side, layers_done, parts):
         torch.testing.assert_close(got[5][0].cpu(), want[5][0], **close)
 
 
+@pytest.mark.parametrize("tokens, hidden, side, layers_done, splits", [
+    (150, 16, 16, 0, 1), (300, 896, 64, 3, 1), (149, 144, 32, 9, 3), (2401, 48, 48, 1, 1), (593, 1568, 64, 0, 2),
+])
+def test_end_of_a_layer_on_the_tensor_cores(dev, tokens, hidden, side, layers_done, splits):
+    """Two to 16 tokens a CTA, widths around the warps' shares, partial sums: off the statement in 64 bits by what its 32-bit
+    sums and norms round, 2^-24 of each of their terms."""
+    from einf_b200 import ops
+
+    generator = torch.Generator().manual_seed(tokens + side)
+    vocab = 50
+    residual = torch.randn((tokens, hidden), generator=generator)
+    pending = [torch.randn((splits, tokens, hidden), generator=generator),
+               torch.randn((tokens, hidden), generator=generator).to(torch.bfloat16)][:1 + splits % 2]
+    ids = torch.randint(0, vocab, (tokens,), generator=generator, dtype=torch.int32)
+    table, proj_t = (torch.randn((n, m), generator=generator).to(torch.bfloat16) for n, m in ((vocab, side), (side, hidden)))
+    gate = (torch.randn((side, hidden), generator=generator) * hidden ** -0.5).to(torch.bfloat16)
+    norm = torch.rand((hidden,), generator=generator) + 0.5
+    history = torch.randn((layers_done + 2, tokens, hidden), generator=generator)
+    weight = torch.randn((layers_done + 2,), generator=generator)
+    x = residual.double() + 0.6 * sum(p.double().reshape(-1, tokens, hidden).sum(0) for p in pending)
+    s = x @ gate.double().T
+    g = 0.5 * s * (1 + torch.tanh(0.7978845608028654 * (s + 0.044715 * s ** 3))) * table[ids.long()].double()
+    y = g @ proj_t.double()
+    x = x + 0.6 * y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * norm.double()
+    for depth in (True, False):
+        got, line = residual.to(dev), history.to(dev)
+        ops.stream_tail(got, [p.to(dev) for p in pending], 0.6, ids.to(dev),
+                        (table.to(dev), gate.to(dev), proj_t.to(dev), norm.to(dev), 1e-5),
+                        (line, layers_done, weight.to(dev)) if depth else None)
+        want = x
+        if depth:
+            torch.testing.assert_close(line[layers_done + 1].cpu().double(), x, rtol=1e-5, atol=1e-5)
+            want = weight[layers_done + 1].double() * x + torch.einsum("j,jth->th", weight[:layers_done + 1].double(),
+                                                                      history[:layers_done + 1].double())
+        torch.testing.assert_close(got.cpu().double(), want, rtol=1e-5, atol=2e-5)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("hidden, taps, lengths", [
     (64, 4, (1, 190, 2, 69)), (516, 2, (8, 8, 264, 3)), (1540, 3, (300,)), (2052, 4, (130, 1)), (72, 5, (66, 2)), (70, 3, (80,)),
