@@ -315,6 +315,297 @@ mixed_prompt_attention_kernel(const __grid_constant__ MixArgs a) {
   }
 }
 
+// The same for requests that bring one token (decoding), up to 16 heads: a product's 16 rows are the token's heads, so a key
+// or value row is read once for all of them, and its columns are all key heads end to end, then all value heads (a row uses
+// those of its own head).  A CTA has a share of the token's keys, a warp 32 keys at a time of its own, brought by the warp
+// alone: no barrier between the first key and the last.  What the warps found (maximum, sum, values) meets in shared memory,
+// what the CTAs of a token found in the join below.
+//
+// Bound by the latencies of a CTA's few chunks.  Measured (B200): 64 tokens behind 2,048, 14 heads of 64 on 2, four CTAs a
+// token: 68 -> 23 us (the FMA kernel of attention_mixed_tiled.cu), the join 2.8 either way.
+constexpr int kSingleChunk = 32, kSingleHeads = 16, kSinglePitch = 256;
+constexpr int kSingleQ = 3 * kSingleHeads * kSinglePitch, kSingleWarp = 2 * kSingleChunk * kSinglePitch;
+constexpr int kSingleSmem = kSingleQ + 4 * kSingleWarp, kSingleOPitch = 136;
+
+struct SingleArgs {
+  MixArgs m;
+  const int* seq_of_token; const int* positions;
+  const int* tokens;                 // token indices; null: token = block
+  int splits, num_tokens;
+  float* part_acc;                   // [splits, tokens, heads * vdim]
+  float* part_ml;                    // [splits, tokens, heads, 2]: maximum (of scores in powers of two), sum
+};
+
+__global__ void __launch_bounds__(kMixThreads, 2)
+mixed_single_attention_kernel(const __grid_constant__ SingleArgs s) {
+  extern __shared__ __align__(128) unsigned char mix_smem[];
+  __shared__ float slopes[kSingleHeads], warp_m[4][kSingleHeads], warp_l[4][kSingleHeads];
+  const MixArgs& a = s.m;
+  pdl_launch_dependents();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, q2 = (lane & 3) * 2;
+  const int in8 = lane & 7, second = (lane >> 3) & 1, third = lane >> 4;
+  const uint32_t base = smem_address(mix_smem), keys_at = base + kSingleQ + warp * kSingleWarp;
+  const uint32_t values_at = keys_at + kSingleChunk * kSinglePitch;
+  const int dim = a.dim, vdim = a.vdim, heads = a.heads, per = heads / a.kv_heads;
+  const int key_width = a.kv_heads * dim, value_width = a.kv_heads * vdim;
+  const int t = s.tokens ? s.tokens[blockIdx.x] : (int)blockIdx.x;
+  const int pos = s.positions[t];
+  const int* table = a.block_table + (long long)s.seq_of_token[t] * a.table_width;
+  const int lowest = a.window > 0 ? max(0, pos - a.window + 1) : 0;
+  const int chunks = pos / kSingleChunk + 1 - lowest / kSingleChunk, share = (chunks + s.splits - 1) / s.splits;
+  const int begin = lowest / kSingleChunk + (int)blockIdx.y * share, end = min(begin + share, pos / kSingleChunk + 1);
+  bool bad_page = false;
+  auto find = [&](int chunk) {       // of this lane's key: the page's first row of head 0 + slot in it, -1: none
+    const int j = chunk * kSingleChunk + lane;
+    if (chunk >= end || j < lowest || j > pos) return -1;
+    const int logical = j / a.page_size, page = table[logical];
+    if (page < 0 || page >= a.num_pages) {
+      bad_page = true;
+      return -1;
+    }
+    return page * a.kv_heads * a.page_size + (j - logical * a.page_size);
+  };
+  int chunk = begin + warp, row = find(chunk);
+  const int piece = lane & 15, half_row = lane >> 4;
+  auto bring = [&](uint32_t at, const __nv_bfloat16* cache, int size, int width, int rows) {
+    const int e = 8 * piece, c = e / size;
+    const __nv_bfloat16* from = cache + (long long)c * a.page_size * size + (e - c * size);
+#pragma unroll
+    for (int i = 0; i < kSingleChunk / 2; ++i) {
+      const int key = 2 * i + half_row, place = __shfl_sync(0xffffffffu, rows, key);
+      const bool there = e < width && place >= 0;
+      cp_async16(at + swizzled(key, piece, kSinglePitch), there ? from + (long long)place * size : cache, there ? 16 : 0);
+    }
+  };
+  pdl_wait();
+  if (chunk < end) bring(keys_at, a.k_cache, dim, key_width, row);
+  cp_async_commit_group();
+  if (chunk < end) bring(values_at, a.v_cache, vdim, value_width, row);
+  cp_async_commit_group();
+
+  // ---- q': a thread has two neighbouring columns of every other head
+  {
+    const int e = 2 * ((int)threadIdx.x & 63), c = e / dim;
+    float qx[kSingleHeads], qy[kSingleHeads];
+#pragma unroll
+    for (int u = 0; u < kSingleHeads; ++u) {
+      const bool there = e < key_width && u < per;
+      const uint32_t pair = there ? *reinterpret_cast<const uint32_t*>(a.q + ((long long)t * heads + c * per + u) * dim + e - c * dim) : 0u;
+      qx[u] = low_bf16(pair);
+      qy[u] = high_bf16(pair);
+    }
+    for (int h = threadIdx.x >> 6; h < kSingleHeads; h += 2) {
+      float x = 0.f, y = 0.f;
+      if (h < heads && e < key_width) {
+#pragma unroll
+        for (int u = 0; u < kSingleHeads; ++u) {
+          if (u >= per) continue;
+          const float w = a.talk ? a.talk[h * heads + c * per + u] : (c * per + u == h ? 1.f : 0.f);
+          x = fmaf(w, qx[u], x);
+          y = fmaf(w, qy[u], y);
+        }
+      }
+      uint32_t part[3];
+      split3(x * a.scale_log2, y * a.scale_log2, part);
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
+        sts_u32(base + p * kSingleHeads * kSinglePitch + swizzled(h, e / 8, kSinglePitch) + (e & 7) * 2, part[p]);
+    }
+    if (threadIdx.x < kSingleHeads) {
+      const int h = threadIdx.x;
+      float slope = 0.f;
+      if (h < heads && a.slopes)
+        for (int other = 0; other < heads; ++other)
+          slope = fmaf(a.talk ? a.talk[h * heads + other] : (other == h ? 1.f : 0.f), a.slopes[other], slope);
+      slopes[h] = slope * 1.4426950408889634f;
+    }
+  }
+  __syncthreads();
+  const float slope[2] = {slopes[g], slopes[g + 8]};
+
+  float O[16][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) O[j][e] = 0.f;
+  for (; chunk < end; chunk += 4) {
+    const int j0 = chunk * kSingleChunk;
+    row = find(chunk + 4);
+    cp_async_wait_groups<1>();                         // the keys are there
+    __syncwarp();
+    float S[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) S[j][e] = 0.f;
+#pragma unroll 2
+    for (int kk = 0; kk < kMixKeySize / 16; ++kk) {
+      if (16 * kk >= key_width) break;
+      uint32_t qf[3][4], kf[2][4];
+      float sum[4][4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        ldsm_x4(kf[j], keys_at + swizzled(16 * j + in8 + 8 * third, 2 * kk + second, kSinglePitch));
+#pragma unroll
+      for (int p = 2; p >= 0; --p) {
+        ldsm_x4(qf[p], base + p * kSingleHeads * kSinglePitch + swizzled(in8 + 8 * second, 2 * kk + third, kSinglePitch));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (p == 2) mma_bf16_16816_zero(sum[j], qf[p], kf[j >> 1][2 * (j & 1)], kf[j >> 1][2 * (j & 1) + 1]);
+          else mma_bf16_16816(sum[j], qf[p], kf[j >> 1][2 * (j & 1)], kf[j >> 1][2 * (j & 1) + 1]);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[j][e] += sum[j][e];
+    }
+    __syncwarp();                                      // the keys are used up
+    if (chunk + 4 < end) bring(keys_at, a.k_cache, dim, key_width, row);
+    cp_async_commit_group();                           // perhaps an empty group: the values are always the second youngest
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {             // heads g and g + 8
+      float top = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int key = j0 + 8 * j + q2 + e;
+          const float z = S[j][2 * half + e] - slope[half] * (float)(pos - key);
+          S[j][2 * half + e] = key >= lowest && key <= pos ? z : -INFINITY;
+          top = fmaxf(top, S[j][2 * half + e]);
+        }
+      top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+      top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+      const float to = fmaxf(m[half], top);
+      const float shift = to == -INFINITY ? 0.f : to;
+      const float factor = exp2f(m[half] - shift);     // nothing seen so far: zero
+      m[half] = to;
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float w = exp2f(S[j][2 * half + e] - shift);
+          S[j][2 * half + e] = w;
+          sum += w;
+        }
+      l[half] = l[half] * factor + sum;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        O[j][2 * half] *= factor;
+        O[j][2 * half + 1] *= factor;
+      }
+    }
+    cp_async_wait_groups<1>();                         // the values are there
+    __syncwarp();
+#pragma unroll
+    for (int kk = 0; kk < 2; ++kk) {
+      uint32_t hi[4], lo[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float x = S[2 * kk + (e >> 1)][2 * (e & 1)], y = S[2 * kk + (e >> 1)][2 * (e & 1) + 1];
+        hi[e] = pack_pair(x, y);
+        lo[e] = pack_pair(x - low_bf16(hi[e]), y - high_bf16(hi[e]));
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (16 * j >= value_width) break;
+        uint32_t vf[4];
+        ldsm_x4_trans(vf, values_at + swizzled(16 * kk + in8 + 8 * second, 2 * j + third, kSinglePitch));
+        mma_bf16_16816(O[2 * j], lo, vf[0], vf[1]);
+        mma_bf16_16816(O[2 * j + 1], lo, vf[2], vf[3]);
+        mma_bf16_16816(O[2 * j], hi, vf[0], vf[1]);
+        mma_bf16_16816(O[2 * j + 1], hi, vf[2], vf[3]);
+      }
+    }
+    __syncwarp();                                      // the values are used up
+    if (chunk + 4 < end) bring(values_at, a.v_cache, vdim, value_width, row);
+    cp_async_commit_group();
+  }
+  cp_async_wait_groups<0>();
+  if (bad_page) atomicOr(a.status, kStatusBadPage);
+  __syncthreads();                                     // everyone is done with the tiles: their place takes the warps' results
+  float* found = reinterpret_cast<float*>(mix_smem + kSingleQ);       // [warp, head, value column]
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const int h = g + 8 * half;
+    float sum = l[half];
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    if (q2 == 0) {
+      warp_m[warp][h] = m[half];
+      warp_l[warp][h] = sum;
+    }
+    float* to = found + (warp * kSingleHeads + h) * kSingleOPitch + q2;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) *reinterpret_cast<float2*>(to + 8 * j) = make_float2(O[j][2 * half], O[j][2 * half + 1]);
+  }
+  __syncthreads();
+  const int outs = heads * vdim;
+  const size_t part = ((size_t)blockIdx.y * s.num_tokens + t);
+  for (int o = threadIdx.x; o < outs; o += kMixThreads) {
+    const int h = o / vdim, d = o - h * vdim, column = (h / per) * vdim + d;
+    const bool whole = s.splits == 1;
+    float best = whole && a.sink ? a.sink[h] * 1.4426950408889634f : -INFINITY;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) best = fmaxf(best, warp_m[w][h]);
+    float sum = whole && a.sink ? exp2f(a.sink[h] * 1.4426950408889634f - best) : 0.f, value = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const float factor = warp_m[w][h] == -INFINITY ? 0.f : exp2f(warp_m[w][h] - best);
+      sum = fmaf(warp_l[w][h], factor, sum);
+      value = fmaf(found[(w * kSingleHeads + h) * kSingleOPitch + column], factor, value);
+    }
+    if (whole) {
+      a.out[(size_t)t * outs + o] = __float2bfloat16_rn(sum > 0.f ? value / sum * a.out_scale : 0.f);
+    } else {
+      s.part_acc[part * outs + o] = value;
+      if (d == 0) *reinterpret_cast<float2*>(s.part_ml + (part * heads + h) * 2) = make_float2(best, sum);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kMixThreads) mixed_single_join_kernel(const __grid_constant__ SingleArgs s) {
+  const MixArgs& a = s.m;
+  pdl_launch_dependents();
+  const int outs = a.heads * a.vdim, o = (int)blockIdx.y * kMixThreads + (int)threadIdx.x;
+  const int t = s.tokens ? s.tokens[blockIdx.x] : (int)blockIdx.x;
+  pdl_wait();
+  if (o >= outs) return;
+  const int h = o / a.vdim;
+  const size_t ml_step = (size_t)s.num_tokens * a.heads, acc_step = (size_t)s.num_tokens * outs;
+  const float2* ml = reinterpret_cast<const float2*>(s.part_ml) + (size_t)t * a.heads + h;
+  const float* acc = s.part_acc + (size_t)t * outs + o;
+  constexpr int kBatch = 8;                            // loads in flight before they are used
+  float best = a.sink ? a.sink[h] * 1.4426950408889634f : -INFINITY;
+  float sum = a.sink ? 1.f : 0.f, value = 0.f;
+  for (int s0 = 0; s0 < s.splits; s0 += kBatch) {
+    float2 of[kBatch];
+    float v[kBatch];
+    float to = best;
+#pragma unroll
+    for (int e = 0; e < kBatch; ++e) {
+      const bool there = s0 + e < s.splits;
+      of[e] = there ? ml[(s0 + e) * ml_step] : make_float2(-INFINITY, 0.f);
+      v[e] = there ? acc[(s0 + e) * acc_step] : 0.f;
+      to = fmaxf(to, of[e].x);
+    }
+    const float factor = best == -INFINITY ? 0.f : exp2f(best - to);
+    sum *= factor;
+    value *= factor;
+    best = to;
+#pragma unroll
+    for (int e = 0; e < kBatch; ++e) {
+      const float w = of[e].x == -INFINITY ? 0.f : exp2f(of[e].x - best);
+      sum = fmaf(of[e].y, w, sum);
+      value = fmaf(v[e], w, value);
+    }
+  }
+  a.out[(size_t)t * outs + o] = __float2bfloat16_rn(sum > 0.f ? value / sum * a.out_scale : 0.f);
+}
+
 template <int VALUE>
 static cudaError_t launch_mixed_prompt(const MixArgs& a, int num_tiles, cudaStream_t stream) {
   auto kernel = mixed_prompt_attention_kernel<VALUE>;
@@ -350,4 +641,37 @@ extern "C" int einf_mixed_prompt_attention(const void* q, const void* k_cache, c
   a.window = window; a.wave = wave;
   a.scale_log2 = scale * 1.4426950408889634f; a.out_scale = out_scale;
   return (int)(vdim <= 64 ? launch_mixed_prompt<64>(a, num_tiles, stream) : launch_mixed_prompt<128>(a, num_tiles, stream));
+}
+
+// One token each of `num_items` requests (`items`: token indices, null: tokens 0 .. num_items - 1); `splits` CTAs share a
+// token's keys and, above one, need part_acc [splits, num_tokens, heads * vdim] and part_ml [splits, num_tokens, heads, 2].
+extern "C" int einf_mixed_single_attention(const void* q, const void* k_cache, const void* v_cache, const int* block_table,
+                                           int table_width, const int* seq_of_token, const int* positions, const int* items,
+                                           int num_items, void* out, int num_tokens, int heads, int kv_heads, int dim, int vdim,
+                                           int page_size, int num_pages, float scale, int window, const float* slopes,
+                                           const float* talk, const float* sink, float out_scale, int splits, float* part_acc,
+                                           float* part_ml, int* status, cudaStream_t stream) {
+  if (num_items == 0) return 0;
+  if (heads <= 0 || heads > kSingleHeads || kv_heads <= 0 || heads % kv_heads || dim <= 0 || dim % 8 ||
+      kv_heads * dim > kMixKeySize || vdim <= 0 || vdim % 8 || kv_heads * vdim > 128 || splits < 1 || splits > 65535 ||
+      (splits > 1 && (!part_acc || !part_ml)) || (long long)num_pages * kv_heads * page_size > 0x7fffffff ||
+      (((uintptr_t)k_cache | (uintptr_t)v_cache) & 15) || ((uintptr_t)q & 3) || ((uintptr_t)part_ml & 7))
+    return (int)cudaErrorInvalidValue;
+  SingleArgs s;
+  MixArgs& a = s.m;
+  a.q = (const __nv_bfloat16*)q;
+  a.k_cache = (const __nv_bfloat16*)k_cache; a.v_cache = (const __nv_bfloat16*)v_cache;
+  a.block_table = block_table; a.table_width = table_width; a.tiles = nullptr; a.out = (__nv_bfloat16*)out;
+  a.slopes = slopes; a.talk = talk; a.sink = sink; a.status = status;
+  a.heads = heads; a.kv_heads = kv_heads; a.dim = dim; a.vdim = vdim; a.page_size = page_size; a.num_pages = num_pages;
+  a.window = window; a.wave = 0;
+  a.scale_log2 = scale * 1.4426950408889634f; a.out_scale = out_scale;
+  s.seq_of_token = seq_of_token; s.positions = positions; s.tokens = items;
+  s.splits = splits; s.num_tokens = num_tokens; s.part_acc = part_acc; s.part_ml = part_ml;
+  cudaError_t e = cudaFuncSetAttribute(mixed_single_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSingleSmem);
+  if (e != cudaSuccess) return (int)e;
+  e = launch_pdl(mixed_single_attention_kernel, dim3(num_items, splits), dim3(kMixThreads), kSingleSmem, stream, s);
+  if (e != cudaSuccess || splits == 1) return (int)e;
+  return (int)launch_pdl(mixed_single_join_kernel, dim3(num_items, (heads * vdim + kMixThreads - 1) / kMixThreads),
+                         dim3(kMixThreads), 0, stream, s);
 }

@@ -2354,6 +2354,30 @@ def mixed_prompt_takes(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
     )
 
 
+def mixed_single_takes(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor) -> bool:
+    """Whether single tokens run with the mixing in the queries and their heads as the rows of a product: bfloat16, up to 16
+    heads, a token's key heads and its value heads of together up to 128 elements each, in multiples of eight."""
+    heads, dim, kv_heads, value_size = q.shape[1], q.shape[2], k_cache.shape[1], v_cache.shape[3]
+    return (
+        q.dtype == torch.bfloat16 and heads <= 16 and dim % 8 == 0 and value_size % 8 == 0
+        and kv_heads * max(dim, value_size) <= MIXED_PROMPT_KEYS
+        and q.data_ptr() % 4 == 0 and all(t.data_ptr() % 16 == 0 for t in (k_cache, v_cache))
+        and k_cache.shape[0] * kv_heads * k_cache.shape[2] <= 0x7fffffff
+    )
+
+
+def _mixed_split_scratch(device, need: int):
+    # Buffers by power-of-two size and never given back: a captured graph keeps the address it saw.
+    bucket = max(1 << 16, 1 << (need - 1).bit_length())
+    key = (str(device), bucket)
+    scratch = _mixed_join_scratch.get(key)
+    if scratch is None:
+        scratch = (torch.empty(bucket, dtype=torch.float32, device=device),
+                   torch.empty(2 * bucket, dtype=torch.float32, device=device))
+        _mixed_join_scratch[key] = scratch
+    return scratch
+
+
 def _mixed_tiled(q, k_cache, v_cache, block_table, seq_of_token, positions, out, scale, window, slopes, talk, sink,
                  out_scale, status, q_tiles, single_tokens, num_singles, max_context) -> bool:
     tokens, heads, key_size = q.shape
@@ -2363,12 +2387,13 @@ def _mixed_tiled(q, k_cache, v_cache, block_table, seq_of_token, positions, out,
     if q_tiles.dtype != torch.int32 or q_tiles.dim() != 2 or q_tiles.shape[1] != 4:
         raise ValueError("q_tiles must be int32 [tiles, 4]")
     launches = []
-    if num_singles:
+    by_rows = num_singles and mixed_single_takes(q, k_cache, v_cache)
+    if num_singles and not by_rows:
         launches.append((single_tokens, num_singles, 1, mixed_tiled_rows(heads, kv_heads, key_size, value_size, True, q.dtype)))
     by_heads = num_tiles and mixed_prompt_takes(q, k_cache, v_cache, out, num_tiles, window, max_context)
     if num_tiles and not by_heads:
         launches.append((q_tiles, num_tiles, 0, mixed_tiled_rows(heads, kv_heads, key_size, value_size, False, q.dtype)))
-    if not (launches or by_heads) or any(rows == 0 for _, _, _, rows in launches):
+    if not (launches or by_heads or by_rows) or any(rows == 0 for _, _, _, rows in launches):
         return False
     if by_heads:
         fn = _fn(
@@ -2384,8 +2409,33 @@ def _mixed_tiled(q, k_cache, v_cache, block_table, seq_of_token, positions, out,
                _opt(sink, "sink", torch.float32), float(out_scale), _sm_count(), _dev(status, "status"), _stream()),
             "mixed_prompt_attention",
         )
-        if not launches:
-            return True
+    global launch_count
+    if by_rows:
+        splits = mixed_tiled_splits(num_singles, 1, window, max_context)
+        part_acc = part_ml = None
+        if splits > 1:
+            part_acc, part_ml = _mixed_split_scratch(q.device, splits * tokens * heads * value_size)
+        fn = _fn(
+            "einf_mixed_single_attention",
+            [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
+             c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p, c_float, c_int, c_void_p, c_void_p,
+             c_void_p, c_void_p],
+        )
+        _check(
+            fn(_dev(q, "q"), _dev(k_cache, "k_cache"), _dev(v_cache, "v_cache"),
+               _opt(block_table, "block_table", torch.int32), block_table.shape[1],
+               _opt(seq_of_token, "seq_of_token", torch.int32), _opt(positions, "positions", torch.int32),
+               _opt(single_tokens, "single_tokens", torch.int32), num_singles, _dev(out, "out"), tokens, heads, kv_heads,
+               key_size, value_size, page_size, num_pages, float(scale), int(window or 0),
+               _opt(slopes, "slopes", torch.float32), _opt(talk, "talk", torch.float32), _opt(sink, "sink", torch.float32),
+               float(out_scale), splits, _opt(part_acc, "part_acc", torch.float32), _opt(part_ml, "part_ml", torch.float32),
+               _dev(status, "status"), _stream()),
+            "mixed_single_attention",
+        )
+        if splits > 1:
+            launch_count += 1      # the kernel that joins the splits
+    if not launches:
+        return True
     variant = mixed_tiled_variant(heads)
     fn = _fn(
         "einf_paged_attention_mixed_tiled",
@@ -2394,7 +2444,6 @@ def _mixed_tiled(q, k_cache, v_cache, block_table, seq_of_token, positions, out,
          c_void_p, c_void_p, c_void_p, c_void_p],
         variant,
     )
-    global launch_count
     for items, count, single, rows in launches:
         per_sm = 2
         if not single and q.dtype == torch.bfloat16:      # the tensor-core kernel runs one or two CTAs an SM
@@ -2403,16 +2452,7 @@ def _mixed_tiled(q, k_cache, v_cache, block_table, seq_of_token, positions, out,
         splits = mixed_tiled_splits(count * (1 if single else -(-128 // rows)), rows, window, max_context, per_sm)
         part_acc = part_ml = None
         if splits > 1:
-            # Buffers by power-of-two size and never given back: a captured graph keeps the address it saw.
-            need = splits * tokens * heads * value_size
-            bucket = max(1 << 16, 1 << (need - 1).bit_length())
-            key = (str(q.device), bucket)
-            scratch = _mixed_join_scratch.get(key)
-            if scratch is None:
-                scratch = (torch.empty(bucket, dtype=torch.float32, device=q.device),
-                           torch.empty(2 * bucket, dtype=torch.float32, device=q.device))
-                _mixed_join_scratch[key] = scratch
-            part_acc, part_ml = scratch
+            part_acc, part_ml = _mixed_split_scratch(q.device, splits * tokens * heads * value_size)
         _check(
             fn(_dev(q, "q"), _dev(k_cache, "k_cache"), _dev(v_cache, "v_cache"), _code(q),
                _opt(block_table, "block_table", torch.int32), block_table.shape[1],

@@ -65,6 +65,7 @@ LAUNCHERS = {
     "einf_paged_attention_mixed_tiled_rows": "attention_mixed_tiled",
     "einf_paged_attention_mixed_mma_ctas": "attention_mixed_tiled",
     "einf_mixed_prompt_attention": "attention_mixed_mma",
+    "einf_mixed_single_attention": "attention_mixed_mma",
     "einf_gated_scan": "recurrence",
     "einf_memory_gates": "recurrence",
     "einf_memory_output": "recurrence",

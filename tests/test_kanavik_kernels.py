@@ -133,6 +133,50 @@ def test_mixing_in_the_queries(dev, heads, kv_heads, size, vsize, window, parts)
         first += n
 
 
+@pytest.mark.parametrize("heads, kv_heads, size, vsize, window", [
+    (14, 2, 64, 64, 100), (16, 1, 128, 128, None), (5, 1, 8, 24, 33), (4, 4, 32, 16, 1), (6, 3, 40, 40, None),
+])
+@pytest.mark.parametrize("parts, splits", [("all", 1), ("all", 3), ("no slopes", 40), ("no mixing", 1)])
+def test_single_tokens_with_their_heads_as_rows(dev, heads, kv_heads, size, vsize, window, parts, splits, monkeypatch):
+    """Contexts around the chunks of 32 keys, CTAs without a key among those that share a token's, a list of tokens in an
+    order of its own."""
+    from einf_b200 import ops
+
+    requests = [(0, 1), (30, 1), (31, 1), (32, 1), (600, 1), (129, 1)]
+    (q, k, v, table, seq, pos), scale, window = _attention_case(dev, torch.bfloat16, heads, kv_heads, size, 16, requests, window)
+    generator = torch.Generator().manual_seed(12)
+    v = torch.randn((*v.shape[:3], vsize), generator=generator).to(torch.bfloat16).to(dev)
+    slopes, talk, sink = _mixing(heads, generator, dev)
+    slopes, talk = None if parts == "no slopes" else slopes, None if parts == "no mixing" else talk
+    assert ops.mixed_single_takes(q, k, v)
+    monkeypatch.setattr(ops, "mixed_tiled_splits", lambda *_: splits)
+    singles = torch.tensor([4, 0, 3, 1, 5], dtype=torch.int32, device=dev)
+    out = torch.full((q.shape[0], heads, vsize), float("nan"), dtype=torch.bfloat16, device=dev)
+    st = status(dev)
+    ops.paged_attention_mixed(q, k, v, table, seq, pos, out, scale, window, slopes, talk, sink, 0.7, st,
+                              q_tiles=torch.empty((0, 4), dtype=torch.int32, device=dev), single_tokens=singles,
+                              num_singles=5, max_context=601)
+    assert int(st) == 0 and bool(out[2].isnan().all())
+    group = torch.arange(heads, device=dev) // (heads // kv_heads)
+    for t in singles.tolist():
+        end = requests[t][0] + 1
+        pages = table[t, :-(-end // 16)].long().clamp(min=0)
+        keys = k[pages].transpose(1, 2).reshape(-1, kv_heads, size)[:end].double()[:, group]
+        values = v[pages].transpose(1, 2).reshape(-1, kv_heads, vsize)[:end].double()[:, group]
+        away = end - 1 - torch.arange(end, device=dev)
+        raw = torch.einsum("hd,jhd->hj", q[t].double(), keys) * scale
+        if slopes is not None:
+            raw = raw - slopes.double()[:, None] * away
+        if talk is not None:
+            raw = talk.double() @ raw
+        if window is not None:
+            raw = raw.masked_fill(away >= window, float("-inf"))
+        weights = torch.softmax(torch.cat([raw, sink.double()[:, None]], dim=1), dim=1)[:, :-1]
+        want = 0.7 * torch.einsum("hj,jhv->hv", weights, values)
+        # the output's rounding, 2^-9 of an element; weights of two bfloat16 parts and 32-bit sums: far below
+        assert bool(((out[t].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-4).all())
+
+
 @pytest.mark.parametrize("batch, context, window", [(1, 3000, None), (3, 1500, 1024), (64, 300, 128), (2, 40, 64)])
 def test_tiled_score_mixing_decode_splits_its_keys(dev, batch, context, window):
     """Single tokens with long contexts: the keys of a token are split over CTAs and joined with the sink."""
