@@ -272,9 +272,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 // out[r] = W[g] x[r] for offsets[g] <= r < offsets[g + 1], W stacked [groups, n, k].  The grid's y
 // dimension is a list of token tiles that never cross a group: tile slot y belongs to the group
 // and the place that a walk over the offsets gives it (slots beyond the last tile leave at once),
-// so the host never has to know how many rows a group got.  A tile's box of x may reach into the
-// next group's rows (or past the end, where TMA fills zeros): those columns of the accumulator are
-// computed and not stored.  With `splits` > 1 (grid z) the CTAs of a tile each take a K range and write
+// so the host never has to know how many rows a group got.  A tile's boxes of x may reach into the
+// next group's rows (or past the end, where TMA fills zeros): columns of the accumulator from the tile's rows on are at most
+// 15, and not stored.  With `splits` > 1 (grid z) the CTAs of a tile each take a K range and write
 // 32-bit partial sums [splits, rows, n] that the consumer adds up in order (a matrix with few row
 // tiles and a handful of rows per group would otherwise run on a third of the GPU).
 // ---------------------------------------------------------------------------
@@ -285,19 +285,23 @@ struct GroupedParams {
   int* status;
   int rows, n, k, groups;
   int token_tile;
+  int box;                // rows of x a load brings
   int stages;
   int out_dtype;
 };
 
+// A group's tiles are of one size, as near as multiples of 16 allow: 520 rows are three tiles of 176, not two of 256 and one
+// of 8, which would read the whole weight tile for its 8 rows.
 __device__ __forceinline__ bool find_group_tile(const GroupedParams& p, int slot, int* group, int* t0, int* valid) {
   for (int g = 0; g < p.groups; ++g) {
     const int begin = p.offsets[g], count = p.offsets[g + 1] - begin;
     const int tiles = (count + p.token_tile - 1) / p.token_tile;
     if (slot < tiles) {
+      const int each = min(p.token_tile, ((count + tiles - 1) / tiles + 15) / 16 * 16);
       *group = g;
-      *t0 = begin + slot * p.token_tile;
-      *valid = min(p.token_tile, count - slot * p.token_tile);
-      return true;
+      *t0 = begin + slot * each;
+      *valid = min(each, count - slot * each);
+      return *valid > 0;
     }
     slot -= tiles;
   }
@@ -353,6 +357,9 @@ gemm_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __g
   int group = 0, t0 = 0, valid = 0;
   const bool have = find_group_tile(p, blockIdx.y, &group, &t0, &valid);
 
+  const int boxes = (valid + p.box - 1) / p.box;       // of x: the rows of this tile alone
+  const int load_bytes = kWTileBytes + boxes * p.box * kBlockK * 2;
+
   if (have && warp == 0) {
     if (lane == 0) {
       bool ok = true;
@@ -360,14 +367,17 @@ gemm_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __g
         const int s = i % p.stages;
         if (i >= p.stages) ok = mbar_wait(empty_bar(s), ((i / p.stages) & 1) ^ 1, p.status);
         if (!ok) break;
-        mbar_expect_tx(full_bar(s), stage_bytes);
+        mbar_expect_tx(full_bar(s), load_bytes);
         tma_load_2d(smem_base + s * stage_bytes, &map_w, (kb_begin + i) * kBlockK, group * p.n + n0, full_bar(s));
-        tma_load_2d(smem_base + s * stage_bytes + kWTileBytes, &map_x, (kb_begin + i) * kBlockK, t0, full_bar(s));
+        for (int b = 0; b < boxes; ++b)
+          tma_load_2d(smem_base + s * stage_bytes + kWTileBytes + b * p.box * kBlockK * 2, &map_x, (kb_begin + i) * kBlockK,
+                      t0 + b * p.box, full_bar(s));
       }
     }
   } else if (have && warp == 1) {
     if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.token_tile >> 3) << 17) |
+      const int columns = (valid + 15) / 16 * 16;      // the products' N: this tile's rows
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(columns >> 3) << 17) |
                              ((uint32_t)(kBlockW >> 4) << 24);
       bool ok = true;
       for (int i = 0; i < num_kblocks && ok; ++i) {
@@ -528,13 +538,16 @@ extern "C" int einf_gemm_tcgen05_splits(int k, int splits) {
   return (total_kblocks + per_split - 1) / per_split;
 }
 
-// The token tile of the grouped product for `rows` rows over `groups` groups: about one and a half
-// times the average rows of a group, a multiple of 16 between 16 and 128 (at 128 two CTAs share an
-// SM, so that one's epilogue runs beside the other's products).
+// The largest token tile of the grouped product for `rows` rows over `groups` groups: about one and a half times the average
+// rows of a group, a multiple of 16 between 16 and 128, above that 192 or 256.  The CTAs' reads of W and x out of L2 bound
+// the product at many rows (2.6 GB at tiles of 128 for the sizes below, 2 GB at 256), so a
+// weight tile meets as many rows as its accumulator holds with two CTAs an SM, one's epilogue beside the other's products.
+// Measured (B200): both products of 4,096 rows on eight experts, n and k of 17,920 and 1,536 and of 1,536 and 8,960:
+// 218 -> 182 us.
 extern "C" int einf_gemm_grouped_tcgen05_token_tile(int rows, int groups) {
   const int average = (rows + groups - 1) / (groups > 0 ? groups : 1);
-  int tile = (average * 3 / 2 + 15) / 16 * 16;
-  return tile < 16 ? 16 : (tile > 128 ? 128 : tile);
+  const int tile = (average * 3 / 2 + 15) / 16 * 16;
+  return tile < 16 ? 16 : (tile <= 128 ? tile : (tile <= 192 ? 192 : 256));
 }
 
 // x: [rows, k] bfloat16 contiguous, sorted by group; w: [groups, n, k] bfloat16 contiguous; offsets: [groups + 1]
@@ -549,12 +562,12 @@ extern "C" int einf_gemm_grouped_tcgen05(const void* x, const void* w, const int
   if (splits != einf_gemm_tcgen05_splits(k, splits)) return (int)cudaErrorInvalidValue;   // the caller sized out for it
   const int per_split = (total_kblocks + splits - 1) / splits;
   int stages = per_split < kMaxStages ? per_split : kMaxStages;
-  while (stages > 3 && smem_bytes(token_tile, stages) > 110 * 1024) --stages;
-  while (stages > 1 && smem_bytes(token_tile, stages) > 200 * 1024) --stages;
+  while (stages > 2 && smem_bytes(token_tile, stages) > 110 * 1024) --stages;      // two CTAs an SM
   CUtensorMap map_w, map_x;
   int rc = make_map(&map_w, w, (long long)groups * n, k, k, kBlockW);
   if (rc) return rc;
-  rc = make_map(&map_x, x, rows, k, k, token_tile);
+  const int box = token_tile <= 128 ? token_tile : 64;
+  rc = make_map(&map_x, x, rows, k, k, box);
   if (rc) return rc;
   GroupedParams p;
   p.out = out;
@@ -565,6 +578,7 @@ extern "C" int einf_gemm_grouped_tcgen05(const void* x, const void* w, const int
   p.k = k;
   p.groups = groups;
   p.token_tile = token_tile;
+  p.box = box;
   p.stages = stages;
   p.out_dtype = out_dtype;
   p.kblocks_per_split = per_split;

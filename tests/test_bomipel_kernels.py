@@ -284,6 +284,26 @@ def test_routed_feed_forward_steps(dev, dtype, tokens, hidden, inter, experts, t
         close(got, want, got.dtype if got.dtype == torch.bfloat16 else (torch.float32 if dtype == torch.float32 else torch.bfloat16))
 
 
+@pytest.mark.parametrize("counts", [(520, 1, 0, 256), (513, 257, 16, 17), (300, 90), (176, 177), (129, 255, 3)])
+def test_grouped_product_in_tiles_of_one_size(dev, counts):
+    """Groups above the largest tile (cut evenly), below one box of loads, empty; rows of another group behind every tile."""
+    from einf_b200 import ops
+
+    generator = torch.Generator().manual_seed(sum(counts))
+    rows, n, k = sum(counts), 136, 200
+    x = torch.randn((rows, k), generator=generator).to(torch.bfloat16).to(dev)
+    weight = (torch.randn((len(counts), n, k), generator=generator) * k ** -0.5).to(torch.bfloat16).to(dev)
+    offsets = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32, device=dev)
+    st = torch.zeros(1, dtype=torch.int32, device=dev)
+    out = torch.full((rows, n), float("nan"), dtype=torch.float32, device=dev)
+    ops.moe_gemm(x, weight, offsets, out, st)
+    assert int(st) == 0
+    for g in range(len(counts)):
+        part = slice(int(offsets[g]), int(offsets[g + 1]))
+        # exact products, 32-bit sums of 200 terms of a total of about one
+        torch.testing.assert_close(out[part].double(), x[part].double() @ weight[g].double().T, rtol=1e-5, atol=2e-5)
+
+
 def test_softcap(dev):
     from einf_b200 import ops
 
