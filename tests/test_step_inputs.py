@@ -7,6 +7,7 @@ figures that launches are sized from.
 """
 import random
 
+import numpy as np
 import pytest
 import torch
 
@@ -170,3 +171,32 @@ def test_the_decode_attention_cuts_the_keys_by_an_estimate_of_each_shape():
                 cluster, splits = plan(tokens, heads, kv_heads, size, context)
                 pairs = tokens * kv_heads
                 assert cluster == 1 and splits == 1 or pairs * splits <= held[size][cluster]
+
+
+@pytest.mark.parametrize("kind", ["list", "tuple", "numpy", "numpy elements", "floats", "strings", "mixed", "iterators"])
+def test_request_like_objects_may_hold_numbers_of_any_kind(kind):
+    """Lists of ints are converted by the binding, everything else as int() takes it."""
+    from types import SimpleNamespace
+
+    from einf_b200.engine.batch import as_plan
+
+    make = {
+        "list": list, "tuple": tuple, "numpy": np.array, "numpy elements": lambda v: [np.int32(x) for x in v],
+        "floats": lambda v: [float(x) for x in v], "strings": lambda v: [str(x) for x in v],
+        "mixed": lambda v: [True if x == 1 else x for x in v], "iterators": iter,
+    }[kind]
+    tokens, tables = [7, 1, -3], [[5, 2 ** 31 - 1], [1, 0, 4]]
+    plan = as_plan([SimpleNamespace(input_token_ids=make(tokens), start_position=2, block_tables=[make(t) for t in tables])])
+    request = plan.requests[0]
+    assert list(request.input_token_ids) == tokens and [list(t) for t in request.block_tables] == tables
+    assert request.start_position == 2 and request.request_id == "0" and request.state_slot == -1
+
+
+def test_request_like_objects_with_numbers_beyond_32_bits_are_refused():
+    from types import SimpleNamespace
+
+    from einf_b200.engine.batch import as_plan
+
+    for tokens, table in (([2 ** 31], [1]), ([1], [2 ** 40]), ([1], [2 ** 70])):
+        with pytest.raises(TypeError):
+            as_plan([SimpleNamespace(input_token_ids=tokens, start_position=0, block_tables=[table])])
