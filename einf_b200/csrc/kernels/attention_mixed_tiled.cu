@@ -10,7 +10,8 @@
 // shared memory and every warp adds its tasks' weighted values into registers, a lane per value column.
 // Scores, weights, sums and the output are 32-bit.  With several splits (grid.y) each CTA takes a share
 // of the key tiles and leaves (maximum, sum, unnormalised output); a second kernel joins them and the
-// sink.  Queries that come alone (decoding) use the same kernel with one query a task.
+// sink.  Queries that come alone (decoding) use the same kernel with one query a task.  What bfloat16 allows goes to
+// attention_mixed_mma.cu instead: single tokens of up to 16 heads, prompt portions of many CTAs.
 // Compiled per HEADS_PAD (4, 8, 16 or 32 >= heads).
 #include "common.cuh"
 

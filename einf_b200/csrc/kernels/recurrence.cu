@@ -5,7 +5,8 @@
 // (state[slot * row_stride + ...]); a request without a slot (-1: padding of a decode graph) reads
 // zeros and writes nothing.  The step's tokens are packed request by request, q_start[r] ..
 // q_start[r + 1], so a prompt portion and a single decoded token take the same code and the same
-// order of additions: what a position computes does not depend on how the prompt was cut.
+// order of additions: what a position computes does not depend on how the prompt was cut.  (bfloat16 portions of 24 tokens
+// and more take recurrence_chunks.cu, which sums a chunk's tokens in another order.)
 #include <type_traits>
 
 #include "conv_run.cuh"
