@@ -25,7 +25,7 @@
 // A row's result depends on that row, its expert and its weight alone: which other tokens share
 // the batch moves nothing.  (The place of a row inside its expert's range is first come, first
 // served; no value depends on it.)
-#include "common.cuh"
+#include "conv_run.cuh"
 
 namespace einf {
 
@@ -423,6 +423,53 @@ moe_combine_kernel(const TY* __restrict__ y, const int* __restrict__ expert_ids,
   }
 }
 
+// The same for hundreds of tokens, rows that come whole (no partial sums) and experts that all compute: four neighbouring
+// columns a thread, the rows of four choices in flight together, added in the same order.
+template <typename TY, typename TA>
+__global__ void __launch_bounds__(128)
+moe_combine_quads_kernel(const TY* __restrict__ y, const int* __restrict__ expert_ids, const int* __restrict__ place,
+                         const float* __restrict__ weights, int scale_outputs, const TA* __restrict__ addend,
+                         float* __restrict__ out, int num_experts, int top_k, int hidden,
+                         const float* __restrict__ gate_logits, int gate_width, int gate_column, int gate_splits,
+                         size_t gate_stride) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.y, d = 4 * (int)(blockIdx.x * 128 + threadIdx.x);
+  if (d >= hidden) return;
+  float4 v = addend ? load_quad(addend + (size_t)t * hidden + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+  if (gate_logits) {
+    const float z = sum_strided(gate_logits + (size_t)t * gate_width + gate_column, gate_splits, gate_stride);
+    const float open = 1.f / (1.f + expf(-z));
+    v.x *= open; v.y *= open; v.z *= open; v.w *= open;
+  }
+  constexpr int kBatch = 4;
+  for (int j0 = 0; j0 < top_k; j0 += kBatch) {
+    int row[kBatch];
+    float w[kBatch];
+    float4 term[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int p = t * top_k + j0 + u;
+      const int e = j0 + u < top_k ? expert_ids[p] : -1;
+      row[u] = e >= 0 && e < num_experts ? place[p] : -1;
+      w[u] = scale_outputs && row[u] >= 0 ? weights[p] : 1.f;
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u)
+      if (row[u] >= 0) term[u] = load_quad(y + (size_t)row[u] * hidden + d);
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      if (row[u] < 0) continue;
+      if (scale_outputs) {
+        v.x += w[u] * term[u].x; v.y += w[u] * term[u].y; v.z += w[u] * term[u].z; v.w += w[u] * term[u].w;
+      } else {
+        v.x += term[u].x; v.y += term[u].y; v.z += term[u].z; v.w += term[u].w;
+      }
+    }
+  }
+  store_quad(out + (size_t)t * hidden + d, v);
+}
+
 }  // namespace einf
 
 using namespace einf;
@@ -503,6 +550,19 @@ extern "C" int einf_moe_combine(const void* y, int y_dtype, const int* expert_id
   if (num_identity < 0 || (num_identity > 0 && (!identity_x || !weights))) return (int)cudaErrorInvalidValue;
   if (gate_logits && (!addend || gate_column < 0 || gate_column >= gate_width)) return (int)cudaErrorInvalidValue;
   const bool many = num_tokens >= 128;
+  // groups of four aligned columns: 2,048 tokens of 1,536 with two experts each 24 -> 9 us
+  const size_t y_quad = y_dtype == kFloat32 ? 16 : 8, addend_quad = addend_dtype == kFloat32 ? 16 : 8;
+  if (many && y_splits <= 1 && num_identity == 0 && (!addend || splits <= 1) && hidden % 4 == 0 && (uintptr_t)y % y_quad == 0 &&
+      (uintptr_t)addend % addend_quad == 0 && (uintptr_t)out % 16 == 0) {
+    EINF_DISPATCH_2(y_dtype, TY, {
+      EINF_DISPATCH_2(addend_dtype, TA, {
+        return (int)launch_pdl(moe_combine_quads_kernel<TY, TA>, dim3((hidden + 511) / 512, num_tokens), dim3(128), 0, stream,
+                               (const TY*)y, expert_ids, place, weights, scale_outputs, (const TA*)addend, out, num_experts,
+                               top_k, hidden, gate_logits, gate_width, gate_column, gate_splits < 1 ? 1 : gate_splits,
+                               (size_t)gate_stride);
+      })
+    })
+  }
   const dim3 grid(many ? (hidden + 511) / 512 : (hidden + 127) / 128, num_tokens);
   EINF_DISPATCH_2(y_dtype, TY, {
     EINF_DISPATCH_2(addend_dtype, TA, {

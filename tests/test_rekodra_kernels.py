@@ -313,3 +313,32 @@ def test_tensor_core_attention_with_a_sink(dev, heads, kv_heads, size, page_size
         assert int(st) == 0
         rows = singles.long().to(dev)
         torch.testing.assert_close(out[rows], want[rows], **tol(dtype))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("tokens, hidden, top, addend, gated", [
+    (128, 4, 1, None, False), (130, 516, 2, torch.bfloat16, False), (200, 520, 5, torch.float32, True), (129, 1028, 9, None, False),
+])
+@pytest.mark.parametrize("scale", [True, False])
+def test_combine_four_columns_a_thread(dev, dtype, tokens, hidden, top, addend, gated, scale):
+    """More choices than are in flight together, choices of no expert, columns that do not fill a CTA: the sums in order."""
+    from einf_b200 import ops
+
+    generator = torch.Generator().manual_seed(hidden)
+    experts = 12
+    ids = torch.stack([torch.randperm(experts + 1, generator=generator)[:top] for _ in range(tokens)])   # `experts`: none
+    place = torch.randperm(tokens * top, generator=generator).view(tokens, top)
+    y = torch.randn((tokens * top, hidden), generator=generator).to(dtype)
+    weights = torch.rand((tokens, top), generator=generator)
+    more = None if addend is None else torch.randn((tokens, hidden), generator=generator).to(addend)
+    logits = torch.randn((tokens, 3), generator=generator)
+    out = torch.full((tokens, hidden), float("nan"), device=dev)
+    ops.moe_combine(y.to(dev), ids.to(torch.int32).to(dev), place.to(torch.int32).to(dev), weights.to(dev), scale,
+                    None if more is None else more.to(dev), out, experts, addend_gate=(logits.to(dev), 1) if gated else None)
+    want = torch.zeros((tokens, hidden), dtype=torch.float64) if more is None else more.double()
+    if gated:
+        want = want * torch.sigmoid(logits[:, 1:2].double())
+    for j in range(top):
+        there = (ids[:, j] < experts).double()[:, None]
+        want = want + there * (weights[:, j:j + 1].double() if scale else 1.0) * y[place[:, j]].double()
+    torch.testing.assert_close(out.cpu().double(), want, rtol=1e-6, atol=1e-5)      # ten terms, sums up to 15: 10 x 15 x 2^-24
