@@ -196,7 +196,8 @@ class LatentAttention(Mixer):
         return min(context, self.window) if self.window else context
 
     def launch_group(self):
-        return ("latent_attention", self.num_heads, self.row, self.fast, self.window)
+        # kv_rank: the splits of single tokens go by it; by_heads: so do the kernels of prompts
+        return ("latent_attention", self.num_heads, self.row, self.kv_rank, self.fast, self.window, self.by_heads)
 
     def cache_need(self):
         # the values are the first kv_rank elements of the rows: no value cache of its own

@@ -359,6 +359,50 @@ def test_the_engines_frequency_table(dims, base, scaling):
     assert part.amplitude == pytest.approx(amplitude)
 
 
+@pytest.mark.parametrize("first, second", [(dict(dim=256), dict(dim=128)), (dict(rank=512), dict(rank=504)), (dict(rot=60), dict(rot=64)),
+                                           (dict(value=128), dict(value=136))])
+@pytest.mark.parametrize("turned", [False, True])
+def test_latent_layers_that_launch_by_one_key_agree_on_it(first, second, turned, monkeypatch):
+    """The runner asks one part of every launch group for its key, so layers of one group must answer alike for every
+    step; here layers of which only one can run fresh prompts head by head, or whose latents differ in size, in either order."""
+    from types import SimpleNamespace
+
+    from einf_b200 import ops
+    from einf_b200.config.specs import PartSpec
+    from einf_b200.parts.base import Runtime, build_part
+
+    monkeypatch.setattr(ops, "_sm_count", lambda: 148)
+
+    def part(dim=128, rank=512, rot=64, value=128, heads=2, hidden=64):
+        spec = PartSpec("latent_attention", {
+            "hidden_size": hidden, "num_heads": heads, "head_size": dim, "rotary_size": rot, "value_head_size": value,
+            "q_rank": 0, "kv_rank": rank, "scale": 0.1, "window": None, "eps": 1e-6,
+            "position": PartSpec("rope", {"rotary_dim": rot, "theta": 1e4})})
+        draw = lambda *shape: torch.zeros(shape, dtype=torch.bfloat16)  # noqa: E731
+        tensors = {"q_proj.weight": draw(heads * (dim + rot), hidden), "kv_down.weight": draw(rank + rot, hidden),
+                   "kv_norm.weight": draw(rank), "k_up.weight": draw(heads * dim, rank),
+                   "v_up.weight": draw(heads * value, rank), "o_proj.weight": draw(hidden, heads * value)}
+        return build_part("mixer", spec, tensors, Runtime(torch.bfloat16, torch.device("cpu")))
+
+    layers = [part(**first), part(**second)]
+    if turned:
+        layers.reverse()
+    on_gpu = lambda n: SimpleNamespace(shape=(n, 4), is_cuda=True)  # noqa: E731
+
+    def step(starts, lens):
+        tiles, singles = sum(n > 1 for n in lens), sum(n == 1 for n in lens)
+        return SimpleNamespace(
+            q_tiles=on_gpu(tiles), single_tokens=on_gpu(singles), q_lens=lens, start_positions=starts,
+            num_tokens=sum(lens), num_requests=len(lens), decode_only=not tiles, max_q_len=max(lens),
+            max_context_len=max(s + n for s, n in zip(starts, lens)),
+            max_portion_start=max((s for s, n in zip(starts, lens) if n > 1), default=0))
+
+    steps = [step((0, 0), (20, 30)), step((0, 300), (20, 30)), step((200, 300), (20, 30)), step((0, 50), (20, 1)),
+             step((9, 50), (20, 1)), step((40, 5000), (1, 1))]
+    agree = all(layers[0].launch_key(s, 128) == layers[1].launch_key(s, 128) for s in steps)
+    assert agree or layers[0].launch_group() != layers[1].launch_group()
+
+
 # ---------------------------------------------------------------------------
 # the engine on the plain statements of the kernels (CPU)
 @pytest.fixture()
