@@ -29,6 +29,11 @@ class BatchError(ValueError):
     """A plan the step function refuses."""
 
 
+def _again(values):
+    """``values``, as something that can be iterated any number of times."""
+    return values if isinstance(values, (list, tuple)) else list(values)
+
+
 def as_plan(requests) -> BatchPlan:
     """A :class:`BatchPlan` from a plan or from request-like objects (``input_token_ids``,
     ``start_position``, ``block_tables``, optional ``state_slot``, ``need_sample``,
@@ -48,15 +53,15 @@ def as_plan(requests) -> BatchPlan:
             getattr(r, "sampling_params", None),
         )
         name, start = str(getattr(r, "request_id", index)), int(r.start_position)
+        # both tries below read the numbers, so what can be read only once (an iterator, a generator) becomes a list here
+        tokens, tables = _again(r.input_token_ids), [_again(table) for table in r.block_tables]
         try:
             # the binding turns sequences of whole numbers into vectors itself; what it refuses (numbers in strings,
             # fractions) goes element by element (64 requests with 129 pages: 757 -> 304 us a plan)
-            request = ScheduledRequest(name, r.input_token_ids, start, r.block_tables, *rest)
+            request = ScheduledRequest(name, tokens, start, tables, *rest)
         except TypeError:
             request = ScheduledRequest(
-                name, [int(t) for t in r.input_token_ids], start, [[int(p) for p in table] for table in r.block_tables],
-                *rest,
-            )
+                name, [int(t) for t in tokens], start, [[int(p) for p in table] for table in tables], *rest)
         converted.append(request)
     return BatchPlan(0, converted)
 

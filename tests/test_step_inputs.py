@@ -173,7 +173,8 @@ def test_the_decode_attention_cuts_the_keys_by_an_estimate_of_each_shape():
                 assert cluster == 1 and splits == 1 or pairs * splits <= held[size][cluster]
 
 
-@pytest.mark.parametrize("kind", ["list", "tuple", "numpy", "numpy elements", "floats", "strings", "mixed", "iterators"])
+@pytest.mark.parametrize("kind", ["list", "tuple", "numpy", "numpy elements", "floats", "strings", "mixed", "iterators", "generators",
+                                  "generators of floats", "generators of strings", "sets", "tensors"])
 def test_request_like_objects_may_hold_numbers_of_any_kind(kind):
     """Lists of ints are converted by the binding, everything else as int() takes it."""
     from types import SimpleNamespace
@@ -183,13 +184,21 @@ def test_request_like_objects_may_hold_numbers_of_any_kind(kind):
     make = {
         "list": list, "tuple": tuple, "numpy": np.array, "numpy elements": lambda v: [np.int32(x) for x in v],
         "floats": lambda v: [float(x) for x in v], "strings": lambda v: [str(x) for x in v],
-        "mixed": lambda v: [True if x == 1 else x for x in v], "iterators": iter,
+        "mixed": lambda v: [True if x == 1 else x for x in v], "iterators": iter, "generators": lambda v: (x for x in v),
+        "generators of floats": lambda v: (float(x) for x in v), "generators of strings": lambda v: (str(x) for x in v),
+        "sets": lambda v: dict.fromkeys(v).keys(), "tensors": torch.tensor,
     }[kind]
     tokens, tables = [7, 1, -3], [[5, 2 ** 31 - 1], [1, 0, 4]]
-    plan = as_plan([SimpleNamespace(input_token_ids=make(tokens), start_position=2, block_tables=[make(t) for t in tables])])
-    request = plan.requests[0]
-    assert list(request.input_token_ids) == tokens and [list(t) for t in request.block_tables] == tables
-    assert request.start_position == 2 and request.request_id == "0" and request.state_slot == -1
+    fraction, plain = (8.0 for _ in range(1)), [8]
+    for of_tokens, of_tables, outer in ((make, make, list), (make, list, list), (list, make, tuple), (make, make, iter),
+                                        (make, lambda t: [float(x) for x in t], lambda v: (t for t in v))):
+        plan = as_plan([SimpleNamespace(input_token_ids=of_tokens(tokens), start_position=2,
+                                        block_tables=outer([of_tables(t) for t in tables]))])
+        request = plan.requests[0]
+        assert list(request.input_token_ids) == tokens and [list(t) for t in request.block_tables] == tables
+        assert request.start_position == 2 and request.request_id == "0" and request.state_slot == -1
+    plan = as_plan([SimpleNamespace(input_token_ids=plain, start_position=0, block_tables=[fraction])])
+    assert list(plan.requests[0].input_token_ids) == [8] and [list(t) for t in plan.requests[0].block_tables] == [[8]]
 
 
 def test_request_like_objects_with_numbers_beyond_32_bits_are_refused():
