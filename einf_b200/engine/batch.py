@@ -54,7 +54,10 @@ def as_plan(requests) -> BatchPlan:
         )
         name, start = str(getattr(r, "request_id", index)), int(r.start_position)
         # both tries below read the numbers, so what can be read only once (an iterator, a generator) becomes a list here
-        tokens, tables = _again(r.input_token_ids), [_again(table) for table in r.block_tables]
+        tokens = r.input_token_ids
+        if type(tokens) is not list:
+            tokens = _again(tokens)
+        tables = [table if type(table) is list else _again(table) for table in r.block_tables]
         try:
             # the binding turns sequences of whole numbers into vectors itself; what it refuses (numbers in strings,
             # fractions) goes element by element (64 requests with 129 pages: 757 -> 304 us a plan)
