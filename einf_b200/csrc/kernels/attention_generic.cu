@@ -26,6 +26,8 @@
 // elements: value_size for a cache of its own, the key size when the values are the leading
 // elements of the key rows (a latent cache that holds one row per token for both).
 // The kernel exists twice: for sizes up to 256 and for sizes up to 640 (more registers a lane).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace einf {
@@ -176,9 +178,11 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
 // heads of 64 in 32 bits, 0.5 GFLOP).  A thread has 4 x 4 of the scores and 4 rows x VALUE / 16 columns of the output; rows
 // of shared memory are four floats longer than a vector, so that eight neighbouring rows meet no bank twice.  The
 // scores are the same sums in the same order; the softmax goes by tiles of 64 keys instead of 32.  Bound by the
-// reads from shared memory and by the longest token's chain of tiles.
+// reads from shared memory and by the longest token's chain of tiles.  A key that a row does not see adds nothing to the
+// row, not even zero times its value: an infinity or NaN among a later token's values reaches no token before it.
 // ---------------------------------------------------------------------------
 constexpr int kPromptRows = 32, kPromptKeys = 64, kPromptThreads = 128;
+constexpr float kHidden = -1.f;      // in a weight's place: the row does not see the key (weights are never negative)
 
 struct PromptArgs {
   const void* q; const void* k_cache; const void* v_cache; void* out;
@@ -290,6 +294,7 @@ paged_attention_prompt_kernel(const __grid_constant__ PromptArgs a) {
     prompt_wait<1>();
     __syncthreads();
     float s[4][4];
+    bool hides = false;                            // a row of the portion does not see a key of the tile
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -315,14 +320,17 @@ paged_attention_prompt_kernel(const __grid_constant__ PromptArgs a) {
     for (int i = 0; i < 4; ++i) {
       const int pos = pos0 + ty + 8 * i, lo = low_of(pos);
       float top = -INFINITY;
+      unsigned hidden = 0;                         // bit j: the row does not see key j
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int key = base + tx + 16 * j;
         const bool seen = key <= pos && (key >= lo || key < kept) && pages[tx + 16 * j] >= 0;
         const float capped = a.softcap > 0.f ? a.softcap * tanhf(s[i][j] * inv_cap) : s[i][j];
+        hidden |= seen ? 0u : 1u << j;
         s[i][j] = seen ? capped : -INFINITY;
         top = fmaxf(top, s[i][j]);
       }
+      hides |= hidden != 0 && ty + 8 * i < rows;
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
       const float m_new = fmaxf(m[i], top);
@@ -331,7 +339,7 @@ paged_attention_prompt_kernel(const __grid_constant__ PromptArgs a) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float p = s[i][j] == -INFINITY ? 0.f : expf(s[i][j] - m_new);
-        ps[(ty + 8 * i) * kScorePitch + tx + 16 * j] = p;
+        ps[(ty + 8 * i) * kScorePitch + tx + 16 * j] = (hidden >> j) & 1u ? kHidden : p;
         sum += p;
       }
 #pragma unroll
@@ -343,28 +351,32 @@ paged_attention_prompt_kernel(const __grid_constant__ PromptArgs a) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[i][c][e] *= correction;
     }
-    prompt_wait<0>();
-    __syncthreads();
+    auto add_values = [&](auto with_hidden) {
 #pragma unroll 2
-    for (int j = 0; j < kPromptKeys; j += 4) {
-      float4 pv[4];
+      for (int j = 0; j < kPromptKeys; j += 4) {
+        float4 pv[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) pv[i] = *reinterpret_cast<const float4*>(ps + (ty + 8 * i) * kScorePitch + j);
+        for (int i = 0; i < 4; ++i) pv[i] = *reinterpret_cast<const float4*>(ps + (ty + 8 * i) * kScorePitch + j);
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int c = 0; c < COLS; ++c) {
-          const float4 v = *reinterpret_cast<const float4*>(vs + (j + u) * value_pitch + 64 * c + 4 * tx);
+          for (int c = 0; c < COLS; ++c) {
+            const float4 v = *reinterpret_cast<const float4*>(vs + (j + u) * value_pitch + 64 * c + 4 * tx);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float p = u == 0 ? pv[i].x : u == 1 ? pv[i].y : u == 2 ? pv[i].z : pv[i].w;
-            acc[i][c][0] = fmaf(p, v.x, acc[i][c][0]);
-            acc[i][c][1] = fmaf(p, v.y, acc[i][c][1]);
-            acc[i][c][2] = fmaf(p, v.z, acc[i][c][2]);
-            acc[i][c][3] = fmaf(p, v.w, acc[i][c][3]);
+            for (int i = 0; i < 4; ++i) {
+              const float p = u == 0 ? pv[i].x : u == 1 ? pv[i].y : u == 2 ? pv[i].z : pv[i].w;
+              if (decltype(with_hidden)::value && p == kHidden) continue;
+              acc[i][c][0] = fmaf(p, v.x, acc[i][c][0]);
+              acc[i][c][1] = fmaf(p, v.y, acc[i][c][1]);
+              acc[i][c][2] = fmaf(p, v.z, acc[i][c][2]);
+              acc[i][c][3] = fmaf(p, v.w, acc[i][c][3]);
+            }
           }
-        }
-    }
+      }
+    };
+    prompt_wait<0>();
+    if (__syncthreads_or(hides)) add_values(std::true_type{});
+    else add_values(std::false_type{});
   }
   if (bad_page) atomicOr(a.status, kStatusBadPage);
 #pragma unroll

@@ -280,6 +280,44 @@ def test_linear_recurrence_keeps_its_state(dev, dtype, heads, groups, dim, vdim,
         torch.testing.assert_close(state_got, state_want, rtol=2e-4, atol=2e-4)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("options", [{}, {"window": 37}, {"window": 20, "keep_first": 9}, {"chunk": 48}])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_attention_of_portions_keeps_a_value_from_rows_that_do_not_see_it(dev, dtype, options, bad):
+    """A value that is not finite reaches the tokens that see its key and no other: those before it, those whose window has
+    passed it and those of the next chunk are bit for bit what they are beside a finite one."""
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(5)
+    start, tokens, heads, size, page = 30, 100, 2, 32, 16
+    options = dict(options)
+    window, keep, chunk = options.pop("window", None), options.get("keep_first", 0), options.get("chunk")
+    pages = -(-(start + tokens) // page)
+    table = torch.randperm(pages, generator=gen).to(torch.int32).view(1, -1).to(dev)
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device=dev)  # noqa: E731
+    q, k, v = (torch.randn(shape, generator=gen).to(dtype).to(dev) for shape in (
+        (tokens, heads, size), (pages, heads, page, size), (pages, heads, page, size)))
+    tiles, none, st = ints([(0, 0, tokens, start)]), ints([]), status(dev)
+    seq, pos = ints([0] * tokens), ints(range(start, start + tokens))
+
+    def run(values):
+        out = torch.empty((tokens, heads, size), dtype=dtype, device=dev)
+        ops.paged_attention_generic(q, k, values, table, seq, pos, out, size ** -0.5, window, st, q_tiles=tiles,
+                                    single_tokens=none, **options)
+        return out
+
+    clean = run(v)
+    assert bool(torch.isfinite(clean).all()) and int(st) == 0
+    for key in (5, 31, 64, 95, 129):
+        broken = v.clone()
+        broken[int(table[0, key // page]), :, key % page] = bad
+        got, at = run(broken), pos.long()
+        sees = (at >= key) & ((at < key + window) | (key < keep) if window else at >= 0)
+        if chunk:
+            sees &= at // chunk == key // chunk
+        assert not bool(torch.isfinite(got[sees]).any()) and torch.equal(got[~sees], clean[~sees]), key
+
+
 @pytest.mark.parametrize("heads, groups, dim, vdim, per_token, silu, pad", [
     (2, 2, 64, 64, False, True, 8), (4, 1, 128, 64, True, False, 8), (1, 1, 128, 260, True, False, 4), (3, 3, 64, 132, True, True, 4),
     (2, 2, 16, 12, True, False, 4), (2, 1, 40, 100, False, False, 8), (1, 1, 100, 36, False, True, 4),
