@@ -30,8 +30,11 @@
 // memory, 6 heads of 128 x 260, prompts of 2,048 and 500 tokens 332 -> 93 us (7 heads of 64 x 132, 1,500 and 301: 121 -> 37
 // us).  The error against 64 bits is no larger: 0.9, 0.9 and 1.1e-7 of y's norm (before: 1.7, 1.0 and 1.4e-7).  What bounds
 // it now are its instructions beside the products (taking values apart into parts, rounded additions) and, at two CTAs
-// an SM, the latency of its loads.  A value that is not finite reaches all tokens of its tile of 16 (the weights
-// beyond the diagonal are zeros, not left out).
+// an SM, the latency of its loads.
+//
+// The weights beyond the diagonal of a tile of 16 tokens are zeros, and zero times a value that is not finite is NaN: such
+// values leave the product of their own tile and are added one by one to the tokens they belong to, so that none reaches a
+// token before its own.
 #include <type_traits>
 
 #include "mma_sync.cuh"
@@ -62,6 +65,9 @@ __device__ __forceinline__ int first_segment(const ChunkArgs& a, int r) { return
 // SiLU with the quick division: two units in the last place at most (the division that rounds exactly is a third of this
 // kernel's instructions where the inputs pass a SiLU; y and state stay closer to 64 bits than the token-by-token kernel's).
 __device__ __forceinline__ float silu_quick(float z) { return __fdividef(z, 1.f + expf(-z)); }
+
+// The halves of a pair of bfloat16 that are infinite or NaN, as their highest bits.
+__device__ __forceinline__ uint32_t not_finite(uint32_t pair) { return ((pair & 0x7f807f80u) + 0x00800080u) & 0x80008000u; }
 
 // Shared memory of a CTA, in bytes from its start.  ROWS: rows of the state (filled up); NT: tiles of eight columns;
 // with kAct the inputs are 32-bit values in three parts.  Rows of q and k (and of v and the state at 64 columns) are a
@@ -407,11 +413,24 @@ recurrence_chunk_kernel(const __grid_constant__ ChunkArgs a) {
           for (int i = 0; i < 3; ++i) wf[i][2 * e + 1] = part[i];
         }
         if (kk < tile) between_tiles *= whole[kk];
+        uint32_t odd = 0;                          // values of this warp's own tokens that are not finite
+        auto keep_finite = [&](uint32_t (&v)[kIn][2]) {     // (such a value's other parts are zeros)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const uint32_t bad = not_finite(v[0][e]);
+            odd |= bad;
+            v[0][e] &= ~((bad >> 15) * 0xffffu);
+          }
+        };
 #pragma unroll
         for (int j = 0; j < NH / 2; ++j) {
           uint32_t v0[kIn][2], v1[kIn][2];
 #pragma unroll
           for (int p = 0; p < kIn; ++p) column_tiles(v0[p], v1[p], L::kValue + p * L::kValuePart, 16 * kk, n0 + 2 * j);
+          if (kk == tile) {
+            keep_finite(v0);
+            keep_finite(v1);
+          }
           mma_parts<3, kIn>(Y[2 * j], wf, v0);
           mma_parts<3, kIn>(Y[2 * j + 1], wf, v1);
         }
@@ -419,7 +438,38 @@ recurrence_chunk_kernel(const __grid_constant__ ChunkArgs a) {
           uint32_t v0[kIn][2];
 #pragma unroll
           for (int p = 0; p < kIn; ++p) column_tile(v0[p], L::kValue + p * L::kValuePart, 16 * kk, n0 + NH - 1);
+          if (kk == tile) keep_finite(v0);
           mma_parts<3, kIn>(Y[NH - 1], wf, v0);
+        }
+        if (kk == tile && __any_sync(0xffffffffu, odd != 0)) {   // what was left out, token after token (seldom: never for finite inputs)
+#pragma unroll 1
+          for (int quarter = 0; quarter < 4; ++quarter)
+#pragma unroll
+            for (int place = 0; place < 4; ++place) {
+              const int e = place >> 1, s = 8 * e + 2 * quarter + (place & 1);
+              auto weight_of = [&](int row_half) {   // of token s for this lane's row, from the lane that made it
+                float sum = 0.f;
+#pragma unroll
+                for (int i = 2; i >= 0; --i)
+                  sum += place & 1 ? high_bf16(wf[i][2 * e + row_half]) : low_bf16(wf[i][2 * e + row_half]);
+                return __shfl_sync(0xffffffffu, sum, (lane & ~3) | quarter);
+              };
+              const float w_low = weight_of(0), w_high = weight_of(1);
+#pragma unroll
+              for (int j = 0; j < NH; ++j) {
+                const int row = 16 * tile + s;
+                const uint32_t pair = lds_u32(base + L::kValue + row * L::kColPitch + L::column(row, n0 + j) + q2 * 2);
+                const uint32_t bad = not_finite(pair);
+                if (bad & 0x8000u) {
+                  if (s <= g) Y[j][0] = fmaf(w_low, low_bf16(pair), Y[j][0]);
+                  if (s <= g + 8) Y[j][2] = fmaf(w_high, low_bf16(pair), Y[j][2]);
+                }
+                if (bad & 0x80000000u) {
+                  if (s <= g) Y[j][1] = fmaf(w_low, high_bf16(pair), Y[j][1]);
+                  if (s <= g + 8) Y[j][3] = fmaf(w_high, high_bf16(pair), Y[j][3]);
+                }
+              }
+            }
         }
       }
       float* y_out = a.y + ((long long)t0 * a.heads + head) * vdim;

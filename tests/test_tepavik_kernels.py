@@ -368,6 +368,56 @@ def test_chunked_recurrence(dev, heads, groups, dim, vdim, per_token, silu, pad,
         assert torch.equal(state[:, :4], base[:, :4])
 
 
+@pytest.mark.parametrize("silu", [False, True])
+@pytest.mark.parametrize("dim, vdim", [(64, 64), (128, 20), (40, 132)])
+@pytest.mark.parametrize("lengths", [(60,), (40, 150)])
+@pytest.mark.parametrize("what", ["v", "k", "q", "scale", "decay"])
+def test_chunked_recurrence_keeps_what_is_not_finite_from_earlier_tokens(dev, silu, dim, vdim, lengths, what):
+    """An infinity in one token's inputs leaves the tokens before it, the other requests and, in a value, the other columns bit
+    for bit as they were, and what it belongs to is no number afterwards (the token's own output with a query, everything
+    from the token on and the state otherwise)."""
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(dim + vdim)
+    heads, requests, tokens = 2, len(lengths), sum(lengths)
+    q_start, _ = _packed(lengths, dev)
+    slots = torch.arange(requests, dtype=torch.int32, device=dev)
+    base = torch.randn((requests, heads, dim, vdim), generator=gen).to(dev)
+    inputs = {name: torch.rand((tokens, heads * n), generator=gen).add(0.1).to(torch.bfloat16).to(dev)
+              for name, n in (("q", dim), ("k", dim), ("v", vdim))}
+    inputs["decay"], inputs["scale"] = (torch.rand((tokens, heads), generator=gen).add(0.1).to(dev) for _ in range(2))
+
+    def run(with_inputs):
+        state, y = base.clone(), torch.empty((tokens, heads * vdim), device=dev)
+        ops.linear_recurrence(with_inputs["q"], with_inputs["k"], with_inputs["v"], state, q_start, slots, y, heads, heads, dim,
+                              vdim, token_decay=with_inputs["decay"], token_scale=with_inputs["scale"], silu_inputs=silu,
+                              max_q_len=max(lengths), chunks=True)
+        return y.view(tokens, heads, vdim), state
+
+    clean_y, clean_state = run(inputs)
+    assert bool(torch.isfinite(clean_y).all()) and bool(torch.isfinite(clean_state).all())
+    last_first = tokens - lengths[-1]                  # of the last request, which holds every token below
+    for token in (last_first + 5, last_first + 31, tokens - 1):
+        broken = {name: t.clone() for name, t in inputs.items()}
+        head, column = 1, 3                            # the first head stays as it is
+        width = {"q": dim, "k": dim, "v": vdim}.get(what, 1)
+        broken[what][token, head * width + (column if width > 1 else 0)] = float("inf")
+        y, state = run(broken)
+        touched = torch.zeros_like(clean_y, dtype=torch.bool)
+        end = token + 1 if what == "q" else tokens
+        touched[token:end, head, column if what == "v" else slice(None)] = True
+        assert torch.equal(y[~touched], clean_y[~touched]), (token, "reaches what it does not belong to")
+        assert not bool(torch.isfinite(y[touched]).any()), (token, "is lost")
+        of_state = torch.zeros_like(base, dtype=torch.bool)
+        if what == "v":
+            of_state[-1, head, :, column] = True
+        elif what == "k":
+            of_state[-1, head, column] = True
+        elif what != "q":
+            of_state[-1, head] = True
+        assert torch.equal(state[~of_state], clean_state[~of_state]) and not bool(torch.isfinite(state[of_state]).any())
+
+
 def _recurrence64(q, k, v, state, q_start, slots, heads, groups, of, head_decay=None, token_decay=None, token_scale=None,
                   skip=None, silu_inputs=False):
     """y and the states after the loop over tokens in 64 bits, of ``of`` the inputs (torch.abs: the sums of the sizes)."""
