@@ -6,7 +6,8 @@
 // zeros and writes nothing.  The step's tokens are packed request by request, q_start[r] ..
 // q_start[r + 1], so a prompt portion and a single decoded token take the same code and the same
 // order of additions: what a position computes does not depend on how the prompt was cut.  (bfloat16 portions of 24 tokens
-// and more take recurrence_chunks.cu, which sums a chunk's tokens in another order.)
+// and more take recurrence_chunks.cu, which sums a chunk's tokens in another order; the shorter portions of the same step
+// stay here, so a portion's kernel goes by its own length and not by what stands beside it.)
 #include <type_traits>
 
 #include "conv_run.cuh"
@@ -179,6 +180,7 @@ struct RecurrenceArgs {
   float* segment_state;    // [requests * segments, heads, dim, vdim]: B after the first pass, start states after the walk
   float* segment_decay;    // [requests * segments, heads]
   int num_slots, heads, groups, dim, vdim, act, lanes_per_column, dim_pad, batch, segments, segment_len;
+  int below;               // portions of so many tokens and more are another kernel's (0: none are)
 };
 
 // kEmit false: the first pass (no queries, no output, state from zero into segment_state).
@@ -204,7 +206,7 @@ linear_recurrence_kernel(const __grid_constant__ RecurrenceArgs a) {
   const int request_first = a.q_start[r], request_last = a.q_start[r + 1];
   const int count = request_last - request_first;
   const int num_segments = (count + a.segment_len - 1) / a.segment_len;
-  if (segment >= num_segments || (!kEmit && num_segments <= 1)) return;
+  if (segment >= num_segments || (!kEmit && num_segments <= 1) || (a.below && count >= a.below)) return;
   const int first = request_first + segment * a.segment_len;
   const int last = min(request_last, first + a.segment_len);
   const int slot = a.state_slots[r];
@@ -1032,8 +1034,9 @@ extern "C" int einf_linear_recurrence(const void* q, const void* k, const void* 
                                       const int* state_slots, int num_requests, float* y, int heads, int groups,
                                       int dim, int vdim, int act, int rows, int columns, int segments,
                                       int segment_len, float* segment_state, float* segment_decay, int y_splits,
-                                      long long y_split_stride, cudaStream_t stream) {
+                                      long long y_split_stride, int below, cudaStream_t stream) {
   if (num_requests == 0) return 0;
+  if (below < 0 || (below && segments > 1)) return (int)cudaErrorInvalidValue;
   if (y_splits < 1 || y_splits > 64) return (int)cudaErrorInvalidValue;
   if (heads <= 0 || groups <= 0 || heads % groups || dim <= 0 || vdim <= 0 || dim > 512 || heads > 65535 ||
       segments < 1 || segment_len < 1 || (long long)num_requests * segments > 65535 ||
@@ -1054,8 +1057,8 @@ extern "C" int einf_linear_recurrence(const void* q, const void* k, const void* 
   a.y_splits = y_splits; a.y_split_stride = y_split_stride;
   a.segment_state = segment_state; a.segment_decay = segment_decay;
   a.num_slots = num_slots; a.heads = heads; a.groups = groups; a.dim = dim; a.vdim = vdim; a.act = act;
-  a.segments = segments; a.segment_len = segment_len;
-  // A step of single tokens (segment_len 1 says so): the streaming kernel, where it takes the sizes.
+  a.segments = segments; a.segment_len = segment_len; a.below = below;
+  // Single tokens (segment_len 1 says that there is nothing else to do): the streaming kernel, where it takes the sizes.
   if (segments == 1 && segment_len == 1 && vdim % 4 == 0 && vdim / 4 <= kRecurrenceThreads &&
       state_stride % 4 == 0 && ((uintptr_t)state & 15) == 0) {
     a.lanes_per_column = 0; a.dim_pad = dim; a.batch = 1;

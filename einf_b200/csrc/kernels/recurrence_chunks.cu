@@ -22,8 +22,10 @@
 // w % 4 of the chunk's 64 in the first three products and a quarter of the state's rows in the last, of half the columns.
 // Long portions are cut into segments as in recurrence.cu: a pass over all segments from a zero state, a walk that
 // leaves every segment's start state (here as three bfloat16 parts, which the last pass brings straight into shared
-// memory), the emitting pass.  Segments are numbered q_start[r] / segment_len + r + (segment of the request), which leaves
-// no two requests a common number and is at most tokens / segment_len + requests, however long the longest portion.
+// memory), the emitting pass.  Only portions of min_len tokens and more are taken (the others are recurrence.cu's).  Their
+// segments are numbered q_start[r] / segment_len + (such portions before r) + (segment of the portion), which leaves no two
+// portions a common number and stays below tokens / segment_len + portions, however long the longest of them: users
+// that decode beside a prompt cost neither segments nor CTAs.
 //
 // Measured (B200, bfloat16, the three launches of a call, token-by-token kernel before): lightning attention, 14 heads of
 // 64 x 64, prompts of 4,096 and 1,000 tokens 222 -> 105 us; Mamba-2, 24 heads of 128 x 64, 2,048 tokens 242 -> 70 us; matrix
@@ -56,11 +58,37 @@ struct ChunkArgs {
   __nv_bfloat16* segment_start;     // [segments, heads, 3, dim, vdim]: the state it starts from, in parts
   float* segment_decay;             // [segments, heads]
   int num_slots, num_requests, heads, groups, dim, vdim, segment_len;
+  int min_len;                      // tokens of the shortest portion that is taken (at least one)
   int wide;                         // operands with 16-byte rows (bits: q, k, v, the segments' start states)
 };
 
-// The number of a request's first segment.
-__device__ __forceinline__ int first_segment(const ChunkArgs& a, int r) { return a.q_start[r] / a.segment_len + r; }
+// Which portion a CTA has: the request whose segments' numbers hold `number` or, with kByRank, the number-th that is taken
+// (-1: none).  first_segment: the number of its first.  Every warp looks for itself, 32 requests at a time.
+template <bool kByRank>
+__device__ __forceinline__ int find_portion(const ChunkArgs& a, int number, int* first_segment) {
+  const int lane = threadIdx.x & 31;
+  int before = 0;                                // portions taken among the requests so far
+#pragma unroll 4
+  for (int base = 0; base < a.num_requests; base += 32) {
+    const int i = base + lane;
+    const int begin = i < a.num_requests ? a.q_start[i] : 0;
+    const int count = i < a.num_requests ? a.q_start[i + 1] - begin : 0;
+    const bool taken = count >= a.min_len;
+    const uint32_t all = __ballot_sync(0xffffffffu, taken);
+    const int rank = before + __popc(all & ((1u << lane) - 1u));
+    const int first = begin / a.segment_len + rank;
+    const bool mine = taken && (kByRank ? rank == number
+                                        : first <= number && number < first + (count + a.segment_len - 1) / a.segment_len);
+    const uint32_t found = __ballot_sync(0xffffffffu, mine);
+    if (found) {
+      const int at = __ffs(found) - 1;
+      *first_segment = __shfl_sync(0xffffffffu, first, at);
+      return base + at;
+    }
+    before += __popc(all);
+  }
+  return -1;
+}
 
 // SiLU with the quick division: two units in the last place at most (the division that rounds exactly is a third of this
 // kernel's instructions where the inputs pass a SiLU; y and state stay closer to 64 bits than the token-by-token kernel's).
@@ -175,22 +203,15 @@ recurrence_chunk_kernel(const __grid_constant__ ChunkArgs a) {
   const int g = lane >> 2, q2 = (lane & 3) * 2;  // a fragment's row and first column of this lane
   const int n0 = half * NH;                      // this warp's first column tile
   const int column0 = blockIdx.x * kColumns, head = blockIdx.y;
-  int r = 0;
-  if (a.num_requests > 1) {                      // whose segment this CTA has
-    __shared__ int whose;
-    if (threadIdx.x == 0) whose = 0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < a.num_requests; i += kChunkThreads)
-      if (first_segment(a, i) <= (int)blockIdx.z && (int)blockIdx.z < first_segment(a, i + 1)) whose = i;
-    __syncthreads();
-    r = whose;
-  }
-  const int segment = (int)blockIdx.z - first_segment(a, r);
+  int numbered;
+  const int r = find_portion<false>(a, (int)blockIdx.z, &numbered);      // whose segment this CTA has
+  if (r < 0) return;
+  const int segment = (int)blockIdx.z - numbered;
   const int request_first = a.q_start[r], request_last = a.q_start[r + 1];
   const int slot = a.state_slots[r];
   const int count = request_last - request_first;
   const int num_segments = (count + a.segment_len - 1) / a.segment_len;
-  if (segment >= num_segments || (!kEmit && num_segments <= 1)) return;
+  if (!kEmit && num_segments <= 1) return;
   const int first = request_first + segment * a.segment_len;
   const int last = min(request_last, first + a.segment_len);
   const int dim = a.dim, vdim = a.vdim;
@@ -659,13 +680,15 @@ __global__ void __launch_bounds__(128)
 recurrence_chunk_walk_kernel(const __grid_constant__ ChunkArgs a) {
   pdl_launch_dependents();
   pdl_wait();
-  const int head = blockIdx.y, r = blockIdx.z;
+  const int head = blockIdx.y;
+  int first;
+  const int r = find_portion<true>(a, (int)blockIdx.z, &first);
+  if (r < 0) return;
   const int count = a.q_start[r + 1] - a.q_start[r];
   const int num_segments = (count + a.segment_len - 1) / a.segment_len;
   if (num_segments <= 1) return;
   const int slot = a.state_slots[r];
   const long long per_head = (long long)a.dim * a.vdim;
-  const int first = first_segment(a, r);
   constexpr int kAtOnce = 8;       // segments whose B and P are in registers before the chain of products starts
   for (long long e = 4 * ((long long)blockIdx.x * blockDim.x + threadIdx.x); e < per_head; e += 4ll * gridDim.x * blockDim.x) {
     float* slot_state = (slot >= 0 && slot < a.num_slots) ? a.state + (long long)slot * a.state_stride + head * per_head + e : nullptr;
@@ -712,13 +735,13 @@ static cudaError_t launch_chunks(const ChunkArgs& a, int slots, cudaStream_t str
 
 // `slots`: CTAs along z, one per segment number; 0 says that no portion is longer than a segment.
 template <int ROWS, int NT, bool kAct>
-static cudaError_t run_chunks(const ChunkArgs& a, int slots, cudaStream_t stream) {
-  if (slots == 0) return launch_chunks<ROWS, NT, kAct, true>(a, a.num_requests, stream);
+static cudaError_t run_chunks(const ChunkArgs& a, int portions, int slots, cudaStream_t stream) {
+  if (slots == 0) return launch_chunks<ROWS, NT, kAct, true>(a, portions, stream);
   cudaError_t e = launch_chunks<ROWS, NT, kAct, false>(a, slots, stream);
   if (e != cudaSuccess) return e;
-  // requests of one segment have nothing to walk: with many of them the CTAs of a request take more each
-  const long long blocks = ((long long)a.dim * a.vdim / 4 + 127) / 128, most = 1 + 4096 / ((long long)a.heads * a.num_requests);
-  e = launch_pdl(recurrence_chunk_walk_kernel, dim3((unsigned)(blocks < most ? blocks : most), a.heads, a.num_requests), dim3(128),
+  // portions of one segment have nothing to walk: with many portions the CTAs of one take more each
+  const long long blocks = ((long long)a.dim * a.vdim / 4 + 127) / 128, most = 1 + 4096 / ((long long)a.heads * portions);
+  e = launch_pdl(recurrence_chunk_walk_kernel, dim3((unsigned)(blocks < most ? blocks : most), a.heads, portions), dim3(128),
                  0, stream, a);
   if (e != cudaSuccess) return e;
   return launch_chunks<ROWS, NT, kAct, true>(a, slots, stream);
@@ -729,19 +752,20 @@ static cudaError_t run_chunks(const ChunkArgs& a, int slots, cudaStream_t stream
 using namespace einf;
 
 // q, k, v: bfloat16, 8-byte aligned rows (strides and sizes in multiples of four elements), the state 16-byte aligned; dim
-// up to 128.  `slots`: 0 where no portion is longer than segment_len; else tokens / segment_len + num_requests, with
-// segment_len a multiple of 64.  `tiles`: columns of the state that a CTA takes, in eights (4, 8 or 10).
+// up to 128.  Portions of min_len tokens and more are taken, `portions` of them at most.  `slots`: 0 where none of them is
+// longer than segment_len; else tokens / segment_len + portions, with segment_len a multiple of 64.  `tiles`: columns of the state that a CTA takes, in eights (4, 8 or 10).
 extern "C" int einf_linear_recurrence_chunks(const void* q, const void* k, const void* v, long long q_stride,
                                              long long k_stride, long long v_stride, const float* head_decay,
                                              const float* token_decay, const float* token_scale, const float* skip,
                                              float* state, long long state_stride, int num_slots, const int* q_start,
-                                             const int* state_slots, int num_requests, float* y, int heads, int groups,
-                                             int dim, int vdim, int act, int tiles, int slots, int segment_len,
+                                             const int* state_slots, int num_requests, int portions, int min_len, float* y,
+                                             int heads, int groups, int dim, int vdim, int act, int tiles, int slots,
+                                             int segment_len,
                                              float* segment_state, void* segment_start, float* segment_decay,
                                              cudaStream_t stream) {
-  if (num_requests == 0) return 0;
+  if (num_requests == 0 || portions == 0) return 0;
   if (heads <= 0 || groups <= 0 || heads % groups || dim <= 0 || dim > 128 || dim % 4 || vdim <= 0 || vdim % 4 ||
-      heads > 65535 || num_requests > 65535 || slots < 0 || slots > 65535 || segment_len < 1 ||
+      heads > 65535 || portions < 0 || portions > 65535 || min_len < 1 || slots < 0 || slots > 65535 || segment_len < 1 ||
       (slots && (!segment_state || !segment_start || !segment_decay || segment_len % kChunk)) || state_stride % 4 ||
       ((uintptr_t)state & 15) || ((uintptr_t)y & 7) || ((uintptr_t)q & 7) || ((uintptr_t)k & 7) || ((uintptr_t)v & 7) ||
       q_stride % 4 || k_stride % 4 || v_stride % 4)
@@ -755,18 +779,18 @@ extern "C" int einf_linear_recurrence_chunks(const void* q, const void* k, const
   a.y = y;
   a.segment_state = segment_state; a.segment_start = (__nv_bfloat16*)segment_start; a.segment_decay = segment_decay;
   a.num_slots = num_slots; a.heads = heads; a.groups = groups; a.dim = dim; a.vdim = vdim;
-  a.num_requests = num_requests;
-  a.segment_len = slots ? segment_len : 1 << 30;     // one segment each: numbered by the request alone
+  a.num_requests = num_requests; a.min_len = min_len;
+  a.segment_len = slots ? segment_len : 1 << 30;     // one segment each: numbered by the portions alone
   a.wide = (!((uintptr_t)q & 15) && q_stride % 8 == 0 && dim % 8 == 0 ? 1 : 0) |
            (!((uintptr_t)k & 15) && k_stride % 8 == 0 && dim % 8 == 0 ? 2 : 0) |
            (!((uintptr_t)v & 15) && v_stride % 8 == 0 && vdim % 8 == 0 ? 4 : 0) | (vdim % 8 == 0 ? 8 : 0);
 #define EINF_CHUNKS(NT_)                                                                              \
   if (tiles == NT_) {                                                                                 \
     if (dim <= 64)                                                                                    \
-      return act ? (int)run_chunks<64, NT_, true>(a, slots, stream)                                   \
-                 : (int)run_chunks<64, NT_, false>(a, slots, stream);                          \
-    return act ? (int)run_chunks<128, (NT_ > 8 ? 8 : NT_), true>(a, slots, stream)                    \
-               : (int)run_chunks<128, NT_, false>(a, slots, stream);                           \
+      return act ? (int)run_chunks<64, NT_, true>(a, portions, slots, stream)                                   \
+                 : (int)run_chunks<64, NT_, false>(a, portions, slots, stream);                          \
+    return act ? (int)run_chunks<128, (NT_ > 8 ? 8 : NT_), true>(a, portions, slots, stream)                    \
+               : (int)run_chunks<128, NT_, false>(a, portions, slots, stream);                           \
   }
   EINF_CHUNKS(4)
   EINF_CHUNKS(8)

@@ -13,7 +13,7 @@ from __future__ import annotations
 import ctypes
 import functools
 from ctypes import c_float, c_int, c_longlong, c_void_p
-from typing import Optional, Tuple
+from typing import Optional, Sequence, Tuple
 
 import torch
 
@@ -1650,9 +1650,10 @@ def recurrence_plan(num_requests: int, max_q_len: Optional[int], heads: int, dim
 
 #: tokens that the chunked recurrence takes at a time
 RECURRENCE_CHUNK = 64
-#: shortest longest portion that takes the chunked kernel (kernels alone, us, one request / eight; token by token against
+#: shortest portion that takes the chunked kernel (kernels alone, us, one request / eight; token by token against
 #: chunked: 16 tokens 7.6 / 10.7 against 9.6 / 11.3 (14 heads of 64 x 64), 9.4 / 15.8 against 9.2 / 11.5 (24 of 128 x 64); 24 tokens
-#: 12.3 / 16.7 against 10.8 / 15.1, 12.1 / 20.1 against 10.1 / 13.9; 64 tokens 20.5 / 30.3 against 14.9 / 21.2)
+#: 12.3 / 16.7 against 10.8 / 15.1, 12.1 / 20.1 against 10.1 / 13.9; 64 tokens 20.5 / 30.3 against 14.9 / 21.2).  The shorter
+#: portions of a step run token by token beside it, single tokens through the streaming kernel of decoding steps
 RECURRENCE_CHUNK_MIN = 24
 #: bytes that the states of a launch's segments may take (10 an element: the sum and the start state in parts)
 RECURRENCE_SEGMENT_BYTES = 128 << 20
@@ -1670,16 +1671,28 @@ def recurrence_takes_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, s
     )
 
 
-def recurrence_chunk_plan(tokens: int, num_requests: int, max_q_len: int, heads: int, dim: int, vdim: int) -> tuple[int, int]:
-    """``(segments, segment_len)`` of a chunked recurrence launch; no segments where no portion is longer than one.  A
-    segment is one chunk (longer ones repeat the state's product in both passes: Mamba-2, 24 heads of 128 x 64 over 2,048
-    tokens 70 us with 64, 71 with 128, 83 with 256 tokens) until the segments' states would outgrow the L2."""
+def recurrence_portions(q_lens: Sequence[int]) -> tuple[int, int]:
+    """``(long, short)`` of a step's portions for :func:`linear_recurrence`: how many take the chunked kernel, and what the
+    others are: 0 none, 1 single tokens alone, 2 longer ones too."""
+    long = short = 0
+    for n in q_lens:
+        if n >= RECURRENCE_CHUNK_MIN:
+            long += 1
+        elif n > 0:
+            short = max(short, 1 if n == 1 else 2)
+    return long, short
+
+
+def recurrence_chunk_plan(tokens: int, portions: int, max_q_len: int, heads: int, dim: int, vdim: int) -> tuple[int, int]:
+    """``(segments, segment_len)`` of a chunked recurrence launch for that many portions; no segments where none is longer
+    than one.  A segment is one chunk (longer ones repeat the state's product in both passes: Mamba-2, 24 heads of 128 x 64 over
+    2,048 tokens 70 us with 64, 71 with 128, 83 with 256 tokens) until the segments' states would outgrow the L2."""
     segment_len = RECURRENCE_CHUNK
     while segment_len < max_q_len and (
-            10 * heads * dim * vdim * (tokens // segment_len + num_requests) > RECURRENCE_SEGMENT_BYTES
-            or tokens // segment_len + num_requests > 65535):
+            10 * heads * dim * vdim * (tokens // segment_len + portions) > RECURRENCE_SEGMENT_BYTES
+            or tokens // segment_len + portions > 65535):
         segment_len *= 2
-    return (tokens // segment_len + num_requests if max_q_len > segment_len else 0), segment_len
+    return (tokens // segment_len + portions if max_q_len > segment_len else 0), segment_len
 
 
 def _recurrence_tiles(dim: int, vdim: int) -> int:
@@ -1728,6 +1741,7 @@ def linear_recurrence(
     segment_len: Optional[int] = None,
     columns: int = 0,
     chunks: Optional[bool] = None,
+    q_lens: Optional[Sequence[int]] = None,
 ) -> None:
     """Per request and head, over its tokens in order, with a float32 state ``S [dim, vdim]``::
 
@@ -1744,8 +1758,10 @@ def linear_recurrence(
     consumer to add up.  ``max_q_len`` is the longest portion of the step as the host knows it (None: unknown,
     no portion is cut into segments); ``rows`` (0, 4, 8, 16), ``columns`` (0, 1, 2) and ``segment_len``
     override the launch's own choices (:func:`recurrence_plan`), for tests and measurements.  ``chunks``: whether the
-    tokens are taken 64 at a time on the tensor cores (None: where :func:`recurrence_takes_chunks` says so and none
-    of the overrides is given; ``segment_len`` is then a multiple of 64)."""
+    tokens are taken 64 at a time on the tensor cores (None: those of portions of ``RECURRENCE_CHUNK_MIN`` tokens and more, where
+    :func:`recurrence_takes_chunks` says so and none of the overrides is given; True: all, ``segment_len`` is then a
+    multiple of 64).  ``q_lens``: the portions' lengths as the host knows them, which spare such a step the launch for
+    shorter portions where it has none."""
     tokens = v.shape[0]
     if q.shape != (tokens, groups * dim) or k.shape != q.shape or v.shape != (tokens, heads * vdim):
         raise ValueError(f"q, k must be [{tokens}, {groups * dim}] and v [{tokens}, {heads * vdim}]")
@@ -1774,14 +1790,27 @@ def linear_recurrence(
     requests = state_slots.shape[0]
     if tokens == 0 or requests == 0:
         return
+    below, short = 0, None
     if chunks is None:
         chunks = rows == 0 and columns == 0 and segment_len is None and \
             recurrence_takes_chunks(q, k, v, state, y, dim, vdim, max_q_len)
-    if chunks:
+        if chunks:
+            if q_lens is not None:
+                long, short = recurrence_portions(q_lens)
+            else:
+                long, short = min(requests, tokens // RECURRENCE_CHUNK_MIN), 0 if tokens == requests * max_q_len else 2
+            _recurrence_chunks(q, k, v, state, q_start, state_slots, y, heads, groups, dim, vdim, head_decay, token_decay,
+                               token_scale, skip, silu_inputs, max_q_len, None, long, RECURRENCE_CHUNK_MIN)
+            if not short:
+                return
+            below = 2 if short == 1 else RECURRENCE_CHUNK_MIN
+    elif chunks:
         _recurrence_chunks(q, k, v, state, q_start, state_slots, y, heads, groups, dim, vdim, head_decay, token_decay,
-                           token_scale, skip, silu_inputs, max_q_len or tokens, segment_len)
+                           token_scale, skip, silu_inputs, max_q_len or tokens, segment_len, requests, 1)
         return
-    if segment_len is not None:
+    if below:
+        segments, segment_len = 1, below - 1
+    elif segment_len is not None:
         longest = max_q_len or tokens
         segments, segment_len = -(-longest // int(segment_len)), int(segment_len)
     else:
@@ -1799,7 +1828,7 @@ def linear_recurrence(
         "einf_linear_recurrence",
         [c_void_p, c_void_p, c_void_p, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p,
          c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
-         c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_longlong, c_void_p],
+         c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_longlong, c_int, c_void_p],
     )
     _check(
         fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), _code(q), _rows_of(q, "q"), _rows_of(k, "k"), _rows_of(v, "v"),
@@ -1809,20 +1838,21 @@ def linear_recurrence(
            _opt(state_slots, "state_slots", torch.int32), requests, _dev(y, "y"), heads, groups, dim,
            vdim, 1 if silu_inputs else 0, int(rows), int(columns), segments, segment_len,
            _opt(segment_state, "segment_state", torch.float32), _opt(segment_decay, "segment_decay", torch.float32),
-           y_splits, tokens * heads * vdim, _stream()),
+           y_splits, tokens * heads * vdim, below, _stream()),
         "linear_recurrence",
     )
 
 
 def _recurrence_chunks(q, k, v, state, q_start, state_slots, y, heads, groups, dim, vdim, head_decay, token_decay,
-                       token_scale, skip, silu_inputs, max_q_len, segment_len) -> None:
-    """The chunked form of :func:`linear_recurrence`, which has checked the operands."""
+                       token_scale, skip, silu_inputs, max_q_len, segment_len, portions, min_len) -> None:
+    """The chunked form of :func:`linear_recurrence`, which has checked the operands, for the portions of ``min_len`` tokens
+    and more, of which there are ``portions`` at most."""
     global launch_count
-    requests, device = state_slots.shape[0], y.device
-    slots, planned = recurrence_chunk_plan(v.shape[0], requests, max_q_len, heads, dim, vdim)
+    device = y.device
+    slots, planned = recurrence_chunk_plan(v.shape[0], portions, max_q_len, heads, dim, vdim)
     if segment_len is not None:
         planned = int(segment_len)
-        slots = v.shape[0] // planned + requests if max_q_len > planned else 0
+        slots = v.shape[0] // planned + portions if max_q_len > planned else 0
     segment_state = segment_start = segment_decay = None
     if slots:
         segment_state = torch.empty((slots, heads, dim, vdim), dtype=torch.float32, device=device)
@@ -1832,16 +1862,16 @@ def _recurrence_chunks(q, k, v, state, q_start, state_slots, y, heads, groups, d
     fn = _fn(
         "einf_linear_recurrence_chunks",
         [c_void_p, c_void_p, c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p,
-         c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
-         c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
+         c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int,
+         c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
     )
     _check(
         fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), _rows_of(q, "q"), _rows_of(k, "k"), _rows_of(v, "v"),
            _opt(head_decay, "head_decay", torch.float32), _opt(token_decay, "token_decay", torch.float32),
            _opt(token_scale, "token_scale", torch.float32), _opt(skip, "skip", torch.float32),
            state.data_ptr(), state.stride(0), state.shape[0], _opt(q_start, "q_start", torch.int32),
-           _opt(state_slots, "state_slots", torch.int32), requests, _dev(y, "y"), heads, groups, dim, vdim,
-           1 if silu_inputs else 0, _recurrence_tiles(dim, vdim), slots, planned,
+           _opt(state_slots, "state_slots", torch.int32), state_slots.shape[0], portions, min_len, _dev(y, "y"), heads, groups,
+           dim, vdim, 1 if silu_inputs else 0, _recurrence_tiles(dim, vdim), slots, planned,
            _opt(segment_state, "segment_state", torch.float32), _opt(segment_start, "segment_start", torch.bfloat16),
            _opt(segment_decay, "segment_decay", torch.float32), _stream()),
         "linear_recurrence",

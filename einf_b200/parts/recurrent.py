@@ -38,12 +38,13 @@ class _RecurrentMixer(Mixer):
     state_shape: tuple[int, int, int] = (0, 0, 0)
 
     def launch_key(self, ctx: StepContext, page_size: int) -> tuple:
-        """Long portions are cut into segments by the step's longest portion, a host-side figure (which of the two forms of
-        the recurrence runs goes by it too)."""
+        """Long portions are cut into segments by the step's longest portion, a host-side figure; how many portions take which
+        form of the recurrence, and into how many segments those are cut, goes by all of their lengths."""
         plan = ops.recurrence_plan(ctx.num_requests, ctx.max_q_len, *self.state_shape)
         if ctx.max_q_len < ops.RECURRENCE_CHUNK_MIN:
             return plan
-        return plan + ops.recurrence_chunk_plan(ctx.num_tokens, ctx.num_requests, ctx.max_q_len, *self.state_shape)
+        long, short = ops.recurrence_portions(ctx.q_lens)
+        return plan + (long, short) + ops.recurrence_chunk_plan(ctx.num_tokens, long, ctx.max_q_len, *self.state_shape)
 
     def launch_group(self):
         return ("recurrence",) + self.state_shape
@@ -102,7 +103,7 @@ class LightningAttention(_RecurrentMixer):
         ops.linear_recurrence(
             q, k, v, state.view(state.shape[0], self.heads, self.dim, self.vdim), ctx.q_start, ctx.state_slots, y,
             self.heads, self.heads, self.dim, self.vdim, head_decay=self.decay, silu_inputs=True,
-            max_q_len=ctx.max_q_len,
+            max_q_len=ctx.max_q_len, q_lens=ctx.q_lens,
         )
         out = torch.empty((tokens, values), dtype=self.runtime.dtype, device=x.device)
         ops.gated_norm(y, gate, self.norm_weight, out, 1, self.eps, gate_first=False, gate_kind="sigmoid")
@@ -182,7 +183,7 @@ class Mamba2(_RecurrentMixer):
         y = torch.empty((tokens, inner), dtype=torch.float32, device=device)
         ops.linear_recurrence(
             c, b, xs, recurrent, ctx.q_start, ctx.state_slots, y, heads, self.groups, self.state_size, self.vdim,
-            token_decay=decay, token_scale=dt, skip=self.skip, max_q_len=ctx.max_q_len,
+            token_decay=decay, token_scale=dt, skip=self.skip, max_q_len=ctx.max_q_len, q_lens=ctx.q_lens,
         )
         out = torch.empty((tokens, inner), dtype=self.runtime.dtype, device=device)
         ops.gated_norm(y, z, self.norm_weight, out, self.norm_groups, self.eps, gate_first=True, gate_kind="silu")
@@ -371,7 +372,7 @@ class MatrixMemory(_RecurrentMixer):
         y = torch.empty(shape, dtype=torch.float32, device=device)
         ops.linear_recurrence(
             q, k, v_wide, memory, ctx.q_start, ctx.state_slots, y, heads, heads, self.dim, self.columns,
-            token_decay=decay, token_scale=scale, max_q_len=ctx.max_q_len,
+            token_decay=decay, token_scale=scale, max_q_len=ctx.max_q_len, q_lens=ctx.q_lens,
         )
         out = torch.empty((tokens, values), dtype=self.runtime.dtype, device=device)
         ops.memory_output(y, floor, gate, self.norm_weight, out, heads, self.vdim, self.query_scale, self.eps,

@@ -449,7 +449,7 @@ def qkv_conv_store(qkv, bias, conv_weight, conv_state, seq_of_token, q_start, st
 
 def linear_recurrence(q, k, v, state, q_start, state_slots, y, heads, groups, dim, vdim, head_decay=None,
                       token_decay=None, token_scale=None, skip=None, silu_inputs=False, max_q_len=None, rows=0,
-                      segment_len=None, columns=0):
+                      segment_len=None, columns=0, q_lens=None):
     def act(t):
         t = t.float()
         return t / (1 + torch.exp(-t)) if silu_inputs else t

@@ -218,6 +218,40 @@ def test_long_portions_are_cut_into_segments_only_where_that_fills_the_gpu():
     assert 4000 * segments <= 65535 and segments * length >= 300
 
 
+def test_the_chunked_recurrences_segments_go_by_its_own_portions():
+    """Segments are numbered q_start / segment_len + (long portions before) + (segment): no two long portions share a number
+    and all stay below the launch's CTAs, whatever stands between them; and single tokens beside a prompt leave its
+    segments as short as they are without them."""
+    import random
+
+    from einf_b200 import ops
+
+    rng = random.Random(1)
+    for _ in range(300):
+        lens = [rng.choice([0, 1, 1, 2, 23, 24, 63, 64, 65, 130, 700]) for _ in range(rng.randint(1, 40))]
+        long, short = ops.recurrence_portions(lens)
+        assert long == sum(n >= 24 for n in lens) and short == (2 if set(lens) & {2, 23} else 1 if 1 in lens else 0)
+        if not long:
+            continue
+        slots, segment = ops.recurrence_chunk_plan(sum(lens), long, max(lens), 4, 64, 64)
+        if not slots:
+            assert max(lens) <= segment
+            continue
+        used, first, rank = [], 0, 0
+        for n in lens:
+            if n >= 24:
+                used += [first // segment + rank + i for i in range(-(-n // segment))]
+                rank += 1
+            first += n
+        assert len(set(used)) == len(used) and max(used) < slots
+    alone = ops.recurrence_chunk_plan(2048, 1, 2048, 24, 128, 64)
+    for users in (16, 64, 128):
+        long, short = ops.recurrence_portions([2048] + [1] * users)
+        assert (long, short) == (1, 1)
+        slots, segment = ops.recurrence_chunk_plan(2048 + users, long, 2048, 24, 128, 64)
+        assert segment == alone[1] == 64 and slots <= alone[0] + users // segment
+
+
 # ---------------------------------------------------------------------------
 # the engine on the plain statements of the kernels (CPU)
 @pytest.fixture()

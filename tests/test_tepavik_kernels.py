@@ -368,6 +368,44 @@ def test_chunked_recurrence(dev, heads, groups, dim, vdim, per_token, silu, pad,
         assert torch.equal(state[:, :4], base[:, :4])
 
 
+@pytest.mark.parametrize("known", [False, True])
+@pytest.mark.parametrize("dim, vdim, silu", [(64, 64, True), (128, 260, False), (40, 20, True), (16, 516, False)])
+@pytest.mark.parametrize("lengths", [
+    (130,) + (1,) * 40, (1, 24, 0, 193, 1, 64), (23, 24, 2, 65, 1, 0), (300, 17, 1) * 15, (1,) * 33 + (70,), (64, 64, 64)])
+def test_a_portions_recurrence_goes_by_its_own_length(dev, dim, vdim, silu, lengths, known):
+    """Every portion of a step gives bit for bit what it gives alone: those of 24 tokens and more through the chunked kernel,
+    the others token by token, whatever stands beside them and whether the host knows the lengths."""
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(dim + vdim)
+    heads, requests, tokens = 2, len(lengths), sum(lengths)
+    q_start, _ = _packed(lengths, dev)
+    slots = torch.randperm(requests, generator=gen).to(torch.int32).to(dev)
+    base = torch.randn((requests, heads, dim, vdim), generator=gen).to(dev)
+    q, k, v = ((torch.randn((tokens, heads * n), generator=gen) * 0.3).to(torch.bfloat16).to(dev) for n in (dim, dim, vdim))
+    decay = torch.rand((tokens, heads), generator=gen).add(0.1).to(dev)
+
+    def run(first, last, q_start, slots, state, lens, **options):
+        y = torch.full((last - first, heads * vdim), float("nan"), device=dev)
+        ops.linear_recurrence(q[first:last], k[first:last], v[first:last], state, q_start, slots, y, heads, heads, dim, vdim,
+                              token_decay=decay[first:last], silu_inputs=silu, max_q_len=max(lens), **options)
+        return y
+
+    state, alone = base.clone(), base.clone()
+    y = run(0, tokens, q_start, slots, state, lengths, **(dict(q_lens=lengths) if known else {}))
+    for r, n in enumerate(lengths):
+        if n == 0:
+            continue
+        first = int(q_start[r])
+        # a single token beside a prompt takes the streaming kernel only where the host knows of nothing but single tokens
+        only_singles = known and not any(1 < m < 24 for m in lengths)
+        options = {} if n >= 24 or (n == 1 and only_singles) else dict(segment_len=23)
+        got = y[first:first + n]
+        want = run(first, first + n, torch.tensor([0, n], dtype=torch.int32, device=dev), slots[r:r + 1], alone, [n], **options)
+        assert torch.equal(got, want), (r, n)
+    assert torch.equal(state, alone)
+
+
 @pytest.mark.parametrize("silu", [False, True])
 @pytest.mark.parametrize("dim, vdim", [(64, 64), (128, 20), (40, 132)])
 @pytest.mark.parametrize("lengths", [(60,), (40, 150)])
