@@ -538,16 +538,22 @@ extern "C" int einf_gemm_tcgen05_splits(int k, int splits) {
   return (total_kblocks + per_split - 1) / per_split;
 }
 
-// The largest token tile of the grouped product for `rows` rows over `groups` groups: about one and a half times the average
-// rows of a group, a multiple of 16 between 16 and 128, above that 192 or 256.  The CTAs' reads of W and x out of L2 bound
-// the product at many rows (2.6 GB at tiles of 128 for the sizes below, 2 GB at 256), so a
-// weight tile meets as many rows as its accumulator holds with two CTAs an SM, one's epilogue beside the other's products.
+// The largest token tile of the grouped product for `rows` rows over `groups` groups of n outputs: about one and a half
+// times the average rows of a group, a multiple of 16 between 16 and 128, above that 192 or 256.  The CTAs' reads of W and x
+// out of L2 bound the product at many rows (2.6 GB at tiles of 128 for the sizes below, 2 GB at 256), so a weight tile meets
+// as many rows as its accumulator holds with two CTAs an SM, one's epilogue beside the other's products.
 // Measured (B200): both products of 4,096 rows on eight experts, n and k of 17,920 and 1,536 and of 1,536 and 8,960:
-// 218 -> 182 us.
-extern "C" int einf_gemm_grouped_tcgen05_token_tile(int rows, int groups) {
+// 218 -> 182 us.  Not where tiles of 128 are one wave of CTAs or less (two an SM): fewer and larger tiles then leave
+// multiprocessors empty, and the ring of a larger tile has two stages where that of 128 rows has three.  Eight experts, n
+// 1,536, k 8,960, us with 128 / larger: 100 rows an expert (96 CTAs of 128) 80 / 100, 200 (192) 82 / 119, 340 (288) 84 / 113, 512
+// (384) 139 / 123; sixteen, n 1,024, k 896: 160 (256) 20.5 / 22.5, 340 (384) 33 / 25; sixty, n 2,816, k 2,048: 160 (2,640) 217 / 193.
+extern "C" int einf_gemm_grouped_tcgen05_token_tile(int rows, int groups, int n) {
   const int average = (rows + groups - 1) / (groups > 0 ? groups : 1);
   const int tile = (average * 3 / 2 + 15) / 16 * 16;
-  return tile < 16 ? 16 : (tile <= 128 ? tile : (tile <= 192 ? 192 : 256));
+  if (tile <= 128) return tile < 16 ? 16 : tile;
+  const long long ctas = (long long)((n + kBlockW - 1) / kBlockW) * groups * ((average + 127) / 128);
+  if (ctas <= 2 * 148) return 128;
+  return tile <= 192 ? 192 : 256;
 }
 
 // x: [rows, k] bfloat16 contiguous, sorted by group; w: [groups, n, k] bfloat16 contiguous; offsets: [groups + 1]
@@ -557,7 +563,7 @@ extern "C" int einf_gemm_grouped_tcgen05(const void* x, const void* w, const int
                                          cudaStream_t stream) {
   if (rows == 0 || n == 0 || groups == 0) return 0;
   if (k % 8 != 0 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15)) return (int)cudaErrorInvalidValue;
-  const int token_tile = einf_gemm_grouped_tcgen05_token_tile(rows, groups);
+  const int token_tile = einf_gemm_grouped_tcgen05_token_tile(rows, groups, n);
   const int total_kblocks = (k + kBlockK - 1) / kBlockK;
   if (splits != einf_gemm_tcgen05_splits(k, splits)) return (int)cudaErrorInvalidValue;   // the caller sized out for it
   const int per_split = (total_kblocks + splits - 1) / splits;

@@ -10,6 +10,7 @@ scheduler), and, marked ``gpu``, on the kernels in float32 and bfloat16.
 from __future__ import annotations
 
 import copy
+import ctypes
 import json
 import math
 
@@ -643,3 +644,15 @@ def test_greedy_generation_through_the_entry_point(lookahead, graphs, folders):
     prompts, got = generation(folder, config, weights, "float32", "cuda:0", lookahead, graphs)
     for prompt, tokens in zip(prompts, got):
         assert tokens == greedy_plain(config, weights, prompt, 8)
+
+
+def test_the_routed_products_larger_tiles_are_for_launches_of_more_than_a_wave():
+    """Tiles of 192 and 256 rows only where tiles of 128 would be more CTAs than run at once (two on each of 148
+    multiprocessors): 1,536 outputs of eight experts are 96 CTAs a tile of rows."""
+    from einf_b200 import ops
+
+    tile = ops._fn("einf_gemm_grouped_tcgen05_token_tile", [ctypes.c_int] * 3)
+    assert [tile(rows, 8, 1536) for rows in (8, 64 * 8, 85 * 8, 86 * 8, 200 * 8, 384 * 8)] == [16, 96, 128, 128, 128, 128]
+    assert [tile(rows, 8, 1536) for rows in (385 * 8, 512 * 8)] == [256, 256]
+    assert [tile(rows, 8, 17920) for rows in (64 * 8, 86 * 8, 128 * 8, 129 * 8, 4096)] == [96, 192, 192, 256, 256]
+    assert tile(5, 64, 128) == 16
