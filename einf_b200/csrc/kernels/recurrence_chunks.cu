@@ -753,7 +753,8 @@ using namespace einf;
 
 // q, k, v: bfloat16, 8-byte aligned rows (strides and sizes in multiples of four elements), the state 16-byte aligned; dim
 // up to 128.  Portions of min_len tokens and more are taken, `portions` of them at most.  `slots`: 0 where none of them is
-// longer than segment_len; else tokens / segment_len + portions, with segment_len a multiple of 64.  `tiles`: columns of the state that a CTA takes, in eights (4, 8 or 10).
+// longer than segment_len; else tokens / segment_len + portions, with segment_len a multiple of 64.  `tiles`: columns of the
+// state that a CTA takes, in eights (4 or 8; 10 where dim is 64 at most).
 extern "C" int einf_linear_recurrence_chunks(const void* q, const void* k, const void* v, long long q_stride,
                                              long long k_stride, long long v_stride, const float* head_decay,
                                              const float* token_decay, const float* token_scale, const float* skip,
@@ -784,17 +785,15 @@ extern "C" int einf_linear_recurrence_chunks(const void* q, const void* k, const
   a.wide = (!((uintptr_t)q & 15) && q_stride % 8 == 0 && dim % 8 == 0 ? 1 : 0) |
            (!((uintptr_t)k & 15) && k_stride % 8 == 0 && dim % 8 == 0 ? 2 : 0) |
            (!((uintptr_t)v & 15) && v_stride % 8 == 0 && vdim % 8 == 0 ? 4 : 0) | (vdim % 8 == 0 ? 8 : 0);
-#define EINF_CHUNKS(NT_)                                                                              \
-  if (tiles == NT_) {                                                                                 \
-    if (dim <= 64)                                                                                    \
-      return act ? (int)run_chunks<64, NT_, true>(a, portions, slots, stream)                                   \
-                 : (int)run_chunks<64, NT_, false>(a, portions, slots, stream);                          \
-    return act ? (int)run_chunks<128, (NT_ > 8 ? 8 : NT_), true>(a, portions, slots, stream)                    \
-               : (int)run_chunks<128, NT_, false>(a, portions, slots, stream);                           \
-  }
-  EINF_CHUNKS(4)
-  EINF_CHUNKS(8)
-  EINF_CHUNKS(10)
+#define EINF_CHUNKS(ROWS_, NT_)                                                                                  \
+  if (dim <= ROWS_ && tiles == NT_)                                                                             \
+    return act ? (int)run_chunks<ROWS_, NT_, true>(a, portions, slots, stream)                                  \
+               : (int)run_chunks<ROWS_, NT_, false>(a, portions, slots, stream);
+  EINF_CHUNKS(64, 4)
+  EINF_CHUNKS(64, 8)
+  EINF_CHUNKS(64, 10)
+  EINF_CHUNKS(128, 4)
+  EINF_CHUNKS(128, 8)
 #undef EINF_CHUNKS
   return (int)cudaErrorInvalidValue;
 }
