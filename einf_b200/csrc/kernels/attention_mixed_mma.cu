@@ -5,17 +5,20 @@
 // it is sum_c q'_(h, c) . k_c - slope'_h distance, one query [q'_(h, 0) | q'_(h, 1) ..] against the key heads' rows end to end.
 // So the heads meet in the queries, once a query, and not in every score (heads^2 FMAs a key, which with the exchange of all
 // heads' scores through shared memory bounded the kernel of attention_mixed_tiled.cu), and a head's softmax and values
-// are those of plain attention.  q' is 32-bit and enters the products as three bfloat16 parts (mma_sync.cuh), the weights
-// enter the second product as two, as they did; scores, sums and the output are 32-bit.
+// are those of plain attention.  q' is 32-bit and enters the products as three bfloat16 parts (mma_sync.cuh).  The weights
+// of up to 16 heads' prompts enter the second product as two, as in the tensor-core kernel of attention_mixed_tiled.cu;
+// those of more heads and of single tokens, whose kernels there hold them in 32 bits, as three, whose sums are added to
+// the output by rounded additions.  Scores, sums and the output are 32-bit.
 //
 // A CTA has 64 queries of one head, a warp 16 of them; 64 keys a tile; the next tile's keys are brought while this one's
 // values are used and the other way round.  The parts of q' stay in shared memory: in registers (96 of them) they leave two
 // CTAs an SM and no room for sums that do not wait for one another.  Takes key heads of together up to 128 elements (a
 // multiple of 16 each) and value heads up to 64 or 128 (a multiple of 8).
 //
-// Measured (B200): 14 heads of 64 on 2 key heads, window 1,024, 2,048 tokens: 283 -> 128 us (with q' in registers 163); 32
-// heads of 32 on 4, 1,024 tokens: 685 -> 119 us.  Of the products (256 a tile and warp) a third of the time; the rest is
-// the softmax between them and what a tile's four barriers cost three CTAs an SM.
+// Measured (B200): 14 heads of 64 on 2 key heads, window 1,024, 2,048 tokens: 283 -> 117 us (with q' in registers 163); 32
+// heads of 32 on 4, 1,024 tokens: 685 -> 136 us (119 with weights of two parts).  The tensor pipe is active 40 and 31 % of the
+// time, a scheduler issues in 46 % of its cycles: the rest is the softmax between the products and what a tile's four
+// barriers cost three CTAs an SM.
 #include <type_traits>
 
 #include "mma_sync.cuh"
@@ -45,8 +48,35 @@ __device__ __forceinline__ uint32_t swizzled(int row, int piece, int pitch) {
 template <int VALUE>
 constexpr int kMixSmem = 3 * kMixRows * kMixKeySize * 2 + kMixKeys * (kMixKeySize + VALUE) * 2;
 
-// VALUE: vdim filled up to 64 or 128.
-template <int VALUE>
+// Weights x and y as PARTS pairs of bfloat16, largest first: two are 16 bits of each, three all 24.
+template <int PARTS>
+__device__ __forceinline__ void split_weights(float x, float y, uint32_t (&part)[PARTS][4], int e) {
+#pragma unroll
+  for (int p = 0; p < PARTS; ++p) {
+    part[p][e] = pack_pair(x, y);
+    x -= low_bf16(part[p][e]);
+    y -= high_bf16(part[p][e]);
+  }
+}
+
+// O += P V of 16 keys for four column tiles, P in three parts: as mma_parts does it, the tiles side by side.
+__device__ __forceinline__ void add_weighted(float (*O)[4], const uint32_t (&P)[3][4], const uint32_t (&vf)[2][4]) {
+  float sum[4][4];
+#pragma unroll
+  for (int p = 2; p >= 0; --p)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (p == 2) mma_bf16_16816_zero(sum[j], P[p], vf[j >> 1][2 * (j & 1)], vf[j >> 1][2 * (j & 1) + 1]);
+      else mma_bf16_16816(sum[j], P[p], vf[j >> 1][2 * (j & 1)], vf[j >> 1][2 * (j & 1) + 1]);
+    }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) O[j][e] += sum[j][e];
+}
+
+// VALUE: vdim filled up to 64 or 128; PARTS: of the weights.
+template <int VALUE, int PARTS>
 __global__ void __launch_bounds__(kMixThreads, VALUE <= 64 ? 3 : 2)
 mixed_prompt_attention_kernel(const __grid_constant__ MixArgs a) {
   extern __shared__ __align__(128) unsigned char mix_smem[];
@@ -269,24 +299,33 @@ mixed_prompt_attention_kernel(const __grid_constant__ MixArgs a) {
     __syncthreads();
     if (seen) {
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {                 // the weights are the first operand as they lie in registers, two parts
-        uint32_t hi[4], lo[4];
+      for (int kk = 0; kk < 4; ++kk) {                 // the weights are the first operand as they lie in registers
+        uint32_t P[PARTS][4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float x = S[2 * kk + (e >> 1)][2 * (e & 1)], y = S[2 * kk + (e >> 1)][2 * (e & 1) + 1];
-          hi[e] = pack_pair(x, y);
-          lo[e] = pack_pair(x - low_bf16(hi[e]), y - high_bf16(hi[e]));
-        }
+        for (int e = 0; e < 4; ++e)
+          split_weights<PARTS>(S[2 * kk + (e >> 1)][2 * (e & 1)], S[2 * kk + (e >> 1)][2 * (e & 1) + 1], P, e);
+        if constexpr (PARTS == 3) {
 #pragma unroll
-        for (int j0v = 0; j0v < VALUE / 16; j0v += 4) {
-          uint32_t vf[4][4];
+          for (int j = 0; j < VALUE / 16; j += 2) {
+            uint32_t vf[2][4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            ldsm_x4_trans(vf[j], base + kV + swizzled(16 * kk + in8 + 8 * second, 2 * (j0v + j) + third, kValuePitch));
+            for (int u = 0; u < 2; ++u)
+              ldsm_x4_trans(vf[u], base + kV + swizzled(16 * kk + in8 + 8 * second, 2 * (j + u) + third, kValuePitch));
+            add_weighted(O + 2 * j, P, vf);
+          }
+        } else {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) mma_bf16_16816(O[2 * j0v + j], lo, vf[j >> 1][2 * (j & 1)], vf[j >> 1][2 * (j & 1) + 1]);
+          for (int j0v = 0; j0v < VALUE / 16; j0v += 4) {
+            uint32_t vf[4][4];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) mma_bf16_16816(O[2 * j0v + j], hi, vf[j >> 1][2 * (j & 1)], vf[j >> 1][2 * (j & 1) + 1]);
+            for (int j = 0; j < 4; ++j)
+              ldsm_x4_trans(vf[j], base + kV + swizzled(16 * kk + in8 + 8 * second, 2 * (j0v + j) + third, kValuePitch));
+#pragma unroll
+            for (int p = PARTS - 1; p >= 0; --p)
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                mma_bf16_16816(O[2 * j0v + j], P[p], vf[j >> 1][2 * (j & 1)], vf[j >> 1][2 * (j & 1) + 1]);
+          }
         }
       }
     }
@@ -322,7 +361,7 @@ mixed_prompt_attention_kernel(const __grid_constant__ MixArgs a) {
 // what the CTAs of a token found in the join below.
 //
 // Bound by the latencies of a CTA's few chunks.  Measured (B200): 64 tokens behind 2,048, 14 heads of 64 on 2, four CTAs a
-// token: 68 -> 23 us (the FMA kernel of attention_mixed_tiled.cu), the join 2.8 either way.
+// token: 68 -> 25 us (the FMA kernel of attention_mixed_tiled.cu; 23 with weights of two parts), the join 2.8 either way.
 constexpr int kSingleChunk = 32, kSingleHeads = 16, kSinglePitch = 256;
 constexpr int kSingleQ = 3 * kSingleHeads * kSinglePitch, kSingleWarp = 2 * kSingleChunk * kSinglePitch;
 constexpr int kSingleSmem = kSingleQ + 4 * kSingleWarp, kSingleOPitch = 136;
@@ -502,22 +541,18 @@ mixed_single_attention_kernel(const __grid_constant__ SingleArgs s) {
     __syncwarp();
 #pragma unroll
     for (int kk = 0; kk < 2; ++kk) {
-      uint32_t hi[4], lo[4];
+      uint32_t P[3][4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float x = S[2 * kk + (e >> 1)][2 * (e & 1)], y = S[2 * kk + (e >> 1)][2 * (e & 1) + 1];
-        hi[e] = pack_pair(x, y);
-        lo[e] = pack_pair(x - low_bf16(hi[e]), y - high_bf16(hi[e]));
-      }
+      for (int e = 0; e < 4; ++e)
+        split_weights<3>(S[2 * kk + (e >> 1)][2 * (e & 1)], S[2 * kk + (e >> 1)][2 * (e & 1) + 1], P, e);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (16 * j >= value_width) break;
-        uint32_t vf[4];
-        ldsm_x4_trans(vf, values_at + swizzled(16 * kk + in8 + 8 * second, 2 * j + third, kSinglePitch));
-        mma_bf16_16816(O[2 * j], lo, vf[0], vf[1]);
-        mma_bf16_16816(O[2 * j + 1], lo, vf[2], vf[3]);
-        mma_bf16_16816(O[2 * j], hi, vf[0], vf[1]);
-        mma_bf16_16816(O[2 * j + 1], hi, vf[2], vf[3]);
+      for (int j = 0; j < 8; j += 2) {
+        if (16 * j >= value_width) break;              // the last pair may reach into columns of zeros
+        uint32_t vf[2][4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          ldsm_x4_trans(vf[u], values_at + swizzled(16 * kk + in8 + 8 * second, 2 * (j + u) + third, kSinglePitch));
+        add_weighted(O + 2 * j, P, vf);
       }
     }
     __syncwarp();                                      // the values are used up
@@ -606,9 +641,9 @@ __global__ void __launch_bounds__(kMixThreads) mixed_single_join_kernel(const __
   a.out[(size_t)t * outs + o] = __float2bfloat16_rn(sum > 0.f ? value / sum * a.out_scale : 0.f);
 }
 
-template <int VALUE>
+template <int VALUE, int PARTS>
 static cudaError_t launch_mixed_prompt(const MixArgs& a, int num_tiles, cudaStream_t stream) {
-  auto kernel = mixed_prompt_attention_kernel<VALUE>;
+  auto kernel = mixed_prompt_attention_kernel<VALUE, PARTS>;
   constexpr int kBytes = kMixSmem<VALUE>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
   if (e != cudaSuccess) return e;
@@ -640,7 +675,9 @@ extern "C" int einf_mixed_prompt_attention(const void* q, const void* k_cache, c
   a.heads = heads; a.kv_heads = kv_heads; a.dim = dim; a.vdim = vdim; a.page_size = page_size; a.num_pages = num_pages;
   a.window = window; a.wave = wave;
   a.scale_log2 = scale * 1.4426950408889634f; a.out_scale = out_scale;
-  return (int)(vdim <= 64 ? launch_mixed_prompt<64>(a, num_tiles, stream) : launch_mixed_prompt<128>(a, num_tiles, stream));
+  if (heads <= 16)
+    return (int)(vdim <= 64 ? launch_mixed_prompt<64, 2>(a, num_tiles, stream) : launch_mixed_prompt<128, 2>(a, num_tiles, stream));
+  return (int)(vdim <= 64 ? launch_mixed_prompt<64, 3>(a, num_tiles, stream) : launch_mixed_prompt<128, 3>(a, num_tiles, stream));
 }
 
 // One token each of `num_items` requests (`items`: token indices, null: tokens 0 .. num_items - 1); `splits` CTAs share a

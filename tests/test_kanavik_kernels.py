@@ -133,6 +133,47 @@ def test_mixing_in_the_queries(dev, heads, kv_heads, size, vsize, window, parts)
         first += n
 
 
+@pytest.mark.parametrize("heads, kv_heads, size, vsize, n", [
+    (14, 2, 64, 64, 1), (16, 1, 128, 128, 1), (4, 4, 16, 24, 1), (20, 2, 64, 64, 5), (32, 4, 32, 128, 4), (24, 8, 16, 8, 2)])
+def test_mixed_weights_hold_32_bits(dev, heads, kv_heads, size, vsize, n):
+    """Single tokens of up to 16 heads and portions of more, over five keys whose values (chosen one after the other, for the last
+    token and the first head of every key head) nearly cancel under the weights, so that what is left shows the weights'
+    own rounding.  The bound: the output's rounding (2^-8 of it) and 12 roundings to 32 bits of the sum of the terms' sizes
+    (scores below one: a score's sums, exp2 and the sum of values; weights of 16 bits are off by up to 2^-16, 256 of those)."""
+    from einf_b200 import ops
+
+    requests = [(5 - n, n)] * 12
+    (q, k, v, table, seq, pos), scale, _ = _attention_case(dev, torch.bfloat16, heads, kv_heads, size, 16, requests, None)
+    scale, per = scale / 4, heads // kv_heads
+    generator = torch.Generator().manual_seed(13)
+    v = torch.zeros((*k.shape[:3], vsize), dtype=torch.bfloat16, device=dev)
+    group, exact = torch.arange(heads, device=dev) // per, []
+    for r in range(len(requests)):
+        page = int(table[r, 0])
+        keys = k[page].transpose(0, 1)[:5].double()[:, group]
+        scores = torch.einsum("ihd,jhd->hij", q[n * r:n * (r + 1)].double(), keys) * scale
+        seen = torch.arange(5, device=dev)[None, :] <= torch.arange(5 - n, 5, device=dev)[:, None]
+        weights = torch.softmax(scores.masked_fill(~seen, float("-inf")), dim=2)
+        last = weights[::per, -1]                                          # [kv_heads, 5]
+        v[page, :, 0] = (1 + torch.rand((kv_heads, vsize), generator=generator)).to(torch.bfloat16).to(dev)
+        for j in range(1, 4):
+            so_far = torch.einsum("gj,gjd->gd", last[:, :j], v[page, :, :j].double())
+            v[page, :, j] = (-so_far / last[:, j, None]).to(torch.bfloat16)
+        exact.append((weights, v[page].transpose(0, 1)[:5].double()[:, group]))
+    q_tiles, singles = _step_split(requests)
+    out = torch.full((q.shape[0], heads, vsize), float("nan"), dtype=torch.bfloat16, device=dev)
+    st = status(dev)
+    assert ops.mixed_single_takes(q, k, v) if n == 1 else ops.mixed_prompt_takes(q, k, v, out, q_tiles.shape[0], None, 5)
+    ops.paged_attention_mixed(q, k, v, table, seq, pos, out, scale, None, None, None, None, 1.0, st, q_tiles=q_tiles.to(dev),
+                              single_tokens=singles.to(dev), num_singles=singles.shape[0], max_context=5)
+    assert int(st) == 0
+    for r, (weights, values) in enumerate(exact):
+        want, size_of = (torch.einsum("hij,jhv->ihv", weights, t) for t in (values, values.abs()))
+        assert float(want[-1, ::per].abs().max()) < 2.0 ** -14
+        error = (out[n * r:n * (r + 1)].double() - want).abs()
+        assert bool((error <= 2.0 ** -8 * want.abs() + 12 * 2.0 ** -24 * size_of).all()), float((error / size_of).max() * 2 ** 24)
+
+
 @pytest.mark.parametrize("heads, kv_heads, size, vsize, window", [
     (14, 2, 64, 64, 100), (16, 1, 128, 128, None), (5, 1, 8, 24, 33), (4, 4, 32, 16, 1), (6, 3, 40, 40, None),
 ])
