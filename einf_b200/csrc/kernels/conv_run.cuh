@@ -9,7 +9,7 @@
 namespace einf {
 
 constexpr int kRunTokens = 8, kRunTaps = 4;
-constexpr long long kRunElements = 1 << 19;      // of a launch from which runs are the faster way (einf_conv_silu)
+constexpr long long kRunElements = 1 << 19;      // of a launch above which runs are the faster way (einf_conv_silu)
 
 template <typename T>
 __device__ __forceinline__ float4 load_quad(const T* p) {

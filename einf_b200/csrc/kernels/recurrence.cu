@@ -998,11 +998,11 @@ extern "C" int einf_conv_silu(const void* in, int dtype, long long in_stride, co
   // 64 single tokens of 896 channels took 17 us this way, every thread one chain of state rows, against 7.  And enough of
   // them: a thread's eleven rows are a chain that a small launch does not hide (whole call, us, an element / a run a
   // thread: 100 tokens of 896 channels 10.2 / 16.4, of 3,328 14.3 / 16.4; 512 of 896 14.3 / 16.4; 640 of 896 16.4 / 16.4; 300 of
-  // 3,328 20.5 / 18.4; 2,048 of 256 16.4 / 14.4), so from 2^19 elements on.
+  // 3,328 20.5 / 18.4; 2,048 of 256 16.4 / 14.4), so above 2^19 elements.
   const size_t quad = dtype == kFloat32 ? 16 : 8;
   const long long run_threads = (long long)((num_tokens + kRunTokens - 1) / kRunTokens) * (channels / 4) +
                                 (long long)num_tokens * heads;
-  if (num_tokens >= 64ll * num_requests && (long long)num_tokens * channels >= kRunElements && taps <= kRunTaps &&
+  if (num_tokens >= 64ll * num_requests && (long long)num_tokens * channels > kRunElements && taps <= kRunTaps &&
       channels % 4 == 0 && in_stride % 4 == 0 && run_threads < (1ll << 31) && (uintptr_t)in % quad == 0 && (uintptr_t)out % quad == 0) {
     EINF_DISPATCH_2(dtype, T, {
       cudaError_t e = launch_pdl(conv_silu_run_kernel<T>, (int)((run_threads + 127) / 128), 128, 0, stream, (const T*)in,

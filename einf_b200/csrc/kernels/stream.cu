@@ -977,9 +977,10 @@ extern "C" int einf_norm_conv(const void* pend_a, int a_dtype, int a_splits, lon
       e = launch_pdl(norm_row_kernel<T>, num_tokens, threads, smem, stream, pending, scale, residual, weight, eps, conv_weight,
                      taps, conv_state, state_stride, num_slots, seq_of_token, state_slots, (T*)out, scratch, hidden, mode);
     if (e != cudaSuccess || mode != 2) return (int)e;
-    // runs of eight tokens for portions of 64 and more on average: 2,048 tokens of 896 channels 16 -> 7.4 us
+    // runs of eight tokens for portions of 64 and more on average: 2,048 tokens of 896 channels 16 -> 7.4 us (small launches as
+    // in einf_conv_silu: whole call, an element / a run a thread, 256 tokens of 896 16.4 / 18.4, 600 22.5 / 18.9)
     const long long run_threads = (long long)((num_tokens + kRunTokens - 1) / kRunTokens) * (hidden / 4);
-    if (quads && num_tokens >= 64ll * num_requests && run_threads < (1ll << 31)) {
+    if (quads && num_tokens >= 64ll * num_requests && (long long)num_tokens * hidden > kRunElements && run_threads < (1ll << 31)) {
       e = launch_pdl(conv_rows_run_kernel<T>, (int)((run_threads + 127) / 128), 128, 0, stream, (const float*)scratch,
                      conv_weight, taps, (const float*)conv_state, state_stride, num_slots, seq_of_token, q_start, state_slots,
                      (T*)out, hidden, num_tokens);
