@@ -276,18 +276,30 @@ static int launch(const SimtArgs& g, int share, int out_dtype, cudaStream_t stre
   return (int)launch_simt<TA, TW, __nv_bfloat16>(g, share, stream);
 }
 
-// How many CTAs share K: 1 while the output's tiles fill the GPU twice over; else enough to do so, each with
-// at least one block of 256 terms, as far as the blocks' sums take no more than `limit` bytes.  (545 x 896 outputs, 63 tiles,
-// K = 4,864: 291 us alone, 177 / 123 / 116 us with 4 / 8 / 16; 545 x 9,728, 684 tiles: 210 us alone, 242 with 2.)
+// How many CTAs share K, as far as the blocks' sums take no more than `limit` bytes.  CTAs run three an SM, but an SM's rate does
+// not grow with them, so a launch takes as long as the SM with the most blocks of 256 terms: CTAs an SM, rounded up, times
+// blocks a CTA.  Sharing costs three quarters of a block more (the workspace and the second kernel); of equal shares the
+// larger one, whose CTAs hide one another's waits better.  Measured (us, alone / the rule): 63 tiles, K = 4,864 295 / 129; 81, K =
+// 896 61 / 43; 200, K = 2,048 217 / 158; 288, K = 1,024 115 / alone (126 by two); 300, K = 896 136 / 118; 384, K = 1,024 160 / 164 (178
+// by two); 440, K = 515 95 / alone (112 by two); 448, K = 1,024 207 / 190.
 extern "C" int einf_gemm_simt_shares(int m, int n, int k, long long limit) {
   const long long tiles = (long long)((m + kRows - 1) / kRows) * ((n + kCols - 1) / kCols);
   const int blocks = (k + kBlock - 1) / kBlock;
-  int share = 1;
   if (tiles <= 0 || 4ll * blocks * m * n > limit) return 1;
-  while (share < blocks && tiles * share < 4 * 148) ++share;
-  // no CTA without a block
-  const int each = (blocks + share - 1) / share;
-  return each > 0 ? (blocks + each - 1) / each : 1;
+  constexpr int kSms = 148;
+  int share = 1;
+  long long best = 4 * ((tiles + kSms - 1) / kSms) * blocks;          // in quarters of a block
+  const long long alone = best;
+  for (int s = 2; s <= blocks; ++s) {
+    const int each = (blocks + s - 1) / s;
+    if ((blocks + each - 1) / each != s) continue;                    // no CTA without a block
+    const long long cost = 4 * ((tiles * s + kSms - 1) / kSms) * each + 3;
+    if (cost < alone && cost <= best) {
+      best = cost;
+      share = s;
+    }
+  }
+  return share;
 }
 
 // lda / ldo: row strides of A and out in elements (rows of A may be a strided view).  block_sums: [blocks of 256
