@@ -180,6 +180,12 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
 // scores are the same sums in the same order; the softmax goes by tiles of 64 keys instead of 32.  Bound by the
 // reads from shared memory and by the longest token's chain of tiles.  A key that a row does not see adds nothing to the
 // row, not even zero times its value: an infinity or NaN among a later token's values reaches no token before it.
+// The single tokens of the same step are the kernel above, launched first: an ordinary launch, which starts when everything
+// before it is complete and at once lets this one in.  With `beside` this kernel therefore reads and writes without a
+// wait (other rows of the output) and waits for that one at its end, so that what follows finds both complete.  (64 tokens and
+// 32 single ones, each behind 2,048, us, all by the kernel above / one behind the other / beside: 14 heads of 64 in 32 bits
+// 1,334 / 1,557 / 1,372, of 72 in bfloat16 1,471 / 2,098 / 1,539; 28 heads of 128 2,497 / 2,756 / 2,773, where the single
+// tokens' CTAs fill the GPU and the two do not help each other.)
 // ---------------------------------------------------------------------------
 constexpr int kPromptRows = 32, kPromptKeys = 64, kPromptThreads = 128;
 constexpr float kHidden = -1.f;      // in a weight's place: the row does not see the key (weights are never negative)
@@ -192,6 +198,7 @@ struct PromptArgs {
   int num_heads, num_kv_heads, head_size, value_size, value_stride, page_size, num_pages, table_width;
   float scale, softcap;
   int window, keep_first, chunk;
+  int beside;                                     // runs beside the kernel launched before it, see below
 };
 
 __device__ __forceinline__ void prompt_copy16(float* smem, const float* gmem) {
@@ -208,7 +215,7 @@ __global__ void __launch_bounds__(kPromptThreads)
 paged_attention_prompt_kernel(const __grid_constant__ PromptArgs a) {
   extern __shared__ __align__(16) float prompt_smem[];
   pdl_launch_dependents();
-  pdl_wait();
+  if (!a.beside) pdl_wait();
   const int head_size = a.head_size, value_size = a.value_size;
   const int key_pitch = head_size + 4, value_pitch = 64 * COLS + 4;
   constexpr int kScorePitch = kPromptKeys + 4;
@@ -405,6 +412,7 @@ paged_attention_prompt_kernel(const __grid_constant__ PromptArgs a) {
         out[d] = from_float<T>(o);
       }
   }
+  if (a.beside) pdl_wait();
 }
 
 template <typename T, int COLS>
@@ -648,17 +656,14 @@ extern "C" int einf_paged_attention_generic(const void* q, const void* k_cache, 
   const int blocks = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
   if (value_stride < value_size) return (int)cudaErrorInvalidValue;
   EINF_DISPATCH_2(dtype, T, {
-    if (head_size <= 256 && value_size <= 256) {
-      paged_attention_generic_kernel<T, 256><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(
+    auto launch = [&](auto kernel) {
+      kernel<<<blocks, kWarpsPerBlock * 32, 0, stream>>>(
           (const T*)q, (const T*)k_cache, (const T*)v_cache, block_table, seq_of_token, positions, (T*)out,
           rows, num_heads, num_kv_heads, head_size, value_size, value_stride, page_size, num_pages, table_width,
           scale, window, keep_first, chunk, softcap, sink, gate, (const T*)value_gate, value_gate_stride, tokens, status);
-    } else {
-      paged_attention_generic_kernel<T, kMaxHeadSize><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(
-          (const T*)q, (const T*)k_cache, (const T*)v_cache, block_table, seq_of_token, positions, (T*)out,
-          rows, num_heads, num_kv_heads, head_size, value_size, value_stride, page_size, num_pages, table_width,
-          scale, window, keep_first, chunk, softcap, sink, gate, (const T*)value_gate, value_gate_stride, tokens, status);
-    }
+    };
+    if (head_size <= 256 && value_size <= 256) launch(paged_attention_generic_kernel<T, 256>);
+    else launch(paged_attention_generic_kernel<T, kMaxHeadSize>);
   })
   return (int)cudaGetLastError();
 }
@@ -713,13 +718,14 @@ extern "C" int einf_latent_decode_merge(const float* part_acc, const float* part
   })
 }
 
-// Portions of prompts: the tokens that `q_tiles` lists.  Key and value sizes up to 128, multiples of four.
+// Portions of prompts: the tokens that `q_tiles` lists.  Key and value sizes up to 128, multiples of four.  `beside`: the launch
+// before this one on the stream is einf_paged_attention_generic on other tokens of the same step.
 extern "C" int einf_paged_attention_prompt(const void* q, const void* k_cache, const void* v_cache, int dtype,
                                            const int* block_table, const int* q_tiles, int num_tiles, void* out,
                                            int num_heads, int num_kv_heads, int head_size, int value_size, int value_stride,
                                            int page_size, int num_pages, int table_width, float scale, int window,
                                            int keep_first, int chunk, float softcap, const float* sink, const float* gate,
-                                           const void* value_gate, long long value_gate_stride, int* status,
+                                           const void* value_gate, long long value_gate_stride, int beside, int* status,
                                            cudaStream_t stream) {
   if (num_tiles == 0) return 0;
   if (head_size <= 0 || head_size > 128 || head_size % 4 || value_size <= 0 || value_size > 128 || value_size % 4 ||
@@ -736,6 +742,7 @@ extern "C" int einf_paged_attention_prompt(const void* q, const void* k_cache, c
   a.value_stride = value_stride; a.page_size = page_size; a.num_pages = num_pages; a.table_width = table_width;
   a.scale = scale; a.softcap = softcap;
   a.window = window; a.keep_first = window > 0 ? keep_first : 0; a.chunk = chunk;
+  a.beside = beside;
   EINF_DISPATCH_2(dtype, T, {
     if (value_size <= 64) return (int)launch_prompt<T, 1>(a, num_tiles, stream);
     return (int)launch_prompt<T, 2>(a, num_tiles, stream);

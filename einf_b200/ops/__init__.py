@@ -591,6 +591,7 @@ def paged_attention_generic(
     value_gate: Optional[torch.Tensor] = None,
     q_tiles: Optional[torch.Tensor] = None,
     single_tokens: Optional[torch.Tensor] = None,
+    cached_before: Optional[int] = None,
 ) -> None:
     """Causal attention of every token of the batch over the pages of its request.
 
@@ -608,8 +609,9 @@ def paged_attention_generic(
     a wider matrix): every element of the mixed heads is multiplied by the sigmoid of its own logit.
 
     ``q_tiles`` (int32 ``[tiles, 4]``: request, first token, rows up to 128, first position) and ``single_tokens``
-    (int32) list the step's tokens by portions: portions of ``PROMPT_TILE_MIN`` tokens a tile or more, on average, then
-    take a kernel that shares key rows between their tokens, where it takes the sizes.
+    (int32) list the step's tokens by portions: portions of :func:`prompt_tile_min` tokens a tile or more, on average, then
+    take a kernel that shares key rows between their tokens, where it takes the sizes, beside the single tokens'.
+    ``cached_before``: the longest cached prefix of a portion, where the host knows it.
     """
     tokens, num_heads, head_size = q.shape
     if sink is not None and (sink.dtype != torch.float32 or sink.shape != (num_heads,)):
@@ -638,40 +640,39 @@ def paged_attention_generic(
     options = (float(scale), int(window) if window else 0, int(keep_first) if window else 0, int(chunk) if chunk else 0,
                float(softcap) if softcap else 0.0, _opt(sink, "sink", torch.float32), _opt(gate, "gate", torch.float32),
                *_value_gate(value_gate, q, value_size, False))
-    singles = None
-    if q_tiles is not None and single_tokens is not None and _takes_prompt_tiles(
-            q_tiles, tokens - single_tokens.shape[0], head_size, value_size, value_stride, k_cache, v_cache):
+    tiled = q_tiles is not None and single_tokens is not None and _takes_prompt_tiles(
+        q_tiles, tokens - single_tokens.shape[0], head_size, value_size, value_stride, k_cache, v_cache,
+        prompt_tile_min(q.dtype, cached_before))
+    listed = tokens if not tiled else single_tokens.shape[0]
+    if listed:
+        fn = _fn(
+            "einf_paged_attention_generic",
+            [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+             c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p,
+             c_longlong, c_void_p, c_void_p, c_void_p],
+        )
+        _check(
+            fn(_dev(q, "q"), _dev(k_cache, "k_cache"), _dev(v_cache, "v_cache"), _code(q),
+               _opt(block_table, "block_table", torch.int32), _opt(seq_of_token, "seq_of_token", torch.int32),
+               _opt(positions, "positions", torch.int32), _dev(out, "out"), listed, num_heads, num_kv_heads,
+               head_size, value_size, value_stride, page_size, num_pages, block_table.shape[1], *options,
+               _opt(single_tokens if tiled else None, "single_tokens", torch.int32), _dev(status, "status"), _stream()),
+            "paged_attention_generic",
+        )
+    if tiled:
         fn = _fn(
             "einf_paged_attention_prompt",
             [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int,
              c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p, c_longlong,
-             c_void_p, c_void_p],
+             c_int, c_void_p, c_void_p],
         )
         _check(
             fn(_dev(q, "q"), _dev(k_cache, "k_cache"), _dev(v_cache, "v_cache"), _code(q),
                _opt(block_table, "block_table", torch.int32), _opt(q_tiles, "q_tiles", torch.int32), q_tiles.shape[0],
                _dev(out, "out"), num_heads, num_kv_heads, head_size, value_size, value_stride, page_size, num_pages,
-               block_table.shape[1], *options, _dev(status, "status"), _stream()),
+               block_table.shape[1], *options, 1 if listed else 0, _dev(status, "status"), _stream()),
             "paged_attention_prompt",
         )
-        tokens = single_tokens.shape[0]
-        if tokens == 0:
-            return
-        singles = single_tokens
-    fn = _fn(
-        "einf_paged_attention_generic",
-        [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
-         c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p,
-         c_longlong, c_void_p, c_void_p, c_void_p],
-    )
-    _check(
-        fn(_dev(q, "q"), _dev(k_cache, "k_cache"), _dev(v_cache, "v_cache"), _code(q),
-           _opt(block_table, "block_table", torch.int32), _opt(seq_of_token, "seq_of_token", torch.int32),
-           _opt(positions, "positions", torch.int32), _dev(out, "out"), tokens, num_heads, num_kv_heads,
-           head_size, value_size, value_stride, page_size, num_pages, block_table.shape[1], *options,
-           _opt(singles, "single_tokens", torch.int32), _dev(status, "status"), _stream()),
-        "paged_attention_generic",
-    )
 
 
 #: tokens of prompt portions per tile of ``q_tiles``, on average, from which they take the kernel that shares key rows (a
@@ -679,10 +680,22 @@ def paged_attention_generic(
 PROMPT_TILE_MIN = 8
 
 
+def prompt_tile_min(dtype: torch.dtype, cached_before: Optional[int]) -> int:
+    """From how many tokens of prompt portions a tile on the kernel that shares key rows is the faster one: ``PROMPT_TILE_MIN``
+    behind a cached prefix, where the general kernel's chain of keys is the longer one (us, general / shared, 14 heads of 64 in
+    32 bits: 8 tokens behind 2,048 keys 1,018 / 199; of 72 in bfloat16 1,169 / 596); at the start of a prompt more (8 tokens
+    12.8 / 14.3 and 14.3 / 18.4, 16 tokens 18.4 / 14.3 and 18.4 / 20.5, 64 tokens 41 / 16 and 43 / 27).  A prefix counts as
+    one from where the other prefill launches take it for one (:func:`prefill_prefix_bucket`), so that steps that are
+    captured as one launch alike."""
+    if cached_before is None or prefill_prefix_bucket(cached_before) > 1:
+        return PROMPT_TILE_MIN
+    return 16 if dtype == torch.float32 else 32
+
+
 def _takes_prompt_tiles(q_tiles: torch.Tensor, tokens: int, head_size: int, value_size: int, value_stride: int,
-                        k_cache: torch.Tensor, v_cache: torch.Tensor) -> bool:
+                        k_cache: torch.Tensor, v_cache: torch.Tensor, least: int = PROMPT_TILE_MIN) -> bool:
     return (
-        q_tiles.shape[0] > 0 and tokens >= PROMPT_TILE_MIN * q_tiles.shape[0] and head_size <= 128 and head_size % 4 == 0
+        q_tiles.shape[0] > 0 and tokens >= least * q_tiles.shape[0] and head_size <= 128 and head_size % 4 == 0
         and value_size <= 128 and value_size % 4 == 0 and value_stride % 4 == 0
         and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0
         and k_cache.shape[0] * k_cache.shape[1] * k_cache.shape[2] <= 0x7fffffff

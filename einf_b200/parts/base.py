@@ -216,7 +216,7 @@ class StepContext:
         the plain statements that stand in for them there take every token alone)."""
         if not self.q_tiles.is_cuda:
             return {}
-        return {"q_tiles": self.q_tiles, "single_tokens": self.single_tokens}
+        return {"q_tiles": self.q_tiles, "single_tokens": self.single_tokens, "cached_before": self.max_portion_start}
 
 
 class Part:

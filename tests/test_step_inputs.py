@@ -136,6 +136,14 @@ def test_the_prefix_bucket_is_what_a_prefill_launch_keeps_of_the_contexts():
     assert [ops.prefill_prefix_bucket(n) for n in (None, 0, 511, 512, 1023, 1024, 10 ** 6)] == [1, 1, 1, 4, 4, 8, 8]
 
 
+def test_short_portions_share_key_rows_behind_a_prefix_alone():
+    """From how many tokens a tile the general attention takes portions 32 tokens at a time: what is captured by the prefix
+    bucket decides, so that a graph holds the kernel that its steps would take."""
+    f32, bf16 = torch.float32, torch.bfloat16
+    assert [ops.prompt_tile_min(f32, n) for n in (None, 0, 511, 512, 10 ** 6)] == [8, 16, 16, 8, 8]
+    assert [ops.prompt_tile_min(bf16, n) for n in (None, 0, 511, 512, 10 ** 6)] == [8, 32, 32, 8, 8]
+
+
 def test_the_context_bucket_is_what_a_decode_launch_keeps_of_the_contexts():
     assert [ops.decode_context_bucket(n) for n in (None, 0, 1, 4096, 4097, 8192, 8193, 32768, 100000)] == [
         4096, 4096, 4096, 4096, 8192, 8192, 16384, 32768, 131072]
