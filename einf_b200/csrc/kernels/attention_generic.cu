@@ -63,7 +63,7 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
                                int table_width, float scale, int window, int keep_first, int chunk, float softcap,
                                const float* __restrict__ sink, const float* __restrict__ gate,
                                const T* __restrict__ value_gate, long long value_gate_stride,
-                               const int* __restrict__ tokens, int* status) {
+                               const int* __restrict__ tokens, const int* __restrict__ q_start, int* status) {
   __shared__ float q_smem[kWarpsPerBlock][kHeadLimit];
   pdl_launch_dependents();
   pdl_wait();
@@ -76,6 +76,8 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
   const int kv_head = h / (num_heads / num_kv_heads);
   const int r = seq_of_token[t];
   const int pos = positions[t];
+  // a portion of several tokens that starts at position 0 is another kernel's
+  if (q_start && q_start[r + 1] - q_start[r] > 1 && positions[q_start[r]] == 0) return;
   int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
   if (chunk > 0) lo = max(lo, (pos / chunk) * chunk);
   const bool vectors = head_size % Vec<T>::N == 0;
@@ -193,6 +195,7 @@ constexpr float kHidden = -1.f;      // in a weight's place: the row does not se
 struct PromptArgs {
   const void* q; const void* k_cache; const void* v_cache; void* out;
   const int* block_table; const int* q_tiles;     // [tiles, 4]: request, first token, rows (up to 128), first position
+  const int* q_start;                             // as in the kernel above
   const float* sink; const float* gate; const void* value_gate; long long value_gate_stride;
   int* status;
   int num_heads, num_kv_heads, head_size, value_size, value_stride, page_size, num_pages, table_width;
@@ -230,6 +233,10 @@ paged_attention_prompt_kernel(const __grid_constant__ PromptArgs a) {
   const int rows = min(kPromptRows, tile[2] - sub);
   if (rows <= 0) return;
   const int t0 = tile[1] + sub, pos0 = tile[3] + sub;
+  if (a.q_start && a.q_start[request] == t0 - pos0) {
+    if (a.beside) pdl_wait();
+    return;
+  }
   const int h = blockIdx.y, kv_head = h / (a.num_heads / a.num_kv_heads);
   const int* table = a.block_table + (long long)request * a.table_width;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;       // scores: rows ty + 8 i, keys tx + 16 j
@@ -640,7 +647,8 @@ __global__ void latent_decode_merge_kernel(const float* __restrict__ part_acc, c
 
 using namespace einf;
 
-// `tokens`: the tokens to take (num_tokens of them), or null for all.
+// `tokens`: the tokens to take (num_tokens of them), or null for all.  `q_start`: the requests' first tokens, for portions of
+// several tokens that start at position 0 to be left out, or null.
 extern "C" int einf_paged_attention_generic(const void* q, const void* k_cache, const void* v_cache,
                                             int dtype, const int* block_table, const int* seq_of_token,
                                             const int* positions, void* out, int num_tokens,
@@ -648,7 +656,8 @@ extern "C" int einf_paged_attention_generic(const void* q, const void* k_cache, 
                                             int value_stride, int page_size, int num_pages, int table_width,
                                             float scale, int window, int keep_first, int chunk, float softcap,
                                             const float* sink, const float* gate, const void* value_gate,
-                                            long long value_gate_stride, const int* tokens, int* status, cudaStream_t stream) {
+                                            long long value_gate_stride, const int* tokens, const int* q_start, int* status,
+                                            cudaStream_t stream) {
   const int rows = num_tokens * num_heads;
   if (rows == 0) return 0;
   if (head_size > kMaxHeadSize || value_size > kMaxHeadSize || head_size <= 0 || value_size <= 0)
@@ -660,7 +669,8 @@ extern "C" int einf_paged_attention_generic(const void* q, const void* k_cache, 
       kernel<<<blocks, kWarpsPerBlock * 32, 0, stream>>>(
           (const T*)q, (const T*)k_cache, (const T*)v_cache, block_table, seq_of_token, positions, (T*)out,
           rows, num_heads, num_kv_heads, head_size, value_size, value_stride, page_size, num_pages, table_width,
-          scale, window, keep_first, chunk, softcap, sink, gate, (const T*)value_gate, value_gate_stride, tokens, status);
+          scale, window, keep_first, chunk, softcap, sink, gate, (const T*)value_gate, value_gate_stride, tokens,
+          q_start, status);
     };
     if (head_size <= 256 && value_size <= 256) launch(paged_attention_generic_kernel<T, 256>);
     else launch(paged_attention_generic_kernel<T, kMaxHeadSize>);
@@ -725,8 +735,8 @@ extern "C" int einf_paged_attention_prompt(const void* q, const void* k_cache, c
                                            int num_heads, int num_kv_heads, int head_size, int value_size, int value_stride,
                                            int page_size, int num_pages, int table_width, float scale, int window,
                                            int keep_first, int chunk, float softcap, const float* sink, const float* gate,
-                                           const void* value_gate, long long value_gate_stride, int beside, int* status,
-                                           cudaStream_t stream) {
+                                           const void* value_gate, long long value_gate_stride, int beside, const int* q_start,
+                                           int* status, cudaStream_t stream) {
   if (num_tiles == 0) return 0;
   if (head_size <= 0 || head_size > 128 || head_size % 4 || value_size <= 0 || value_size > 128 || value_size % 4 ||
       value_stride < value_size || value_stride % 4 || num_heads <= 0 || num_heads > 65535 || num_kv_heads <= 0 ||
@@ -742,7 +752,7 @@ extern "C" int einf_paged_attention_prompt(const void* q, const void* k_cache, c
   a.value_stride = value_stride; a.page_size = page_size; a.num_pages = num_pages; a.table_width = table_width;
   a.scale = scale; a.softcap = softcap;
   a.window = window; a.keep_first = window > 0 ? keep_first : 0; a.chunk = chunk;
-  a.beside = beside;
+  a.beside = beside; a.q_start = q_start;
   EINF_DISPATCH_2(dtype, T, {
     if (value_size <= 64) return (int)launch_prompt<T, 1>(a, num_tiles, stream);
     return (int)launch_prompt<T, 2>(a, num_tiles, stream);

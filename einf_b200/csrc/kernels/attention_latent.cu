@@ -45,6 +45,7 @@ struct LatentParams {
   const int* token_list;      // single tokens by their packed index (null: 0 .. n - 1)
   const int* seq_of_token;
   const int* positions;
+  const int* q_start;         // where given, tiles of portions that start at position 0 are another kernel's
   const int* block_table;     // [requests, table_width]
   __nv_bfloat16* out;         // [tokens, heads, value_size]
   float* part_acc;            // [single tokens, heads, splits, value_size], with splits > 1
@@ -82,6 +83,10 @@ latent_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const
     token0 = info.y;
     tokens = info.z;
     pos0 = info.w;
+    if (p.q_start && p.q_start[request] == token0 - pos0) {
+      pdl_wait();
+      return;
+    }
   } else {
     token0 = p.token_list ? p.token_list[blockIdx.x] : (int)blockIdx.x;
     tokens = 1;
@@ -401,13 +406,14 @@ extern "C" int einf_latent_attention_tcgen05_parts(int value_size) {
 
 // q: [tokens, heads, row] bfloat16, cache: [pages, 1, page_size, row]; out: [tokens, heads, value_size].  Either `tiles`
 // [num_tiles, 4] (prompt portions of up to 128 tokens each) or num_tiles single tokens (token_list, or 0 .. num_tiles - 1;
-// then seq_of_token and positions are read).  With splits > 1 the shares go to part_acc and part_ml.
+// then seq_of_token and positions are read).  With splits > 1 the shares go to part_acc and part_ml.  `q_start`: the requests'
+// first tokens, for `tiles` to be left out whose portion starts at position 0, or null.
 extern "C" int einf_latent_attention_tcgen05(const void* q, const void* cache, const int* block_table, const int* tiles,
                                              const int* token_list, const int* seq_of_token, const int* positions,
                                              int num_tiles, void* out, float* part_acc, float* part_ml, int num_tokens,
                                              int num_heads, int row_size, int value_size, int page_size, int num_pages,
                                              int table_width, float scale, int window, int splits, const float* sink,
-                                             const float* gate, int* status, cudaStream_t stream) {
+                                             const float* gate, const int* q_start, int* status, cudaStream_t stream) {
   if (num_tiles == 0) return 0;
   if (row_size % 64 || row_size <= 0 || row_size > 64 * kMaxSlices || value_size <= 0 || value_size > row_size ||
       num_heads <= 0 || page_size < 8 || page_size > 128 || (page_size & (page_size - 1)) || splits < 1 ||
@@ -427,6 +433,7 @@ extern "C" int einf_latent_attention_tcgen05(const void* q, const void* cache, c
   p.sink = sink;
   p.gate = gate;
   p.status = status;
+  p.q_start = q_start;
   p.num_heads = num_heads;
   p.value_size = value_size;
   p.page_size = page_size;

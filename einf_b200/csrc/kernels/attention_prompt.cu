@@ -6,7 +6,8 @@
 // Head by head, with keys [W_uk c | r] and values W_uv c, it is dim + rot_dim + value_size, a third of that at rows of
 // 512 + 64 and heads of 128, for one more product over the rows.  That pays for a prompt that is all there: every row is
 // projected once and met by all later queries.  (A portion with cached tokens before it would project those anew in
-// every step, a single token would project all it sees: both stay on the rows.)
+// every step, a single token would project all it sees: both stay on the rows.  Which portions of a step are which is told
+// here, by q_start, tile by tile: what a prompt gets does not depend on what stands beside it.)
 //
 // A CTA has 64 queries of one head, a warp 16 of them with its queries in registers; 64 keys a tile; the next tile's keys
 // are brought while this one's values are used and the other way round.  Keys come from two places (the head's plain part
@@ -32,6 +33,7 @@ struct HeadPromptArgs {
   const __nv_bfloat16* k_rot;                                              // [tokens, rot_dim]
   const __nv_bfloat16* v; long long v_token, v_head;
   const int4* tiles;                 // request, first token, tokens (up to 128), first position
+  const int* q_start;                // where given, tiles of portions that do not start at position 0 are another kernel's
   __nv_bfloat16* out;                // [tokens, heads, value_size]
   const float* sink; const float* gate;
   int heads, dim, rot_dim, value_size, window, wave;
@@ -60,12 +62,12 @@ head_prompt_attention_kernel(const __grid_constant__ HeadPromptArgs a) {
   const int4 tile = a.tiles[row_tile >> 1];
   const int sub = (row_tile & 1) * kPromptRows;
   const int rows = min(kPromptRows, tile.z - sub);
-  if (rows <= 0) {
+  const int key_token = tile.y - tile.w;                  // packed index of the request's position 0
+  if (rows <= 0 || (a.q_start && a.q_start[tile.x] != key_token)) {
     pdl_wait();
     return;
   }
   const int t0 = tile.y + sub, pos0 = tile.w + sub;
-  const int key_token = tile.y - tile.w;                  // packed index of the request's position 0
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, q2 = (lane & 3) * 2;
   const uint32_t base = smem_address(prompt_smem);
@@ -296,13 +298,15 @@ extern "C" int einf_latent_rows(const void* cache, const int* slots, long long n
                          (__nv_bfloat16*)rest, second, tokens);
 }
 
-// Every request listed in `tiles` starts at position 0 in this step, its tokens packed one after the other.  Sizes and
+// Portions that start at position 0 in this step, their tokens packed one after the other; with `q_start`, the requests' first
+// tokens, `tiles` of other portions are left out (without it there must be none).  Sizes and
 // strides in multiples of eight elements, pointers on 16-byte borders; dim + rot_dim up to 192, value_size up to 128.
 // `wave`: multiprocessors of the device.
 extern "C" int einf_head_prompt_attention(const void* q_plain, long long q_plain_token, long long q_plain_head,
                                           const void* q_rot, long long q_rot_token, long long q_rot_head, const void* k_plain,
                                           long long k_token, long long k_head, const void* k_rot, const void* v,
-                                          long long v_token, long long v_head, const int* tiles, int num_tiles, void* out,
+                                          long long v_token, long long v_head, const int* tiles, int num_tiles,
+                                          const int* q_start, void* out,
                                           const float* sink, const float* gate, int heads, int dim, int rot_dim,
                                           int value_size, int window, float scale, int wave, cudaStream_t stream) {
   if (num_tiles == 0) return 0;
@@ -318,7 +322,7 @@ extern "C" int einf_head_prompt_attention(const void* q_plain, long long q_plain
   a.k_plain = (const __nv_bfloat16*)k_plain; a.k_token = k_token; a.k_head = k_head;
   a.k_rot = (const __nv_bfloat16*)k_rot;
   a.v = (const __nv_bfloat16*)v; a.v_token = v_token; a.v_head = v_head;
-  a.tiles = (const int4*)tiles; a.out = (__nv_bfloat16*)out; a.sink = sink; a.gate = gate;
+  a.tiles = (const int4*)tiles; a.q_start = q_start; a.out = (__nv_bfloat16*)out; a.sink = sink; a.gate = gate;
   a.heads = heads; a.dim = dim; a.rot_dim = rot_dim; a.value_size = value_size; a.window = window; a.wave = wave;
   a.scale_log2 = scale * 1.4426950408889634f;
   if (dim + rot_dim <= 128)

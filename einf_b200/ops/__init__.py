@@ -592,6 +592,7 @@ def paged_attention_generic(
     q_tiles: Optional[torch.Tensor] = None,
     single_tokens: Optional[torch.Tensor] = None,
     cached_before: Optional[int] = None,
+    leave_first: Optional[torch.Tensor] = None,
 ) -> None:
     """Causal attention of every token of the batch over the pages of its request.
 
@@ -611,7 +612,8 @@ def paged_attention_generic(
     ``q_tiles`` (int32 ``[tiles, 4]``: request, first token, rows up to 128, first position) and ``single_tokens``
     (int32) list the step's tokens by portions: portions of :func:`prompt_tile_min` tokens a tile or more, on average, then
     take a kernel that shares key rows between their tokens, where it takes the sizes, beside the single tokens'.
-    ``cached_before``: the longest cached prefix of a portion, where the host knows it.
+    ``cached_before``: the longest cached prefix of a portion, where the host knows it.  ``leave_first`` (the step's
+    ``q_start``, int32): portions of several tokens that start at position 0 are left out, for another kernel.
     """
     tokens, num_heads, head_size = q.shape
     if sink is not None and (sink.dtype != torch.float32 or sink.shape != (num_heads,)):
@@ -649,14 +651,15 @@ def paged_attention_generic(
             "einf_paged_attention_generic",
             [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
              c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p,
-             c_longlong, c_void_p, c_void_p, c_void_p],
+             c_longlong, c_void_p, c_void_p, c_void_p, c_void_p],
         )
         _check(
             fn(_dev(q, "q"), _dev(k_cache, "k_cache"), _dev(v_cache, "v_cache"), _code(q),
                _opt(block_table, "block_table", torch.int32), _opt(seq_of_token, "seq_of_token", torch.int32),
                _opt(positions, "positions", torch.int32), _dev(out, "out"), listed, num_heads, num_kv_heads,
                head_size, value_size, value_stride, page_size, num_pages, block_table.shape[1], *options,
-               _opt(single_tokens if tiled else None, "single_tokens", torch.int32), _dev(status, "status"), _stream()),
+               _opt(single_tokens if tiled else None, "single_tokens", torch.int32),
+               _opt(leave_first, "leave_first", torch.int32), _dev(status, "status"), _stream()),
             "paged_attention_generic",
         )
     if tiled:
@@ -664,13 +667,14 @@ def paged_attention_generic(
             "einf_paged_attention_prompt",
             [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int,
              c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p, c_longlong,
-             c_int, c_void_p, c_void_p],
+             c_int, c_void_p, c_void_p, c_void_p],
         )
         _check(
             fn(_dev(q, "q"), _dev(k_cache, "k_cache"), _dev(v_cache, "v_cache"), _code(q),
                _opt(block_table, "block_table", torch.int32), _opt(q_tiles, "q_tiles", torch.int32), q_tiles.shape[0],
                _dev(out, "out"), num_heads, num_kv_heads, head_size, value_size, value_stride, page_size, num_pages,
-               block_table.shape[1], *options, 1 if listed else 0, _dev(status, "status"), _stream()),
+               block_table.shape[1], *options, 1 if listed else 0, _opt(leave_first, "leave_first", torch.int32),
+               _dev(status, "status"), _stream()),
             "paged_attention_prompt",
         )
 
@@ -815,13 +819,14 @@ def latent_attention(
     max_context: Optional[int] = None,
     sink: Optional[torch.Tensor] = None,
     gate: Optional[torch.Tensor] = None,
+    leave_first: Optional[torch.Tensor] = None,
 ) -> None:
     """Causal attention of a whole step on the tensor cores over rows that all query heads share: ``q [tokens,
     heads, row]``, ``cache [pages, 1, page_size, row]`` whose first ``out.shape[2]`` elements are the values.  The
     prompt portions' ``q_tiles`` (see :func:`paged_prefill_attention`) and the ``singles`` single tokens
     (``token_list``: their packed indices; None: the step has no other) are a launch each; a few single
     tokens' keys are cut in shares (:func:`latent_attention_splits` of the longest context) that one more launch adds
-    up.  ``window``, ``sink`` and ``gate``: see :func:`paged_attention_generic`."""
+    up.  ``window``, ``sink``, ``gate`` and ``leave_first``: see :func:`paged_attention_generic`."""
     tokens, heads, row = q.shape
     pages, kv_heads, page_size, size = cache.shape
     value_size = out.shape[2]
@@ -838,7 +843,7 @@ def latent_attention(
     _check_gate(gate, tokens, heads)
     fn = _fn(
         "einf_latent_attention_tcgen05",
-        [c_void_p] * 7 + [c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 7 + [c_float, c_int, c_int] + [c_void_p] * 4,
+        [c_void_p] * 7 + [c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 7 + [c_float, c_int, c_int] + [c_void_p] * 5,
     )
 
     def launch(tiles, listed, count, splits, shares):
@@ -848,7 +853,8 @@ def latent_attention(
                _opt(seq_of_token, "seq_of_token", torch.int32), _opt(positions, "positions", torch.int32), count,
                _dev(out, "out"), shares[0], shares[1], tokens, heads, row, value_size, page_size, pages,
                block_table.shape[1], float(scale), int(window) if window else 0, splits,
-               _opt(sink, "sink", torch.float32), _opt(gate, "gate", torch.float32), _dev(status, "status"), _stream()),
+               _opt(sink, "sink", torch.float32), _opt(gate, "gate", torch.float32),
+               _opt(leave_first, "leave_first", torch.int32), _dev(status, "status"), _stream()),
             "latent_attention",
         )
 
@@ -914,13 +920,15 @@ def head_prompt_attention(
     window: Optional[int],
     sink: Optional[torch.Tensor] = None,
     gate: Optional[torch.Tensor] = None,
+    q_start: Optional[torch.Tensor] = None,
 ) -> None:
     """Causal attention of prompts that start in this step, every head with keys and values of its own: query head h
     scores key head h, ``q_plain . k_plain + q_rot . k_rot``, where all heads share ``k_rot``.  ``q_plain``, ``k_plain``
     ``[tokens, heads, dim]``, ``q_rot [tokens, heads, rot]``, ``v [tokens, heads, value]`` (views of wider rows are fine),
     ``k_rot [tokens, rot]``, ``out [tokens, heads, value]``, all bfloat16; ``q_tiles`` as for
-    :func:`paged_prefill_attention`, of requests whose first token in the step is at position 0.  ``window``, ``sink`` and
-    ``gate``: see :func:`paged_attention_generic`."""
+    :func:`paged_prefill_attention`, of requests whose first token in the step is at position 0; with ``q_start`` (int32
+    ``[requests + 1]``) other requests may be among them and are left out.  ``window``, ``sink`` and ``gate``: see
+    :func:`paged_attention_generic`."""
     tokens, heads, dim = q_plain.shape
     rot_dim, value_size = q_rot.shape[2], v.shape[2]
     if q_rot.shape[:2] != (tokens, heads) or k_plain.shape != (tokens, heads, dim) or k_rot.shape != (tokens, rot_dim) or \
@@ -940,14 +948,14 @@ def head_prompt_attention(
     fn = _fn(
         "einf_head_prompt_attention",
         [c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p,
-         c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
-         c_float, c_int, c_void_p],
+         c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+         c_int, c_float, c_int, c_void_p],
     )
     _check(
         fn(q_plain.data_ptr(), q_plain.stride(0), q_plain.stride(1), q_rot.data_ptr(), q_rot.stride(0), q_rot.stride(1),
            k_plain.data_ptr(), k_plain.stride(0), k_plain.stride(1), _dev(k_rot, "k_rot"), v.data_ptr(), v.stride(0),
-           v.stride(1), _opt(q_tiles, "q_tiles", torch.int32), q_tiles.shape[0], _dev(out, "out"),
-           _opt(sink, "sink", torch.float32), _opt(gate, "gate", torch.float32), heads, dim, rot_dim, value_size,
+           v.stride(1), _opt(q_tiles, "q_tiles", torch.int32), q_tiles.shape[0], _opt(q_start, "q_start", torch.int32),
+           _dev(out, "out"), _opt(sink, "sink", torch.float32), _opt(gate, "gate", torch.float32), heads, dim, rot_dim, value_size,
            int(window) if window else 0, float(scale), _sm_count(), _stream()),
         "head_prompt_attention",
     )

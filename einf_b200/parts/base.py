@@ -211,6 +211,11 @@ class StepContext:
     decode_only: bool = False
     extras: dict[str, Any] = field(default_factory=dict)
 
+    def starts_and_goes_on(self) -> tuple[bool, bool]:
+        """Whether portions of several tokens start at position 0 in this step, and whether others go on behind cached tokens."""
+        portions = [start for n, start in zip(self.q_lens, self.start_positions) if n > 1]
+        return 0 in portions, any(portions)
+
     def portions(self) -> dict:
         """What the general attention kernels take to tell portions of prompts from single tokens (nothing off the GPU:
         the plain statements that stand in for them there take every token alone)."""

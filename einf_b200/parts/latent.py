@@ -25,9 +25,12 @@ the cached rows as keys and values at once: the mixed rows then carry ``rot_dim`
 reads (a fifth to a quarter more work in the second product, none in memory traffic).  Other row
 sizes, and the 32-bit path, run the general kernel, which reads the values out of the key rows.
 
-A step of prompts alone that all start in it (no cached tokens before them, no single tokens beside them) runs head
-by head instead where the layer is not on the attention mixer's kernels: the up-projections are applied to the step's
-rows, one product for keys and values, and ``ops.head_prompt_attention`` meets queries and keys as they are.
+A portion of several tokens that starts its prompt runs head by head instead where the layer is not on the attention
+mixer's kernels: the up-projections are applied to the step's rows, one product for keys and values, and
+``ops.head_prompt_attention`` meets queries and keys as they are.  Single tokens and portions behind cached tokens
+stay on the rows, in the same step; the kernels tell the portions apart, so that what a prompt gets does not depend on
+what stands beside it (only on where it is cut: keys and values per head are rounded to bfloat16 in the one case, the
+absorbed queries and the mixed latents in the other).
 """
 from __future__ import annotations
 
@@ -160,8 +163,9 @@ class LatentAttention(Mixer):
     def launch_key(self, ctx: StepContext, page_size: int) -> tuple:
         """As for the attention mixer: the decode kernel's shape follows the batch and the longest context."""
         singles = int(ctx.single_tokens.shape[0])
-        if not singles:
-            return ("heads",) if self._runs_by_heads(ctx) else ()
+        return self._ways(ctx) + (self._singles_key(ctx, page_size, singles) if singles else ())
+
+    def _singles_key(self, ctx: StepContext, page_size: int, singles: int) -> tuple:
         context = self._visible(ctx.max_context_len)
         if not self.fast and ops.has_latent_attention(self.runtime.dtype, self.row, page_size):
             return ("latent", ops.latent_attention_splits(singles, self.num_heads, self.kv_rank, context))
@@ -170,13 +174,15 @@ class LatentAttention(Mixer):
             return ("shares", ops.latent_decode_splits(singles, self.num_heads, context)) if ctx.decode_only else ()
         return ops.decode_plan(singles, self.num_heads, 1, self.row, page_size, context)
 
-    def _runs_by_heads(self, ctx: StepContext) -> bool:
-        """A step of prompts alone that all start in it."""
-        return self.by_heads and not ctx.single_tokens.shape[0] and ctx.q_tiles.shape[0] > 0 \
-            and ctx.max_portion_start == 0 and ctx.q_tiles.is_cuda
+    def _ways(self, ctx: StepContext) -> tuple[bool, bool]:
+        """Whether portions of the step run head by head, and whether portions of several tokens run on the rows."""
+        if not self.by_heads or not ctx.q_tiles.is_cuda or not ctx.q_lens:
+            return False, ctx.q_tiles.shape[0] > 0
+        return ctx.starts_and_goes_on()
 
-    def _prompts(self, q_plain, q_full, gate, ctx: StepContext, cache: CacheView) -> torch.Tensor:
-        """Prompts head by head: the step's rows through both up-projections, then attention; ``[T, H, value]``."""
+    def _prompts(self, q_plain, q_full, gate, ctx: StepContext, cache: CacheView, mixed: torch.Tensor) -> None:
+        """Prompts that start in the step, head by head: its rows through both up-projections, then attention into those
+        portions' rows of ``mixed [T, H, value]``."""
         tokens, heads, device = q_full.shape[0], self.num_heads, q_full.device
         rows = torch.empty((tokens, self.kv_rank), dtype=q_full.dtype, device=device)
         part = torch.empty((tokens, self.rot_dim), dtype=q_full.dtype, device=device)
@@ -184,13 +190,11 @@ class LatentAttention(Mixer):
         kv = torch.empty((tokens, self.kv_up.shape[0]), dtype=q_full.dtype, device=device)
         ops.linear(rows, self.kv_up, None, kv)
         keys = heads * self.dim
-        mixed = torch.empty((tokens, heads, self.value_size), dtype=q_full.dtype, device=device)
         ops.head_prompt_attention(
             q_plain, q_full[:, :, self.kv_rank:self.kv_rank + self.rot_dim], kv[:, :keys].unflatten(1, (heads, self.dim)),
             part, kv[:, keys:].unflatten(1, (heads, self.value_size)), ctx.q_tiles, mixed, self.scale, self.window,
-            sink=self.sink, gate=gate,
+            sink=self.sink, gate=gate, q_start=ctx.q_start,
         )
-        return mixed
 
     def _visible(self, context: int) -> int:
         return min(context, self.window) if self.window else context
@@ -242,9 +246,21 @@ class LatentAttention(Mixer):
         dtype, device = self.runtime.dtype, x.device
         heads = self.num_heads
         q_plain, q_full, gate = self._queries_and_store(x, ctx, cache)
-        if self._runs_by_heads(ctx):
-            mixed = self._prompts(q_plain, q_full, gate, ctx, cache)
-            return ops.project(mixed.view(tokens, -1), self.out_weight, ctx.status)
+        by_heads, on_rows = self._ways(ctx)
+        mixed = torch.empty((tokens, heads, self.value_size), dtype=dtype, device=device)
+        if on_rows or ctx.single_tokens.shape[0]:
+            self._on_rows(q_plain, q_full, gate, ctx, cache, mixed, by_heads, on_rows)
+        if by_heads:      # after the others: those leave something in every row of `mixed`
+            self._prompts(q_plain, q_full, gate, ctx, cache, mixed)
+        return ops.project(mixed.view(tokens, -1), self.out_weight, ctx.status)
+
+    def _on_rows(self, q_plain, q_full, gate, ctx: StepContext, cache: CacheView, mixed: torch.Tensor, by_heads: bool,
+                 portions: bool) -> None:
+        """Attention over the cached rows into ``mixed``: of every token or, ``by_heads``, of all but the portions that start
+        their prompts; ``portions``: whether that leaves any of several tokens."""
+        tokens, heads = mixed.shape[:2]
+        dtype, device = self.runtime.dtype, mixed.device
+        leave_first = ctx.q_start if by_heads else None
         ops.per_head_project(q_plain, self.k_up_t, q_full[:, :, : self.kv_rank])
         table = ctx.block_tables[cache.group]
         if self.fast and ops.has_tcgen05_attention(self.row, cache.k.shape[2]):
@@ -265,9 +281,10 @@ class LatentAttention(Mixer):
         elif ops.has_latent_attention(dtype, self.row, cache.k.shape[2]):
             mixed_latent = torch.empty((tokens, heads, self.kv_rank), dtype=dtype, device=device)
             ops.latent_attention(
-                q_full, cache.k, table, ctx.seq_of_token, ctx.positions, ctx.q_tiles,
+                q_full, cache.k, table, ctx.seq_of_token, ctx.positions, ctx.q_tiles if portions else None,
                 None if ctx.decode_only else ctx.single_tokens, int(ctx.single_tokens.shape[0]), mixed_latent, self.scale,
                 self.window, ctx.status, max_context=ctx.max_context_len, sink=self.sink, gate=gate,
+                **({"leave_first": leave_first} if by_heads else {}),
             )
         elif ctx.decode_only:
             # every token stands alone: sixteen heads a CTA share the rows it stages, the keys are cut in shares
@@ -282,7 +299,6 @@ class LatentAttention(Mixer):
             ops.paged_attention_generic(
                 q_full, cache.k, None, table, ctx.seq_of_token, ctx.positions, mixed_latent,
                 self.scale, self.window, ctx.status, values_in_keys=self.kv_rank, sink=self.sink, gate=gate, **ctx.portions(),
+                **({"leave_first": leave_first} if by_heads else {}),
             )
-        mixed = torch.empty((tokens, heads, self.value_size), dtype=dtype, device=device)
         ops.per_head_project(mixed_latent, self.v_up, mixed)
-        return ops.project(mixed.view(tokens, -1), self.out_weight, ctx.status)

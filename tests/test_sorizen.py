@@ -369,7 +369,7 @@ def test_latent_layers_that_launch_by_one_key_agree_on_it(first, second, turned,
 
     from einf_b200 import ops
     from einf_b200.config.specs import PartSpec
-    from einf_b200.parts.base import Runtime, build_part
+    from einf_b200.parts.base import Runtime, StepContext, build_part
 
     monkeypatch.setattr(ops, "_sm_count", lambda: 148)
 
@@ -391,11 +391,10 @@ def test_latent_layers_that_launch_by_one_key_agree_on_it(first, second, turned,
 
     def step(starts, lens):
         tiles, singles = sum(n > 1 for n in lens), sum(n == 1 for n in lens)
-        return SimpleNamespace(
-            q_tiles=on_gpu(tiles), single_tokens=on_gpu(singles), q_lens=lens, start_positions=starts,
-            num_tokens=sum(lens), num_requests=len(lens), decode_only=not tiles, max_q_len=max(lens),
-            max_context_len=max(s + n for s, n in zip(starts, lens)),
-            max_portion_start=max((s for s, n in zip(starts, lens) if n > 1), default=0))
+        return StepContext(
+            sum(lens), len(lens), *[None] * 9, q_tiles=on_gpu(tiles), single_tokens=on_gpu(singles), status=None, q_lens=lens,
+            start_positions=starts, max_q_len=max(lens), max_context_len=max(s + n for s, n in zip(starts, lens)),
+            max_portion_start=max((s for s, n in zip(starts, lens) if n > 1), default=0), decode_only=not tiles)
 
     steps = [step((0, 0), (20, 30)), step((0, 300), (20, 30)), step((200, 300), (20, 30)), step((0, 50), (20, 1)),
              step((9, 50), (20, 1)), step((40, 5000), (1, 1))]

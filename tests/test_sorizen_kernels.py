@@ -323,7 +323,7 @@ def test_latent_attention_reports_a_page_outside_the_pool(dev):
 @pytest.mark.parametrize("lengths", [(2,), (63, 64, 65), (130, 2, 257)])
 @pytest.mark.parametrize("options", [False, True])
 def test_prompts_head_by_head(dev, heads, dim, rot, value, window, lengths, options):
-    """Prompts with keys and values of their own per head against the plain statement in 32 bits: lengths around the
+    """Prompts with keys and values of their own per head against the plain statement in 64 bits: lengths around the
     kernel's tiles of 64 and the tiles of 128 it is given, keys that fill no tile of 64 elements, views of wider rows."""
     from einf_b200 import ops
 
@@ -348,19 +348,81 @@ def test_prompts_head_by_head(dev, heads, dim, rot, value, window, lengths, opti
     first = 0
     for n in lengths:
         part = slice(first, first + n)
-        scores = torch.einsum("ihd,jhd->hij", q_plain[part].float(), k_plain[part].float())
-        scores = (scores + torch.einsum("ihr,jr->hij", q_rot[part].float(), k_rot[part].float())) * scale
+        scores = torch.einsum("ihd,jhd->hij", q_plain[part].double(), k_plain[part].double())
+        scores = (scores + torch.einsum("ihr,jr->hij", q_rot[part].double(), k_rot[part].double())) * scale
         i, j = torch.arange(n, device=dev)[:, None], torch.arange(n, device=dev)[None, :]
         seen = (j <= i) if window is None else (j <= i) & (j > i - window)
         scores = scores.masked_fill(~seen, float("-inf"))
         if sink is not None:
             scores = torch.cat([scores, sink[:, None, None].expand(heads, n, 1)], dim=2)
         weights = torch.softmax(scores, dim=2)[:, :, :n]
-        want = torch.einsum("hij,jhv->ihv", weights, v[part].float())
+        want = torch.einsum("hij,jhv->ihv", weights, v[part].double())
+        size = torch.einsum("hij,jhv->ihv", weights, v[part].double().abs())
         if gate is not None:
-            want = want * gate[part][:, :, None]
-        torch.testing.assert_close(out[part].float(), want, rtol=2e-2, atol=2e-2)
+            want, size = want * gate[part][:, :, None], size * gate[part][:, :, None]
+        # the output's rounding, the weights' (each to bfloat16), and 2^-16 of the terms' sizes for scores, exponentials and sums
+        bound = 2.0 ** -8 * want.abs() + (2.0 ** -8 + 2.0 ** -16) * size
+        assert bool(((out[part].double() - want).abs() <= bound).all())
         first += n
+
+
+@pytest.mark.parametrize("heads, dim, rot, value, rank, q_rank, page", [
+    (3, 128, 64, 128, 512, None, 16), (4, 40, 24, 72, 32, 64, 16), (2, 64, 16, 64, 192, 40, 8), (2, 64, 8, 40, 176, 40, 5)])
+@pytest.mark.parametrize("window", [None, 60])
+def test_a_prompt_gets_what_it_gets_beside_prompts(dev, heads, dim, rot, value, rank, q_rank, page, window):
+    """A latent layer's prompts that start in a step are bit for bit the same beside single tokens and portions that go on as
+    beside a prompt of as many tokens that starts with them (equal counts: equal products); and those others are
+    what a layer that runs everything on the rows makes of them."""
+    from einf_b200 import ops
+    from einf_b200.config.specs import PartSpec
+    from einf_b200.engine.batch import StepInputBuilder
+    from einf_b200.parts.base import CacheView, Runtime, build_part, part_class, walk_part_specs
+    from types import SimpleNamespace
+
+    gen = torch.Generator().manual_seed(rank + rot)
+    hidden = 128
+    spec = PartSpec("latent_attention", {
+        "hidden_size": hidden, "num_heads": heads, "head_size": dim, "rotary_size": rot, "value_head_size": value,
+        "kv_rank": rank, "q_rank": q_rank, "scale": (dim + rot) ** -0.5, "eps": 1e-6, "window": window, "sink": True,
+        "position": PartSpec("rope", {"rotary_dim": rot, "theta": 1e4})})
+    draw = lambda *shape: (torch.randn(shape, generator=gen) * shape[-1] ** -0.5).to(torch.bfloat16).to(dev)  # noqa: E731
+    tensors = {"kv_down.weight": draw(rank + rot, hidden), "k_up.weight": draw(heads * dim, rank), "v_up.weight": draw(heads * value, rank),
+               "o_proj.weight": draw(hidden, heads * value), "sink": torch.randn(heads, generator=gen).to(dev),
+               "kv_norm.weight": torch.ones(rank, dtype=torch.bfloat16, device=dev)}
+    if q_rank:
+        tensors.update({"q_down.weight": draw(q_rank, hidden), "q_up.weight": draw(heads * (dim + rot), q_rank),
+                        "q_norm.weight": torch.ones(q_rank, dtype=torch.bfloat16, device=dev)})
+    else:
+        tensors["q_proj.weight"] = draw(heads * (dim + rot), hidden)
+    runtime = Runtime(torch.bfloat16, dev)
+    names = []
+    for category, nested in walk_part_specs("mixer", spec):
+        names += part_class(category, nested.kind).kernel_libraries(nested, runtime)
+    ops.ensure_built(tuple(dict.fromkeys(names)))
+    part = build_part("mixer", spec, tensors, runtime)
+    assert part.by_heads
+    fresh, others = [(0, 150), (0, 2), (0, 64)], [(40, 1), (70, 33), (300, 1), (129, 140), (0, 1)]
+    count, rest = sum(n for _, n in fresh), sum(n for _, n in others)
+    x = torch.randn((count + rest, hidden), generator=gen).to(torch.bfloat16).to(dev)
+
+    def run(requests):
+        needs = [-(-(start + n) // page) for start, n in requests]
+        order = torch.randperm(sum(needs), generator=torch.Generator().manual_seed(1)).tolist()
+        cache = torch.randn((sum(needs), 1, page, part.row), generator=torch.Generator().manual_seed(2)).to(torch.bfloat16).to(dev)
+        builder = StepInputBuilder(dev, page, [sum(needs)], [window], 1000, max(needs), x.shape[0], len(requests))
+        ctx, _ = builder.build([SimpleNamespace(input_token_ids=[1] * n, start_position=start, need_sample=False,
+                                                block_tables=[[order.pop() for _ in range(need)]])
+                                for (start, n), need in zip(requests, needs)])
+        out = part.forward(x, ctx, CacheView(group=0, k=cache, v=None, writes=True, page_size=page))
+        assert int(ctx.status) == 0
+        return out.float().sum(dim=0) if out.dim() == 3 else out.float()
+
+    mixed, together = run(fresh + others), run(fresh + [(0, rest)])
+    part.by_heads = False
+    on_rows = run(fresh + others)
+    assert torch.equal(mixed[:count], together[:count]) and torch.equal(mixed[count:], on_rows[count:])
+    assert not torch.equal(mixed[:count], on_rows[:count])                  # the two ways round in different places
+    torch.testing.assert_close(mixed[:count], on_rows[:count], rtol=2e-2, atol=2e-2)
 
 
 def test_latent_rows(dev):
