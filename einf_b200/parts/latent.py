@@ -176,7 +176,7 @@ class LatentAttention(Mixer):
 
     def _ways(self, ctx: StepContext) -> tuple[bool, bool]:
         """Whether portions of the step run head by head, and whether portions of several tokens run on the rows."""
-        if not self.by_heads or not ctx.q_tiles.is_cuda or not ctx.q_lens:
+        if not self.by_heads or not ctx.q_tiles.shape[0] or not ctx.q_tiles.is_cuda or not ctx.q_lens:
             return False, ctx.q_tiles.shape[0] > 0
         return ctx.starts_and_goes_on()
 
