@@ -40,10 +40,6 @@ struct MixArgs {
   float scale_log2, out_scale;
 };
 
-__device__ __forceinline__ uint32_t swizzled(int row, int piece, int pitch) {
-  return (uint32_t)(row * pitch + ((piece & ~7) | ((piece ^ row) & 7)) * 16);
-}
-
 // Three parts of q', a tile's keys, its values.
 template <int VALUE>
 constexpr int kMixSmem = 3 * kMixRows * kMixKeySize * 2 + kMixKeys * (kMixKeySize + VALUE) * 2;
@@ -84,10 +80,8 @@ mixed_prompt_attention_kernel(const __grid_constant__ MixArgs a) {
   constexpr int kKeyPitch = kMixKeySize * 2, kValuePitch = VALUE * 2;
   constexpr int kQPart = kMixRows * kKeyPitch, kK = 3 * kQPart, kV = kK + kMixKeys * kKeyPitch, kSteps = kMixKeySize / 16;
   pdl_launch_dependents();
-  // which rows: see attention_prompt.cu
-  const int total = (int)gridDim.x, wave = (int)blockIdx.x / a.wave, place = (int)blockIdx.x - wave * a.wave;
-  const int rank = wave & 1 ? total - 1 - ((wave >> 1) * a.wave + place) : ((wave + 1) >> 1) * a.wave + place;
-  const int row_tiles = total / a.heads, row_tile = row_tiles - 1 - rank / a.heads, h = rank % a.heads;
+  int row_tile, h;
+  rows_of_cta(a.wave, a.heads, &row_tile, &h);
   const int4 tile = a.tiles[row_tile >> 1];
   const int sub = (row_tile & 1) * kMixRows;
   const int rows = min(kMixRows, tile.z - sub);

@@ -40,12 +40,6 @@ struct HeadPromptArgs {
   float scale_log2;
 };
 
-// Byte of a 16-byte piece of a row whose rows are 128-byte lines: exchanged by the row's last three bits, so that the eight
-// rows of an ldmatrix meet no bank twice.
-__device__ __forceinline__ uint32_t swizzled(int row, int piece, int pitch) {
-  return (uint32_t)(row * pitch + ((piece & ~7) | ((piece ^ row) & 7)) * 16);
-}
-
 // KEY: dim + rot_dim filled up to 128 or 192; VALUE: value_size filled up to 64 or 128.
 template <int KEY, int VALUE>
 __global__ void __launch_bounds__(kPromptThreads, 3)
@@ -54,11 +48,8 @@ head_prompt_attention_kernel(const __grid_constant__ HeadPromptArgs a) {
   constexpr int kKeyPitch = KEY * 2, kValuePitch = VALUE * 2;
   constexpr int kK = 0, kV = kPromptKeys * kKeyPitch;
   pdl_launch_dependents();
-  // Which rows: (tile, head) pairs in the order of their keys, the last tiles first; every second wave of CTAs takes them
-  // from the other end, so that an SM's CTAs, which all run at once, are long and short ones.
-  const int total = (int)gridDim.x, wave = (int)blockIdx.x / a.wave, place = (int)blockIdx.x - wave * a.wave;
-  const int rank = wave & 1 ? total - 1 - ((wave >> 1) * a.wave + place) : ((wave + 1) >> 1) * a.wave + place;
-  const int row_tiles = total / a.heads, row_tile = row_tiles - 1 - rank / a.heads, h = rank % a.heads;
+  int row_tile, h;
+  rows_of_cta(a.wave, a.heads, &row_tile, &h);
   const int4 tile = a.tiles[row_tile >> 1];
   const int sub = (row_tile & 1) * kPromptRows;
   const int rows = min(kPromptRows, tile.z - sub);

@@ -95,6 +95,22 @@ __device__ __forceinline__ uint32_t pack_pair(float low, float high) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// Byte of a 16-byte piece of a row whose rows are 128-byte lines: exchanged by the row's last three bits, so that the eight
+// rows of an ldmatrix meet no bank twice.
+__device__ __forceinline__ uint32_t swizzled(int row, int piece, int pitch) {
+  return (uint32_t)(row * pitch + ((piece & ~7) | ((piece ^ row) & 7)) * 16);
+}
+
+// Which rows of a prompt a CTA of (row tiles x heads) has: pairs in the order of their keys, the last tiles first; every second
+// wave of CTAs (`wave`: multiprocessors) takes them from the other end, so that an SM's CTAs, which all run at once, are
+// long and short ones.
+__device__ __forceinline__ void rows_of_cta(int wave_size, int heads, int* row_tile, int* head) {
+  const int total = (int)gridDim.x, wave = (int)blockIdx.x / wave_size, place = (int)blockIdx.x - wave * wave_size;
+  const int rank = wave & 1 ? total - 1 - ((wave >> 1) * wave_size + place) : ((wave + 1) >> 1) * wave_size + place;
+  *row_tile = total / heads - 1 - rank / heads;
+  *head = rank % heads;
+}
+
 // x and y as three pairs of bfloat16 whose sums are x and y to 24 bits (x in the low halves).  A value whose first
 // part is not finite (infinite, NaN, or rounded up to infinity) has no further parts.
 __device__ __forceinline__ void split3(float x, float y, uint32_t (&part)[3]) {

@@ -1673,7 +1673,9 @@ def recurrence_plan(num_requests: int, max_q_len: Optional[int], heads: int, dim
 RECURRENCE_CHUNK = 64
 #: shortest portion that takes the chunked kernel (kernels alone, us, one request / eight; token by token against
 #: chunked: 16 tokens 7.6 / 10.7 against 9.6 / 11.3 (14 heads of 64 x 64), 9.4 / 15.8 against 9.2 / 11.5 (24 of 128 x 64); 24 tokens
-#: 12.3 / 16.7 against 10.8 / 15.1, 12.1 / 20.1 against 10.1 / 13.9; 64 tokens 20.5 / 30.3 against 14.9 / 21.2).  The shorter
+#: 12.3 / 16.7 against 10.8 / 15.1, 12.1 / 20.1 against 10.1 / 13.9; 64 tokens 20.5 / 30.3 against 14.9 / 21.2; 12 heads of 128 x 128
+#: behind a SiLU, whose chunked CTAs have an SM each, four requests / eight: 24 tokens 22.5 / 24.1 against 16.9 / 30.7, 32 27.1 /
+#: 29.2 against 16.9 / 31.2, 48 37.4 / 39.4 against 20.6 / 37.9: eight requests are a second wave of 44 CTAs).  The shorter
 #: portions of a step run token by token beside it, single tokens through the streaming kernel of decoding steps
 RECURRENCE_CHUNK_MIN = 24
 #: bytes that the states of a launch's segments may take (10 an element: the sum and the start state in parts)
