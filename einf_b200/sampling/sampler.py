@@ -23,19 +23,22 @@ class Sampler:
         self.max_rows = max_rows
         self.tokens = torch.zeros(max_rows, dtype=torch.int32, device=self.device)
         pin = self.device.type == "cuda"
-        # [temperature, top_p, min_p] as float32, [top_k] as int32, [seed, sample_index] as int64.
-        # The copies to the device are asynchronous and a caller may sample several steps before it
+        # A row's parameters lie in one buffer, so that a step copies once: [seed, sample_index] as int64,
+        # [temperature, top_p, min_p] as float32, [top_k] as int32.
+        # The copy to the device is asynchronous and a caller may sample several steps before it
         # waits for the device, so the pinned staging is a ring: a slot is written again only after
         # the copy that read it last has run (its event).
         self._ring = 8
         self._turn = 0
         self._events = [None] * self._ring
-        self._host_f = torch.zeros((self._ring, 3, max_rows), dtype=torch.float32, pin_memory=pin)
-        self._host_i = torch.zeros((self._ring, 1, max_rows), dtype=torch.int32, pin_memory=pin)
-        self._host_l = torch.zeros((self._ring, 2, max_rows), dtype=torch.int64, pin_memory=pin)
-        self._dev_f = torch.zeros((3, max_rows), dtype=torch.float32, device=self.device)
-        self._dev_i = torch.zeros((1, max_rows), dtype=torch.int32, device=self.device)
-        self._dev_l = torch.zeros((2, max_rows), dtype=torch.int64, device=self.device)
+        self._host = torch.zeros((self._ring, 32 * max_rows), dtype=torch.uint8, pin_memory=pin)
+        self._dev = torch.zeros(32 * max_rows, dtype=torch.uint8, device=self.device)
+        n, host = max_rows, self._host.numpy()
+        self._wide = host[:, :16 * n].view(np.int64).reshape(self._ring, 2, n)
+        self._real = host[:, 16 * n:28 * n].view(np.float32).reshape(self._ring, 3, n)
+        self._whole = host[:, 28 * n:].view(np.int32)
+        wide, real = self._dev[:16 * n].view(torch.int64), self._dev[16 * n:28 * n].view(torch.float32)
+        self._columns = (real[:n], self._dev[28 * n:].view(torch.int32), real[n:2 * n], real[2 * n:], wide[:n], wide[n:])
 
     def sample(self, logits: torch.Tensor, params: Sequence, sample_indices: Sequence[int]) -> torch.Tensor:
         """One token per row of ``logits`` (float32 ``[rows, vocab]``); returns an
@@ -54,23 +57,15 @@ class Sampler:
         self._turn = (turn + 1) % self._ring
         if self._events[turn] is not None:
             self._events[turn].synchronize()
-        f, i, l = self._host_f[turn].numpy(), self._host_i[turn].numpy(), self._host_l[turn].numpy()
-        for r, (p, index) in enumerate(zip(params, sample_indices)):
-            f[0, r] = p.temperature
-            f[1, r] = p.top_p
-            f[2, r] = p.min_p
-            i[0, r] = p.top_k or 0
-            l[0, r] = np.int64(p.seed)
-            l[1, r] = index
-        self._dev_f.copy_(self._host_f[turn], non_blocking=True)
-        self._dev_i.copy_(self._host_i[turn], non_blocking=True)
-        self._dev_l.copy_(self._host_l[turn], non_blocking=True)
+        wide, real = self._wide[turn], self._real[turn]
+        wide[0, :rows] = [np.int64(p.seed) for p in params]
+        wide[1, :rows] = sample_indices
+        real[:, :rows] = [[p.temperature for p in params], [p.top_p for p in params], [p.min_p for p in params]]
+        self._whole[turn, :rows] = [p.top_k or 0 for p in params]
+        self._dev.copy_(self._host[turn], non_blocking=True)
         if self.device.type == "cuda":
             if self._events[turn] is None:
                 self._events[turn] = torch.cuda.Event()
             self._events[turn].record(ops.current_stream())
-        ops.sample(
-            logits, self.tokens, self._dev_f[0], self._dev_i[0], self._dev_f[1], self._dev_f[2],
-            self._dev_l[0], self._dev_l[1],
-        )
+        ops.sample(logits, self.tokens, *self._columns)
         return self.tokens[:rows]

@@ -1254,6 +1254,35 @@ def test_sampling_random_rows_and_filters(dev, first_case):
                 assert low - 1e-4 <= u <= float(cumulative[token]) + 1e-4, (case, r, index, u)
 
 
+@pytest.mark.parametrize("top_k", [1, 5, 255, 256, 257, 0])
+def test_sampling_where_few_tokens_are_looked_at(dev, top_k):
+    """Both sides of what one CTA settles by itself and of what a CTA lists: more tied tokens than it takes, a row
+    that lies in one bin, fewer threads with a token near the maximum than k, a minus infinite bulk."""
+    from einf_b200 import ops
+
+    torch.manual_seed(top_k)
+    vocab = 80003
+    logits = torch.randn(5, vocab, device=dev) * 3
+    logits[1, torch.randperm(vocab, device=dev)[:600]] = 30.0
+    logits[2] *= 0.001
+    logits[3] = -float("inf")
+    logits[3, torch.randperm(vocab, device=dev)[:40]] = torch.linspace(0, 3, 40, device=dev)
+    logits[4, :3] += 60.0
+    columns = (torch.full((5,), 0.9, device=dev), torch.full((5,), top_k, dtype=torch.int32, device=dev),
+               torch.full((5,), 0.85, device=dev), torch.zeros(5, device=dev))
+    tokens = torch.zeros(5, dtype=torch.int32, device=dev)
+    weights = [ref.kept_weights(logits[r].cpu(), 0.9, top_k, 0.85, 0.0).double() for r in range(5)]
+    for index in range(6):
+        ops.sample(logits, tokens, *columns, torch.full((5,), 7, dtype=torch.int64, device=dev),
+                   torch.full((5,), index, dtype=torch.int64, device=dev))
+        u = ref.keyed_uniform(7, index)
+        for r, token in enumerate(tokens.tolist()):
+            assert weights[r][token] > 0, (r, index, token)
+            cumulative = weights[r].cumsum(0) / weights[r].sum()
+            low = float(cumulative[token] - weights[r][token] / weights[r].sum())
+            assert low - 1e-4 <= u <= float(cumulative[token]) + 1e-4, (r, index, u)
+
+
 def test_sampling_frequencies(dev):
     from einf_b200 import ops
 
