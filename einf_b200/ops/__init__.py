@@ -549,6 +549,93 @@ def project(
     return out
 
 
+#: A layer's products for up to this many tokens run with what stands before and behind them in one launch, where
+#: the stream is narrow enough (measured, a layer of 0.5B sizes for 1 / 8 / 16 tokens: 24.4 -> 17.6, 29.0 -> 22.8,
+#: 27.9 -> 26.1 us; of 1.5B sizes, 1,536 wide, 34.2 -> 34.9, 40.3 -> 45.0: the separate products stream its 94 MB better).
+FEW_TOKENS = 16
+FEW_NORM_WIDTH = 1024
+#: and the rows of the down projection short enough for two CTAs an SM
+FEW_WIDTH = 5120
+
+
+def few_tokens_fit(k: int, norm: bool) -> bool:
+    """Whether the kernels for a few tokens take products over K elements (with a norm in front)."""
+    return k % 32 == 0 and k <= (FEW_NORM_WIDTH if norm else FEW_WIDTH)
+
+
+def few_qkv(residual: torch.Tensor, pending: Optional[torch.Tensor], norm_weight: torch.Tensor, eps: float,
+            weight: torch.Tensor, bias: Optional[torch.Tensor], positions: torch.Tensor, inv_freq: torch.Tensor,
+            slots: Optional[torch.Tensor], q_out: torch.Tensor, k_cache: Optional[torch.Tensor],
+            v_cache: Optional[torch.Tensor], num_heads: int, num_kv_heads: int, head_size: int, status: torch.Tensor) -> None:
+    """RMS norm of ``residual + pending`` (float32 ``[tokens, hidden]`` both; the stream is not written), the QKV
+    product, bias, rotation of whole heads in halves (none with an empty ``inv_freq``) and the cache write, as
+    :func:`rope_kv_write` does it, in one launch for up to :data:`FEW_TOKENS` tokens."""
+    tokens, hidden = residual.shape
+    rows = (num_heads + 2 * num_kv_heads) * head_size
+    if not 0 < tokens <= FEW_TOKENS or not few_tokens_fit(hidden, True) or head_size % 8:
+        raise UnsupportedSize(f"few_qkv: {tokens} tokens of {hidden}, heads of {head_size}")
+    if weight.dtype != torch.bfloat16 or weight.shape != (rows, hidden) or q_out.dtype != torch.bfloat16:
+        raise ValueError(f"few_qkv takes a bfloat16 weight {(rows, hidden)} and bfloat16 queries")
+    if q_out.numel() != tokens * num_heads * head_size or norm_weight.shape != (hidden,):
+        raise ValueError("few_qkv: queries or norm weight of another size")
+    if pending is not None and pending.shape != residual.shape:
+        raise ValueError(f"pending is {tuple(pending.shape)}, residual {tuple(residual.shape)}")
+    if inv_freq.shape[0] not in (0, head_size // 2):
+        raise UnsupportedSize("few_qkv rotates whole heads or none")
+    page_size = num_pages = k_ptr = v_ptr = 0
+    if slots is not None:
+        if k_cache is None or v_cache is None or k_cache.dtype != torch.bfloat16 or v_cache.dtype != torch.bfloat16:
+            raise ValueError("slots need bfloat16 caches")
+        num_pages, heads, page_size, size = k_cache.shape
+        if (heads, size) != (num_kv_heads, head_size) or v_cache.shape != k_cache.shape or slots.shape[0] < tokens:
+            raise ValueError(f"cache is {tuple(k_cache.shape)}, expected [pages, {num_kv_heads}, page, {head_size}]")
+        k_ptr, v_ptr = _dev(k_cache, "k_cache"), _dev(v_cache, "v_cache")
+    if positions.shape[0] < tokens or (bias is not None and bias.shape != (rows,)):
+        raise ValueError("few_qkv: positions or bias of another size")
+    fn = _fn("einf_few_qkv", [c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(fn(_opt(residual, "residual", torch.float32), _opt(pending, "pending", torch.float32),
+              _opt(norm_weight, "norm_weight", torch.float32), float(eps), _dev(weight, "weight"),
+              _opt(bias, "bias", torch.float32), _opt(positions, "positions", torch.int32),
+              _opt(inv_freq, "inv_freq", torch.float32), _opt(slots, "slots", torch.int32), _dev(q_out, "q_out"), k_ptr, v_ptr,
+              tokens, hidden, num_heads, num_kv_heads, head_size, int(inv_freq.shape[0] > 0), page_size, num_pages,
+              _dev(status, "status"), _stream()), "few_qkv")
+
+
+def few_gate_up(residual: torch.Tensor, norm_weight: torch.Tensor, eps: float, weight: torch.Tensor, out: torch.Tensor,
+                status: torch.Tensor) -> None:
+    """RMS norm of ``residual``, the product with the gate rows and the up rows behind them, ``out = silu(gate) * up``
+    (bfloat16 ``[tokens, intermediate]``), in one launch for up to :data:`FEW_TOKENS` tokens."""
+    tokens, hidden = residual.shape
+    inter = out.shape[1]
+    if not 0 < tokens <= FEW_TOKENS or not few_tokens_fit(hidden, True) or inter % 16:
+        raise UnsupportedSize(f"few_gate_up: {tokens} tokens of {hidden}, {inter} columns a branch")
+    if weight.dtype != torch.bfloat16 or weight.shape != (2 * inter, hidden) or out.dtype != torch.bfloat16 or out.shape[0] != tokens:
+        raise ValueError(f"few_gate_up takes a bfloat16 weight {(2 * inter, hidden)} and a bfloat16 result of {tokens} rows")
+    if norm_weight.shape != (hidden,):
+        raise ValueError("few_gate_up: norm weight of another size")
+    fn = _fn("einf_few_gate_up", [c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(fn(_opt(residual, "residual", torch.float32), _opt(norm_weight, "norm_weight", torch.float32), float(eps),
+              _dev(weight, "weight"), _dev(out, "out"), tokens, hidden, inter, _dev(status, "status"), _stream()), "few_gate_up")
+
+
+def few_product(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, status: torch.Tensor, add_to_stream: bool = False,
+                pending: Optional[torch.Tensor] = None) -> None:
+    """``out = x weight^T`` in float32 for up to :data:`FEW_TOKENS` tokens; ``add_to_stream``: ``out`` is the residual
+    stream and becomes ``out + pending + x weight^T``."""
+    tokens, k = x.shape
+    rows = weight.shape[0]
+    if not 0 < tokens <= FEW_TOKENS or not few_tokens_fit(k, False) or rows % 8:
+        raise UnsupportedSize(f"few_product: {tokens} tokens of {k}, {rows} rows")
+    if x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or weight.shape[1] != k or out.shape != (tokens, rows):
+        raise ValueError(f"few_product takes bfloat16 operands and a result of {(tokens, rows)}")
+    if pending is not None and (not add_to_stream or pending.shape != out.shape):
+        raise ValueError("what is pending has the stream's size and is added to it")
+    fn = _fn("einf_few_product", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(fn(_dev(x, "x"), _dev(weight, "weight"), _opt(pending, "pending", torch.float32), _opt(out, "out", torch.float32),
+              int(add_to_stream), tokens, k, rows, _dev(status, "status"), _stream()), "few_product")
+
+
 def _value_gate(value_gate: Optional[torch.Tensor], q: torch.Tensor, value_size: int, aligned: bool) -> tuple[int, int]:
     """Pointer and row stride of the logits of an output gate, one per element of the mixed heads:
     ``[tokens, heads * value_size]`` of q's dtype, rows contiguous (columns of a wider matrix are fine);

@@ -71,6 +71,9 @@ LAUNCHERS = {
     "einf_memory_gates": "recurrence",
     "einf_memory_output": "recurrence",
     "einf_norm_join": "pointwise",
+    "einf_few_qkv": "few_tokens",
+    "einf_few_gate_up": "few_tokens",
+    "einf_few_product": "few_tokens",
     "einf_argmax": "sampling",
     "einf_sample": "sampling",
     "einf_report": "sampling",

@@ -133,7 +133,7 @@ class PagedAttention(Mixer):
         if ops.has_fast_attention(runtime.dtype, int(spec["head_size"])):
             # the page size is the engine's choice: ask for both prefill kernels of this head size
             libraries = ops.attention_libraries(int(spec["head_size"]), 16)
-            return ("pointwise", "gemm_simt", "gemm_tcgen05") + libraries
+            return ("pointwise", "gemm_simt", "gemm_tcgen05", "few_tokens") + libraries
         return ("pointwise", "attention_generic", "gemm_simt") + cls._product_libraries(runtime)
 
     @staticmethod
@@ -308,6 +308,29 @@ class PagedAttention(Mixer):
         out = torch.empty((tokens, self.hidden_size), dtype=dtype, device=device)
         ops.linear(mixed.view(tokens, -1), self.out_weight, self.out_bias, out)
         return out
+
+    def takes_few(self) -> bool:
+        """Whether the layer's products run in the kernels for a few tokens."""
+        return bool(
+            self.fast and self.out_bias is None and self.qkv_weight.dtype == self.out_weight.dtype == torch.bfloat16
+            and self.position.kind in ("rope", "none") and self.position.inv_freq.shape[0] in (0, self.head_size // 2)
+            and not getattr(self.position, "interleaved", False)
+            and ops.few_tokens_fit(self.hidden_size, True) and ops.few_tokens_fit(self.num_heads * self.head_size, False)
+            and self.hidden_size % 8 == 0
+        )
+
+    def forward_few(self, residual, pending, norm, ctx: StepContext, cache: CacheView) -> None:
+        """``residual += pending + mixer(norm(residual + pending))`` for a few tokens: the norm runs in the launch of the
+        QKV product with the rotation and the cache write, the sum in that of the output product."""
+        tokens = residual.shape[0]
+        q = torch.empty((tokens, self.num_heads, self.head_size), dtype=self.runtime.dtype, device=residual.device)
+        writes = cache.writes and cache.k is not None
+        ops.few_qkv(residual, pending, norm.weight, norm.eps, self.qkv_weight, self.qkv_bias, ctx.positions,
+                    self.position.inv_freq, ctx.slots[cache.group] if writes else None, q, cache.k if writes else None,
+                    cache.v if writes else None, self.num_heads, self.num_kv_heads, self.head_size, ctx.status)
+        mixed = torch.empty_like(q)
+        self.attend(q, ctx, cache, mixed)
+        ops.few_product(mixed.view(tokens, -1), self.out_weight, residual, ctx.status, add_to_stream=True, pending=pending)
 
     def _convolve_and_store(self, qkv, q, ctx: StepContext, cache: CacheView):
         """Queries into ``q``, keys and values into the pages; returns the logits of the output gate

@@ -16,6 +16,7 @@ import torch
 
 from .. import ops
 from .base import CacheView, Part, StepContext, build_part, join_needs, part_class, register_part
+from .norm import RMSNorm
 from .stream import NormedPending
 
 
@@ -52,6 +53,9 @@ class PreNormBlock(Block):
         self.spec = layer_spec
         for role, category in self.part_categories().items():
             setattr(self, role, build_part(category, layer_spec.parts[role], tensors, runtime))
+        self._few = type(self) is PreNormBlock and all(
+            type(norm) is RMSNorm for norm in (self.mixer_norm, self.feed_forward_norm)) and all(
+            part.takes_few() if hasattr(part, "takes_few") else False for part in (self.mixer, self.feed_forward))
 
     @staticmethod
     def _normalise(norm, pending, residual, ctx):
@@ -61,6 +65,10 @@ class PreNormBlock(Block):
         return norm.forward(pending, residual)
 
     def forward(self, residual, pending, ctx, cache):
+        if self._few and residual.shape[0] <= ops.FEW_TOKENS and (
+                pending is None or (pending.dtype == torch.float32 and pending.shape == residual.shape)):
+            self.mixer.forward_few(residual, pending, self.mixer_norm, ctx, cache)
+            return self.feed_forward.forward_few(residual, self.feed_forward_norm, ctx)
         x = self._normalise(self.mixer_norm, pending, residual, ctx)
         mixed = self.mixer.forward(x, ctx, cache)
         x = self._normalise(self.feed_forward_norm, mixed, residual, ctx)

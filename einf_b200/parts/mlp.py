@@ -54,7 +54,7 @@ class GatedMLP(FeedForward):
 
     @classmethod
     def kernel_libraries(cls, spec, runtime):
-        return ("pointwise", "gemm_simt") + (("gemm_tcgen05",) if runtime.dtype == torch.bfloat16 else ())
+        return ("pointwise", "gemm_simt") + (("gemm_tcgen05", "few_tokens") if runtime.dtype == torch.bfloat16 else ())
 
     def __init__(self, spec, tensors, runtime):
         super().__init__(spec, tensors, runtime)
@@ -74,6 +74,24 @@ class GatedMLP(FeedForward):
         hidden = torch.empty((tokens, self.intermediate_size), dtype=dtype, device=device)
         self.activation(gate_up, hidden)
         return ops.project(hidden, self.down_weight, ctx.status)
+
+    def takes_few(self) -> bool:
+        """Whether the products run in the kernels for a few tokens."""
+        return bool(
+            self.activation.kind == "silu" and self.gate_up_weight.dtype == self.down_weight.dtype == torch.bfloat16
+            and self.runtime.dtype == torch.bfloat16 and self.intermediate_size % 32 == 0 and self.hidden_size % 8 == 0
+            and ops.few_tokens_fit(self.hidden_size, True) and ops.few_tokens_fit(self.intermediate_size, False)
+        )
+
+    def forward_few(self, residual, norm, ctx):
+        """``feed_forward(norm(residual))`` for a few tokens, as float32: the norm and the activation run in the
+        launch of the gate/up product."""
+        tokens, device = residual.shape[0], residual.device
+        hidden = torch.empty((tokens, self.intermediate_size), dtype=self.runtime.dtype, device=device)
+        ops.few_gate_up(residual, norm.weight, norm.eps, self.gate_up_weight, hidden, ctx.status)
+        out = torch.empty((tokens, self.hidden_size), dtype=torch.float32, device=device)
+        ops.few_product(hidden, self.down_weight, out, ctx.status)
+        return out
 
 
 @register_part("feed_forward", "dense_mlp")
