@@ -1,0 +1,285 @@
+// out[M, N] = A[M, K] . W[N, K]^T (+ bias[N]) for 32-bit operands and a 32-bit result on the fifth-generation tensor cores
+// (gemm_simt.cu has the FMA product for operands of mixed type and rows that are not aligned).
+//
+// A 32-bit value is the sum of three bfloat16 parts (8 bits of the significand each), so a product of two is nine bfloat16
+// products, of which the six largest count: what is left out is below 2^-24 of a term.  The instruction cuts its sums
+// off where FMA rounds them, so a chain of it drifts.  Therefore 32 elements of K are summed at a time, products of the
+// smaller parts first, into a tensor-memory accumulator that starts at zero, and its result is added to a running sum in
+// registers by a rounded addition; every 512 elements that sum joins a total in tensor memory.  Error against 64 bits (2-norm,
+// normal values, this / FMA): K = 896 0.97e-7 / 2.8e-7, 4,864 1.1e-7 / 3.0e-7, 18,944 1.5e-7 / 3.3e-7; where all terms are
+// positive 0.96e-7 / 1.28e-7, 1.0e-7 / 0.9e-7, 1.3e-7 / 1.4e-7 (64 elements at a time 1.8e-7; without the total 2.1e-7 at 4,864).
+//
+// A CTA has 128 rows of W (the instruction's M) and 128 rows of A (its N).  Its sixteen warps read the next 64 columns of
+// both operands into registers, split them and write the parts into swizzled K-major tiles (two stages of 96 KB), one
+// thread issues the 24 products, and while they run the warps split the 64 columns after.  Bound by shared memory: the 24
+// products read 192 KB of it and the parts are 96 KB to write, 2,300 cycles at 128 bytes each; 64 columns take 3,200.  (Eight warps
+// of twice the work each 90 us where this takes 84.)  Where the tiles are too few for the GPU, CTAs share K and a second
+// kernel adds their sums in order.
+//
+// Measured (B200, us, FMA before): 545 rows, 896 -> 1,152 42 -> 21, 896 -> 896 41 -> 18, 896 -> 9,728 211 -> 84 (113 TFLOP/s),
+// 4,864 -> 896 118 -> 45; 2,048 rows, 3,584 -> 4,608 1,300 -> 395 (171 TFLOP/s); one row, 896 -> 9,728 40 -> 26.
+//
+// A value that is not finite, or rounds to infinity as bfloat16, has no such parts: a CTA that met one computes its outputs again
+// by FMA (slow; rare).  Of values below 2^-109 parts are lost to the smallest bfloat16.
+#include "mma_sync.cuh"
+#include "tcgen05.cuh"
+
+namespace einf {
+
+constexpr int kPartRows = 128, kPartK = 64, kPartThreads = 512;
+constexpr int kPartTile = kPartRows * kPartK * 2;                 // bytes of one part of one operand
+constexpr int kPartStage = 6 * kPartTile;                         // W's parts, then A's
+constexpr int kPartSmem = 2 * kPartStage + 1024;
+constexpr int kPartFold = 8;                                      // blocks of 64 columns whose sums are added up before they join the total
+
+struct PartsArgs {
+  const float* a; const float* w; const float* bias;
+  float* out;                 // [m, n], rows ldo apart; or sums [shares][m][n]
+  int m, n, k;
+  long long lda, ldo;
+  int blocks_each;            // blocks of 64 columns that a CTA takes
+  int shared;
+  int* status;                // may be null
+};
+
+// Eight values as four pairs of each part; false if one has none.
+__device__ __forceinline__ bool split_eight(const float4& x, const float4& y, uint4 (&part)[3]) {
+  constexpr float kLargest = 3.3895314e38f;
+  const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+  bool fine = true;
+  uint32_t p[3][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float a = v[2 * i], b = v[2 * i + 1];
+    fine = fine && fabsf(a) <= kLargest && fabsf(b) <= kLargest;
+    p[0][i] = pack_pair(a, b);
+    a -= low_bf16(p[0][i]);
+    b -= high_bf16(p[0][i]);
+    p[1][i] = pack_pair(a, b);
+    p[2][i] = pack_pair(a - low_bf16(p[1][i]), b - high_bf16(p[1][i]));
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) part[j] = make_uint4(p[j][0], p[j][1], p[j][2], p[j][3]);
+  return fine;
+}
+
+__device__ __forceinline__ bool parts_wait(uint32_t bar, uint32_t parity) {
+  for (int poll = 0; poll < kPolls; ++poll) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+
+__global__ void __launch_bounds__(kPartThreads, 1) gemm_parts_kernel(const __grid_constant__ PartsArgs g) {
+  extern __shared__ unsigned char parts_smem[];
+  __shared__ __align__(8) unsigned long long bars[1];
+  __shared__ uint32_t tmem_address;
+  const uint32_t tiles = (smem_address(parts_smem) + 1023u) & ~1023u;
+  const uint32_t bar = smem_address(bars);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int row0 = (int)blockIdx.y * kPartRows, col0 = (int)blockIdx.x * kPartRows;
+  const int blocks = (g.k + kPartK - 1) / kPartK, first = (int)blockIdx.z * g.blocks_each, last = min(blocks, first + g.blocks_each);
+  if (tid == 0) {
+    bar_init(bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_address(&tmem_address)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_address;
+  pdl_launch_dependents();
+  pdl_wait();
+  // this thread brings eight columns of rows 64 apart, two of either operand
+  const int chunk = tid & 7, first_row = tid >> 3;
+  float4 w_next[2][2], a_next[2][2];
+  auto fetch = [&](int block) {
+    const int at = block * kPartK + chunk * 8;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int wr = col0 + first_row + 64 * i, ar = row0 + first_row + 64 * i;
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4* from = reinterpret_cast<const float4*>(g.w + (long long)wr * g.k + at);
+      const bool there = wr < g.n && at < g.k;                    // k is a multiple of eight
+      w_next[i][0] = there ? __ldg(from) : zero;
+      w_next[i][1] = there ? __ldg(from + 1) : zero;
+      const float4* rows = reinterpret_cast<const float4*>(g.a + (long long)ar * g.lda + at);
+      const bool in = ar < g.m && at < g.k;
+      a_next[i][0] = in ? rows[0] : zero;
+      a_next[i][1] = in ? rows[1] : zero;
+    }
+  };
+  bool fine = true, ended = true;
+  auto store = [&](uint32_t stage) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int row = first_row + 64 * i;
+      const uint32_t at = stage + row * 128 + ((chunk ^ (row & 7)) << 4);
+      uint4 part[3];
+      fine = split_eight(w_next[i][0], w_next[i][1], part) && fine;
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at + j * kPartTile), "r"(part[j].x), "r"(part[j].y), "r"(part[j].z), "r"(part[j].w) : "memory");
+      fine = split_eight(a_next[i][0], a_next[i][1], part) && fine;
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at + (3 + j) * kPartTile), "r"(part[j].x), "r"(part[j].y), "r"(part[j].z), "r"(part[j].w) : "memory");
+    }
+  };
+  // D = F32, A = B = BF16, both K-major, N = 128, M = 128
+  constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kPartRows >> 3) << 17) | ((uint32_t)(kPartRows >> 4) << 24);
+  // this thread's 32 outputs: row col0 + 32 (warp & 3) + lane of W with 32 rows of A
+  float sums[32];
+#pragma unroll
+  for (int e = 0; e < 32; ++e) sums[e] = 0.f;
+  const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * 32), total = mine + 256;
+  // the sums of the i-th block of this CTA: of its first 32 columns, and of the others
+  auto promote = [&](int i) {
+    ended = parts_wait(bar, i & 1) && ended;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+    for (int part = 0; part < 4; ++part) {
+      float v[16];
+      tmem_ld16(mine + (part & 1) * 128 + (part >> 1) * 16, v);
+      tmem_ld_wait();
+#pragma unroll
+      for (int e = 0; e < 16; ++e) sums[(part >> 1) * 16 + e] += v[e];
+    }
+    if (i % kPartFold == kPartFold - 1) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        if (i >= kPartFold) {
+          float v[16];
+          tmem_ld16(total + half * 16, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) sums[half * 16 + e] += v[e];
+        }
+        uint32_t r[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(sums[half * 16 + e]);
+        tmem_st16(total + half * 16, r);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) sums[half * 16 + e] = 0.f;
+      }
+      tmem_st_wait();
+    }
+  };
+  const int count = last - first;
+  if (count > 0) fetch(first);
+  for (int i = 0; i < count; ++i) {
+    const uint32_t stage = tiles + (i & 1) * kPartStage;
+    store(stage);                       // its products of two blocks ago are over: their sums have been added
+    if (i + 1 < count) fetch(first + i + 1);
+    if (i > 0) promote(i - 1);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint64_t w0 = desc_k_major(stage), a0 = desc_k_major(stage + 3 * kPartTile);
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int order = 2; order >= 0; --order)
+#pragma unroll
+          for (int p = 0; p <= order; ++p)
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) {
+              const uint32_t step = (half * 2 + kk) * 32;
+              mma_ss(tmem + half * 128, desc_advance(w0, p * kPartTile + step), desc_advance(a0, (order - p) * kPartTile + step),
+                     kIdesc, order < 2 || p > 0 || kk > 0);
+            }
+      mma_commit(bar);
+    }
+    __syncwarp();
+  }
+  if (count > 0) promote(count - 1);
+  if (count >= kPartFold) {
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      float v[16];
+      tmem_ld16(total + half * 16, v);
+      tmem_ld_wait();
+#pragma unroll
+      for (int e = 0; e < 16; ++e) sums[half * 16 + e] += v[e];
+    }
+  }
+  const bool all_fine = __syncthreads_and(fine), all_ended = __syncthreads_and(ended);
+  if (!all_ended && tid == 0 && g.status) atomicOr(g.status, kStatusWaitExpired);
+  const int col = col0 + (warp & 3) * 32 + lane;
+  if (col < g.n) {
+    float* out = g.out + (g.shared ? (long long)blockIdx.z * g.m * g.n : 0);
+    const long long ldo = g.shared ? g.n : g.ldo;
+    const float bias = g.bias && !g.shared ? g.bias[col] : 0.f;
+    const int first_token = row0 + (warp >> 2) * 32;
+    if (all_fine && all_ended) {
+#pragma unroll
+      for (int e = 0; e < 32; ++e)
+        if (first_token + e < g.m) out[(long long)(first_token + e) * ldo + col] = sums[e] + bias;
+    } else {
+      const int k0 = first * kPartK, k1 = min(g.k, last * kPartK);
+      for (int e = 0; e < 32 && first_token + e < g.m; ++e) {
+        const float* x = g.a + (long long)(first_token + e) * g.lda;
+        const float* y = g.w + (long long)col * g.k;
+        float sum = 0.f;
+        for (int kk = k0; kk < k1; ++kk) sum = fmaf(x[kk], y[kk], sum);
+        out[(long long)(first_token + e) * ldo + col] = all_ended ? sum + bias : __int_as_float(0x7fffffff);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+}
+
+// The shares' sums in the order of K, and bias.
+__global__ void __launch_bounds__(256) gemm_parts_sum_kernel(const __grid_constant__ PartsArgs g, const float* sums, int shares) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long total = (long long)g.m * g.n;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    float v[16], sum = 0.f;
+#pragma unroll
+    for (int s = 0; s < 16; ++s) v[s] = s < shares ? sums[s * total + i] : 0.f;
+#pragma unroll
+    for (int s = 0; s < 16; ++s)
+      if (s < shares) sum += v[s];
+    const int r = (int)(i / g.n), c = (int)(i - (long long)r * g.n);
+    g.out[(long long)r * g.ldo + c] = g.bias ? sum + g.bias[c] : sum;
+  }
+}
+
+}  // namespace einf
+
+using namespace einf;
+
+// sums: [shares][m][n] floats where shares (up to 8) is more than one.
+extern "C" int einf_gemm_parts(const float* a, const float* w, const float* bias, float* out, int m, int n, int k, long long lda,
+                               long long ldo, int shares, float* sums, int* status, cudaStream_t stream) {
+  if (m <= 0 || n <= 0) return 0;
+  const int blocks = (k + kPartK - 1) / kPartK;
+  if (k <= 0 || k % 8 || lda % 4 || ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || shares < 1 || shares > 16 || shares > blocks ||
+      (shares > 1 && !sums) || (m + kPartRows - 1) / kPartRows > 65535)
+    return (int)cudaErrorInvalidValue;
+  PartsArgs g{a, w, bias, shares > 1 ? sums : out, m, n, k, lda, ldo, (blocks + shares - 1) / shares, shares > 1, status};
+  cudaError_t e = cudaFuncSetAttribute(gemm_parts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPartSmem);
+  if (e != cudaSuccess) return (int)e;
+  const dim3 grid((n + kPartRows - 1) / kPartRows, (m + kPartRows - 1) / kPartRows, shares);
+  e = launch_pdl(gemm_parts_kernel, grid, dim3(kPartThreads), kPartSmem, stream, g);
+  if (e != cudaSuccess || shares == 1) return (int)e;
+  g.out = out;
+  const long long ctas = ((long long)m * n + 255) / 256;
+  return (int)launch_pdl(gemm_parts_sum_kernel, dim3((unsigned)(ctas < 148 * 8 ? ctas : 148 * 8)), dim3(256), 0, stream, g, (const float*)sums, shares);
+}

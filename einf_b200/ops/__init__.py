@@ -371,6 +371,59 @@ def gemm_simt(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
     )
 
 
+def gemm_parts_takes(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether :func:`gemm_parts` takes these operands: all float32, K a multiple of eight, rows that start on 16 bytes."""
+    return (
+        x.dtype == weight.dtype == out.dtype == torch.float32 and x.shape[1] % 8 == 0 and x.shape[1] > 0
+        and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and x.shape[0] < 8 << 20
+    )
+
+
+@functools.lru_cache(maxsize=4096)
+def _gemm_parts_shares(row_tiles: int, col_tiles: int, k: int) -> int:
+    """How many CTAs share K in :func:`gemm_parts`: whichever takes the fewest microseconds by what was measured, 1.7 for 64
+    columns of K and 3 beside them for every wave of tiles of 128 x 128, and where K is shared 3.5 for the second
+    launch and its bytes at 4 TB/s (545 rows, 896 -> 896: 28.7 alone, 17.7 by four, 22.5 by five; 128 rows, 4,864 -> 896: 132
+    alone, 25 by eight, 18 by sixteen).  Made of whole tiles, so that up to 128 rows all get the same sums."""
+    tiles, blocks = row_tiles * col_tiles, -(-k // 64)
+    best, shares = float("inf"), 1
+    for s in range(1, min(blocks, 16) + 1):
+        each = -(-blocks // s)
+        if -(-blocks // each) != s or (s > 1 and 4 * s * tiles << 14 > GEMM_SIMT_SUM_BYTES):
+            continue
+        cost = -(-tiles * s // _sm_count()) * (1.7 * each + 3) + (3.5 + 2e-6 * (s * tiles << 14) if s > 1 else 0)
+        if cost < best:
+            best, shares = cost, s
+    return shares
+
+
+def gemm_parts(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
+               status: Optional[torch.Tensor] = None, shares: Optional[int] = None) -> None:
+    """``out = x @ weight.T (+ bias)``, all float32 (:func:`gemm_parts_takes`), on the tensor cores as products of three
+    bfloat16 parts of either operand.  ``shares`` (up to 16, none without a block of 64 columns): CTAs that share K."""
+    m, k = x.shape
+    n = weight.shape[0]
+    if shares is None:
+        shares = _gemm_parts_shares(-(-m // 128), -(-n // 128), k)
+    if weight.shape != (n, k) or out.shape != (m, n):
+        raise ValueError(f"gemm: x {tuple(x.shape)}, weight {tuple(weight.shape)}, out {tuple(out.shape)}")
+    if x.stride(1) != 1 or out.stride(1) != 1:
+        raise ValueError("gemm operands must have unit stride in their last dimension")
+    if not gemm_parts_takes(x, weight, out):
+        raise UnsupportedSize("gemm_parts takes float32 operands and results, K a multiple of eight, rows that start on 16 bytes")
+    if not (x.is_cuda and out.is_cuda):
+        raise KernelError("gemm operands must be on a CUDA device: there is no CPU path")
+    sums = None
+    if shares > 1:
+        sums = torch.empty((shares, m, n), dtype=torch.float32, device=x.device)
+        global launch_count
+        launch_count += 1
+    fn = _fn("einf_gemm_parts", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_int,
+                                 c_void_p, c_void_p, c_void_p])
+    _check(fn(x.data_ptr(), _dev(weight, "weight"), _opt(bias, "bias", torch.float32), out.data_ptr(), m, n, k, x.stride(0),
+              out.stride(0), shares, _opt(sums, "sums", torch.float32), _opt(status, "status", torch.int32), _stream()), "gemm_parts")
+
+
 #: most bytes of block sums a 32-bit product leaves for its second kernel (beyond that K is not shared: such outputs
 #: have tiles enough)
 GEMM_SIMT_SUM_BYTES = 64 << 20
@@ -453,13 +506,17 @@ def linear(
     weight: torch.Tensor,
     bias: Optional[torch.Tensor],
     out: torch.Tensor,
+    status: Optional[torch.Tensor] = None,
 ) -> None:
     """``out = x @ weight.T (+ bias)``.
 
     bfloat16 activations against a bfloat16 matrix go to the tensor cores through
     the library matrix product (as the reference's ``F.linear`` does,
-    ``src/einf/executors/torch/packed_qkv.py:148``); everything else, the whole
-    32-bit path included, runs the FMA kernel, which rounds no input.
+    ``src/einf/executors/torch/packed_qkv.py:148``); the 32-bit path goes there as three
+    bfloat16 parts of either operand, which together are the operand
+    (:func:`gemm_parts`; faster than FMA at every size measured, 1 to 1,024 rows against 8 to 17,920 columns: 1,152 x 896
+    20 -> 13 us for one row and 42 -> 21 for 545, 9,728 x 896 40 -> 26 and 211 -> 85, 896 x 4,864 24 -> 15 and 118 -> 45);
+    operands of mixed type, and rows that are not aligned, run the FMA kernel, which rounds no input.
     """
     if x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.is_contiguous():
         if not x.is_cuda:
@@ -470,6 +527,9 @@ def linear(
             torch.mm(x, weight.t(), out_dtype=torch.float32, out=out)
         if bias is not None:
             add_bias(out, bias)
+        return
+    if x.is_cuda and gemm_parts_takes(x, weight, out):
+        gemm_parts(x, weight, bias, out, status)
         return
     gemm_simt(x, weight, bias, out)
 
@@ -545,7 +605,7 @@ def project(
         gemm_tcgen05(x, weight, None, out, status, splits)
         return out
     out = torch.empty((tokens, n), dtype=out_dtype, device=x.device)
-    linear(x, weight, None, out)
+    linear(x, weight, None, out, status)
     return out
 
 

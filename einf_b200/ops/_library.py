@@ -35,6 +35,7 @@ LAUNCHERS = {
     "einf_head_prompt_attention": "attention_prompt",
     "einf_gemm_simt": "gemm_simt",
     "einf_gemm_simt_shares": "gemm_simt",
+    "einf_gemm_parts": "gemm_parts",
     "einf_gemm_tcgen05": "gemm_tcgen05",
     "einf_gemm_tcgen05_splits": "gemm_tcgen05",
     "einf_gemm_grouped_tcgen05": "gemm_tcgen05",

@@ -124,17 +124,17 @@ class PagedAttention(Mixer):
                 tiled = ("attention_mixed_tiled:" + ops.mixed_tiled_variant(int(spec["num_heads"])),)
             if runtime.dtype == torch.bfloat16:
                 tiled += ("attention_mixed_mma",)
-            return ("pointwise", "attention_mixed", "gemm_simt") + tiled + cls._product_libraries(runtime)
+            return ("pointwise", "attention_mixed", "gemm_simt", "gemm_parts") + tiled + cls._product_libraries(runtime)
         if cls._is_general(spec):
             fast = (f"attention_tcgen05:HEAD_SIZE={int(spec['head_size'])}",) \
                 if cls._general_on_tensor_cores(spec, runtime.dtype) else ()
             store = ("qkv_conv",) if spec.get("conv_taps") or spec.get("output_gate") else ("pointwise",)
-            return store + ("attention_generic", "gemm_simt") + cls._product_libraries(runtime) + fast
+            return store + ("attention_generic", "gemm_simt", "gemm_parts") + cls._product_libraries(runtime) + fast
         if ops.has_fast_attention(runtime.dtype, int(spec["head_size"])):
             # the page size is the engine's choice: ask for both prefill kernels of this head size
             libraries = ops.attention_libraries(int(spec["head_size"]), 16)
-            return ("pointwise", "gemm_simt", "gemm_tcgen05", "few_tokens") + libraries
-        return ("pointwise", "attention_generic", "gemm_simt") + cls._product_libraries(runtime)
+            return ("pointwise", "gemm_simt", "gemm_parts", "gemm_tcgen05", "few_tokens") + libraries
+        return ("pointwise", "attention_generic", "gemm_simt", "gemm_parts") + cls._product_libraries(runtime)
 
     @staticmethod
     def _product_libraries(runtime):

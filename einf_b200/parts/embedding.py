@@ -62,7 +62,7 @@ class LinearHead(Part):
 
     @classmethod
     def kernel_libraries(cls, spec, runtime):
-        return ("gemm_simt",) + (("gemm_tcgen05",) if runtime.dtype == torch.bfloat16 else ()) + \
+        return ("gemm_simt", "gemm_parts",) + (("gemm_tcgen05",) if runtime.dtype == torch.bfloat16 else ()) + \
             (("pointwise",) if spec.get("softcap") or spec.get("scale") else ())
 
     def __init__(self, spec, tensors, runtime, tied=None):

@@ -79,7 +79,7 @@ class LatentAttention(Mixer):
             fast = ("attention_latent",)
         if cls._prompts_by_heads(spec, row, runtime.dtype):
             fast += ("attention_prompt",)
-        return ("pointwise", "latent", "attention_generic", "gemm_simt") + \
+        return ("pointwise", "latent", "attention_generic", "gemm_simt", "gemm_parts") + \
             (("gemm_tcgen05",) if runtime.dtype == torch.bfloat16 else ()) + fast
 
     @staticmethod

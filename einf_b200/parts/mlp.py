@@ -54,7 +54,7 @@ class GatedMLP(FeedForward):
 
     @classmethod
     def kernel_libraries(cls, spec, runtime):
-        return ("pointwise", "gemm_simt") + (("gemm_tcgen05", "few_tokens") if runtime.dtype == torch.bfloat16 else ())
+        return ("pointwise", "gemm_simt", "gemm_parts") + (("gemm_tcgen05", "few_tokens") if runtime.dtype == torch.bfloat16 else ())
 
     def __init__(self, spec, tensors, runtime):
         super().__init__(spec, tensors, runtime)
@@ -105,7 +105,7 @@ class DenseMLP(FeedForward):
 
     @classmethod
     def kernel_libraries(cls, spec, runtime):
-        return ("pointwise", "gemm_simt") + (("gemm_tcgen05",) if runtime.dtype == torch.bfloat16 else ())
+        return ("pointwise", "gemm_simt", "gemm_parts") + (("gemm_tcgen05",) if runtime.dtype == torch.bfloat16 else ())
 
     def __init__(self, spec, tensors, runtime):
         super().__init__(spec, tensors, runtime)

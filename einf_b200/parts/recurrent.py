@@ -30,7 +30,7 @@ from .base import CacheView, Mixer, StateNeed, StepContext, register_part
 class _RecurrentMixer(Mixer):
     @classmethod
     def kernel_libraries(cls, spec, runtime):
-        return ("pointwise", "recurrence", "gemm_simt") + (
+        return ("pointwise", "recurrence", "gemm_simt", "gemm_parts") + (
             ("gemm_tcgen05", "recurrence_chunks") if runtime.dtype == torch.bfloat16 else ()
         )
 
@@ -223,7 +223,7 @@ class GatedLinearRecurrence(Mixer):
 
     @classmethod
     def kernel_libraries(cls, spec, runtime):
-        return ("pointwise", "recurrence", "gemm_simt") + (("gemm_tcgen05",) if runtime.dtype == torch.bfloat16 else ())
+        return ("pointwise", "recurrence", "gemm_simt", "gemm_parts") + (("gemm_tcgen05",) if runtime.dtype == torch.bfloat16 else ())
 
     def __init__(self, spec, tensors, runtime):
         super().__init__(spec, tensors, runtime)

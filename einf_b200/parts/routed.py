@@ -63,7 +63,7 @@ class RoutedMLP(FeedForward):
 
     @classmethod
     def kernel_libraries(cls, spec, runtime):
-        return ("pointwise", "routed", "gemm_simt") + (("gemm_tcgen05",) if runtime.dtype == torch.bfloat16 else ())
+        return ("pointwise", "routed", "gemm_simt", "gemm_parts") + (("gemm_tcgen05",) if runtime.dtype == torch.bfloat16 else ())
 
     def __init__(self, spec, tensors, runtime):
         super().__init__(spec, tensors, runtime)

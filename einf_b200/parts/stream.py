@@ -81,7 +81,7 @@ class TokenSideInput(Part):
 
     @classmethod
     def kernel_libraries(cls, spec, runtime):
-        return ("stream", "gemm_simt") + (("gemm_tcgen05",) if runtime.dtype == torch.bfloat16 else ())
+        return ("stream", "gemm_simt", "gemm_parts") + (("gemm_tcgen05",) if runtime.dtype == torch.bfloat16 else ())
 
     def __init__(self, spec, tensors, runtime):
         super().__init__(spec, tensors, runtime)

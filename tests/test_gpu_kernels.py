@@ -1254,6 +1254,45 @@ def test_sampling_random_rows_and_filters(dev, first_case):
                 assert low - 1e-4 <= u <= float(cumulative[token]) + 1e-4, (case, r, index, u)
 
 
+@pytest.mark.parametrize("m,n,k,shares", [
+    (1, 8, 8, None), (128, 128, 64, 1), (129, 127, 72, 2), (7, 300, 1024, 16), (300, 200, 4864, None), (130, 1000, 520, 3),
+    (64, 128, 512, 1), (33, 257, 576, 1), (5, 130, 1088, 1),
+])
+def test_gemm_of_three_parts(dev, m, n, k, shares):
+    """Edges of tiles, K of fewer and more than 512 elements a CTA (where sums join the total) and of a remainder;
+    strided rows; K shared; values of very different sizes."""
+    from einf_b200 import ops
+
+    torch.manual_seed(m * 7 + n + k)
+    wide = torch.randn(m, k + 12, device=dev) * 10 ** (torch.rand(m, k + 12, device=dev) * 4 - 2)
+    x, w, bias = wide[:, :k], torch.randn(n, k, device=dev), torch.randn(n, device=dev)
+    out, status = torch.full((m, n + 3), 7.0, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    ops.gemm_parts(x, w, bias, out[:, :n], status, shares)
+    want = x.double() @ w.double().T + bias.double()
+    # what the parts leave out is 2^-23 of a term at most; the sums of 32 elements are cut off twice, the others rounded
+    bound = (x.double().abs() @ w.double().abs().T + bias.double().abs()) * 2 ** -22
+    assert bool(((out[:, :n].double() - want).abs() <= bound).all()) and int(status) == 0
+    assert bool((out[:, n:] == 7.0).all())
+    if shares is None:                # a row's sums do not depend on the rows beside it, up to a tile of them
+        one = torch.empty(1, n, device=dev)
+        ops.gemm_parts(x[:1], w, bias, one, status)
+        assert m > 128 or torch.equal(one[0], out[0, :n])
+
+
+def test_gemm_of_three_parts_with_values_that_have_none(dev):
+    from einf_b200 import ops
+
+    torch.manual_seed(5)
+    x, w = torch.randn(150, 128, device=dev), torch.randn(260, 128, device=dev)
+    x[3, 5], x[140, 7], w[7, 9], w[200, 1], w[100, 2] = float("inf"), -float("inf"), float("nan"), 3.4e38, 1e-42
+    x[:, 1] *= 0.01
+    for shares in (1, 2):
+        got, want = torch.empty(150, 260, device=dev), torch.empty(150, 260, device=dev)
+        ops.gemm_parts(x, w, None, got, shares=shares)
+        ops.gemm_simt(x, w, None, want)
+        torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-5, equal_nan=True)
+
+
 @pytest.mark.parametrize("top_k", [1, 5, 255, 256, 257, 0])
 def test_sampling_where_few_tokens_are_looked_at(dev, top_k):
     """Both sides of what one CTA settles by itself and of what a CTA lists: more tied tokens than it takes, a row
