@@ -684,6 +684,24 @@ __global__ void silu_mul_kernel(const TIn* __restrict__ gate_up, int splits, siz
   }
 }
 
+// The same, as exact, for dense 32-bit rows whose width is a multiple of 4: 16-byte loads and stores, block = (token, chunk of
+// the row), so that no element needs a division for its place (the kernel above spends most of its time on those: 545
+// rows of 4,864 28 us, here 8).
+__global__ void silu_mul_f32x4_kernel(const float* __restrict__ gate_up, float* __restrict__ out, int intermediate,
+                                      int chunks_per_row) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const unsigned t = blockIdx.x / (unsigned)chunks_per_row;
+  const unsigned chunk = blockIdx.x - t * (unsigned)chunks_per_row;
+  const int i = (int)(chunk * blockDim.x + threadIdx.x) << 2;
+  if (i >= intermediate) return;
+  const float* row = gate_up + (size_t)t * 2 * intermediate;
+  const float4 g = *reinterpret_cast<const float4*>(row + i), u = *reinterpret_cast<const float4*>(row + intermediate + i);
+  *reinterpret_cast<float4*>(out + (size_t)t * intermediate + i) =
+      make_float4(g.x / (1.f + expf(-g.x)) * u.x, g.y / (1.f + expf(-g.y)) * u.y, g.z / (1.f + expf(-g.z)) * u.z,
+                  g.w / (1.f + expf(-g.w)) * u.w);
+}
+
 // The same for dense bfloat16 rows whose width is a multiple of 8: 16-byte loads and stores, one
 // vector per thread, block = (token, chunk of the row).  At thousands of tokens this kernel is
 // bound by arithmetic, not by memory, if it divides and calls expf exactly; the result is
@@ -1576,6 +1594,13 @@ extern "C" int einf_silu_mul(const void* gate_up, int in_dtype, int splits, long
     if ((long long)chunks * num_tokens < (1ll << 31))
       return (int)launch_pdl(silu_mul_bf16x8_kernel, (int)(chunks * num_tokens), threads, 0, stream,
                              (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)out, intermediate, chunks);
+  }
+  if (splits == 1 && in_dtype == kFloat32 && dtype == kFloat32 && intermediate % 4 == 0 && ((uintptr_t)gate_up & 15) == 0 &&
+      ((uintptr_t)out & 15) == 0) {
+    const int chunks = ((intermediate >> 2) + threads - 1) / threads;
+    if ((long long)chunks * num_tokens < (1ll << 31))
+      return (int)launch_pdl(silu_mul_f32x4_kernel, (int)(chunks * num_tokens), threads, 0, stream, (const float*)gate_up,
+                             (float*)out, intermediate, chunks);
   }
   size_t blocks = (total + threads - 1) / threads;
   if (blocks > 148 * 16) blocks = 148 * 16;

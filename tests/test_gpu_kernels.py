@@ -224,6 +224,19 @@ def test_silu_mul_vector_kernel(dev, rows, intermediate):
     torch.testing.assert_close(out, want, **tol(torch.bfloat16))
 
 
+@pytest.mark.parametrize("rows, intermediate", [(1, 4), (3, 1028), (545, 4864)])
+def test_silu_mul_of_wide_32_bit_rows(dev, rows, intermediate):
+    from einf_b200 import ops
+
+    torch.manual_seed(rows)
+    gate_up = torch.randn(rows, 2 * intermediate, device=dev) * 4
+    gate_up[0, :4] = torch.tensor([-200.0, -90.0, 90.0, -1e30], device=dev)
+    out, want = torch.full((rows, intermediate), float("nan"), device=dev), torch.empty(rows, intermediate, device=dev)
+    ops.silu_mul(gate_up, out)
+    ref.silu_mul(gate_up, want)
+    torch.testing.assert_close(out, want, **tol(torch.float32))
+
+
 def test_report_writes_pinned_host_memory(dev):
     from einf_b200 import ops
 
