@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "mma_sync.cuh"
+#include "tcgen05.cuh"
 
 namespace einf {
 
@@ -38,6 +39,8 @@ struct HeadPromptArgs {
   const float* sink; const float* gate;
   int heads, dim, rot_dim, value_size, window, wave;
   float scale_log2;
+  int* status;                       // may be null
+  int short_rows;                    // portions of up to this many tokens (0: none) are the other kernel's
 };
 
 // KEY: dim + rot_dim filled up to 128 or 192; VALUE: value_size filled up to 64 or 128.
@@ -54,7 +57,7 @@ head_prompt_attention_kernel(const __grid_constant__ HeadPromptArgs a) {
   const int sub = (row_tile & 1) * kPromptRows;
   const int rows = min(kPromptRows, tile.z - sub);
   const int key_token = tile.y - tile.w;                  // packed index of the request's position 0
-  if (rows <= 0 || (a.q_start && a.q_start[tile.x] != key_token)) {
+  if (rows <= 0 || (a.q_start && a.q_start[tile.x] != key_token) || (a.short_rows && (tile.w > 0 || tile.z > a.short_rows))) {
     pdl_wait();
     return;
   }
@@ -245,6 +248,315 @@ head_prompt_attention_kernel(const __grid_constant__ HeadPromptArgs a) {
   }
 }
 
+// The same on the fifth-generation tensor cores, for heads in whole 128-byte lines (dim, rot_dim and value_size multiples of
+// 64): a CTA has 128 queries of one head and takes its keys 128 at a time, in turn by two warpgroups, each with scores, sums
+// and an accumulator of its own, which meet at the end.  One warp brings keys and values (TMA, two stages each), one lane of
+// another issues the products: scores into the group's 128 columns of tensor memory; the group's threads (a row each)
+// take them out, and put the weights, as bfloat16 pairs, into the same columns, where the second product reads them as its
+// first operand.  While one group is at its softmax the other's products run.  A row's reference moves only when a tile's
+// maximum is more than 2^8 above it, so that the accumulator is rarely taken out and multiplied.  Values behind the last key
+// of the request are cleared in shared memory: the tile's other rows are another request's, and zero times infinity is not zero.
+// Measured (B200, us, the kernel above / this one): 12 heads, keys of 128 + 64, values of 128: 2,048 tokens 124 / 33 (490
+// TFLOP/s), 4,096 283 / 92, 300 18.4 / 11.8, 128 10.1 / 8.1; 14 heads of 64 + 64, values of 64, 2,048 tokens 80 / 32.  Portions of up to
+// 64 tokens fill half a tile of this one at most and stay above: 40 of 30 tokens 14.8 / 31.7, one of 20 6.4 / 8.2.  What bounds it
+// now: a tile's softmax, 128 exponentials a thread between two passes through tensor memory.
+constexpr int kHeadThreads = 320, kHeadSlice = 128 * 64 * 2;
+
+template <int KS, int VS>
+struct HeadLayout {
+  static constexpr int kQ = 0, kK = KS * kHeadSlice, kV = kK + 2 * KS * kHeadSlice, kBars = kV + 2 * VS * kHeadSlice;
+  static constexpr int kShared = kBars + 8 * 16 + 16, kSums = kShared, kBytes = kSums + 4 * 128 * 4 + 1024;
+};
+
+__device__ __forceinline__ bool head_wait(uint32_t bar, uint32_t parity, int* status) {
+  for (int poll = 0; poll < kPolls; ++poll) {
+    if (bar_test(bar, parity)) return true;
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  if (status) atomicOr(status, kStatusWaitExpired);
+  return false;
+}
+
+template <int KS, int VS>
+__global__ void __launch_bounds__(kHeadThreads, 1)
+head_prompt_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_qr,
+                           const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_kr,
+                           const __grid_constant__ CUtensorMap map_v, const __grid_constant__ HeadPromptArgs a) {
+  using L = HeadLayout<KS, VS>;
+  constexpr int kValue = VS * 64;
+  extern __shared__ unsigned char head_smem[];
+  int row_tile, h;
+  rows_of_cta(a.wave, a.heads, &row_tile, &h);
+  const int4 tile = a.tiles[row_tile];
+  const int rows = tile.z, key_token = tile.y - tile.w;
+  if (rows <= 0 || (a.q_start && a.q_start[tile.x] != key_token) || (tile.w == 0 && rows <= a.short_rows)) {
+    pdl_launch_dependents();
+    pdl_wait();
+    return;
+  }
+  const uint32_t raw = smem_address(head_smem), base = (raw + 1023u) & ~1023u;
+  unsigned char* generic = head_smem + (base - raw);
+  const uint32_t bars = base + L::kBars;
+  const uint32_t q_full = bars, k_full = bars + 8, k_empty = bars + 24, v_full = bars + 40, v_empty = bars + 56, s_full = bars + 72,
+                 p_full = bars + 88, o_done = bars + 104, holder = bars + 128;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int pos0 = tile.w, last_pos = pos0 + rows - 1;
+  const int first_tile = a.window > 0 ? max(0, pos0 - a.window + 1) / 128 : 0, n = last_pos / 128 + 1 - first_tile;
+  if (tid == 0) {
+    bar_init(q_full, 1);
+    for (int s = 0; s < 2; ++s) {
+      bar_init(k_full + 8 * s, 1);
+      bar_init(k_empty + 8 * s, 1);
+      bar_init(v_full + 8 * s, 1);
+      bar_init(v_empty + 8 * s, 1);
+      bar_init(s_full + 8 * s, 1);
+      bar_init(p_full + 8 * s, 128);
+      bar_init(o_done + 8 * s, 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 9) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(holder) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(generic + L::kBars + 128);
+  pdl_launch_dependents();
+  pdl_wait();
+  const int dim_lines = a.dim / 64;
+  bool ok = true;
+  if (warp == 8) {
+    if (lane == 0) {
+      bar_expect_tx(q_full, KS * kHeadSlice);
+      for (int c = 0; c < KS; ++c) {
+        if (c < dim_lines) tma_2d(base + L::kQ + c * kHeadSlice, &map_q, (int)(h * a.q_plain_head) + 64 * c, tile.y, q_full);
+        else tma_2d(base + L::kQ + c * kHeadSlice, &map_qr, (int)(h * a.q_rot_head) + 64 * (c - dim_lines), tile.y, q_full);
+      }
+      for (int i = 0; i < n && ok; ++i) {
+        const int s = i & 1, token = key_token + (first_tile + i) * 128;
+        const uint32_t again = ((i >> 1) & 1) ^ 1;
+        if (i >= 2) ok = head_wait(k_empty + 8 * s, again, a.status);
+        if (!ok) break;
+        bar_expect_tx(k_full + 8 * s, KS * kHeadSlice);
+        for (int c = 0; c < KS; ++c) {
+          const uint32_t to = base + L::kK + (s * KS + c) * kHeadSlice;
+          if (c < dim_lines) tma_2d(to, &map_k, (int)(h * a.k_head) + 64 * c, token, k_full + 8 * s);
+          else tma_2d(to, &map_kr, 64 * (c - dim_lines), token, k_full + 8 * s);
+        }
+        if (i >= 2) ok = head_wait(v_empty + 8 * s, again, a.status);
+        if (!ok) break;
+        bar_expect_tx(v_full + 8 * s, VS * kHeadSlice);
+        for (int c = 0; c < VS; ++c)
+          tma_2d(base + L::kV + (s * VS + c) * kHeadSlice, &map_v, (int)(h * a.v_head) + 64 * c, token, v_full + 8 * s);
+      }
+    }
+  } else if (warp == 9) {
+    constexpr uint32_t kScores = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+    constexpr uint32_t kMix = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(kValue >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+    ok = head_wait(q_full, 0, a.status);
+    auto scores = [&](int i) {
+      const int s = i & 1, turn = i >> 1;
+      ok = ok && head_wait(k_full + 8 * s, turn & 1, a.status);
+      if (turn > 0) ok = ok && head_wait(o_done + 8 * s, (turn - 1) & 1, a.status);   // the group's weights are used up
+      if (!ok || lane != 0) return;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int c = 0; c < KS; ++c) {
+        const uint64_t q = desc_k_major(base + L::kQ + c * kHeadSlice), k = desc_k_major(base + L::kK + (s * KS + c) * kHeadSlice);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) mma_ss(tmem + 128 * s, desc_advance(q, kk * 32), desc_advance(k, kk * 32), kScores, c > 0 || kk > 0);
+      }
+      mma_commit(k_empty + 8 * s);
+      mma_commit(s_full + 8 * s);
+    };
+    if (n > 0) scores(0);
+    for (int i = 0; i < n; ++i) {
+      const int s = i & 1, turn = i >> 1;
+      if (i + 1 < n) scores(i + 1);
+      ok = ok && head_wait(v_full + 8 * s, turn & 1, a.status);
+      const int real = last_pos + 1 - (first_tile + i) * 128;
+      if (real < 128) {
+        for (int e = lane; e < (128 - real) * 8 * VS; e += 32) {
+          const int c = e / ((128 - real) * 8), in = e - c * ((128 - real) * 8);
+          asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(base + L::kV + (s * VS + c) * kHeadSlice + (real + (in >> 3)) * 128 + (in & 7) * 16), "r"(0u) : "memory");
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
+      __syncwarp();
+      ok = ok && head_wait(p_full + 8 * s, turn & 1, a.status);
+      if (ok && lane == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint64_t v = desc_mn_major(base + L::kV + s * VS * kHeadSlice, kHeadSlice);
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) mma_ts(tmem + 256 + 128 * s, tmem + 128 * s + kk * 8, desc_advance(v, kk * 2048), kMix, turn > 0 || kk > 0);
+        mma_commit(v_empty + 8 * s);
+        mma_commit(o_done + 8 * s);
+      }
+      __syncwarp();
+    }
+  }
+  float m = -INFINITY, l = 0.f;
+  const int group = (warp >> 2) & 1, r = (warp & 3) * 32 + lane;
+  const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16), mine = lanes + 128 * group, mixed = lanes + 256 + 128 * group;
+  const int turns = (n - group + 1) >> 1;
+  if (warp < 8) {
+    const int pos = pos0 + r;
+    for (int turn = 0; turn < turns && ok; ++turn) {
+      ok = head_wait(s_full + 8 * group, turn & 1, a.status);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int j0 = (first_tile + 2 * turn + group) * 128;
+      float z[128];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld32(mine + 32 * c, z + 32 * c);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_wait32(z + 32 * c);
+      if (j0 + 127 > pos0 || (a.window > 0 && j0 <= last_pos - a.window)) {
+        const int to = pos - j0, from = a.window > 0 ? to - a.window : -1;        // visible: from < key <= to
+#pragma unroll
+        for (int e = 0; e < 128; ++e) z[e] = e <= to && e > from ? z[e] : -INFINITY;
+      }
+      float top = -INFINITY;
+#pragma unroll
+      for (int e = 0; e < 128; ++e) top = fmaxf(top, z[e]);
+      top *= a.scale_log2;
+      const bool moves = top > m + 8.f || (m == -INFINITY && top > -INFINITY);
+      if (__any_sync(0xffffffffu, moves)) {
+        const float factor = moves ? exp2f(m - top) : 1.f;       // nothing seen so far: zero
+        if (moves) m = top;
+        l *= factor;
+        if (turn > 0) {                                           // the scores' arrival says that the last product is over
+#pragma unroll
+          for (int c = 0; c < kValue / 32; ++c) {
+            float o[32];
+            tmem_ld32(mixed + 32 * c, o);
+            tmem_ld_wait32(o);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) o[e] *= factor;
+            tmem_st32(mixed + 32 * c, o);
+          }
+        }
+      }
+      const float shift = m == -INFINITY ? 0.f : m;
+      float sum = 0.f;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t pairs[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          const float x = fast_exp2(fmaf(z[32 * c + 2 * e], a.scale_log2, -shift)), y = fast_exp2(fmaf(z[32 * c + 2 * e + 1], a.scale_log2, -shift));
+          sum += x + y;
+          pairs[e] = pack_pair(x, y);
+        }
+        tmem_st16(mine + 16 * c, pairs);
+      }
+      l += sum;
+      tmem_st_wait();
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      bar_arrive(p_full + 8 * group);
+    }
+    if (turns > 0) ok = ok && head_wait(o_done + 8 * group, (turns - 1) & 1, a.status);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    float* shared = reinterpret_cast<float*>(generic + L::kSums);
+    shared[group * 128 + r] = m;
+    shared[256 + group * 128 + r] = l;
+  }
+  __syncthreads();
+  float factor = 0.f;
+  float* half = reinterpret_cast<float*>(generic + L::kK);        // the second group's share: every load and product is over
+  constexpr int kPitch = kValue + 1;
+  static_assert(128 * kPitch * 4 <= (2 * KS + 2 * VS) * kHeadSlice, "the share fits the keys' and values' place");
+  if (warp < 8) {
+    const float* shared = reinterpret_cast<const float*>(generic + L::kSums);
+    const float m0 = shared[r], m1 = shared[128 + r], top = fmaxf(m0, m1), at = top == -INFINITY ? 0.f : top;
+    float total = shared[256 + r] * exp2f(m0 - at) + shared[384 + r] * exp2f(m1 - at);
+    if (a.sink) total += exp2f(a.sink[h] * 1.4426950408889634f - top);
+    factor = total > 0.f && m != -INFINITY ? exp2f(m - at) / total : 0.f;
+    if (a.gate && r < rows) factor *= a.gate[(long long)(tile.y + r) * a.heads + h];
+    if (group == 1 && turns > 0) {
+#pragma unroll
+      for (int c = 0; c < kValue / 32; ++c) {
+        float o[32];
+        tmem_ld32(mixed + 32 * c, o);
+        tmem_ld_wait32(o);
+#pragma unroll
+        for (int e = 0; e < 32; ++e) half[r * kPitch + 32 * c + e] = factor != 0.f ? o[e] * factor : 0.f;
+      }
+    }
+  }
+  __syncthreads();
+  if (warp < 4) {
+    __nv_bfloat16* out = a.out + ((long long)(tile.y + r) * a.heads + h) * kValue;
+#pragma unroll
+    for (int c = 0; c < kValue / 32; ++c) {
+      float o[32];
+      tmem_ld32(mixed + 32 * c, o);
+      tmem_ld_wait32(o);
+      uint32_t pairs[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        float x = factor != 0.f ? o[2 * e] * factor : 0.f, y = factor != 0.f ? o[2 * e + 1] * factor : 0.f;
+        if (n > 1) {
+          x += half[r * kPitch + 32 * c + 2 * e];
+          y += half[r * kPitch + 32 * c + 2 * e + 1];
+        }
+        pairs[e] = pack_pair(x, y);
+      }
+      if (r < rows) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          *reinterpret_cast<uint4*>(out + 32 * c + 8 * e) = make_uint4(pairs[4 * e], pairs[4 * e + 1], pairs[4 * e + 2], pairs[4 * e + 3]);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 9) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+  }
+}
+
+// rows x cols bfloat16, unit stride along cols, rows `stride` elements apart, box of (64 cols x 128 rows), 128-byte swizzle
+static int head_map(CUtensorMap* map, const void* base, long long rows, long long cols, long long stride) {
+  EncodeTiledFn encode = encode_tiled();
+  if (!encode) return (int)cudaErrorNotSupported;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)stride * 2};
+  cuuint32_t box[2] = {64, 128};
+  cuuint32_t element_strides[2] = {1, 1};
+  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, element_strides,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+}
+
+template <int KS, int VS>
+static int launch_head_tcgen05(const HeadPromptArgs& a, int tokens, int num_tiles, cudaStream_t stream) {
+  CUtensorMap q, qr, k, kr, v;
+  int e = head_map(&q, a.q_plain, tokens, (a.heads - 1) * a.q_plain_head + a.dim, a.q_plain_token);
+  if (!e) e = head_map(&qr, a.q_rot, tokens, (a.heads - 1) * a.q_rot_head + a.rot_dim, a.q_rot_token);
+  if (!e) e = head_map(&k, a.k_plain, tokens, (a.heads - 1) * a.k_head + a.dim, a.k_token);
+  if (!e) e = head_map(&kr, a.k_rot, tokens, a.rot_dim, a.rot_dim);
+  if (!e) e = head_map(&v, a.v, tokens, (a.heads - 1) * a.v_head + a.value_size, a.v_token);
+  if (e) return e;
+  auto kernel = head_prompt_tcgen05_kernel<KS, VS>;
+  constexpr int kBytes = HeadLayout<KS, VS>::kBytes;
+  const cudaError_t set = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+  if (set != cudaSuccess) return (int)set;
+  return (int)launch_pdl(kernel, dim3(num_tiles * a.heads), dim3(kHeadThreads), kBytes, stream, q, qr, k, kr, v, a);
+}
+
 // Cached rows of the step's tokens, taken apart: rows[t] = the first `first` elements of the row in slot t, rest[t] the next
 // `second` (multiples of eight; a token without a slot gets zeros).
 __global__ void __launch_bounds__(256)
@@ -289,6 +601,8 @@ extern "C" int einf_latent_rows(const void* cache, const int* slots, long long n
                          (__nv_bfloat16*)rest, second, tokens);
 }
 
+// `tensor_memory`: by the kernel on tcgen05 (sizes multiples of 64, rot_dim above 0), `short_rows`: of it and the other kernel,
+// the other one has the portions of up to that many tokens and this one the longer ones (0: the kernel has all).
 // Portions that start at position 0 in this step, their tokens packed one after the other; with `q_start`, the requests' first
 // tokens, `tiles` of other portions are left out (without it there must be none).  Sizes and
 // strides in multiples of eight elements, pointers on 16-byte borders; dim + rot_dim up to 192, value_size up to 128.
@@ -299,7 +613,8 @@ extern "C" int einf_head_prompt_attention(const void* q_plain, long long q_plain
                                           long long v_token, long long v_head, const int* tiles, int num_tiles,
                                           const int* q_start, void* out,
                                           const float* sink, const float* gate, int heads, int dim, int rot_dim,
-                                          int value_size, int window, float scale, int wave, cudaStream_t stream) {
+                                          int value_size, int window, float scale, int wave, int tokens, int tensor_memory, int short_rows, int* status,
+                                          cudaStream_t stream) {
   if (num_tiles == 0) return 0;
   const long long strides = q_plain_token | q_plain_head | q_rot_token | q_rot_head | k_token | k_head | v_token | v_head;
   if (heads <= 0 || 2ll * num_tiles * heads > 0x7fffffff || dim <= 0 || rot_dim < 0 || dim + rot_dim > 192 ||
@@ -316,6 +631,14 @@ extern "C" int einf_head_prompt_attention(const void* q_plain, long long q_plain
   a.tiles = (const int4*)tiles; a.q_start = q_start; a.out = (__nv_bfloat16*)out; a.sink = sink; a.gate = gate;
   a.heads = heads; a.dim = dim; a.rot_dim = rot_dim; a.value_size = value_size; a.window = window; a.wave = wave;
   a.scale_log2 = scale * 1.4426950408889634f;
+  a.status = status;
+  a.short_rows = short_rows;
+  if (tensor_memory) {
+    if (dim % 64 || rot_dim % 64 || rot_dim == 0 || value_size % 64 || tokens <= 0) return (int)cudaErrorInvalidValue;
+    if (dim + rot_dim == 128)
+      return value_size == 64 ? launch_head_tcgen05<2, 1>(a, tokens, num_tiles, stream) : launch_head_tcgen05<2, 2>(a, tokens, num_tiles, stream);
+    return value_size == 64 ? launch_head_tcgen05<3, 1>(a, tokens, num_tiles, stream) : launch_head_tcgen05<3, 2>(a, tokens, num_tiles, stream);
+  }
   if (dim + rot_dim <= 128)
     return (int)(value_size <= 64 ? launch_head_prompt<128, 64>(a, num_tiles, stream)
                                   : launch_head_prompt<128, 128>(a, num_tiles, stream));

@@ -1055,6 +1055,17 @@ def latent_rows(cache: torch.Tensor, slots: torch.Tensor, rows: torch.Tensor, re
     )
 
 
+#: portions of up to this many tokens take :func:`head_prompt_attention`'s kernel with tiles of 64 queries
+HEAD_PROMPT_SHORT = 64
+
+
+def head_prompt_ways(lengths: Optional[Sequence[int]]) -> tuple[bool, bool]:
+    """Whether portions of these lengths (None: unknown) hold any for the kernel of short and of long ones."""
+    if lengths is None:
+        return True, True
+    return any(n <= HEAD_PROMPT_SHORT for n in lengths), any(n > HEAD_PROMPT_SHORT for n in lengths)
+
+
 def head_prompt_attention(
     q_plain: torch.Tensor,
     q_rot: torch.Tensor,
@@ -1068,6 +1079,9 @@ def head_prompt_attention(
     sink: Optional[torch.Tensor] = None,
     gate: Optional[torch.Tensor] = None,
     q_start: Optional[torch.Tensor] = None,
+    status: Optional[torch.Tensor] = None,
+    tensor_memory: Optional[bool] = None,
+    lengths: Optional[Sequence[int]] = None,
 ) -> None:
     """Causal attention of prompts that start in this step, every head with keys and values of its own: query head h
     scores key head h, ``q_plain . k_plain + q_rot . k_rot``, where all heads share ``k_rot``.  ``q_plain``, ``k_plain``
@@ -1075,7 +1089,11 @@ def head_prompt_attention(
     ``k_rot [tokens, rot]``, ``out [tokens, heads, value]``, all bfloat16; ``q_tiles`` as for
     :func:`paged_prefill_attention`, of requests whose first token in the step is at position 0; with ``q_start`` (int32
     ``[requests + 1]``) other requests may be among them and are left out.  ``window``, ``sink`` and ``gate``: see
-    :func:`paged_attention_generic`."""
+    :func:`paged_attention_generic`.
+
+    Heads in whole 128-byte lines run on tcgen05 where a portion has more than :data:`HEAD_PROMPT_SHORT` tokens, each by
+    its own length; ``lengths``: those portions' lengths where the host knows them, which spares a launch with
+    nothing to do.  ``tensor_memory`` (True or False) sends all portions to one kernel."""
     tokens, heads, dim = q_plain.shape
     rot_dim, value_size = q_rot.shape[2], v.shape[2]
     if q_rot.shape[:2] != (tokens, heads) or k_plain.shape != (tokens, heads, dim) or k_rot.shape != (tokens, rot_dim) or \
@@ -1092,20 +1110,29 @@ def head_prompt_attention(
     if sink is not None and (sink.dtype != torch.float32 or sink.shape != (heads,)):
         raise ValueError(f"sink must be float32 [{heads}]")
     _check_gate(gate, tokens, heads)
+    if tensor_memory is not None:
+        ways = [(int(tensor_memory), 0)]
+    elif dim % 64 or rot_dim != 64 or value_size % 64:
+        ways = [(0, 0)]
+    else:
+        short, long = head_prompt_ways(lengths)
+        ways = [(0, HEAD_PROMPT_SHORT)] * short + [(1, HEAD_PROMPT_SHORT)] * long
     fn = _fn(
         "einf_head_prompt_attention",
         [c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p,
          c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-         c_int, c_float, c_int, c_void_p],
+         c_int, c_float, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     )
-    _check(
-        fn(q_plain.data_ptr(), q_plain.stride(0), q_plain.stride(1), q_rot.data_ptr(), q_rot.stride(0), q_rot.stride(1),
-           k_plain.data_ptr(), k_plain.stride(0), k_plain.stride(1), _dev(k_rot, "k_rot"), v.data_ptr(), v.stride(0),
-           v.stride(1), _opt(q_tiles, "q_tiles", torch.int32), q_tiles.shape[0], _opt(q_start, "q_start", torch.int32),
-           _dev(out, "out"), _opt(sink, "sink", torch.float32), _opt(gate, "gate", torch.float32), heads, dim, rot_dim, value_size,
-           int(window) if window else 0, float(scale), _sm_count(), _stream()),
-        "head_prompt_attention",
-    )
+    for way, short_rows in ways:
+        _check(
+            fn(q_plain.data_ptr(), q_plain.stride(0), q_plain.stride(1), q_rot.data_ptr(), q_rot.stride(0), q_rot.stride(1),
+               k_plain.data_ptr(), k_plain.stride(0), k_plain.stride(1), _dev(k_rot, "k_rot"), v.data_ptr(), v.stride(0),
+               v.stride(1), _opt(q_tiles, "q_tiles", torch.int32), q_tiles.shape[0], _opt(q_start, "q_start", torch.int32),
+               _dev(out, "out"), _opt(sink, "sink", torch.float32), _opt(gate, "gate", torch.float32), heads, dim, rot_dim, value_size,
+               int(window) if window else 0, float(scale), _sm_count(), tokens, way, short_rows,
+               _opt(status, "status", torch.int32), _stream()),
+            "head_prompt_attention",
+        )
 
 
 #: activations of :func:`activation` by name

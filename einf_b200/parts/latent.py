@@ -163,7 +163,8 @@ class LatentAttention(Mixer):
     def launch_key(self, ctx: StepContext, page_size: int) -> tuple:
         """As for the attention mixer: the decode kernel's shape follows the batch and the longest context."""
         singles = int(ctx.single_tokens.shape[0])
-        return self._ways(ctx) + (self._singles_key(ctx, page_size, singles) if singles else ())
+        ways = self._ways(ctx)
+        return ways + (ops.head_prompt_ways(self._fresh(ctx)) if ways[0] else ()) + (self._singles_key(ctx, page_size, singles) if singles else ())
 
     def _singles_key(self, ctx: StepContext, page_size: int, singles: int) -> tuple:
         context = self._visible(ctx.max_context_len)
@@ -180,6 +181,11 @@ class LatentAttention(Mixer):
             return False, ctx.q_tiles.shape[0] > 0
         return ctx.starts_and_goes_on()
 
+    @staticmethod
+    def _fresh(ctx: StepContext) -> list[int]:
+        """Lengths of the portions of several tokens that start their prompts."""
+        return [n for n, start in zip(ctx.q_lens, ctx.start_positions) if n > 1 and start == 0]
+
     def _prompts(self, q_plain, q_full, gate, ctx: StepContext, cache: CacheView, mixed: torch.Tensor) -> None:
         """Prompts that start in the step, head by head: its rows through both up-projections, then attention into those
         portions' rows of ``mixed [T, H, value]``."""
@@ -188,12 +194,13 @@ class LatentAttention(Mixer):
         part = torch.empty((tokens, self.rot_dim), dtype=q_full.dtype, device=device)
         ops.latent_rows(cache.k, ctx.slots[cache.group], rows, part)
         kv = torch.empty((tokens, self.kv_up.shape[0]), dtype=q_full.dtype, device=device)
-        ops.linear(rows, self.kv_up, None, kv)
+        ops.linear(rows, self.kv_up, None, kv, ctx.status)
         keys = heads * self.dim
         ops.head_prompt_attention(
             q_plain, q_full[:, :, self.kv_rank:self.kv_rank + self.rot_dim], kv[:, :keys].unflatten(1, (heads, self.dim)),
             part, kv[:, keys:].unflatten(1, (heads, self.value_size)), ctx.q_tiles, mixed, self.scale, self.window,
-            sink=self.sink, gate=gate, q_start=ctx.q_start,
+            sink=self.sink, gate=gate, q_start=ctx.q_start, status=ctx.status,
+            lengths=self._fresh(ctx),
         )
 
     def _visible(self, context: int) -> int:

@@ -366,6 +366,47 @@ def test_prompts_head_by_head(dev, heads, dim, rot, value, window, lengths, opti
         first += n
 
 
+@pytest.mark.parametrize("heads, dim, value, window, lengths", [
+    (3, 128, 128, None, (700, 129, 1)), (2, 64, 64, 200, (900,)), (1, 128, 64, None, (256, 384)), (2, 64, 128, 130, (385, 5))])
+def test_prompts_head_by_head_in_tensor_memory(dev, heads, dim, value, window, lengths):
+    """Prompts of many key tiles, both groups' turns and one group's alone, scores that grow along the prompt (so that the
+    rows' references move), and values that are not finite in the request behind, whose rows fill up the last tile."""
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(dim + value)
+    tokens, rot = sum(lengths), 64
+    draw = lambda *shape: torch.randn(shape, generator=gen).to(torch.bfloat16).to(dev)  # noqa: E731
+    q_plain, q_rot, k_rot, v = draw(tokens, heads, dim), draw(tokens, heads, rot), draw(tokens, rot), draw(tokens, heads, value)
+    grow = torch.cat([torch.linspace(0.1, 8.0, n) for n in lengths])[:, None, None].to(dev)
+    k_plain = (draw(tokens, heads, dim).float() * grow).to(torch.bfloat16)
+    tiles, first = [], 0
+    for r, n in enumerate(lengths):
+        tiles += [(r, first + at, min(128, n - at), at) for at in range(0, n, 128)]
+        first += n
+    tiles, scale = torch.tensor(tiles, dtype=torch.int32, device=dev), (dim + rot) ** -0.5
+    out, status = torch.full((tokens, heads, value), float("nan"), dtype=torch.bfloat16, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    ops.head_prompt_attention(q_plain, q_rot, k_plain, k_rot, v, tiles, out, scale, window, status=status, tensor_memory=True)
+    first = 0
+    for n in lengths:
+        part = slice(first, first + n)
+        scores = torch.einsum("ihd,jhd->hij", q_plain[part].double(), k_plain[part].double())
+        scores = (scores + torch.einsum("ihr,jr->hij", q_rot[part].double(), k_rot[part].double())) * scale
+        i, j = torch.arange(n, device=dev)[:, None], torch.arange(n, device=dev)[None, :]
+        scores = scores.masked_fill(~((j <= i) & (j > i - (window or tokens))), float("-inf"))
+        weights = torch.softmax(scores, dim=2)
+        want = torch.einsum("hij,jhv->ihv", weights, v[part].double())
+        size = torch.einsum("hij,jhv->ihv", weights, v[part].double().abs())
+        bound = 2.0 ** -8 * want.abs() + (2.0 ** -8 + 2.0 ** -14) * size      # as above; scores of up to fifty
+        assert bool(((out[part].double() - want).abs() <= bound).all())
+        first += n
+    if len(lengths) > 1:
+        again, begin = torch.empty_like(out), lengths[0]
+        v[begin:], k_plain[begin:] = float("inf"), float("nan")
+        ops.head_prompt_attention(q_plain, q_rot, k_plain, k_rot, v, tiles, again, scale, window, status=status, tensor_memory=True)
+        assert torch.equal(again[:begin], out[:begin])
+    assert int(status) == 0
+
+
 @pytest.mark.parametrize("heads, dim, rot, value, rank, q_rank, page", [
     (3, 128, 64, 128, 512, None, 16), (4, 40, 24, 72, 32, 64, 16), (2, 64, 16, 64, 192, 40, 8), (2, 64, 8, 40, 176, 40, 5)])
 @pytest.mark.parametrize("window", [None, 60])
