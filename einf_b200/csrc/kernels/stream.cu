@@ -560,13 +560,33 @@ stream_tail_tokens_kernel(float* __restrict__ residual, const __grid_constant__ 
   float* y = x + TB * hidden;        // [TB, hidden]
   float* g = y + TB * hidden;        // [TB, side]
   float* red = g + TB * side;        // [TB, warps]
+  float* rows = red + TB * (kTailThreads / 32);   // [TB, side]: the tokens' rows of the table
   pdl_launch_dependents();
-  pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int kWarps = kTailThreads / 32;
   const int t0 = blockIdx.x * TB;
   const int count = min(TB, num_tokens - t0);
   const bool adds = pending.a != nullptr || pending.b != nullptr;
+  // Before the wait: the tokens' rows of the table (two loads one behind the other, out of HBM), and a hint for the lines of
+  // the matrices, which every CTA reads: the next layer's are in L2 by the time this layer's stream is there.
+  if (table) {
+    for (int idx = tid; idx < TB * side; idx += kTailThreads) {
+      const int i = idx / side;
+      float v = 0.f;
+      if (i < count) {
+        int token = token_ids[t0 + i];
+        token = token < 0 ? 0 : (token >= vocab ? vocab - 1 : token);     // a bad id was reported by the embedding
+        v = to_float(table[(size_t)token * side + idx - i * side]);
+      }
+      rows[idx] = v;
+    }
+    constexpr int kLine = 128 / (int)sizeof(TW);
+    for (int line = blockIdx.x * kTailThreads + tid; line < side * hidden / kLine; line += gridDim.x * kTailThreads) {
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(gate + (size_t)line * kLine));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(proj_t + (size_t)line * kLine));
+    }
+  }
+  pdl_wait();
   for (int idx = tid; idx < TB * hidden; idx += kTailThreads) {
     const int i = idx / hidden;
     float v = 0.f;
@@ -610,11 +630,7 @@ stream_tail_tokens_kernel(float* __restrict__ residual, const __grid_constant__ 
 #pragma unroll
         for (int i = 0; i < TB; ++i) {
           const float total = warp_sum(dot[r][i]);
-          if (lane == 0 && d0 + r < side && i < count) {
-            int token = token_ids[t0 + i];
-            token = token < 0 ? 0 : (token >= vocab ? vocab - 1 : token);     // a bad id was reported by the embedding
-            g[i * side + d0 + r] = gelu_tanh_f(total) * to_float(table[(size_t)token * side + d0 + r]);
-          }
+          if (lane == 0 && d0 + r < side && i < count) g[i * side + d0 + r] = gelu_tanh_f(total) * rows[i * side + d0 + r];
         }
     }
     __syncthreads();
@@ -1079,7 +1095,7 @@ extern "C" int einf_stream_tail(float* residual, const void* pend_a, int a_dtype
   if (hidden % 8 == 0 && side > 0 && ((uintptr_t)gate | (uintptr_t)proj_t) % 16 == 0) {
     // tokens a CTA: eight for a long step where they fit beside a second CTA, else four; one while every token
     // still gets an SM of its own (the step is then bound by one CTA's instructions, not by the matrices' bytes)
-    auto bytes = [&](int each) { return (size_t)(2 * each * hidden + each * side + each * (kTailThreads / 32)) * sizeof(float); };
+    auto bytes = [&](int each) { return (size_t)(2 * each * hidden + 2 * each * side + each * (kTailThreads / 32)) * sizeof(float); };
     const int each = (num_tokens >= 1024 && bytes(8) <= 100 * 1024) ? 8 : (num_tokens <= 148 ? 1 : 4);
     if (bytes(each) <= 200 * 1024) {
       const int blocks = (num_tokens + each - 1) / each;
