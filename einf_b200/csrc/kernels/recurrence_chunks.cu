@@ -112,7 +112,9 @@ struct ChunkLayout {
   static constexpr int kValue = kKey + kInParts * kKeyPart;      // in the first pass the weighted values take their place
   static constexpr int kValuePart = kChunk * kColPitch;
   static constexpr int kQuery = kValue + (kEmit ? kInParts : 3) * kValuePart;
-  static constexpr int kState = kQuery + (kEmit ? kInParts * kKeyPart : 0);
+  // the queries' place, and behind them that of the ten 16 x 16 tiles of q . k, which the halves of the warps exchange there
+  static constexpr int kQueryBytes = kInParts * kKeyPart > 10 * 1024 ? kInParts * kKeyPart : 10 * 1024;
+  static constexpr int kState = kQuery + (kEmit ? kQueryBytes : 0);
   static constexpr int kStatePart = ROWS * kColPitch;
   static constexpr int kDiagonal = kState + (kEmit ? 3 * kStatePart : 0);
   static constexpr int kVectors = kDiagonal + (kEmit ? kChunk * kDiagonalPitch * 4 : 0);   // 64 floats each
@@ -329,35 +331,42 @@ recurrence_chunk_kernel(const __grid_constant__ ChunkArgs a) {
     cp_async_wait_groups<0>();
     __syncthreads();
 
-    if (kEmit && 16 * tile < n) {
-      // (q_t . k_s) for this warp's 16 tokens t and the tokens s up to the last of them
-      float G[8][4];
+    if constexpr (kEmit) {
+      // (q_t . k_s) for this warp's 16 tokens t and the tokens s up to the last of them, every other tile of 16: the warp with
+      // the same tokens and the other columns has the others (both made all of them before: of the last tokens' warps,
+      // whose products are the CTA's longest chain, 96 products in place of 192 where both operands have three parts)
+      const bool here = 16 * tile < n;
+      float G[2][2][4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
+      for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) G[j][e] = 0.f;
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) G[i][j][e] = 0.f;
       const uint32_t q_at = base + L::kQuery + (16 * tile + in8 + 8 * second) * L::kRowPitch;
-      const uint32_t k_at = base + L::kKey + (in8 + 8 * third) * L::kRowPitch;
+      const uint32_t k_at = base + L::kKey + (in8 + 8 * third + 16 * half) * L::kRowPitch;
       auto query = [&](uint32_t (&f)[kIn][4], int kk) {
 #pragma unroll
         for (int p = 0; p < kIn; ++p) ldsm_x4(f[p], q_at + p * L::kKeyPart + ((2 * kk + third) ^ in8) * 16);
       };
+      if (here) {
 #pragma unroll 1
-      for (int kk = 0; kk < ROWS / 16; ++kk) {
-        uint32_t qf[kIn][4];
-        query(qf, kk);
+        for (int kk = 0; kk < ROWS / 16; ++kk) {
+          uint32_t qf[kIn][4];
+          query(qf, kk);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (j > tile) break;
-          uint32_t k0[kIn][2], k1[kIn][2];
+          for (int i = 0; i < 2; ++i) {
+            if (half + 2 * i > tile) break;
+            uint32_t k0[kIn][2], k1[kIn][2];
 #pragma unroll
-          for (int p = 0; p < kIn; ++p) {
-            uint32_t f[4];
-            ldsm_x4(f, k_at + p * L::kKeyPart + 16 * j * L::kRowPitch + ((2 * kk + second) ^ in8) * 16);
-            k0[p][0] = f[0]; k0[p][1] = f[1]; k1[p][0] = f[2]; k1[p][1] = f[3];
+            for (int p = 0; p < kIn; ++p) {
+              uint32_t f[4];
+              ldsm_x4(f, k_at + p * L::kKeyPart + 32 * i * L::kRowPitch + ((2 * kk + second) ^ in8) * 16);
+              k0[p][0] = f[0]; k0[p][1] = f[1]; k1[p][0] = f[2]; k1[p][1] = f[3];
+            }
+            mma_parts<kIn, kIn>(G[i][0], qf, k0);
+            mma_parts<kIn, kIn>(G[i][1], qf, k1);
           }
-          mma_parts<kIn, kIn>(G[2 * j], qf, k0);
-          mma_parts<kIn, kIn>(G[2 * j + 1], qf, k1);
         }
       }
       // what the chunk's start state gives: d0[t] S0^T q_t
@@ -367,7 +376,7 @@ recurrence_chunk_kernel(const __grid_constant__ ChunkArgs a) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) Y[j][e] = 0.f;
 #pragma unroll 1
-      for (int kk = 0; kk < ROWS / 16; ++kk) {
+      for (int kk = 0; kk < (here ? ROWS / 16 : 0); ++kk) {
         uint32_t qf[kIn][4];
         query(qf, kk);
 #pragma unroll
@@ -385,6 +394,21 @@ recurrence_chunk_kernel(const __grid_constant__ ChunkArgs a) {
           mma_parts<kIn, 3>(Y[NH - 1], qf, s0);
         }
       }
+      __syncthreads();                             // everyone has read the queries
+      auto exchanged = [&](int j, int e) {         // this lane's four of the tokens 16 j + 8 e on
+        return chunk_smem + L::kQuery + ((tile * (tile + 1) / 2 + j) * 2 + e) * 512 + lane * 16;
+      };
+      if (here) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int j = half + 2 * i;
+          if (j > tile) break;
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            *reinterpret_cast<float4*>(exchanged(j, e)) = make_float4(G[i][e][0], G[i][e][1], G[i][e][2], G[i][e][3]);
+        }
+      }
+      __syncthreads();
       const int t_low = 16 * tile + g, t_high = t_low + 8;
       const float before_low = before[t_low], before_high = before[t_high];
       double earlier_tiles = 1.;                   // the whole tiles before this one
@@ -403,13 +427,14 @@ recurrence_chunk_kernel(const __grid_constant__ ChunkArgs a) {
       double between_tiles = 1.;                   // the whole tiles between s's and t's
 #pragma unroll
       for (int kk = 3; kk >= 0; --kk) {
-        if (kk > tile) continue;
+        if (kk > tile || !here) continue;
         uint32_t wf[3][4];
         const float between = (float)between_tiles;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {              // the eight tokens s of each half of the 16
           const int s = 8 * e + q2;
-          const float* p = G[2 * kk + e];
+          const float4 scores = *reinterpret_cast<const float4*>(exchanged(kk, e));
+          const float p[4] = {scores.x, scores.y, scores.z, scores.w};
           float w[4];
           if (kk == tile) {
             const float2 low = *reinterpret_cast<const float2*>(diagonal + t_low * kDiagonalPitch + s);
