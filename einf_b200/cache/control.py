@@ -42,4 +42,5 @@ SchedulerStats = _control.SchedulerStats
 PackConfig = _control.PackConfig
 PackedStep = _control.PackedStep
 pack_plan = _control.pack_plan
+pack_sampling = _control.pack_sampling
 step_buffer_size = _control.step_buffer_size

@@ -168,6 +168,29 @@ PYBIND11_MODULE(_control, m) {
       .def_readonly("num_logprobs", &SamplingParams::num_logprobs)
       .def_property_readonly("is_greedy", &SamplingParams::greedy);
 
+  // A sampled step's parameters into the sampler's staging buffer of `max_rows` rows: seeds and sample indices as int64,
+  // temperatures, top-p and min-p as float32, top-k as int32.  Anything but SamplingParams and integers: TypeError.
+  m.def("pack_sampling", [](py::sequence params, py::sequence indices, uintptr_t address, int max_rows) {
+    const int rows = (int)py::len(params);
+    if (rows > max_rows || (int)py::len(indices) != rows) throw std::invalid_argument("one set of parameters and one index per row");
+    auto* wide = reinterpret_cast<int64_t*>(address);
+    auto* real = reinterpret_cast<float*>(wide + 2 * (size_t)max_rows);
+    auto* whole = reinterpret_cast<int32_t*>(real + 3 * (size_t)max_rows);
+    for (int r = 0; r < rows; ++r) {
+      py::object item = params[r], index = indices[r];
+      if (!py::isinstance<SamplingParams>(item) || !PyLong_Check(index.ptr())) throw py::type_error("SamplingParams and integers");
+      const auto& p = item.cast<const SamplingParams&>();
+      if (p.seed > (uint64_t)INT64_MAX) throw std::overflow_error("seed beyond 63 bits");
+      wide[r] = (int64_t)p.seed;
+      wide[max_rows + r] = PyLong_AsLongLong(index.ptr());
+      if (PyErr_Occurred()) throw py::error_already_set();
+      real[r] = p.temperature;
+      real[max_rows + r] = p.top_p;
+      real[2 * max_rows + r] = p.min_p;
+      whole[r] = p.top_k;
+    }
+  });
+
   py::class_<RequestSpec>(m, "RequestSpec")
       .def(py::init([](RequestId id, std::vector<int> prompt, int max_new_len, py::object sampling) {
              RequestSpec spec;

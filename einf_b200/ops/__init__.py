@@ -60,19 +60,22 @@ def _dev(t: torch.Tensor, name: str) -> int:
 def _opt(t: Optional[torch.Tensor], name: str, dtype: torch.dtype) -> int:
     if t is None:
         return 0
+    if t.dtype is dtype and t.is_cuda and t.is_contiguous():
+        return t.data_ptr()
     if t.dtype != dtype:
         raise TypeError(f"{name} must be {dtype}, got {t.dtype}")
     return _dev(t, name)
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_get_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
 
 
 def _stream() -> int:
     """The current stream's handle.  Asked for at every launch, so by the short road where torch
     has one (the public ``current_stream()`` builds an object: 7 us, more than a launch costs)."""
-    if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+    if _raw_stream is not None and torch.cuda.is_initialized():
+        return _raw_stream(_get_device())
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -604,6 +607,8 @@ def project(
             out = torch.empty((tokens, n), dtype=out_dtype, device=x.device)
         gemm_tcgen05(x, weight, None, out, status, splits)
         return out
+    if x.dtype == weight.dtype == out_dtype == torch.bfloat16 and x.is_cuda and x.is_contiguous():
+        return torch.mm(x, weight.t())      # as in linear(); the result's allocation inside the call is 3 us shorter
     out = torch.empty((tokens, n), dtype=out_dtype, device=x.device)
     linear(x, weight, None, out, status)
     return out

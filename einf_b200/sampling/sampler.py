@@ -15,6 +15,7 @@ import numpy as np
 import torch
 
 from .. import ops
+from ..cache.control import pack_sampling
 
 
 class Sampler:
@@ -31,12 +32,10 @@ class Sampler:
         self._ring = 8
         self._turn = 0
         self._events = [None] * self._ring
-        self._host = torch.zeros((self._ring, 32 * max_rows), dtype=torch.uint8, pin_memory=pin)
+        staging = torch.zeros((self._ring, 32 * max_rows), dtype=torch.uint8, pin_memory=pin)
+        self._host, self._staging = staging.unbind(0), staging.numpy()
         self._dev = torch.zeros(32 * max_rows, dtype=torch.uint8, device=self.device)
-        n, host = max_rows, self._host.numpy()
-        self._wide = host[:, :16 * n].view(np.int64).reshape(self._ring, 2, n)
-        self._real = host[:, 16 * n:28 * n].view(np.float32).reshape(self._ring, 3, n)
-        self._whole = host[:, 28 * n:].view(np.int32)
+        n = max_rows
         wide, real = self._dev[:16 * n].view(torch.int64), self._dev[16 * n:28 * n].view(torch.float32)
         self._columns = (real[:n], self._dev[28 * n:].view(torch.int32), real[n:2 * n], real[2 * n:], wide[:n], wide[n:])
 
@@ -57,15 +56,24 @@ class Sampler:
         self._turn = (turn + 1) % self._ring
         if self._events[turn] is not None:
             self._events[turn].synchronize()
-        wide, real = self._wide[turn], self._real[turn]
-        wide[0, :rows] = [np.int64(p.seed) for p in params]
-        wide[1, :rows] = sample_indices
-        real[:, :rows] = [[p.temperature for p in params], [p.top_p for p in params], [p.min_p for p in params]]
-        self._whole[turn, :rows] = [p.top_k or 0 for p in params]
-        self._dev.copy_(self._host[turn], non_blocking=True)
+        staging = self._host[turn]
+        try:
+            pack_sampling(params, sample_indices, staging.data_ptr(), self.max_rows)
+        except TypeError:               # other objects with the same attributes
+            self._pack(turn, rows, params, sample_indices)
+        self._dev.copy_(staging, non_blocking=True)
         if self.device.type == "cuda":
             if self._events[turn] is None:
                 self._events[turn] = torch.cuda.Event()
             self._events[turn].record(ops.current_stream())
         ops.sample(logits, self.tokens, *self._columns)
         return self.tokens[:rows]
+
+    def _pack(self, turn: int, rows: int, params: Sequence, sample_indices: Sequence[int]) -> None:
+        """What ``pack_sampling`` does, for any objects with the attributes of sampling parameters."""
+        n, host = self.max_rows, self._staging[turn]
+        wide, real = host[:16 * n].view(np.int64).reshape(2, n), host[16 * n:28 * n].view(np.float32).reshape(3, n)
+        wide[0, :rows] = [np.int64(p.seed) for p in params]
+        wide[1, :rows] = sample_indices
+        real[:, :rows] = [[p.temperature for p in params], [p.top_p for p in params], [p.min_p for p in params]]
+        host[28 * n:].view(np.int32)[:rows] = [p.top_k or 0 for p in params]
