@@ -32,13 +32,17 @@ __device__ __forceinline__ void store_quad(T* p, float4 v) {
 }
 
 // finish(token, input, sum): what becomes of a token's sum (`input` its own row); start(): what the sum starts from, or the
-// input itself with kFromInput.  `state` rows are the taps - 1 inputs before a request's tokens, oldest first.
+// input itself with kFromInput.  `state` rows are the taps - 1 inputs before a request's tokens, oldest first.  `updates`: the
+// step has one request, whose first tokens, and with them all that reads its state row, are the first run's: its thread then
+// leaves the last taps - 1 inputs there (of more requests a run may begin behind another's first token: a kernel behind
+// this one does it).
 template <typename T, bool kFromInput, typename Finish>
 __device__ __forceinline__ void conv_run(const T* __restrict__ in, long long in_stride, int c, int t0, int num_tokens, int taps,
                                          const float* __restrict__ weight, float4 bias, float4 start,
-                                         const float* __restrict__ state, long long state_stride, int channels,
+                                         float* state, long long state_stride, int channels,
                                          const int* __restrict__ seq_of_token, const int* __restrict__ q_start,
-                                         const int* __restrict__ state_slots, int num_slots, Finish finish) {
+                                         const int* __restrict__ state_slots, int num_slots, bool updates,
+                                         Finish finish) {
   constexpr int kRows = kRunTokens + kRunTaps - 1;
   const int n = min(kRunTokens, num_tokens - t0);
   float4 x[kRows];                                       // x[i]: the input of token t0 - 3 + i
@@ -89,6 +93,19 @@ __device__ __forceinline__ void conv_run(const T* __restrict__ in, long long in_
       acc.w = fmaf(w[3][j], v.w, acc.w);
     }
     finish(t, acc);
+  }
+  if (!updates || t0 != 0) return;
+  const int slot = state_slots[0];
+  if (slot < 0 || slot >= num_slots) return;
+#pragma unroll
+  for (int u = 0; u < kRunTaps - 1; ++u) {
+    if (u >= taps - 1) break;
+    float4 v = load_quad(in + (long long)(num_tokens - (taps - 1) + u) * in_stride + c);
+    float* row = state + (long long)slot * state_stride + (long long)u * channels + c;
+    row[0] = v.x + bias.x;
+    row[1] = v.y + bias.y;
+    row[2] = v.z + bias.z;
+    row[3] = v.w + bias.w;
   }
 }
 

@@ -74,12 +74,12 @@ __global__ void conv_silu_kernel(const T* __restrict__ in, long long in_stride, 
 template <typename T>
 __global__ void __launch_bounds__(128)
 conv_silu_run_kernel(const T* __restrict__ in, long long in_stride, const float* __restrict__ weight,
-                     const float* __restrict__ bias, const float* __restrict__ conv_state, long long state_stride,
+                     const float* __restrict__ bias, float* conv_state, long long state_stride,
                      const int* __restrict__ seq_of_token, const int* __restrict__ q_start,
                      const int* __restrict__ state_slots, int num_slots, T* __restrict__ out, int channels, int taps,
                      int num_tokens, const T* __restrict__ dt_in, const float* __restrict__ dt_bias,
                      const float* __restrict__ a_log, float* __restrict__ dt_out, float* __restrict__ decay_out, int heads,
-                     int act, const float* __restrict__ input_bias) {
+                     int act, const float* __restrict__ input_bias, bool updates) {
   pdl_launch_dependents();
   pdl_wait();
   const int pieces = channels / 4, runs = (num_tokens + kRunTokens - 1) / kRunTokens;
@@ -90,7 +90,7 @@ conv_silu_run_kernel(const T* __restrict__ in, long long in_stride, const float*
     if (bias) start = make_float4(bias[c], bias[c + 1], bias[c + 2], bias[c + 3]);
     if (input_bias) before = make_float4(input_bias[c], input_bias[c + 1], input_bias[c + 2], input_bias[c + 3]);
     conv_run<T, false>(in, in_stride, c, run * kRunTokens, num_tokens, taps, weight, before, start, conv_state, state_stride,
-                       channels, seq_of_token, q_start, state_slots, num_slots, [&](int t, float4 v) {
+                       channels, seq_of_token, q_start, state_slots, num_slots, updates, [&](int t, float4 v) {
                          if (act) v = make_float4(silu_f(v.x), silu_f(v.y), silu_f(v.z), silu_f(v.w));
                          store_quad(out + (long long)t * channels + c, v);
                        });
@@ -1006,10 +1006,10 @@ extern "C" int einf_conv_silu(const void* in, int dtype, long long in_stride, co
       channels % 4 == 0 && in_stride % 4 == 0 && run_threads < (1ll << 31) && (uintptr_t)in % quad == 0 && (uintptr_t)out % quad == 0) {
     EINF_DISPATCH_2(dtype, T, {
       cudaError_t e = launch_pdl(conv_silu_run_kernel<T>, (int)((run_threads + 127) / 128), 128, 0, stream, (const T*)in,
-                                 in_stride, weight, bias, (const float*)conv_state, state_stride, seq_of_token, q_start,
+                                 in_stride, weight, bias, conv_state, state_stride, seq_of_token, q_start,
                                  state_slots, num_slots, (T*)out, channels, taps, num_tokens, (const T*)dt_in, dt_bias, a_log,
-                                 dt_out, decay_out, heads, act, input_bias);
-      if (e != cudaSuccess || taps == 1) return (int)e;
+                                 dt_out, decay_out, heads, act, input_bias, num_requests == 1 && taps > 1);
+      if (e != cudaSuccess || taps == 1 || num_requests == 1) return (int)e;
       const dim3 grid((channels + 127) / 128, num_requests);
       return (int)launch_pdl(conv_state_update_kernel<T>, grid, 128, 0, stream, (const T*)in, in_stride, conv_state,
                              state_stride, q_start, state_slots, num_slots, channels, taps, input_bias);

@@ -269,9 +269,10 @@ __global__ void conv_rows_kernel(const float* __restrict__ h, const float* __res
 template <typename TOut>
 __global__ void __launch_bounds__(128)
 conv_rows_run_kernel(const float* __restrict__ h, const float* __restrict__ conv_weight, int taps,
-                     const float* __restrict__ conv_state, long long state_stride, int num_slots,
+                     float* conv_state, long long state_stride, int num_slots,
                      const int* __restrict__ seq_of_token, const int* __restrict__ q_start,
-                     const int* __restrict__ state_slots, TOut* __restrict__ out, int hidden, int num_tokens) {
+                     const int* __restrict__ state_slots, TOut* __restrict__ out, int hidden, int num_tokens,
+                     bool updates) {
   pdl_launch_dependents();
   pdl_wait();
   const int pieces = hidden / 4, runs = (num_tokens + kRunTokens - 1) / kRunTokens;
@@ -280,7 +281,7 @@ conv_rows_run_kernel(const float* __restrict__ h, const float* __restrict__ conv
   const int run = index / pieces, c = 4 * (index - run * pieces);
   const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
   conv_run<float, true>(h, hidden, c, run * kRunTokens, num_tokens, taps, conv_weight, none, none, conv_state, state_stride,
-                        hidden, seq_of_token, q_start, state_slots, num_slots,
+                        hidden, seq_of_token, q_start, state_slots, num_slots, updates,
                         [&](int t, float4 v) { store_quad(out + (size_t)t * hidden + c, v); });
 }
 
@@ -998,8 +999,9 @@ extern "C" int einf_norm_conv(const void* pend_a, int a_dtype, int a_splits, lon
     const long long run_threads = (long long)((num_tokens + kRunTokens - 1) / kRunTokens) * (hidden / 4);
     if (quads && num_tokens >= 64ll * num_requests && (long long)num_tokens * hidden > kRunElements && run_threads < (1ll << 31)) {
       e = launch_pdl(conv_rows_run_kernel<T>, (int)((run_threads + 127) / 128), 128, 0, stream, (const float*)scratch,
-                     conv_weight, taps, (const float*)conv_state, state_stride, num_slots, seq_of_token, q_start, state_slots,
-                     (T*)out, hidden, num_tokens);
+                     conv_weight, taps, conv_state, state_stride, num_slots, seq_of_token, q_start, state_slots, (T*)out, hidden,
+                     num_tokens, num_requests == 1 && taps > 1);
+      if (e != cudaSuccess || num_requests == 1) return (int)e;
     } else {
       const long long total = (long long)num_tokens * hidden;
       long long blocks = (total + 255) / 256;

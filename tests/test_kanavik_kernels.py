@@ -384,6 +384,7 @@ def test_end_of_a_layer_on_the_tensor_cores(dev, tokens, hidden, side, layers_do
 @pytest.mark.parametrize("hidden, taps, lengths", [
     (64, 4, (1, 190, 2, 69)), (516, 2, (8, 8, 264, 3)), (1540, 3, (300,)), (2052, 4, (130, 1)), (72, 5, (66, 2)), (70, 3, (80,)),
     (2004, 4, (1, 190, 2, 69)), (1856, 2, (8, 8, 264, 3)), (4100, 3, (130, 1)),      # above 2^19 elements
+    (2004, 4, (262,)), (1856, 2, (283,)), (4100, 3, (131,)),                          # one request
     (64, 4, (1, 1, 1)), (516, 2, (1, 1)), (896, 3, (1, 1, 1, 1)), (2052, 4, (1,)), (72, 5, (1, 1)),
 ])
 def test_norm_and_convolution(dev, dtype, hidden, taps, lengths):

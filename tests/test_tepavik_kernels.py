@@ -505,6 +505,7 @@ def test_gated_norm(dev, dtype, width, parts, gate_first, kind):
 @pytest.mark.parametrize("channels, taps, heads, lengths", [
     (24, 4, 3, (1, 190, 2, 69)), (40, 2, 0, (8, 8, 264, 3)), (64, 1, 1, (65,)), (132, 3, 2, (3, 1, 191)),
     (2004, 4, 3, (1, 190, 2, 69)), (1856, 2, 0, (8, 8, 264, 3)), (8068, 1, 1, (65,)), (2692, 3, 2, (3, 1, 191)),    # 2^19 elements
+    (2004, 4, 3, (262,)), (1856, 2, 0, (283,)), (2692, 3, 2, (195,)),     # one request: the same launch moves its state on
 ])
 def test_conv_silu_over_runs_of_tokens(dev, dtype, channels, taps, heads, lengths):
     """Portions of 64 tokens and more on average, from 2^19 elements on four channels of eight tokens a thread: requests that
