@@ -151,7 +151,8 @@ latent_qkv_store_kernel(const TIn* __restrict__ in, int splits, size_t split_str
                         int num_heads, int dim, int row, int heads_per_cta, const float* __restrict__ kv_norm_weight,
                         float eps, const int* __restrict__ positions, const float* __restrict__ inv_freq, float amplitude,
                         int interleaved, const int* __restrict__ slots, T* __restrict__ q_plain, T* __restrict__ q_full,
-                        float* __restrict__ gate, T* __restrict__ cache, int page_size, int num_pages, int* status) {
+                        float* __restrict__ gate, T* __restrict__ cache, int page_size, int num_pages, T* __restrict__ rows_out,
+                        T* __restrict__ part_out, int* status) {
   extern __shared__ float smem[];
   const int half = rot_dim >> 1;
   float* cos_t = smem;                       // [half]
@@ -186,21 +187,34 @@ latent_qkv_store_kernel(const TIn* __restrict__ in, int splits, size_t split_str
     const float factor = rsqrtf(block_sum(squares, scratch) / (float)kv_rank + eps);   // has barriers: latent[] is complete
     const int slot = slots ? slots[t] : -1;
     const int page = slot >= 0 ? slot / page_size : -1;
-    if (page >= num_pages) {
-      if (threadIdx.x == 0) atomicOr(status, kStatusBadPage);
-    } else if (page >= 0) {
-      T* dst = cache + ((size_t)page * page_size + (slot - page * page_size)) * row;
-      for (int i = threadIdx.x; i < kv_rank; i += blockDim.x) dst[i] = from_float<T>(latent[i] * factor * kv_norm_weight[i]);
-      const float* part = latent + kv_rank;
-      for (int i = threadIdx.x; i < half; i += blockDim.x) {
-        int a, b;
-        pair_of(i, half, interleaved, &a, &b);
-        const float u = part[a], v = part[b], cs = cos_t[i], sn = sin_t[i];
-        dst[kv_rank + a] = from_float<T>(u * cs - v * sn);
-        dst[kv_rank + b] = from_float<T>(v * cs + u * sn);
-      }
-      for (int i = size + threadIdx.x; i < row; i += blockDim.x) dst[i] = from_float<T>(0.f);
+    if (page >= num_pages && threadIdx.x == 0) atomicOr(status, kStatusBadPage);
+    T* dst = page >= 0 && page < num_pages ? cache + ((size_t)page * page_size + (slot - page * page_size)) * row : nullptr;
+    // the same row in two parts for the prompts' products (of a token without a slot, zeros)
+    T* rows = rows_out ? rows_out + (size_t)t * kv_rank : nullptr;
+    T* rotated = rows_out ? part_out + (size_t)t * rot_dim : nullptr;
+    const T zero = from_float<T>(0.f);
+    for (int i = threadIdx.x; i < kv_rank; i += blockDim.x) {
+      const T v = from_float<T>(latent[i] * factor * kv_norm_weight[i]);
+      if (dst) dst[i] = v;
+      if (rows) rows[i] = dst ? v : zero;
     }
+    const float* part = latent + kv_rank;
+    for (int i = threadIdx.x; i < half; i += blockDim.x) {
+      int a, b;
+      pair_of(i, half, interleaved, &a, &b);
+      const float u = part[a], v = part[b], cs = cos_t[i], sn = sin_t[i];
+      const T x = from_float<T>(u * cs - v * sn), y = from_float<T>(v * cs + u * sn);
+      if (dst) {
+        dst[kv_rank + a] = x;
+        dst[kv_rank + b] = y;
+      }
+      if (rotated) {
+        rotated[a] = dst ? x : zero;
+        rotated[b] = dst ? y : zero;
+      }
+    }
+    if (dst)
+      for (int i = size + threadIdx.x; i < row; i += blockDim.x) dst[i] = zero;
     if (gridDim.y > 1) return;
   }
   const int head0 = gridDim.y > 1 ? ((int)blockIdx.y - 1) * heads_per_cta : 0;
@@ -237,14 +251,15 @@ latent_qkv_store_kernel(const TIn* __restrict__ in, int splits, size_t split_str
 using namespace einf;
 
 // in: [T, width] (or `splits` float32 partial sums of it), of which kv_rank + rot_dim + H * (dim + rot_dim) (+ H gate
-// logits, where gate [T, H] is given) elements are read; cache: [pages, 1, page_size, row]; q_plain: [T, H, dim] or null (the caller
+// logits, where gate [T, H] is given) elements are read; cache: [pages, 1, page_size, row]; rows_out [T, kv_rank] and part_out
+// [T, rot_dim], both or neither: the cache rows' two parts once more; q_plain: [T, H, dim] or null (the caller
 // reads the product's own rows); q_full: [T, H, row], of which this writes the elements from kv_rank on.
 extern "C" int einf_latent_qkv_store(const void* in, int in_dtype, int splits, long long split_stride, int dtype,
                                      int num_tokens, int width, int kv_rank, int rot_dim, int num_heads, int dim, int row,
                                      const float* kv_norm_weight, float eps, const int* positions, const float* inv_freq,
                                      float amplitude, int interleaved, const int* slots, void* q_plain, void* q_full,
-                                     float* gate, void* cache, int page_size, int num_pages, int* status,
-                                     cudaStream_t stream) {
+                                     float* gate, void* cache, int page_size, int num_pages, void* rows_out, void* part_out,
+                                     int* status, cudaStream_t stream) {
   if (num_tokens == 0) return 0;
   if (kv_rank <= 0 || rot_dim < 0 || (rot_dim & 1) || num_heads <= 0 || dim <= 0 || row < kv_rank + rot_dim)
     return (int)cudaErrorInvalidValue;
@@ -260,7 +275,7 @@ extern "C" int einf_latent_qkv_store(const void* in, int in_dtype, int splits, l
       return (int)launch_pdl(latent_qkv_store_kernel<TIn, T>, dim3(num_tokens, blocks), dim3(128), smem, stream,
                              (const TIn*)in, splits, (size_t)split_stride, width, kv_rank, rot_dim, num_heads, dim, row,
                              heads_per_cta, kv_norm_weight, eps, positions, inv_freq, amplitude, interleaved, slots,
-                             (T*)q_plain, (T*)q_full, gate, (T*)cache, page_size, num_pages, status);
+                             (T*)q_plain, (T*)q_full, gate, (T*)cache, page_size, num_pages, (T*)rows_out, (T*)part_out, status);
     })
   })
 }

@@ -1066,9 +1066,9 @@ HEAD_PROMPT_SHORT = 64
 
 def head_prompt_ways(lengths: Optional[Sequence[int]]) -> tuple[bool, bool]:
     """Whether portions of these lengths (None: unknown) hold any for the kernel of short and of long ones."""
-    if lengths is None:
-        return True, True
-    return any(n <= HEAD_PROMPT_SHORT for n in lengths), any(n > HEAD_PROMPT_SHORT for n in lengths)
+    if not lengths:
+        return lengths is None, lengths is None
+    return min(lengths) <= HEAD_PROMPT_SHORT, max(lengths) > HEAD_PROMPT_SHORT
 
 
 def head_prompt_attention(
@@ -1128,16 +1128,15 @@ def head_prompt_attention(
          c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
          c_int, c_float, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     )
+    arguments = (
+        q_plain.data_ptr(), q_plain.stride(0), q_plain.stride(1), q_rot.data_ptr(), q_rot.stride(0), q_rot.stride(1),
+        k_plain.data_ptr(), k_plain.stride(0), k_plain.stride(1), _dev(k_rot, "k_rot"), v.data_ptr(), v.stride(0),
+        v.stride(1), _opt(q_tiles, "q_tiles", torch.int32), q_tiles.shape[0], _opt(q_start, "q_start", torch.int32),
+        _dev(out, "out"), _opt(sink, "sink", torch.float32), _opt(gate, "gate", torch.float32), heads, dim, rot_dim, value_size,
+        int(window) if window else 0, float(scale), _sm_count(), tokens)
+    ends = (_opt(status, "status", torch.int32), _stream())
     for way, short_rows in ways:
-        _check(
-            fn(q_plain.data_ptr(), q_plain.stride(0), q_plain.stride(1), q_rot.data_ptr(), q_rot.stride(0), q_rot.stride(1),
-               k_plain.data_ptr(), k_plain.stride(0), k_plain.stride(1), _dev(k_rot, "k_rot"), v.data_ptr(), v.stride(0),
-               v.stride(1), _opt(q_tiles, "q_tiles", torch.int32), q_tiles.shape[0], _opt(q_start, "q_start", torch.int32),
-               _dev(out, "out"), _opt(sink, "sink", torch.float32), _opt(gate, "gate", torch.float32), heads, dim, rot_dim, value_size,
-               int(window) if window else 0, float(scale), _sm_count(), tokens, way, short_rows,
-               _opt(status, "status", torch.int32), _stream()),
-            "head_prompt_attention",
-        )
+        _check(fn(*arguments, way, short_rows, *ends), "head_prompt_attention")
 
 
 #: activations of :func:`activation` by name
@@ -1481,6 +1480,8 @@ def latent_qkv_store(
     cache: Optional[torch.Tensor],
     status: torch.Tensor,
     dim: int,
+    rows: Optional[torch.Tensor] = None,
+    part: Optional[torch.Tensor] = None,
 ) -> None:
     """The two functions above in one launch, for queries without a latent of their own.  A row of
     ``product`` (or of its float32 split-K partial sums) is ``[kv latent kv_rank | key part rot_dim | heads *
@@ -1488,7 +1489,8 @@ def latent_qkv_store(
     head, whose sigmoid goes there (further elements are not looked at).  The cache row ``[normed latent | rotated key part | zeros]`` goes into
     the token's page slot (``cache [pages, 1, page_size, row]``; ``slots`` None writes none), the rotated query
     parts and zeros behind them into ``q_full [tokens, heads, row]`` from ``kv_rank`` on, the plain parts into
-    ``q_plain [tokens, heads, dim]`` (None: the caller reads them out of ``product`` itself)."""
+    ``q_plain [tokens, heads, dim]`` (None: the caller reads them out of ``product`` itself).  With slots, ``rows [tokens,
+    kv_rank]`` and ``part [tokens, rot_dim]`` get the cache rows' two parts as :func:`latent_rows` gives them."""
     tokens, heads, row = q_full.shape
     used = kv_rank + rot_dim + heads * (dim + rot_dim) + (heads if gate is not None else 0)
     width = product.shape[-1]
@@ -1512,15 +1514,19 @@ def latent_qkv_store(
     fn = _fn(
         "einf_latent_qkv_store",
         [c_void_p, c_int, c_int, c_longlong, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_float, c_void_p,
-         c_void_p, c_float, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p],
+         c_void_p, c_float, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,
+         c_void_p],
     )
+    if rows is not None and (slots is None or part is None or rows.shape != (tokens, kv_rank) or part.shape != (tokens, rot_dim)):
+        raise ValueError(f"rows {(tokens, kv_rank)} and part {(tokens, rot_dim)} come with slots")
     _check(
         fn(_dev(product, "product"), _code(product), splits, stride, _code(q_full), tokens, width, kv_rank, rot_dim, heads,
            int(dim), row, _opt(kv_norm_weight, "kv_norm_weight", torch.float32), float(eps),
            _opt(positions, "positions", torch.int32), _opt(inv_freq, "inv_freq", torch.float32), float(amplitude),
            1 if interleaved else 0, _opt(slots, "slots", torch.int32) if cache_ptr else 0,
            0 if q_plain is None else _dev(q_plain, "q_plain"), _dev(q_full, "q_full"),
-           _opt(gate, "gate", torch.float32), cache_ptr, page_size, num_pages, _dev(status, "status"), _stream()),
+           _opt(gate, "gate", torch.float32), cache_ptr, page_size, num_pages, _opt(rows, "rows", q_full.dtype),
+           0 if rows is None else _opt(part, "part", q_full.dtype), _dev(status, "status"), _stream()),
         "latent_qkv_store",
     )
 

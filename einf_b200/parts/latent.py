@@ -186,13 +186,14 @@ class LatentAttention(Mixer):
         """Lengths of the portions of several tokens that start their prompts."""
         return [n for n, start in zip(ctx.q_lens, ctx.start_positions) if n > 1 and start == 0]
 
-    def _prompts(self, q_plain, q_full, gate, ctx: StepContext, cache: CacheView, mixed: torch.Tensor) -> None:
+    def _prompts(self, q_plain, q_full, gate, rows, part, ctx: StepContext, cache: CacheView, mixed: torch.Tensor) -> None:
         """Prompts that start in the step, head by head: its rows through both up-projections, then attention into those
         portions' rows of ``mixed [T, H, value]``."""
         tokens, heads, device = q_full.shape[0], self.num_heads, q_full.device
-        rows = torch.empty((tokens, self.kv_rank), dtype=q_full.dtype, device=device)
-        part = torch.empty((tokens, self.rot_dim), dtype=q_full.dtype, device=device)
-        ops.latent_rows(cache.k, ctx.slots[cache.group], rows, part)
+        if rows is None:
+            rows = torch.empty((tokens, self.kv_rank), dtype=q_full.dtype, device=device)
+            part = torch.empty((tokens, self.rot_dim), dtype=q_full.dtype, device=device)
+            ops.latent_rows(cache.k, ctx.slots[cache.group], rows, part)
         kv = torch.empty((tokens, self.kv_up.shape[0]), dtype=q_full.dtype, device=device)
         ops.linear(rows, self.kv_up, None, kv, ctx.status)
         keys = heads * self.dim
@@ -214,9 +215,10 @@ class LatentAttention(Mixer):
         # the values are the first kv_rank elements of the rows: no value cache of its own
         return PagedKVNeed(1, self.row, self.window, 0)
 
-    def _queries_and_store(self, x, ctx: StepContext, cache: CacheView):
+    def _queries_and_store(self, x, ctx: StepContext, cache: CacheView, by_heads: bool):
         """Project, write the step's cache rows, and return the queries' plain parts ``[T, H, dim]``, the full
-        queries ``[T, H, row]`` with the rotated part in place, and the heads' gates."""
+        queries ``[T, H, row]`` with the rotated part in place, the heads' gates, and, ``by_heads``, the two parts of
+        the step's cache rows where the storing launch has left them (else None)."""
         tokens, heads, dim = x.shape[0], self.num_heads, self.dim
         dtype, device = self.runtime.dtype, x.device
         interleaved = getattr(self.position, "interleaved", False)
@@ -233,11 +235,15 @@ class LatentAttention(Mixer):
                 q_plain, copy = down[:, first:first + heads * per_head].unflatten(1, (heads, per_head))[..., :dim], None
             else:
                 q_plain = copy = torch.empty((tokens, heads, dim), dtype=dtype, device=device)
+            rows = part = None
+            if by_heads and writes:
+                rows, part = q_full.new_empty((tokens, self.kv_rank)), q_full.new_empty((tokens, self.rot_dim))
             ops.latent_qkv_store(
                 down, self.kv_rank, self.rot_dim, self.kv_norm, self.eps, ctx.positions, self.position.inv_freq,
                 interleaved, amplitude, slots, copy, q_full, gate, pages, ctx.status, dim,
+                **({} if rows is None else {"rows": rows, "part": part}),
             )
-            return q_plain, q_full, gate
+            return q_plain, q_full, gate, rows, part
         q_latent = torch.empty((tokens, self.q_rank), dtype=dtype, device=device)
         ops.latent_down_store(
             down, self.q_rank, self.kv_rank, self.rot_dim, self.q_norm, self.kv_norm, self.eps, ctx.positions,
@@ -246,19 +252,19 @@ class LatentAttention(Mixer):
         q = ops.project(q_latent, self.q_up, ctx.status)
         q_plain = torch.empty((tokens, heads, dim), dtype=dtype, device=device)
         ops.latent_q_store(q, ctx.positions, self.position.inv_freq, interleaved, q_plain, q_full, amplitude)
-        return q_plain, q_full, None
+        return q_plain, q_full, None, None, None
 
     def forward(self, x: torch.Tensor, ctx: StepContext, cache: CacheView) -> torch.Tensor:
         tokens = x.shape[0]
         dtype, device = self.runtime.dtype, x.device
         heads = self.num_heads
-        q_plain, q_full, gate = self._queries_and_store(x, ctx, cache)
         by_heads, on_rows = self._ways(ctx)
+        q_plain, q_full, gate, rows, part = self._queries_and_store(x, ctx, cache, by_heads)
         mixed = torch.empty((tokens, heads, self.value_size), dtype=dtype, device=device)
         if on_rows or ctx.single_tokens.shape[0]:
             self._on_rows(q_plain, q_full, gate, ctx, cache, mixed, by_heads, on_rows)
         if by_heads:      # after the others: those leave something in every row of `mixed`
-            self._prompts(q_plain, q_full, gate, ctx, cache, mixed)
+            self._prompts(q_plain, q_full, gate, rows, part, ctx, cache, mixed)
         return ops.project(mixed.view(tokens, -1), self.out_weight, ctx.status)
 
     def _on_rows(self, q_plain, q_full, gate, ctx: StepContext, cache: CacheView, mixed: torch.Tensor, by_heads: bool,

@@ -123,6 +123,14 @@ def test_latent_store_without_a_query_latent(dev, dtype, heads, dim, rot, rank, 
             close(got, want, got.dtype if got.dtype == torch.bfloat16 else torch.float32)
         assert bool((results[0][1 if copied else 0][:, :, :rank] == 7.0).all())      # the absorbed part is someone else's
     slots[1] = page * pages + 3                             # beyond the pool: reported, not written
+    rows, part = torch.empty((tokens, rank), dtype=dtype, device=dev), torch.empty((tokens, rot), dtype=dtype, device=dev)
+    again = torch.zeros_like(cache)
+    ops.latent_qkv_store(product, rank, rot, norm, 1e-5, positions, inv_freq, interleaved, 1.0, slots, None, torch.empty_like(full),
+                         gate, again, st, dim, rows=rows, part=part)
+    want = [torch.empty_like(rows), torch.empty_like(part)]      # the cache rows' two parts, bit for bit
+    if dtype == torch.bfloat16 and rank % 8 == 0 and rot % 8 == 0 and again.shape[3] % 8 == 0:
+        ops.latent_rows(again, slots, *want)
+        assert torch.equal(rows, want[0]) and torch.equal(part, want[1])
     ops.latent_qkv_store(product, rank, rot, norm, 1e-5, positions, inv_freq, interleaved, 1.0, slots, None, full, gate,
                          cache, st, dim)
     assert int(st) == ops.STATUS_BAD_PAGE
