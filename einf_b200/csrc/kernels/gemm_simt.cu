@@ -1,7 +1,7 @@
 // out[M, N] = A[M, K] . W[N, K]^T (+ bias[N]) with 32-bit FMA accumulation on the
-// CUDA cores: the matrix product of the true 32-bit path (no tensor-core mode
-// rounds its inputs), and the product for operands of mixed type (bfloat16
-// activations against a matrix the checkpoint stores in 32-bit).  Any M, N, K.
+// CUDA cores: the product for operands of mixed type (bfloat16 activations against a
+// matrix the checkpoint stores in 32-bit) and for 32-bit rows that are not whole
+// aligned groups of four (gemm_parts.cu has the others).  Any M, N, K.
 // Sums over K are blocked: every 256 terms the running sum is folded into a second
 // accumulator, so that the rounding of a long sum (K of 18,944 in a 7B-size down
 // projection) grows like the root of the block plus the root of the number of blocks and
