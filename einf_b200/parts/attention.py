@@ -313,6 +313,7 @@ class PagedAttention(Mixer):
         """Whether the layer's products run in the kernels for a few tokens."""
         return bool(
             self.fast and self.out_bias is None and self.qkv_weight.dtype == self.out_weight.dtype == torch.bfloat16
+            and self.qkv_weight.data_ptr() % 16 == 0 and self.out_weight.data_ptr() % 16 == 0
             and self.position.kind in ("rope", "none") and self.position.inv_freq.shape[0] in (0, self.head_size // 2)
             and not getattr(self.position, "interleaved", False)
             and ops.few_tokens_fit(self.hidden_size, True) and ops.few_tokens_fit(self.num_heads * self.head_size, False)

@@ -54,7 +54,8 @@ class PreNormBlock(Block):
         for role, category in self.part_categories().items():
             setattr(self, role, build_part(category, layer_spec.parts[role], tensors, runtime))
         self._few = type(self) is PreNormBlock and all(
-            type(norm) is RMSNorm for norm in (self.mixer_norm, self.feed_forward_norm)) and all(
+            type(norm) is RMSNorm and norm.weight.data_ptr() % 16 == 0
+            for norm in (self.mixer_norm, self.feed_forward_norm)) and all(
             part.takes_few() if hasattr(part, "takes_few") else False for part in (self.mixer, self.feed_forward))
 
     @staticmethod
@@ -65,8 +66,9 @@ class PreNormBlock(Block):
         return norm.forward(pending, residual)
 
     def forward(self, residual, pending, ctx, cache):
-        if self._few and residual.shape[0] <= ops.FEW_TOKENS and (
-                pending is None or (pending.dtype == torch.float32 and pending.shape == residual.shape)):
+        if self._few and residual.shape[0] <= ops.FEW_TOKENS and residual.data_ptr() % 16 == 0 and (
+                pending is None or (pending.dtype == torch.float32 and pending.shape == residual.shape
+                                    and pending.data_ptr() % 16 == 0)):
             self.mixer.forward_few(residual, pending, self.mixer_norm, ctx, cache)
             return self.feed_forward.forward_few(residual, self.feed_forward_norm, ctx)
         x = self._normalise(self.mixer_norm, pending, residual, ctx)
