@@ -473,6 +473,7 @@ head_prompt_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   }
   __syncthreads();
   float factor = 0.f;
+  bool seen = false;
   float* half = reinterpret_cast<float*>(generic + L::kK);        // the second group's share: every load and product is over
   constexpr int kPitch = kValue + 1;
   static_assert(128 * kPitch * 4 <= (2 * KS + 2 * VS) * kHeadSlice, "the share fits the keys' and values' place");
@@ -481,7 +482,9 @@ head_prompt_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     const float m0 = shared[r], m1 = shared[128 + r], top = fmaxf(m0, m1), at = top == -INFINITY ? 0.f : top;
     float total = shared[256 + r] * exp2f(m0 - at) + shared[384 + r] * exp2f(m1 - at);
     if (a.sink) total += exp2f(a.sink[h] * 1.4426950408889634f - top);
-    factor = total > 0.f && m != -INFINITY ? exp2f(m - at) / total : 0.f;
+    // a sum that is not a number is the row's result: only what has seen nothing, or nothing of any weight, is zero
+    seen = m != -INFINITY || l != 0.f;
+    factor = seen && total != 0.f ? exp2f(m - at) / total : 0.f;
     if (a.gate && r < rows) factor *= a.gate[(long long)(tile.y + r) * a.heads + h];
     if (group == 1 && turns > 0) {
 #pragma unroll
@@ -490,7 +493,7 @@ head_prompt_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         tmem_ld32(mixed + 32 * c, o);
         tmem_ld_wait32(o);
 #pragma unroll
-        for (int e = 0; e < 32; ++e) half[r * kPitch + 32 * c + e] = factor != 0.f ? o[e] * factor : 0.f;
+        for (int e = 0; e < 32; ++e) half[r * kPitch + 32 * c + e] = seen ? o[e] * factor : 0.f;
       }
     }
   }
@@ -505,7 +508,7 @@ head_prompt_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       uint32_t pairs[16];
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
-        float x = factor != 0.f ? o[2 * e] * factor : 0.f, y = factor != 0.f ? o[2 * e + 1] * factor : 0.f;
+        float x = seen ? o[2 * e] * factor : 0.f, y = seen ? o[2 * e + 1] * factor : 0.f;
         if (n > 1) {
           x += half[r * kPitch + 32 * c + 2 * e];
           y += half[r * kPitch + 32 * c + 2 * e + 1];

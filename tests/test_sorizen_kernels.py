@@ -415,6 +415,47 @@ def test_prompts_head_by_head_in_tensor_memory(dev, heads, dim, value, window, l
     assert int(status) == 0
 
 
+def _prompt_in_64_bits(q_plain, q_rot, k_plain, k_rot, v, scale, window):
+    """Which keys a row sees, and the rows' results with values that are not finite left out."""
+    n = q_plain.shape[0]
+    scores = torch.einsum("ihd,jhd->hij", q_plain.double(), k_plain.double())
+    scores = (scores + torch.einsum("ihr,jr->hij", q_rot.double(), k_rot.double())) * scale
+    i, j = torch.arange(n, device=v.device)[:, None], torch.arange(n, device=v.device)[None, :]
+    seen = (j <= i) & (j > i - (window or n))
+    weights = torch.softmax(scores.masked_fill(~seen, float("-inf")), dim=2)
+    return seen, torch.einsum("hij,jhv->ihv", weights, torch.nan_to_num(v.double(), 0.0, 0.0, 0.0))
+
+
+def _prompt_tiles(n, dev):
+    return torch.tensor([(0, at, min(128, n - at), at) for at in range(0, n, 128)], dtype=torch.int32, device=dev)
+
+
+@pytest.mark.parametrize("tensor_memory", [True, False])
+@pytest.mark.parametrize("dim, value, window", [(64, 64, None), (128, 128, 100)])
+def test_scores_that_are_not_finite_are_not_hidden(dev, tensor_memory, dim, value, window):
+    """A row that sees a score which is NaN or plus infinity is NaN, and no other row is: NaN in a key, an infinite key
+    (plus or minus infinite scores, by the query's sign), NaN in a query; in the first, the last and a middle tile."""
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(dim)
+    heads, rot, n, scale = 2, 64, 300, (dim + 64) ** -0.5
+    draw = lambda *shape: torch.randn(shape, generator=gen).to(torch.bfloat16).to(dev)  # noqa: E731
+    q_plain, q_rot, k_plain, k_rot, v = draw(n, heads, dim), draw(n, heads, rot), draw(n, heads, dim), draw(n, rot), draw(n, heads, value)
+    tiles, status = _prompt_tiles(n, dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    for where in (5, 130, 290):
+        q, k = q_plain.clone(), k_plain.clone()
+        k[where, 0, 3] = float("nan")
+        k[where - 3, 1, 7] = float("inf")
+        q[where - 2, 1, 0] = float("nan")
+        out = torch.zeros((n, heads, value), dtype=torch.bfloat16, device=dev)
+        ops.head_prompt_attention(q, q_rot, k, k_rot, v, tiles, out, scale, window, status=status, tensor_memory=tensor_memory)
+        want = _prompt_in_64_bits(q, q_rot, k, k_rot, v, scale, window)[1]
+        assert torch.equal(out.isnan(), want.isnan()) and 0 < int(want.isnan().sum()) < want.numel()
+        fine = ~want.isnan()
+        torch.testing.assert_close(out[fine].double(), want[fine], rtol=2e-2, atol=2e-2)
+    assert int(status) == 0
+
+
 @pytest.mark.parametrize("heads, dim, rot, value, rank, q_rank, page", [
     (3, 128, 64, 128, 512, None, 16), (4, 40, 24, 72, 32, 64, 16), (2, 64, 16, 64, 192, 40, 8), (2, 64, 8, 40, 176, 40, 5)])
 @pytest.mark.parametrize("window", [None, 60])
