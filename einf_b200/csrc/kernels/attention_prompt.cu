@@ -604,7 +604,7 @@ extern "C" int einf_latent_rows(const void* cache, const int* slots, long long n
                          (__nv_bfloat16*)rest, second, tokens);
 }
 
-// `tensor_memory`: by the kernel on tcgen05 (sizes multiples of 64, rot_dim above 0), `short_rows`: of it and the other kernel,
+// `tensor_memory`: by the kernel on tcgen05 (sizes multiples of 64, rot_dim and scale above 0), `short_rows`: of it and the other kernel,
 // the other one has the portions of up to that many tokens and this one the longer ones (0: the kernel has all).
 // Portions that start at position 0 in this step, their tokens packed one after the other; with `q_start`, the requests' first
 // tokens, `tiles` of other portions are left out (without it there must be none).  Sizes and
@@ -637,7 +637,7 @@ extern "C" int einf_head_prompt_attention(const void* q_plain, long long q_plain
   a.status = status;
   a.short_rows = short_rows;
   if (tensor_memory) {
-    if (dim % 64 || rot_dim % 64 || rot_dim == 0 || value_size % 64 || tokens <= 0) return (int)cudaErrorInvalidValue;
+    if (dim % 64 || rot_dim % 64 || rot_dim == 0 || value_size % 64 || tokens <= 0 || !(scale > 0.f)) return (int)cudaErrorInvalidValue;
     if (dim + rot_dim == 128)
       return value_size == 64 ? launch_head_tcgen05<2, 1>(a, tokens, num_tiles, stream) : launch_head_tcgen05<2, 2>(a, tokens, num_tiles, stream);
     return value_size == 64 ? launch_head_tcgen05<3, 1>(a, tokens, num_tiles, stream) : launch_head_tcgen05<3, 2>(a, tokens, num_tiles, stream);

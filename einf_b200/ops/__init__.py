@@ -1096,7 +1096,7 @@ def head_prompt_attention(
     ``[requests + 1]``) other requests may be among them and are left out.  ``window``, ``sink`` and ``gate``: see
     :func:`paged_attention_generic`.
 
-    Heads in whole 128-byte lines run on tcgen05 where a portion has more than :data:`HEAD_PROMPT_SHORT` tokens, each by
+    Heads in whole 128-byte lines run on tcgen05 (with a positive ``scale``: a row's largest score is found before it) where a portion has more than :data:`HEAD_PROMPT_SHORT` tokens, each by
     its own length; ``lengths``: those portions' lengths where the host knows them, which spares a launch with
     nothing to do.  ``tensor_memory`` (True or False) sends all portions to one kernel."""
     tokens, heads, dim = q_plain.shape
@@ -1117,7 +1117,7 @@ def head_prompt_attention(
     _check_gate(gate, tokens, heads)
     if tensor_memory is not None:
         ways = [(int(tensor_memory), 0)]
-    elif dim % 64 or rot_dim != 64 or value_size % 64:
+    elif dim % 64 or rot_dim != 64 or value_size % 64 or not 0.0 < scale < float("inf"):
         ways = [(0, 0)]
     else:
         short, long = head_prompt_ways(lengths)

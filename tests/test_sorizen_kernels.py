@@ -456,6 +456,26 @@ def test_scores_that_are_not_finite_are_not_hidden(dev, tensor_memory, dim, valu
     assert int(status) == 0
 
 
+@pytest.mark.parametrize("scale, heads_first", [(0.0, False), (-0.1, False), (0.1, True)])
+def test_prompts_that_the_tensor_memory_kernel_leaves_to_the_other(dev, scale, heads_first):
+    """Scores that a factor turns round or levels, and heads farther apart than tokens."""
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(3)
+    heads, dim, rot, value, n = 2, 64, 64, 64, 200
+
+    def draw(*shape):
+        t = torch.randn(shape, generator=gen).to(torch.bfloat16).to(dev)
+        return t.transpose(0, 1).contiguous().transpose(0, 1) if heads_first and len(shape) == 3 else t
+
+    q_plain, q_rot, k_plain, k_rot, v = draw(n, heads, dim), draw(n, heads, rot), draw(n, heads, dim), draw(n, rot), draw(n, heads, value)
+    out, status = torch.zeros((n, heads, value), dtype=torch.bfloat16, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    ops.head_prompt_attention(q_plain, q_rot, k_plain, k_rot, v, _prompt_tiles(n, dev), out, scale, None, status=status)
+    want = _prompt_in_64_bits(q_plain, q_rot, k_plain, k_rot, v, scale, None)[1]
+    torch.testing.assert_close(out.double(), want, rtol=2e-2, atol=2e-2)
+    assert int(status) == 0
+
+
 @pytest.mark.parametrize("heads, dim, rot, value, rank, q_rank, page", [
     (3, 128, 64, 128, 512, None, 16), (4, 40, 24, 72, 32, 64, 16), (2, 64, 16, 64, 192, 40, 8), (2, 64, 8, 40, 176, 40, 5)])
 @pytest.mark.parametrize("window", [None, 60])
