@@ -254,10 +254,11 @@ head_prompt_attention_kernel(const __grid_constant__ HeadPromptArgs a) {
 // another issues the products: scores into the group's 128 columns of tensor memory; the group's threads (a row each)
 // take them out, and put the weights, as bfloat16 pairs, into the same columns, where the second product reads them as its
 // first operand.  While one group is at its softmax the other's products run.  A row's reference moves only when a tile's
-// maximum is more than 2^8 above it, so that the accumulator is rarely taken out and multiplied.  Values behind the last key
-// of the request are cleared in shared memory: the tile's other rows are another request's, and zero times infinity is not zero.
-// Measured (B200, us, the kernel above / this one): 12 heads, keys of 128 + 64, values of 128: 2,048 tokens 124 / 33 (490
-// TFLOP/s), 4,096 283 / 92, 300 18.4 / 11.8, 128 10.1 / 8.1; 14 heads of 64 + 64, values of 64, 2,048 tokens 80 / 32.  Portions of up to
+// maximum is more than 2^8 above it, so that the accumulator is rarely taken out and multiplied.  In a tile of which some row
+// does not see every key the warp that brings the tiles clears the values behind the request's last key (another request's) and
+// those that are not finite, since zero times infinity is not zero; the rows that see the latter get them added at the end.
+// Measured (B200, us, the kernel above / this one): 12 heads, keys of 128 + 64, values of 128: 2,048 tokens 124 / 34 (480
+// TFLOP/s), 4,096 283 / 93, 300 18.4 / 10.0, 128 10.1 / 7.8; 14 heads of 64 + 64, values of 64, 2,048 tokens 80 / 33.  Portions of up to
 // 64 tokens fill half a tile of this one at most and stay above: 40 of 30 tokens 14.8 / 31.7, one of 20 6.4 / 8.2.  What bounds it
 // now: a tile's softmax, 128 exponentials a thread between two passes through tensor memory.
 constexpr int kHeadThreads = 320, kHeadSlice = 128 * 64 * 2;
@@ -265,7 +266,7 @@ constexpr int kHeadThreads = 320, kHeadSlice = 128 * 64 * 2;
 template <int KS, int VS>
 struct HeadLayout {
   static constexpr int kQ = 0, kK = KS * kHeadSlice, kV = kK + 2 * KS * kHeadSlice, kBars = kV + 2 * VS * kHeadSlice;
-  static constexpr int kShared = kBars + 8 * 16 + 16, kSums = kShared, kBytes = kSums + 4 * 128 * 4 + 1024;
+  static constexpr int kShared = kBars + 8 * 17 + 24, kSums = kShared, kBytes = kSums + 4 * 128 * 4 + 1024;
 };
 
 __device__ __forceinline__ bool head_wait(uint32_t bar, uint32_t parity, int* status) {
@@ -283,6 +284,48 @@ __device__ __forceinline__ bool head_wait(uint32_t bar, uint32_t parity, int* st
   }
   if (status) atomicOr(status, kStatusWaitExpired);
   return false;
+}
+
+// By a warp: takes what is not finite out of the first `real` rows of a tile of values, and everything out of the rows behind
+// them; true if there was something in the former.  Looked at first, eight loads under way (a store behind each: 3.4 us).
+template <int VS>
+__device__ __forceinline__ bool clear_tile(unsigned char* tile, int real, int lane) {
+  uint4* pieces = reinterpret_cast<uint4*>(tile) + lane;
+  uint32_t any = 0;
+#pragma unroll 8
+  for (int e = 0; e < 32 * VS; ++e) {
+    const uint4 v = pieces[32 * e];
+    any |= not_finite(v.x) | not_finite(v.y) | not_finite(v.z) | not_finite(v.w);
+  }
+  bool found = false;
+  if (__any_sync(0xffffffffu, any != 0u)) {
+#pragma unroll 1
+    for (int e = 0; e < 32 * VS; ++e) {
+      const int row = 4 * (e & 31) + (lane >> 3);
+      uint4 v = pieces[32 * e];
+      const uint4 out = make_uint4(not_finite(v.x), not_finite(v.y), not_finite(v.z), not_finite(v.w));
+      if (row >= real || !(out.x | out.y | out.z | out.w)) continue;
+      v = make_uint4(v.x & ~((out.x >> 15) * 0xffffu), v.y & ~((out.y >> 15) * 0xffffu), v.z & ~((out.z >> 15) * 0xffffu),
+                     v.w & ~((out.w >> 15) * 0xffffu));
+      pieces[32 * e] = v;
+      found = true;
+    }
+  }
+  for (int c = 0; c < VS; ++c)
+    for (int e = real * 8 + lane; e < 128 * 8; e += 32) reinterpret_cast<uint4*>(tile + c * kHeadSlice)[e] = make_uint4(0u, 0u, 0u, 0u);
+  return found;
+}
+
+// What clear_tile took out of the keys from `first` to before `last`, added to a row of the output that this thread has written
+// (seldom; a call, since the loops in the kernel's own text cost the others 1.7 us a CTA).
+__device__ __noinline__ void add_not_finite(const HeadPromptArgs& a, __nv_bfloat16* out, int key_token, int first, int last, int h, float weight) {
+  for (int key = first; key < last; ++key) {
+    const __nv_bfloat16* v = a.v + (key_token + key) * a.v_token + h * a.v_head;
+    for (int e = 0; e < a.value_size; ++e) {
+      const float x = __bfloat162float(v[e]);
+      if (!(fabsf(x) < INFINITY)) out[e] = __float2bfloat16_rn(__bfloat162float(out[e]) + weight * x);
+    }
+  }
 }
 
 template <int KS, int VS>
@@ -306,11 +349,13 @@ head_prompt_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   unsigned char* generic = head_smem + (base - raw);
   const uint32_t bars = base + L::kBars;
   const uint32_t q_full = bars, k_full = bars + 8, k_empty = bars + 24, v_full = bars + 40, v_empty = bars + 56, s_full = bars + 72,
-                 p_full = bars + 88, o_done = bars + 104, holder = bars + 128;
+                 p_full = bars + 88, o_done = bars + 104, v_clear = bars + 120, holder = bars + 136;
+  volatile int* taken_out = reinterpret_cast<volatile int*>(generic + L::kBars + 140);   // values that are not finite
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int pos0 = tile.w, last_pos = pos0 + rows - 1;
   const int first_tile = a.window > 0 ? max(0, pos0 - a.window + 1) / 128 : 0, n = last_pos / 128 + 1 - first_tile;
   if (tid == 0) {
+    *taken_out = 0;
     bar_init(q_full, 1);
     for (int s = 0; s < 2; ++s) {
       bar_init(k_full + 8 * s, 1);
@@ -320,6 +365,7 @@ head_prompt_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       bar_init(s_full + 8 * s, 1);
       bar_init(p_full + 8 * s, 128);
       bar_init(o_done + 8 * s, 1);
+      bar_init(v_clear + 8 * s, 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -330,35 +376,54 @@ head_prompt_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(generic + L::kBars + 128);
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(generic + L::kBars + 136);
   pdl_launch_dependents();
   pdl_wait();
   const int dim_lines = a.dim / 64;
   bool ok = true;
+  // some row does not see some key of a tile (the last one's keys may also be another request's)
+  auto hides = [&](int i) {
+    const int j0 = (first_tile + i) * 128;
+    return j0 + 127 > pos0 || (a.window > 0 && j0 <= last_pos - a.window);
+  };
   if (warp == 8) {
+    auto bring = [&](int i) {
+      const int s = i & 1, token = key_token + (first_tile + i) * 128;
+      const uint32_t again = ((i >> 1) & 1) ^ 1;
+      if (i >= 2) ok = ok && head_wait(k_empty + 8 * s, again, a.status);
+      if (!ok) return;
+      bar_expect_tx(k_full + 8 * s, KS * kHeadSlice);
+      for (int c = 0; c < KS; ++c) {
+        const uint32_t to = base + L::kK + (s * KS + c) * kHeadSlice;
+        if (c < dim_lines) tma_2d(to, &map_k, (int)(h * a.k_head) + 64 * c, token, k_full + 8 * s);
+        else tma_2d(to, &map_kr, 64 * (c - dim_lines), token, k_full + 8 * s);
+      }
+      if (i >= 2) ok = ok && head_wait(v_empty + 8 * s, again, a.status);
+      if (!ok) return;
+      bar_expect_tx(v_full + 8 * s, VS * kHeadSlice);
+      for (int c = 0; c < VS; ++c)
+        tma_2d(base + L::kV + (s * VS + c) * kHeadSlice, &map_v, (int)(h * a.v_head) + 64 * c, token, v_full + 8 * s);
+    };
     if (lane == 0) {
       bar_expect_tx(q_full, KS * kHeadSlice);
       for (int c = 0; c < KS; ++c) {
         if (c < dim_lines) tma_2d(base + L::kQ + c * kHeadSlice, &map_q, (int)(h * a.q_plain_head) + 64 * c, tile.y, q_full);
         else tma_2d(base + L::kQ + c * kHeadSlice, &map_qr, (int)(h * a.q_rot_head) + 64 * (c - dim_lines), tile.y, q_full);
       }
-      for (int i = 0; i < n && ok; ++i) {
-        const int s = i & 1, token = key_token + (first_tile + i) * 128;
-        const uint32_t again = ((i >> 1) & 1) ^ 1;
-        if (i >= 2) ok = head_wait(k_empty + 8 * s, again, a.status);
-        if (!ok) break;
-        bar_expect_tx(k_full + 8 * s, KS * kHeadSlice);
-        for (int c = 0; c < KS; ++c) {
-          const uint32_t to = base + L::kK + (s * KS + c) * kHeadSlice;
-          if (c < dim_lines) tma_2d(to, &map_k, (int)(h * a.k_head) + 64 * c, token, k_full + 8 * s);
-          else tma_2d(to, &map_kr, 64 * (c - dim_lines), token, k_full + 8 * s);
-        }
-        if (i >= 2) ok = head_wait(v_empty + 8 * s, again, a.status);
-        if (!ok) break;
-        bar_expect_tx(v_full + 8 * s, VS * kHeadSlice);
-        for (int c = 0; c < VS; ++c)
-          tma_2d(base + L::kV + (s * VS + c) * kHeadSlice, &map_v, (int)(h * a.v_head) + 64 * c, token, v_full + 8 * s);
-      }
+      bring(0);
+    }
+    for (int i = 0; i < n; ++i) {
+      if (i + 1 < n && lane == 0) bring(i + 1);            // before the look at tile i, which its stages do not wait for
+      ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+      if (!ok) break;
+      if (!hides(i)) continue;
+      const int s = i & 1;
+      ok = __all_sync(0xffffffffu, head_wait(v_full + 8 * s, (i >> 1) & 1, a.status)) != 0;
+      if (!ok) break;
+      if (clear_tile<VS>(generic + L::kV + s * VS * kHeadSlice, last_pos + 1 - (first_tile + i) * 128, lane)) *taken_out = 1;
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) bar_arrive(v_clear + 8 * s);
     }
   } else if (warp == 9) {
     constexpr uint32_t kScores = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
@@ -380,18 +445,12 @@ head_prompt_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       mma_commit(s_full + 8 * s);
     };
     if (n > 0) scores(0);
+    uint32_t cleared = 0;                                  // parity of either stage's tiles that hide something, so far
     for (int i = 0; i < n; ++i) {
       const int s = i & 1, turn = i >> 1;
       if (i + 1 < n) scores(i + 1);
-      ok = ok && head_wait(v_full + 8 * s, turn & 1, a.status);
-      const int real = last_pos + 1 - (first_tile + i) * 128;
-      if (real < 128) {
-        for (int e = lane; e < (128 - real) * 8 * VS; e += 32) {
-          const int c = e / ((128 - real) * 8), in = e - c * ((128 - real) * 8);
-          asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(base + L::kV + (s * VS + c) * kHeadSlice + (real + (in >> 3)) * 128 + (in & 7) * 16), "r"(0u) : "memory");
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      }
+      ok = ok && (hides(i) ? head_wait(v_clear + 8 * s, cleared >> s & 1, a.status) : head_wait(v_full + 8 * s, turn & 1, a.status));
+      if (hides(i)) cleared ^= 1u << s;
       __syncwarp();
       ok = ok && head_wait(p_full + 8 * s, turn & 1, a.status);
       if (ok && lane == 0) {
@@ -521,6 +580,13 @@ head_prompt_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
           *reinterpret_cast<uint4*>(out + 32 * c + 8 * e) = make_uint4(pairs[4 * e], pairs[4 * e + 1], pairs[4 * e + 2], pairs[4 * e + 3]);
       }
     }
+    if (*taken_out && r < rows)
+      for (int i = 0; i < n; ++i) {
+        const int j0 = (first_tile + i) * 128;
+        if (hides(i))
+          add_not_finite(a, out, key_token, a.window > 0 ? max(j0, pos0 + r - a.window + 1) : j0, min(j0 + 128, pos0 + r + 1), h,
+                         a.gate ? a.gate[(long long)(tile.y + r) * a.heads + h] : 1.f);
+      }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

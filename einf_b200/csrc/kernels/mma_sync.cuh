@@ -95,6 +95,9 @@ __device__ __forceinline__ uint32_t pack_pair(float low, float high) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// The halves of a pair of bfloat16 that are infinite or NaN, as their highest bits.
+__device__ __forceinline__ uint32_t not_finite(uint32_t pair) { return ((pair & 0x7f807f80u) + 0x00800080u) & 0x80008000u; }
+
 // Byte of a 16-byte piece of a row whose rows are 128-byte lines: exchanged by the row's last three bits, so that the eight
 // rows of an ldmatrix meet no bank twice.
 __device__ __forceinline__ uint32_t swizzled(int row, int piece, int pitch) {

@@ -94,9 +94,6 @@ __device__ __forceinline__ int find_portion(const ChunkArgs& a, int number, int*
 // kernel's instructions where the inputs pass a SiLU; y and state stay closer to 64 bits than the token-by-token kernel's).
 __device__ __forceinline__ float silu_quick(float z) { return __fdividef(z, 1.f + expf(-z)); }
 
-// The halves of a pair of bfloat16 that are infinite or NaN, as their highest bits.
-__device__ __forceinline__ uint32_t not_finite(uint32_t pair) { return ((pair & 0x7f807f80u) + 0x00800080u) & 0x80008000u; }
-
 // Shared memory of a CTA, in bytes from its start.  ROWS: rows of the state (filled up); NT: tiles of eight columns;
 // with kAct the inputs are 32-bit values in three parts.  Rows of q and k (and of v and the state at 64 columns) are a
 // power of two long, and their 16-byte pieces are exchanged by the row's last three bits; other rows are an odd

@@ -476,6 +476,27 @@ def test_prompts_that_the_tensor_memory_kernel_leaves_to_the_other(dev, scale, h
     assert int(status) == 0
 
 
+@pytest.mark.parametrize("value, window", [(64, None), (128, 100), (64, 130)])
+def test_values_that_are_not_finite_stay_with_the_rows_that_see_them(dev, value, window):
+    """Infinite and NaN values in a prompt on the tensor cores: the columns of the rows that see them, and nothing else."""
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(value)
+    heads, dim, rot, n, scale = 2, 64, 64, 301, 0.1
+    draw = lambda *shape: torch.randn(shape, generator=gen).to(torch.bfloat16).to(dev)  # noqa: E731
+    q_plain, q_rot, k_plain, k_rot, v = draw(n, heads, dim), draw(n, heads, rot), draw(n, heads, dim), draw(n, rot), draw(n, heads, value)
+    v[100, 0, 3], v[127, 0, value - 1], v[128, 1, 0], v[200, 1, 0] = float("inf"), -float("inf"), float("nan"), float("inf")
+    v[300, 1, 33], v[150, 0, 3] = float("inf"), -float("inf")
+    out, status = torch.zeros((n, heads, value), dtype=torch.bfloat16, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    ops.head_prompt_attention(q_plain, q_rot, k_plain, k_rot, v, _prompt_tiles(n, dev), out, scale, window, status=status,
+                              tensor_memory=True)
+    seen, want = _prompt_in_64_bits(q_plain, q_rot, k_plain, k_rot, v, scale, window)
+    for token, head, column in (~torch.isfinite(v)).nonzero().tolist():
+        want[seen[:, token], head, column] += v[token, head, column].double()
+    torch.testing.assert_close(out.double(), want, rtol=2e-2, atol=2e-2, equal_nan=True)
+    assert int(status) == 0
+
+
 @pytest.mark.parametrize("heads, dim, rot, value, rank, q_rank, page", [
     (3, 128, 64, 128, 512, None, 16), (4, 40, 24, 72, 32, 64, 16), (2, 64, 16, 64, 192, 40, 8), (2, 64, 8, 40, 176, 40, 5)])
 @pytest.mark.parametrize("window", [None, 60])
