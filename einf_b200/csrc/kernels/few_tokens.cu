@@ -273,8 +273,9 @@ __global__ void __launch_bounds__(WARPS * 32) few_tokens_kernel(FewArgs a) {
         const int kv = is_v ? head - a.num_heads - a.num_kv_heads : head - a.num_heads;
         to = (is_v ? a.v_cache : a.k_cache) + (((size_t)page * a.num_kv_heads + kv) * a.page_size + offset) * a.head_size;
       }
-      to[dim] = __float2bfloat16_rn(one * cosine - two * sine);
-      to[dim + a.head_size / 2] = __float2bfloat16_rn(two * cosine + one * sine);
+      const bool turns = !is_v && a.rotary;     // else the halves do not meet: zero times infinity would not be zero
+      to[dim] = __float2bfloat16_rn(turns ? one * cosine - two * sine : one);
+      to[dim + a.head_size / 2] = __float2bfloat16_rn(turns ? two * cosine + one * sine : two);
     } else if (END == kFewSilu) {
       a.out[(size_t)token * (a.rows / 2) + tile * kEach + item] = __float2bfloat16_rn(one / (1.f + expf(-one)) * two);
     } else {

@@ -105,6 +105,33 @@ def test_product_into_the_stream_and_alone(dev, tokens, k, rows):
     assert int(status) == 0
 
 
+@pytest.mark.parametrize("rotary", [False, True])
+def test_a_value_that_is_not_finite_stays_in_its_element(dev, rotary):
+    """Values, and heads that are not rotated, do not meet the other half of their head."""
+    from einf_b200 import ops
+
+    torch.manual_seed(11)
+    tokens, hidden, heads, kv_heads, size, page = 3, 64, 2, 1, 32, 16
+    residual, norm = torch.randn(tokens, hidden, device=dev), torch.ones(hidden, device=dev)
+    weight = (torch.randn((heads + 2 * kv_heads) * size, hidden, device=dev) * 0.1).bfloat16()
+    bias = torch.zeros(weight.shape[0], device=dev)
+    inv_freq = 1.0 / (1e4 ** (torch.arange(0, size, 2, device=dev).float() / size)) if rotary else torch.empty(0, device=dev)
+    marked = {"q": 5, "k": heads * size + 20, "v": (heads + kv_heads) * size + 3}
+    for value in (float("inf"), float("nan")):
+        for place in marked.values():
+            bias[place] = value
+        q = torch.zeros(tokens, heads, size, dtype=torch.bfloat16, device=dev)
+        k, v = (torch.zeros(1, kv_heads, page, size, dtype=torch.bfloat16, device=dev) for _ in range(2))
+        status = torch.zeros(1, dtype=torch.int32, device=dev)
+        ops.few_qkv(residual, None, norm, 1e-6, weight, bias, torch.arange(1, tokens + 1, dtype=torch.int32, device=dev), inv_freq,
+                    torch.arange(tokens, dtype=torch.int32, device=dev), q, k, v, heads, kv_heads, size, status)
+        rows = {"q": q.view(tokens, -1), "k": k[0, 0, :tokens], "v": v[0, 0, :tokens]}
+        for name, first in (("q", 0), ("k", heads * size), ("v", (heads + kv_heads) * size)):
+            at = marked[name] - first
+            bad = {at, at + size // 2 if at % size < size // 2 else at - size // 2} if rotary and name != "v" else {at}
+            assert set((~torch.isfinite(rows[name])).any(0).nonzero().flatten().tolist()) == bad, (name, value)
+
+
 def test_a_token_gets_the_same_in_every_batch(dev):
     """A token's sums do not depend on the tokens beside it."""
     from einf_b200 import ops
