@@ -34,7 +34,7 @@ __device__ __forceinline__ void store_quad(T* p, float4 v) {
 // finish(token, input, sum): what becomes of a token's sum (`input` its own row); start(): what the sum starts from, or the
 // input itself with kFromInput.  `state` rows are the taps - 1 inputs before a request's tokens, oldest first.  `updates`: the
 // step has one request, whose first tokens, and with them all that reads its state row, are the first run's: its thread then
-// leaves the last taps - 1 inputs there (of more requests a run may begin behind another's first token: a kernel behind
+// leaves the request's last taps - 1 inputs there (rows may go on behind its end, q_start[1]; of more requests a run may begin behind another's first token: a kernel behind
 // this one does it).
 template <typename T, bool kFromInput, typename Finish>
 __device__ __forceinline__ void conv_run(const T* __restrict__ in, long long in_stride, int c, int t0, int num_tokens, int taps,
@@ -95,17 +95,30 @@ __device__ __forceinline__ void conv_run(const T* __restrict__ in, long long in_
     finish(t, acc);
   }
   if (!updates || t0 != 0) return;
-  const int slot = state_slots[0];
-  if (slot < 0 || slot >= num_slots) return;
+  const int slot = state_slots[0], keep = taps - 1, count = q_start[1] - q_start[0];
+  if (slot < 0 || slot >= num_slots || count <= 0) return;
+  float* rows = state + (long long)slot * state_stride + c;
+  float4 fresh[kRunTaps - 1];
 #pragma unroll
   for (int u = 0; u < kRunTaps - 1; ++u) {
-    if (u >= taps - 1) break;
-    float4 v = load_quad(in + (long long)(num_tokens - (taps - 1) + u) * in_stride + c);
-    float* row = state + (long long)slot * state_stride + (long long)u * channels + c;
-    row[0] = v.x + bias.x;
-    row[1] = v.y + bias.y;
-    row[2] = v.z + bias.z;
-    row[3] = v.w + bias.w;
+    if (u >= keep) break;
+    const int rel = count - keep + u;                    // below zero: of the old state, by a portion shorter than it
+    if (rel >= 0) {
+      const float4 v = load_quad(in + (long long)(q_start[0] + rel) * in_stride + c);
+      fresh[u] = make_float4(v.x + bias.x, v.y + bias.y, v.z + bias.z, v.w + bias.w);
+    } else {
+      const float* row = rows + (long long)(u + count) * channels;
+      fresh[u] = make_float4(row[0], row[1], row[2], row[3]);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kRunTaps - 1; ++u) {
+    if (u >= keep) break;
+    float* row = rows + (long long)u * channels;
+    row[0] = fresh[u].x;
+    row[1] = fresh[u].y;
+    row[2] = fresh[u].z;
+    row[3] = fresh[u].w;
   }
 }
 

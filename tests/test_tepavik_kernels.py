@@ -534,6 +534,30 @@ def test_conv_silu_over_runs_of_tokens(dev, dtype, channels, taps, heads, length
         close(got, want, dtype if got.dtype == dtype else torch.float32)
 
 
+@pytest.mark.parametrize("which", ["conv_silu", "norm_conv"])
+@pytest.mark.parametrize("end", [700, 693, 4, 2, 1])
+def test_one_requests_state_ends_where_the_request_ends(dev, which, end):
+    """Rows behind the end of a step's only request (its tokens moved over runs of eight) are no inputs of its state; a
+    portion shorter than the state keeps the tail of the old one."""
+    from einf_b200 import ops
+
+    gen = torch.Generator().manual_seed(end)
+    tokens, channels, taps = 701, 900, 4
+    x, weight = torch.randn((tokens, channels), generator=gen).to(dev), torch.randn((channels, taps), generator=gen).to(dev)
+    state = torch.randn((3, taps - 1, channels), generator=gen).to(dev)
+    q_start, slots = torch.tensor([0, end], dtype=torch.int32, device=dev), torch.tensor([1], dtype=torch.int32, device=dev)
+    seq, results = torch.zeros(tokens, dtype=torch.int32, device=dev), []
+    for module in (ops, ref):
+        mine, out = state.clone(), torch.zeros((tokens, channels), device=dev)
+        if which == "conv_silu":
+            module.conv_silu(x, weight, None, mine, seq, q_start, slots, out)
+        else:
+            module.norm_conv([], 1.0, x.clone(), torch.ones(channels, device=dev), 1e-5, weight, mine, seq, q_start, slots, out)
+        results.append((mine, out[:end]))
+    for got, want in zip(*results):
+        close(got, want, torch.float32)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("width, parts, kind", [(252, 1, "silu"), (1280, 2, "sigmoid"), (1024, 1, "silu"), (1028, 1, "silu")])
 def test_gated_norm_a_warp_a_row(dev, dtype, width, parts, kind):
