@@ -310,9 +310,10 @@ class PagedAttention(Mixer):
         return out
 
     def takes_few(self) -> bool:
-        """Whether the layer's products run in the kernels for a few tokens."""
+        """Whether the layer's products run in the kernels for a few tokens (:meth:`forward_few` does what this very class's
+        ``forward`` does: a derived one's may do anything else)."""
         return bool(
-            self.fast and self.out_bias is None and self.qkv_weight.dtype == self.out_weight.dtype == torch.bfloat16
+            type(self) is PagedAttention and self.fast and self.out_bias is None and self.qkv_weight.dtype == self.out_weight.dtype == torch.bfloat16
             and self.qkv_weight.data_ptr() % 16 == 0 and self.out_weight.data_ptr() % 16 == 0
             and self.position.kind in ("rope", "none") and self.position.inv_freq.shape[0] in (0, self.head_size // 2)
             and not getattr(self.position, "interleaved", False)

@@ -76,9 +76,10 @@ class GatedMLP(FeedForward):
         return ops.project(hidden, self.down_weight, ctx.status)
 
     def takes_few(self) -> bool:
-        """Whether the products run in the kernels for a few tokens."""
+        """Whether the products run in the kernels for a few tokens (:meth:`forward_few` does what this very class's
+        ``forward`` does: a derived one's may do anything else)."""
         return bool(
-            self.activation.kind == "silu" and self.gate_up_weight.dtype == self.down_weight.dtype == torch.bfloat16
+            type(self) is GatedMLP and self.activation.kind == "silu" and self.gate_up_weight.dtype == self.down_weight.dtype == torch.bfloat16
             and self.gate_up_weight.data_ptr() % 16 == 0 and self.down_weight.data_ptr() % 16 == 0
             and self.runtime.dtype == torch.bfloat16 and self.intermediate_size % 32 == 0 and self.hidden_size % 8 == 0
             and ops.few_tokens_fit(self.hidden_size, True) and ops.few_tokens_fit(self.intermediate_size, False)

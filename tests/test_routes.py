@@ -1,0 +1,53 @@
+"""Which calls go which way, and what the host hands on, on a machine without a GPU."""
+from dataclasses import replace
+
+import pytest
+import torch
+
+
+def test_parts_of_ones_own_keep_their_forward():
+    """Parts derived from the attention mixer and the gated feed-forward, under kinds of their own, run their own
+    ``forward`` for any number of tokens; the built-in ones take the kernels for a few."""
+    from conftest import SIZED
+    from einf_b200.config import config_from_dict
+    from einf_b200.parts import base
+    from einf_b200.parts.attention import PagedAttention
+    from einf_b200.parts.block import build_block
+    from einf_b200.parts.mlp import GatedMLP
+    from einf_b200.parts.model import expected_tensors
+    from einf_b200.weights.random import random_tensors
+
+    config = config_from_dict(dict(SIZED["0.5b"], vocab_size=64, num_hidden_layers=1))
+    spec = config.model_spec()
+    tensors = random_tensors(expected_tensors(spec)[0], 0)
+    runtime, called = base.Runtime(torch.bfloat16, torch.device("cpu")), []
+
+    class Mixer(PagedAttention):
+        def forward(self, x, ctx, cache):
+            called.append("mixer")
+            return x
+
+    class FeedForward(GatedMLP):
+        def forward(self, x, ctx):
+            called.append("feed_forward")
+            return x
+
+    saved = {category: dict(kinds) for category, kinds in base._REGISTRY.items()}
+    try:
+        base.register_part("mixer", "own_mixer")(Mixer)
+        base.register_part("feed_forward", "own_feed_forward")(FeedForward)
+        built_in = build_block(spec.layers[0], tensors, runtime)
+        assert built_in.mixer.takes_few() and built_in.feed_forward.takes_few()
+        for own in ({"mixer"}, {"feed_forward"}, {"mixer", "feed_forward"}):
+            parts = {role: replace(part, kind="own_" + role) if role in own else part for role, part in spec.layers[0].parts.items()}
+            block = build_block(replace(spec.layers[0], parts=parts), tensors, runtime)
+            block.mixer_norm.forward = block.feed_forward_norm.forward = lambda pending, residual, **_: residual
+            for role in {"mixer", "feed_forward"} - own:
+                getattr(block, role).forward = lambda x, *_: x
+            called.clear()
+            block.forward(torch.zeros(4, 896), None, type("Context", (), {"status": None}), None)
+            assert set(called) == own
+    finally:
+        for category, kinds in saved.items():
+            base._REGISTRY[category].clear()
+            base._REGISTRY[category].update(kinds)
