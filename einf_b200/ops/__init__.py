@@ -628,6 +628,16 @@ def few_tokens_fit(k: int, norm: bool) -> bool:
     return k % 32 == 0 and k <= (FEW_NORM_WIDTH if norm else FEW_WIDTH)
 
 
+@functools.lru_cache(maxsize=256)
+def few_tokens_limit(hidden: int, inter: int) -> int:
+    """Up to how many tokens a layer of these sizes runs in the kernels for a few: :data:`FEW_TOKENS`, or eight where gate/up
+    for more has more CTAs than run at once (32 rows of weights and sixteen tokens' sums each: two an SM from 992 elements
+    on, three below).  Twelve layers, 1,024 wide, sixteen tokens, separate products / these: 4,608 a branch (288 CTAs) 355 / 329 us,
+    4,864 (304) 357 / 377, 5,120 362 / 385; 960 wide, 5,120 375 / 359; eight tokens, 1,024 wide, 5,120 343 / 266."""
+    room = 32 * ((2 * hidden + 127) // 128 * 128 + 64) + 4 * hidden + 9 * 1024 + 1024     # and what the system keeps of a CTA's
+    return FEW_TOKENS if -(-inter // 16) <= (228 << 10) // room * _sm_count() else 8
+
+
 def few_qkv(residual: torch.Tensor, pending: Optional[torch.Tensor], norm_weight: torch.Tensor, eps: float,
             weight: torch.Tensor, bias: Optional[torch.Tensor], positions: torch.Tensor, inv_freq: torch.Tensor,
             slots: Optional[torch.Tensor], q_out: torch.Tensor, k_cache: Optional[torch.Tensor],

@@ -66,7 +66,8 @@ class PreNormBlock(Block):
         return norm.forward(pending, residual)
 
     def forward(self, residual, pending, ctx, cache):
-        if self._few and residual.shape[0] <= ops.FEW_TOKENS and residual.data_ptr() % 16 == 0 and (
+        if self._few and residual.shape[0] <= ops.FEW_TOKENS and residual.shape[0] <= self.feed_forward.few_limit() and \
+                residual.data_ptr() % 16 == 0 and (
                 pending is None or (pending.dtype == torch.float32 and pending.shape == residual.shape
                                     and pending.data_ptr() % 16 == 0)):
             self.mixer.forward_few(residual, pending, self.mixer_norm, ctx, cache)

@@ -85,6 +85,10 @@ class GatedMLP(FeedForward):
             and ops.few_tokens_fit(self.hidden_size, True) and ops.few_tokens_fit(self.intermediate_size, False)
         )
 
+    def few_limit(self) -> int:
+        """Up to how many tokens those kernels are the faster ones."""
+        return ops.few_tokens_limit(self.hidden_size, self.intermediate_size)
+
     def forward_few(self, residual, norm, ctx):
         """``feed_forward(norm(residual))`` for a few tokens, as float32: the norm and the activation run in the
         launch of the gate/up product."""

@@ -51,3 +51,13 @@ def test_parts_of_ones_own_keep_their_forward():
         for category, kinds in saved.items():
             base._REGISTRY[category].clear()
             base._REGISTRY[category].update(kinds)
+
+
+@pytest.mark.parametrize("hidden, inter, limit", [(896, 4864, 16), (960, 5120, 16), (1024, 4608, 16), (1024, 4736, 16), (1024, 4768, 8), (992, 5120, 8)])
+def test_more_than_eight_tokens_where_gate_up_is_one_wave(monkeypatch, hidden, inter, limit):
+    from einf_b200 import ops
+
+    monkeypatch.setattr(ops, "_sm_count", lambda: 148)
+    ops.few_tokens_limit.cache_clear()
+    assert ops.few_tokens_limit(hidden, inter) == limit
+    ops.few_tokens_limit.cache_clear()
