@@ -19,8 +19,11 @@
 // Measured (B200, us, FMA before): 545 rows, 896 -> 1,152 42 -> 21, 896 -> 896 41 -> 18, 896 -> 9,728 211 -> 84 (113 TFLOP/s),
 // 4,864 -> 896 118 -> 45; 2,048 rows, 3,584 -> 4,608 1,300 -> 395 (171 TFLOP/s); one row, 896 -> 9,728 40 -> 26.
 //
-// A value that is not finite, or rounds to infinity as bfloat16, has no such parts: a CTA that met one computes its outputs again
-// by FMA (slow; rare).  Of values below 2^-109 parts are lost to the smallest bfloat16.
+// A value that is not finite, rounds to infinity as bfloat16 or has bits below the smallest bfloat16 (values below 2^-110) has no
+// such parts.  The outputs of its row, and any whose sum is not finite (products of parts may overflow where the operands'
+// does not, or to the other infinity), are computed by FMA, the CTA's tile out of shared memory with sums over 256 elements;
+// the outputs beside them keep theirs.  (NaN needs no second sum: its first part is NaN.)  545 rows, 896 -> 9,728, one of them with
+// an infinity: 172 us (FMA alone 210; 8,050 where every thread walked its outputs by itself), all of them 719, with NaN 88.
 #include "mma_sync.cuh"
 #include "tcgen05.cuh"
 
@@ -42,25 +45,26 @@ struct PartsArgs {
   int* status;                // may be null
 };
 
-// Eight values as four pairs of each part; false if one has none.
+// Eight values as four pairs of each part; false if one is not the sum of its parts (an infinity or a NaN on the way is not).
 __device__ __forceinline__ bool split_eight(const float4& x, const float4& y, uint4 (&part)[3]) {
-  constexpr float kLargest = 3.3895314e38f;
   const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-  bool fine = true;
+  uint32_t left = 0;                   // of the third parts: bits that bfloat16 has not (NaN, as it is made, has them all)
   uint32_t p[3][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     float a = v[2 * i], b = v[2 * i + 1];
-    fine = fine && fabsf(a) <= kLargest && fabsf(b) <= kLargest;
     p[0][i] = pack_pair(a, b);
     a -= low_bf16(p[0][i]);
     b -= high_bf16(p[0][i]);
     p[1][i] = pack_pair(a, b);
-    p[2][i] = pack_pair(a - low_bf16(p[1][i]), b - high_bf16(p[1][i]));
+    a -= low_bf16(p[1][i]);
+    b -= high_bf16(p[1][i]);
+    p[2][i] = pack_pair(a, b);
+    left |= __float_as_uint(a) | __float_as_uint(b);
   }
 #pragma unroll
   for (int j = 0; j < 3; ++j) part[j] = make_uint4(p[j][0], p[j][1], p[j][2], p[j][3]);
-  return fine;
+  return (left & 0xffffu) == 0u;
 }
 
 __device__ __forceinline__ bool parts_wait(uint32_t bar, uint32_t parity) {
@@ -78,15 +82,88 @@ __device__ __forceinline__ bool parts_wait(uint32_t bar, uint32_t parity) {
   return false;
 }
 
+__device__ __forceinline__ float* parts_out(const PartsArgs& g, int row, int col) {
+  return g.out + (g.shared ? (long long)blockIdx.z * g.m * g.n + (long long)row * g.n : (long long)row * g.ldo) + col;
+}
+
+// Enters a thread's marked rows among the tile's; those with a NaN, which the thread's columns are looked through for, apart.
+__device__ __noinline__ void parts_mark(const PartsArgs& g, uint32_t marks, int row0, int col0, int first, int k1, uint32_t* odd, uint32_t* nan) {
+  for (int j = 0; j < 4; ++j) {
+    if (!(marks >> j & 1u)) continue;
+    const int row = (j & 1 ? row0 : col0) + 64 * (j >> 1);
+    const float* from = j & 1 ? g.a + (long long)row * g.lda : g.w + (long long)row * g.k;
+    bool is_nan = false;
+    for (int at = first; at < k1; at += kPartK)
+      for (int e = 0; e < 8; ++e) is_nan = is_nan || from[at + e] != from[at + e];
+    atomicOr((is_nan ? nan : odd) + (j & 1) * 4 + (row % kPartRows >> 5), 1u << (row & 31));
+  }
+}
+
+// Outputs of the CTA's tile over the columns from `first` to k1 by FMA: of this thread's 32 (one row of W, 32 rows of A) those marked
+// in `again`.  32 columns of both operands at a time in shared memory, rows side by side.
+__device__ __noinline__ void parts_by_fma(const PartsArgs& g, float* w_tile, int row0, int col0, int first, int k1, uint32_t again) {
+  constexpr int kStep = 32, kPitch = kPartRows + 4;
+  float* a_tile = w_tile + kStep * kPitch;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = tid >> 2, part = (tid & 3) * 8;
+  const int col = col0 + (warp & 3) * 32 + lane, first_token = row0 + (warp >> 2) * 32;
+  const bool busy = __any_sync(0xffffffffu, again != 0u);     // a warp with nothing to do only brings its share
+  const bool w_real = col0 + row < g.n, a_real = row0 + row < g.m;
+  const float* w_row = g.w + (long long)(col0 + row) * g.k;
+  const float* a_row = g.a + (long long)(row0 + row) * g.lda;
+  float block[32], folded[32];
+#pragma unroll
+  for (int e = 0; e < 32; ++e) block[e] = folded[e] = 0.f;
+#pragma unroll 1
+  for (int k0 = first; k0 < k1; k0 += kStep) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int at = k0 + part + e;
+      w_tile[(part + e) * kPitch + row] = w_real && at < k1 ? w_row[at] : 0.f;
+      a_tile[(part + e) * kPitch + row] = a_real && at < k1 ? a_row[at] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll 2
+    for (int kk = 0; kk < (busy ? kStep : 0); ++kk) {
+      const float w = w_tile[kk * kPitch + (warp & 3) * 32 + lane];
+      const float4* a = reinterpret_cast<const float4*>(a_tile + kk * kPitch + (warp >> 2) * 32);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float4 x = a[e];
+        block[4 * e] = fmaf(x.x, w, block[4 * e]);
+        block[4 * e + 1] = fmaf(x.y, w, block[4 * e + 1]);
+        block[4 * e + 2] = fmaf(x.z, w, block[4 * e + 2]);
+        block[4 * e + 3] = fmaf(x.w, w, block[4 * e + 3]);
+      }
+    }
+    __syncthreads();
+    if ((k0 - first) % 256 == 256 - kStep) {
+#pragma unroll
+      for (int e = 0; e < 32; ++e) {
+        folded[e] += block[e];
+        block[e] = 0.f;
+      }
+    }
+  }
+  if (!again) return;
+  float* out = parts_out(g, first_token, col);
+  const long long ldo = g.shared ? g.n : g.ldo;
+  const float bias = g.bias && !g.shared ? g.bias[col] : 0.f;
+#pragma unroll
+  for (int e = 0; e < 32; ++e)
+    if (again >> e & 1u) out[e * ldo] = (folded[e] + block[e]) + bias;
+}
+
 __global__ void __launch_bounds__(kPartThreads, 1) gemm_parts_kernel(const __grid_constant__ PartsArgs g) {
   extern __shared__ unsigned char parts_smem[];
   __shared__ __align__(8) unsigned long long bars[1];
   __shared__ uint32_t tmem_address;
+  __shared__ uint32_t odd[2][4], nan[2][4];        // rows of W and of A, a bit each: with a value that has no parts; with a NaN
   const uint32_t tiles = (smem_address(parts_smem) + 1023u) & ~1023u;
   const uint32_t bar = smem_address(bars);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int row0 = (int)blockIdx.y * kPartRows, col0 = (int)blockIdx.x * kPartRows;
   const int blocks = (g.k + kPartK - 1) / kPartK, first = (int)blockIdx.z * g.blocks_each, last = min(blocks, first + g.blocks_each);
+  if (tid < 8) (&odd[0][0])[tid] = (&nan[0][0])[tid] = 0u;
   if (tid == 0) {
     bar_init(bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -120,18 +197,19 @@ __global__ void __launch_bounds__(kPartThreads, 1) gemm_parts_kernel(const __gri
       a_next[i][1] = in ? rows[1] : zero;
     }
   };
-  bool fine = true, ended = true;
+  bool ended = true;
+  uint32_t marks = 0;                              // which of this thread's four rows (W, A, W, A) had a value without parts
   auto store = [&](uint32_t stage) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int row = first_row + 64 * i;
       const uint32_t at = stage + row * 128 + ((chunk ^ (row & 7)) << 4);
       uint4 part[3];
-      fine = split_eight(w_next[i][0], w_next[i][1], part) && fine;
+      marks |= split_eight(w_next[i][0], w_next[i][1], part) ? 0u : 1u << (2 * i);
 #pragma unroll
       for (int j = 0; j < 3; ++j)
         asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at + j * kPartTile), "r"(part[j].x), "r"(part[j].y), "r"(part[j].z), "r"(part[j].w) : "memory");
-      fine = split_eight(a_next[i][0], a_next[i][1], part) && fine;
+      marks |= split_eight(a_next[i][0], a_next[i][1], part) ? 0u : 2u << (2 * i);
 #pragma unroll
       for (int j = 0; j < 3; ++j)
         asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at + (3 + j) * kPartTile), "r"(part[j].x), "r"(part[j].y), "r"(part[j].z), "r"(part[j].w) : "memory");
@@ -216,29 +294,33 @@ __global__ void __launch_bounds__(kPartThreads, 1) gemm_parts_kernel(const __gri
       for (int e = 0; e < 16; ++e) sums[half * 16 + e] += v[e];
     }
   }
-  const bool all_fine = __syncthreads_and(fine), all_ended = __syncthreads_and(ended);
+  if (marks) parts_mark(g, marks, row0 + first_row, col0 + first_row, first * kPartK + chunk * 8, min(g.k, last * kPartK), &odd[0][0], &nan[0][0]);
+  const bool all_ended = __syncthreads_and(ended);            // and every mark is there
   if (!all_ended && tid == 0 && g.status) atomicOr(g.status, kStatusWaitExpired);
-  const int col = col0 + (warp & 3) * 32 + lane;
-  if (col < g.n) {
-    float* out = g.out + (g.shared ? (long long)blockIdx.z * g.m * g.n : 0);
-    const long long ldo = g.shared ? g.n : g.ldo;
-    const float bias = g.bias && !g.shared ? g.bias[col] : 0.f;
-    const int first_token = row0 + (warp >> 2) * 32;
-    if (all_fine && all_ended) {
+  const int col = col0 + (warp & 3) * 32 + lane, first_token = row0 + (warp >> 2) * 32;
+  const int real = col < g.n ? max(0, min(32, g.m - first_token)) : 0;
+  // this thread's outputs that its sums are not good for
+  uint32_t again = odd[0][warp & 3] >> lane & 1u ? ~0u : odd[1][warp >> 2];
+  float zero[4] = {};
 #pragma unroll
-      for (int e = 0; e < 32; ++e)
-        if (first_token + e < g.m) out[(long long)(first_token + e) * ldo + col] = sums[e] + bias;
-    } else {
-      const int k0 = first * kPartK, k1 = min(g.k, last * kPartK);
-      for (int e = 0; e < 32 && first_token + e < g.m; ++e) {
-        const float* x = g.a + (long long)(first_token + e) * g.lda;
-        const float* y = g.w + (long long)col * g.k;
-        float sum = 0.f;
-        for (int kk = k0; kk < k1; ++kk) sum = fmaf(x[kk], y[kk], sum);
-        out[(long long)(first_token + e) * ldo + col] = all_ended ? sum + bias : __int_as_float(0x7fffffff);
-      }
-    }
+  for (int e = 0; e < 32; ++e) zero[e & 3] = fmaf(sums[e], 0.f, zero[e & 3]);
+  if ((zero[0] + zero[1]) + (zero[2] + zero[3]) != 0.f) {
+#pragma unroll
+    for (int e = 0; e < 32; ++e) again |= (fabsf(sums[e]) < INFINITY ? 0u : 1u) << e;
   }
+  again &= nan[0][warp & 3] >> lane & 1u ? 0u : ~nan[1][warp >> 2];
+  again = all_ended && real > 0 ? again & (~0u >> (32 - real)) : 0u;
+  float* out = parts_out(g, first_token, col);
+  const long long ldo = g.shared ? g.n : g.ldo;
+  const float bias = real > 0 && g.bias && !g.shared ? g.bias[col] : 0.f;
+  const uint32_t good = real == 32 ? ~again : ((1u << real) - 1u) & ~again;
+  if (!all_ended) sums[0] = __int_as_float(0x7fffffff);
+#pragma unroll
+  for (int e = 0; e < 32; ++e)
+    if (good >> e & 1u) out[e * ldo] = (all_ended ? sums[e] : sums[0]) + bias;
+  if (__syncthreads_or(again != 0u))
+    parts_by_fma(g, reinterpret_cast<float*>(parts_smem + (tiles - smem_address(parts_smem))), row0, col0, first * kPartK,
+                 min(g.k, last * kPartK), again);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");

@@ -1306,6 +1306,48 @@ def test_gemm_of_three_parts_with_values_that_have_none(dev):
         torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-5, equal_nan=True)
 
 
+@pytest.mark.parametrize("shares", [1, 3])
+def test_gemm_of_three_parts_keeps_values_without_parts_to_themselves(dev, shares):
+    """Rows and columns beside an infinite, a NaN and a too large value get bit for bit what they get without it; those of the
+    value, and finite operands whose product or whose parts' products overflow, get what FMA gives."""
+    from einf_b200 import ops
+
+    torch.manual_seed(17)
+    m, n, k = 130, 140, 1160
+    x, w = torch.randn(m, k, device=dev), torch.randn(n, k, device=dev)
+    clean, got, want = (torch.empty(m, n, device=dev) for _ in range(3))
+    ops.gemm_parts(x, w, None, clean, shares=shares)
+    x[3, 5], x[129, 700], x[64, 1159], x[70, 0] = float("inf"), float("nan"), -3.4e38, 1e30
+    w[7, 600], w[139, 1], w[70, 0] = -float("inf"), 3.4e38, 1e12
+    rows, columns = torch.ones(m, dtype=torch.bool, device=dev), torch.ones(n, dtype=torch.bool, device=dev)
+    rows[[3, 129, 64, 70]], columns[[7, 139, 70]] = False, False
+    ops.gemm_parts(x, w, None, got, shares=shares)
+    ops.gemm_simt(x, w, None, want)
+    assert torch.equal(got[rows][:, columns], clean[rows][:, columns])
+    for of in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(of(got), of(want))
+    assert got[70, 70] == float("inf")
+    size = torch.nan_to_num(x.double().abs(), 0, 0, 0) @ torch.nan_to_num(w.double().abs(), 0, 0, 0).T
+    fine = torch.isfinite(want)
+    assert bool(((got.double() - want.double()).abs() <= size * 2 ** -20)[fine].all())
+
+
+def test_gemm_of_three_parts_of_very_small_values(dev):
+    """Every bit counts down to the smallest normal value and below it, where the parts would end at the smallest bfloat16."""
+    from einf_b200 import ops
+
+    torch.manual_seed(19)
+    m, n, k = 40, 130, 264
+    base, w = torch.randn(m, k, device=dev), torch.randn(n, k, device=dev) * 2.0 ** 90
+    for power in (-100, -108, -112, -120, -126, -135):
+        x = (base.double() * 2.0 ** power).float()
+        for a, b in ((x, w), (w, x)):
+            got = torch.empty(a.shape[0], b.shape[0], device=dev)
+            ops.gemm_parts(a, b, None, got)
+            want = a.double() @ b.double().T
+            assert float((got.double() - want).norm() / want.norm()) < 4e-7, power
+
+
 @pytest.mark.parametrize("top_k", [1, 5, 255, 256, 257, 0])
 def test_sampling_where_few_tokens_are_looked_at(dev, top_k):
     """Both sides of what one CTA settles by itself and of what a CTA lists: more tied tokens than it takes, a row
