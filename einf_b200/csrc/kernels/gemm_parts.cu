@@ -5,9 +5,10 @@
 // products, of which the six largest count: what is left out is below 2^-24 of a term.  The instruction cuts its sums
 // off where FMA rounds them, so a chain of it drifts.  Therefore 32 elements of K are summed at a time, products of the
 // smaller parts first, into a tensor-memory accumulator that starts at zero, and its result is added to a running sum in
-// registers by a rounded addition; every 512 elements that sum joins a total in tensor memory.  Error against 64 bits (2-norm,
-// normal values, this / FMA): K = 896 0.97e-7 / 2.8e-7, 4,864 1.1e-7 / 3.0e-7, 18,944 1.5e-7 / 3.3e-7; where all terms are
-// positive 0.96e-7 / 1.28e-7, 1.0e-7 / 0.9e-7, 1.3e-7 / 1.4e-7 (64 elements at a time 1.8e-7; without the total 2.1e-7 at 4,864).
+// registers by a rounded addition; every 512 elements that sum joins a total in tensor memory.  Error against 64 bits (2-norm, 1 to 2,048
+// rows against 896, this / FMA, in 1e-7): normal values, K = 896 0.83 to 0.97 / 2.8, 4,864 0.95 to 1.14 / 3.0, 18,944 1.2 / 3.3;
+// where all terms are positive (normal values' magnitudes, uniform ones) 0.64 to 0.76 / 1.1 to 1.3, 0.66 to 0.78 / 0.87, 0.66 to 0.72 / 1.34, or
+// 1.08 by one CTA each (64 elements at a time 1.8; without the total 2.1 at 4,864).
 //
 // A CTA has 128 rows of W (the instruction's M) and 128 rows of A (its N).  Its sixteen warps read the next 64 columns of
 // both operands into registers, split them and write the parts into swizzled K-major tiles (two stages of 96 KB), one
@@ -326,7 +327,8 @@ __global__ void __launch_bounds__(kPartThreads, 1) gemm_parts_kernel(const __gri
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
-// The shares' sums in the order of K, and bias: four columns a thread where rows are whole groups of four (545 x 896 by four
+// The shares' sums, four and four in the order of K (one after the other, sixteen shares of uniform terms, K = 4,864, had an error of
+// 0.874e-7 where FMA has 0.865e-7), and bias: four columns a thread where rows are whole groups of four (545 x 896 by four
 // shares: 8.8 us with a thread and a 64-bit division an element).
 template <int VEC>
 __global__ void __launch_bounds__(256) gemm_parts_sum_kernel(const __grid_constant__ PartsArgs g, const float* sums, int shares) {
@@ -352,10 +354,8 @@ __global__ void __launch_bounds__(256) gemm_parts_sum_kernel(const __grid_consta
       }
     }
 #pragma unroll
-    for (int s = 0; s < 4; ++s)
-#pragma unroll
-      for (int e = 0; e < VEC; ++e)
-        if (s0 + s < shares) sum[e] += v[s][e];
+    for (int e = 0; e < VEC; ++e)
+      sum[e] += (v[0][e] + (s0 + 1 < shares ? v[1][e] : 0.f)) + ((s0 + 2 < shares ? v[2][e] : 0.f) + (s0 + 3 < shares ? v[3][e] : 0.f));
   }
   float* out = g.out + (long long)r * g.ldo + c;
 #pragma unroll

@@ -1348,6 +1348,28 @@ def test_gemm_of_three_parts_of_very_small_values(dev):
             assert float((got.double() - want).norm() / want.norm()) < 4e-7, power
 
 
+@pytest.mark.parametrize("k", [896, 4864])
+@pytest.mark.parametrize("values", ["normal", "positive", "uniform"])
+@pytest.mark.parametrize("rows, shares", [(1, None), (128, None), (160, None), (160, 1), (160, 5)])
+def test_gemm_of_three_parts_is_as_close_to_64_bits_as_fma(dev, k, values, rows, shares):
+    """Relative error (2-norm) against 64 bits, of normal values and where all terms are positive: no larger than that of the
+    FMA product, and below the 2e-7 that a lost part (2^-17 of a term, whatever the sum's length) would pass."""
+    from einf_b200 import ops
+
+    torch.manual_seed(k + rows)
+    x, w = torch.randn(rows, k, device=dev), torch.randn(896, k, device=dev)
+    if values == "positive":
+        x, w = x.abs(), w.abs()
+    if values == "uniform":
+        x, w = torch.rand_like(x), torch.rand_like(w)
+    want, errors = x.double() @ w.double().T, []
+    for product in (lambda out: ops.gemm_parts(x, w, None, out, shares=shares), lambda out: ops.gemm_simt(x, w, None, out)):
+        out = torch.empty(rows, 896, device=dev)
+        product(out)
+        errors.append(float((out.double() - want).norm() / want.norm()))
+    assert errors[0] <= errors[1] and errors[0] < 2e-7, errors
+
+
 @pytest.mark.parametrize("top_k", [1, 5, 255, 256, 257, 0])
 def test_sampling_where_few_tokens_are_looked_at(dev, top_k):
     """Both sides of what one CTA settles by itself and of what a CTA lists: more tied tokens than it takes, a row
