@@ -378,7 +378,7 @@ def gemm_parts_takes(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -
     """Whether :func:`gemm_parts` takes these operands: all float32, K a multiple of eight, rows that start on 16 bytes."""
     return (
         x.dtype == weight.dtype == out.dtype == torch.float32 and x.shape[1] % 8 == 0 and x.shape[1] > 0
-        and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and x.shape[0] < 8 << 20
+        and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and x.shape[0] <= 65535 * 128
     )
 
 

@@ -61,3 +61,12 @@ def test_more_than_eight_tokens_where_gate_up_is_one_wave(monkeypatch, hidden, i
     ops.few_tokens_limit.cache_clear()
     assert ops.few_tokens_limit(hidden, inter) == limit
     ops.few_tokens_limit.cache_clear()
+
+
+@pytest.mark.parametrize("rows", [65535 * 128, 65535 * 128 + 1])
+def test_rows_of_a_32_bit_product_in_parts(rows):
+    """As many tiles of 128 rows as the launcher takes (its grid's second dimension), not one row more."""
+    from einf_b200 import ops
+
+    x, weight, out = (torch.empty(size, device="meta") for size in ((rows, 8), (16, 8), (rows, 16)))
+    assert ops.gemm_parts_takes(x, weight, out) == (rows <= 65535 * 128)
