@@ -169,16 +169,17 @@ PYBIND11_MODULE(_control, m) {
       .def_property_readonly("is_greedy", &SamplingParams::greedy);
 
   // A sampled step's parameters into the sampler's staging buffer of `max_rows` rows: seeds and sample indices as int64,
-  // temperatures, top-p and min-p as float32, top-k as int32.  Anything but SamplingParams and integers: TypeError.
+  // temperatures, top-p and min-p as float32, top-k as int32.  Anything but SamplingParams itself and integers: TypeError.
   m.def("pack_sampling", [](py::sequence params, py::sequence indices, uintptr_t address, int max_rows) {
     const int rows = (int)py::len(params);
     if (rows > max_rows || (int)py::len(indices) != rows) throw std::invalid_argument("one set of parameters and one index per row");
     auto* wide = reinterpret_cast<int64_t*>(address);
     auto* real = reinterpret_cast<float*>(wide + 2 * (size_t)max_rows);
     auto* whole = reinterpret_cast<int32_t*>(real + 3 * (size_t)max_rows);
+    const py::type exact = py::type::of<SamplingParams>();     // a derived class may have properties of its own in the fields' place
     for (int r = 0; r < rows; ++r) {
       py::object item = params[r], index = indices[r];
-      if (!py::isinstance<SamplingParams>(item) || !PyLong_Check(index.ptr())) throw py::type_error("SamplingParams and integers");
+      if (!py::type::of(item).is(exact) || !PyLong_Check(index.ptr())) throw py::type_error("SamplingParams and integers");
       const auto& p = item.cast<const SamplingParams&>();
       if (p.seed > (uint64_t)INT64_MAX) throw std::overflow_error("seed beyond 63 bits");
       wide[r] = (int64_t)p.seed;

@@ -59,8 +59,8 @@ class Sampler:
         staging = self._host[turn]
         try:
             pack_sampling(params, sample_indices, staging.data_ptr(), self.max_rows)
-        except TypeError:               # other objects with the same attributes
-            self._pack(turn, rows, params, sample_indices)
+        except TypeError:               # other objects with the same attributes, other collections than sequences
+            self._pack(turn, params, sample_indices)
         self._dev.copy_(staging, non_blocking=True)
         if self.device.type == "cuda":
             if self._events[turn] is None:
@@ -69,11 +69,12 @@ class Sampler:
         ops.sample(logits, self.tokens, *self._columns)
         return self.tokens[:rows]
 
-    def _pack(self, turn: int, rows: int, params: Sequence, sample_indices: Sequence[int]) -> None:
-        """What ``pack_sampling`` does, for any objects with the attributes of sampling parameters."""
+    def _pack(self, turn: int, params: Sequence, sample_indices: Sequence[int]) -> None:
+        """What ``pack_sampling`` does, for any objects with the attributes of sampling parameters in any collections."""
         n, host = self.max_rows, self._staging[turn]
         wide, real = host[:16 * n].view(np.int64).reshape(2, n), host[16 * n:28 * n].view(np.float32).reshape(3, n)
-        wide[0, :rows] = [np.int64(p.seed) for p in params]
-        wide[1, :rows] = sample_indices
-        real[:, :rows] = [[p.temperature for p in params], [p.top_p for p in params], [p.min_p for p in params]]
-        host[28 * n:].view(np.int32)[:rows] = [p.top_k or 0 for p in params]
+        whole = host[28 * n:].view(np.int32)
+        for r, (p, index) in enumerate(zip(params, sample_indices)):
+            wide[0, r], wide[1, r] = np.int64(p.seed), index
+            real[0, r], real[1, r], real[2, r] = p.temperature, p.top_p, p.min_p
+            whole[r] = p.top_k or 0

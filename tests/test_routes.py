@@ -70,3 +70,42 @@ def test_rows_of_a_32_bit_product_in_parts(rows):
 
     x, weight, out = (torch.empty(size, device="meta") for size in ((rows, 8), (16, 8), (rows, 16)))
     assert ops.gemm_parts_takes(x, weight, out) == (rows <= 65535 * 128)
+
+
+class _Others:
+    """Sampling parameters of another type."""
+
+    def __init__(self, params):
+        for name in ("temperature", "top_p", "min_p", "top_k", "seed"):
+            setattr(self, name, getattr(params, name))
+
+
+@pytest.mark.parametrize("collection", ["list", "views", "others", "derived"])
+def test_sampling_parameters_of_any_collection_and_type(monkeypatch, collection):
+    """The step's staging holds the same for sequences of sampling parameters, for views of a dict, for other objects with
+    their attributes, and for a derived class's own properties."""
+    from einf_b200 import ops
+    from einf_b200.cache.control import SamplingParams
+    from einf_b200.sampling import Sampler
+
+    class Colder(SamplingParams):
+        @property
+        def temperature(self):
+            return 0.25
+
+    seen = {}
+    monkeypatch.setattr(ops, "sample", lambda logits, tokens, *columns: seen.update(columns=[c.clone() for c in columns]))
+    params = [SamplingParams(temperature=0.5 + r, top_k=3 * r or None, top_p=0.9, min_p=0.125, seed=7 + r) for r in range(3)]
+    indices = [5, 6, 2**40]
+    want = [[0.5, 1.5, 2.5], [0, 3, 6], [0.9] * 3, [0.125] * 3, [7, 8, 9], indices]
+    given, places = params, indices
+    if collection == "views":
+        given, places = dict(enumerate(params)).values(), dict(enumerate(indices)).values()
+    elif collection == "others":
+        given = [_Others(p) for p in params]
+    elif collection == "derived":
+        given = params[:2] + [Colder(temperature=2.5, top_k=6, top_p=0.9, min_p=0.125, seed=9)]
+        want[0] = [0.5, 1.5, 0.25]
+    Sampler("cpu", 4).sample(torch.zeros(3, 8), given, places)
+    for column, values in zip(seen["columns"], want):
+        assert column[:3].tolist() == torch.tensor(values, dtype=column.dtype).tolist()
