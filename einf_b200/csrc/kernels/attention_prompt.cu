@@ -270,18 +270,7 @@ struct HeadLayout {
 };
 
 __device__ __forceinline__ bool head_wait(uint32_t bar, uint32_t parity, int* status) {
-  for (int poll = 0; poll < kPolls; ++poll) {
-    if (bar_test(bar, parity)) return true;
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
+  if (bar_test(bar, parity) || bar_poll(bar, parity)) return true;
   if (status) atomicOr(status, kStatusWaitExpired);
   return false;
 }

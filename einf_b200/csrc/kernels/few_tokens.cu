@@ -22,6 +22,7 @@
 // later matrices into L2 by the earlier kernels gained nothing).  Rows above 1,024 elements keep the separate kernels:
 // at 1.5B sizes (94 MB a layer, gate/up 11.5 us) a layer takes 34.9 and 45.0 us here and 34.2 and 40.3 there.
 #include "mma_sync.cuh"
+#include "tcgen05.cuh"
 
 namespace einf {
 
@@ -50,21 +51,6 @@ struct FewArgs {
   const float* add;              // add: pending (may be null)
   int* status;
 };
-
-__device__ __forceinline__ bool few_wait(uint32_t bar) {
-  for (int poll = 0; poll < (1 << 22); ++poll) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
 
 __host__ __device__ constexpr int few_row_bytes(int k) { return ((k * 2 + 127) & ~127) + 64; }
 
@@ -173,7 +159,7 @@ __global__ void __launch_bounds__(WARPS * 32) few_tokens_kernel(FewArgs a) {
           }
         }
       }
-      if (!there) failed = !few_wait(bar);
+      if (!there) failed = !bar_poll(bar, 0);
       there = true;
 #pragma unroll
       for (int u = 0; u < BATCH; ++u) {
@@ -199,7 +185,7 @@ __global__ void __launch_bounds__(WARPS * 32) few_tokens_kernel(FewArgs a) {
         xa[u] = in && g < a.tokens ? *reinterpret_cast<const uint4*>(a.x + (size_t)g * a.k + at) : make_uint4(0u, 0u, 0u, 0u);
         if (HI) xb[u] = in && g + 8 < a.tokens ? *reinterpret_cast<const uint4*>(a.x + (size_t)(g + 8) * a.k + at) : make_uint4(0u, 0u, 0u, 0u);
       }
-      if (!there) failed = !few_wait(bar);
+      if (!there) failed = !bar_poll(bar, 0);
       there = true;
     }
 #pragma unroll
@@ -219,7 +205,7 @@ __global__ void __launch_bounds__(WARPS * 32) few_tokens_kernel(FewArgs a) {
       }
     }
   }
-  if (!there) failed = !few_wait(bar);     // a warp without a piece: no CTA ends with a copy under way
+  if (!there) failed = !bar_poll(bar, 0);     // a warp without a piece: no CTA ends with a copy under way
   if (failed) atomicOr(a.status, kStatusWaitExpired);
 #pragma unroll
   for (int r = 0; r < RT; ++r) {

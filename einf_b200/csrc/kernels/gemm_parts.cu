@@ -68,21 +68,6 @@ __device__ __forceinline__ bool split_eight(const float4& x, const float4& y, ui
   return (left & 0xffffu) == 0u;
 }
 
-__device__ __forceinline__ bool parts_wait(uint32_t bar, uint32_t parity) {
-  for (int poll = 0; poll < kPolls; ++poll) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-
 __device__ __forceinline__ float* parts_out(const PartsArgs& g, int row, int col) {
   return g.out + (g.shared ? (long long)blockIdx.z * g.m * g.n + (long long)row * g.n : (long long)row * g.ldo) + col;
 }
@@ -225,7 +210,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) gemm_parts_kernel(const __gri
   const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * 32), total = mine + 256;
   // the sums of the i-th block of this CTA: of its first 32 columns, and of the others
   auto promote = [&](int i) {
-    ended = parts_wait(bar, i & 1) && ended;
+    ended = bar_poll(bar, i & 1) && ended;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
     for (int part = 0; part < 4; ++part) {

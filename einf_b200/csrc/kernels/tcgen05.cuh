@@ -19,7 +19,8 @@ __device__ __forceinline__ void bar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 constexpr int kPolls = 1 << 22;
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, int* status) {
+// True once the phase with this parity has completed, false if it has not after kPolls looks.
+__device__ __forceinline__ bool bar_poll(uint32_t bar, uint32_t parity) {
   for (int poll = 0; poll < kPolls; ++poll) {
     uint32_t done;
     asm volatile(
@@ -31,6 +32,10 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, int* sta
         : "memory");
     if (done) return true;
   }
+  return false;
+}
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, int* status) {
+  if (bar_poll(bar, parity)) return true;
   atomicOr(status, kStatusWaitExpired);
   return false;
 }
