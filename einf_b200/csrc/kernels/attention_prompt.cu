@@ -9,13 +9,14 @@
 // every step, a single token would project all it sees: both stay on the rows.  Which portions of a step are which is told
 // here, by q_start, tile by tile: what a prompt gets does not depend on what stands beside it.)
 //
-// A CTA has 64 queries of one head, a warp 16 of them with its queries in registers; 64 keys a tile; the next tile's keys
+// Portions of more than 64 tokens of heads in whole 128-byte lines have the kernel on tcgen05 further down; this is the one of the
+// others.  A CTA has 64 queries of one head, a warp 16 of them with its queries in registers; 64 keys a tile; the next tile's keys
 // are brought while this one's values are used and the other way round.  Keys come from two places (the head's plain part
 // and the rotated part that all heads share), queries too.  Three CTAs an SM hide one another's waits (two warps of 32
 // rows, which read half as much shared memory, have no registers left to load ahead of their products).
 //
 // Measured (B200): 12 heads, keys of 128 + 64, values of 128, 2,048 tokens (16 GFLOP): 116 us, against 336 us of
-// attention_latent.cu on the rows of 512 + 64 (55 GFLOP); two warps of 32 rows 184 us.  The mixer as a whole 403 -> 176 us.
+// attention_latent.cu on the rows of 512 + 64 (55 GFLOP); two warps of 32 rows 184 us.
 // What bounds it: the chain of a tile (products, softmax, products) in the CTAs with the most keys, three of which share
 // an SM, and the reads of shared memory (92 a tile and warp, 512 bytes each, against 160 products).
 #include <type_traits>
@@ -257,8 +258,8 @@ head_prompt_attention_kernel(const __grid_constant__ HeadPromptArgs a) {
 // maximum is more than 2^8 above it, so that the accumulator is rarely taken out and multiplied.  In a tile of which some row
 // does not see every key the warp that brings the tiles clears the values behind the request's last key (another request's) and
 // those that are not finite, since zero times infinity is not zero; the rows that see the latter get them added at the end.
-// Measured (B200, us, the kernel above / this one): 12 heads, keys of 128 + 64, values of 128: 2,048 tokens 124 / 34 (480
-// TFLOP/s), 4,096 283 / 93, 300 18.4 / 10.0, 128 10.1 / 7.8; 14 heads of 64 + 64, values of 64, 2,048 tokens 80 / 33.  Portions of up to
+// Measured (B200, us, the kernel above / this one): 12 heads, keys of 128 + 64, values of 128: 2,048 tokens 124 / 32 (500
+// TFLOP/s), 4,096 283 / 91, 300 18.4 / 9.9, 128 10.1 / 7.8; 14 heads of 64 + 64, values of 64, 2,048 tokens 80 / 33.  Portions of up to
 // 64 tokens fill half a tile of this one at most and stay above: 40 of 30 tokens 14.8 / 31.7, one of 20 6.4 / 8.2.  What bounds it
 // now: a tile's softmax, 128 exponentials a thread between two passes through tensor memory.
 constexpr int kHeadThreads = 320, kHeadSlice = 128 * 64 * 2;

@@ -2,7 +2,7 @@
 // (gemm_simt.cu has the FMA product for operands of mixed type and rows that are not aligned).
 //
 // A 32-bit value is the sum of three bfloat16 parts (8 bits of the significand each), so a product of two is nine bfloat16
-// products, of which the six largest count: what is left out is below 2^-24 of a term.  The instruction cuts its sums
+// products, of which the six largest count: what is left out is 2^-24 of a term at most.  The instruction cuts its sums
 // off where FMA rounds them, so a chain of it drifts.  Therefore 32 elements of K are summed at a time, products of the
 // smaller parts first, into a tensor-memory accumulator that starts at zero, and its result is added to a running sum in
 // registers by a rounded addition; every 512 elements that sum joins a total in tensor memory.  Error against 64 bits (2-norm, 1 to 2,048
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(256) gemm_parts_sum_kernel(const __grid_consta
 
 using namespace einf;
 
-// sums: [shares][m][n] floats where shares (up to 8) is more than one.
+// sums: [shares][m][n] floats where shares (up to 16) is more than one.
 extern "C" int einf_gemm_parts(const float* a, const float* w, const float* bias, float* out, int m, int n, int k, long long lda,
                                long long ldo, int shares, float* sums, int* status, cudaStream_t stream) {
   if (m <= 0 || n <= 0) return 0;

@@ -387,7 +387,9 @@ def _gemm_parts_shares(row_tiles: int, col_tiles: int, k: int) -> int:
     """How many CTAs share K in :func:`gemm_parts`: whichever takes the fewest microseconds by what was measured, 1.7 for 64
     columns of K and 3 beside them for every wave of tiles of 128 x 128, and where K is shared 3.5 for the second
     launch and its bytes at 4 TB/s (545 rows, 896 -> 896: 28.7 alone, 17.7 by four, 22.5 by five; 128 rows, 4,864 -> 896: 132
-    alone, 25 by eight, 18 by sixteen).  Made of whole tiles, so that up to 128 rows all get the same sums."""
+    alone, 25 by eight, 18 by sixteen).  Against every other number of shares, 1 to 1,024 rows of nine matrices from 256 x 4,864 to
+    17,920 x 1,536: the fastest in 52 of 63 sizes, within 5 % in 56, within 14 % in 62, 46.5 against 38.4 us at one (545 rows of
+    2,048 x 1,536).  Made of whole tiles, so that up to 128 rows all get the same sums."""
     tiles, blocks = row_tiles * col_tiles, -(-k // 64)
     best, shares = float("inf"), 1
     for s in range(1, min(blocks, 16) + 1):
@@ -516,7 +518,7 @@ def linear(
     bfloat16 activations against a bfloat16 matrix go to the tensor cores through
     the library matrix product (as the reference's ``F.linear`` does,
     ``src/einf/executors/torch/packed_qkv.py:148``); the 32-bit path goes there as three
-    bfloat16 parts of either operand, which together are the operand
+    bfloat16 parts of either operand, which together are the operand (where they are not, by FMA)
     (:func:`gemm_parts`; faster than FMA at every size measured, 1 to 1,024 rows against 8 to 17,920 columns: 1,152 x 896
     20 -> 13 us for one row and 42 -> 21 for 545, 9,728 x 896 40 -> 26 and 211 -> 85, 896 x 4,864 24 -> 15 and 118 -> 45);
     operands of mixed type, and rows that are not aligned, run the FMA kernel, which rounds no input.
@@ -618,8 +620,15 @@ def project(
 #: the stream is narrow enough (measured, a layer of 0.5B sizes for 1 / 8 / 16 tokens: 24.4 -> 17.6, 29.0 -> 22.8,
 #: 27.9 -> 26.1 us; of 1.5B sizes, 1,536 wide, 34.2 -> 34.9, 40.3 -> 45.0: the separate products stream its 94 MB better).
 FEW_TOKENS = 16
+#: Twelve layers at a context of 256, separate products / these, us a step for 1 / 8 / 16 tokens: 640 wide 297 / 211, 320 / 222, 337 / 275;
+#: 1,024 wide (4,608 a branch) 335 / 262 for eight, 355 / 329 for sixteen; 1,152 wide (4,608) 333 / 255, 350 / 278, 371 / 372, (5,120)
+#: 342 / 299, 362 / 331, 379 / 439; 1,280 wide 346 / 334, 369 / 372, 402 / 486; 1,536 wide 379 / 356, 392 / 400, 416 / 518.
+#: So up to 1,024 all numbers of tokens gain (but see :func:`few_tokens_limit`); beyond it sixteen do not, though one and eight
+#: do to 1,152.
 FEW_NORM_WIDTH = 1024
-#: and the rows of the down projection short enough for two CTAs an SM
+#: The rows of the down projection: sixteen warps have one of up to 5,120 elements under way at once, and two CTAs fit an SM.  Longer
+#: rows are allowed by neither reason, not by a loss: 896 wide, 5,120 313 / 228, 336 / 256, 365 / 320; 6,144 321 / 241, 348 / 268, 369 / 335;
+#: 8,192 351 / 285, 374 / 322, 393 / 404.
 FEW_WIDTH = 5120
 
 
@@ -1106,8 +1115,8 @@ def head_prompt_attention(
     ``[requests + 1]``) other requests may be among them and are left out.  ``window``, ``sink`` and ``gate``: see
     :func:`paged_attention_generic`.
 
-    Heads in whole 128-byte lines run on tcgen05 (with a positive ``scale``: a row's largest score is found before it) where a portion has more than :data:`HEAD_PROMPT_SHORT` tokens, each by
-    its own length; ``lengths``: those portions' lengths where the host knows them, which spares a launch with
+    Heads in whole 128-byte lines run on tcgen05 (with a positive ``scale``: a row's largest score is found before it) where a
+    portion has more than :data:`HEAD_PROMPT_SHORT` tokens, each by its own length; ``lengths``: those portions' lengths where the host knows them, which spares a launch with
     nothing to do.  ``tensor_memory`` (True or False) sends all portions to one kernel."""
     tokens, heads, dim = q_plain.shape
     rot_dim, value_size = q_rot.shape[2], v.shape[2]

@@ -1282,7 +1282,7 @@ def test_gemm_of_three_parts(dev, m, n, k, shares):
     out, status = torch.full((m, n + 3), 7.0, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
     ops.gemm_parts(x, w, bias, out[:, :n], status, shares)
     want = x.double() @ w.double().T + bias.double()
-    # what the parts leave out is 2^-23 of a term at most; the sums of 32 elements are cut off twice, the others rounded
+    # what the parts leave out is 2^-24 of a term at most; the sums of 32 elements are cut off twice, the others rounded
     bound = (x.double().abs() @ w.double().abs().T + bias.double().abs()) * 2 ** -22
     assert bool(((out[:, :n].double() - want).abs() <= bound).all()) and int(status) == 0
     assert bool((out[:, n:] == 7.0).all())
